@@ -206,12 +206,18 @@ def _arcs(case: dict) -> int:
     return case["n"] * (case["n"] - 1 if case["graph"] == "clique" else case["degree"])
 
 
-def _solve_work(n: int, arcs: int, k: int) -> tuple[float, float]:
-    """(bytes, operations): the graph once and the table once; an add and a
-    minimum per unordered subset pair and vertex, and per row and arc."""
+def _solve_work(n: int, arcs: int, k: int, table: bool) -> tuple[float, float]:
+    """(bytes, operations): the graph once and, where it is an output, the
+    table once; an add and a minimum per unordered subset pair and vertex, and
+    per row and arc.  A call that returns no table needs the rows of the
+    subsets of the first k - 1 terminals only: the cost is the cell of those
+    k - 1 terminals at the last one, and every row depends only on the rows of
+    its own subsets."""
+    if not table:
+        k = max(1, k - 1)
     rows = (1 << k) - 1
     pairs = (3**k - 2 ** (k + 1) + 1) / 2
-    return 4.0 * (n + 1) + 8.0 * arcs + 4.0 * n * (rows + 1), 2.0 * n * pairs + 2.0 * rows * arcs
+    return 4.0 * (n + 1) + 8.0 * arcs + 4.0 * n * (rows + 1) * table, 2.0 * n * pairs + 2.0 * rows * arcs
 
 
 def work(case: dict) -> dict:
@@ -219,14 +225,14 @@ def work(case: dict) -> dict:
     if call in ("batch", "serve"):
         sizes = [(g.n, g.arcs, g.k) for g in _mixed(case["count"], 1)]
         sizes += [(LARGE["n"], LARGE["n"] * LARGE["degree"], LARGE["k"])] * case.get("large", 0)
-        parts = [_solve_work(*s) for s in sizes]
+        parts = [_solve_work(*s, False) for s in sizes]
         return {"bytes": sum(b for b, _ in parts), "flops": sum(f for _, f in parts)}
     n, arcs = case["n"], _arcs(case)
     if call == "sssp":
         return {"bytes": 4.0 * (n + 1) + 8.0 * arcs + 8.0 * n, "flops": 2.0 * arcs}
     if call == "closure":
         return {"bytes": 4.0 * (n + 1) + 8.0 * arcs + 8.0 * n * case["rows"], "flops": 2.0 * arcs * case["rows"]}
-    b, f = _solve_work(n, arcs, case["k"])
+    b, f = _solve_work(n, arcs, case["k"], case.get("table", call == "device"))
     return {"bytes": b, "flops": f}
 
 
