@@ -216,6 +216,7 @@ int emv_kernel_dev(emv_ctx *ctx, int32_t n, int64_t arcs,
 #define EMV_SOLVE_TREE  0x1   /* recover a tree (R:2301-2310, -list)        */
 #define EMV_SOLVE_TABLE 0x2   /* copy the table to out->table               */
 #define EMV_SOLVE_NOCHECK 0x4 /* skip the admission checks (below)          */
+#define EMV_SOLVE_ALL_ROWS 0x8 /* fill all 2^k rows without returning them (below) */
 
 typedef struct emv_result {
     int64_t cost;          /* d[C][q], INT64_MAX when unreachable / k == 1 */
@@ -238,7 +239,11 @@ typedef struct emv_result {
  * min((n-1) * max_w, sum of edge weights), rejecting EMV_ERR_BAD_INPUT /
  * EMV_ERR_OVERFLOW; a graph that is not connected (a vertex the level-1
  * closures leave unreached) is EMV_ERR_DISCONNECTED after the DP.  The CSR
- * must hold both arcs of every edge. */
+ * must hold both arcs of every edge.
+ * Rows computed: all 2^k when the table is returned (or EMV_SOLVE_ALL_ROWS is
+ * set, for timings comparable with the reference's whole-table DP); otherwise
+ * the 2^(k-1) rows over the first k - 1 terminals, which are all that the
+ * cost d[C][q] and the tree read. */
 int emv_solve(emv_ctx *ctx, const emv_graph *g, const int32_t *terminals,
               int32_t k, int32_t flags, emv_result *out, void *stream);
 
@@ -302,7 +307,9 @@ typedef struct emv_batch_stats {
 /* Solves many independent instances (no counterpart in the reference, which
  * runs one instance per process): one persistent, CUDA-graph-captured launch
  * per DP level over a device work queue of (instance, level) items.  costs_out
- * gets one int64 per instance. */
+ * gets one int64 per instance.  Only the rows that the costs depend on (the
+ * subsets of each instance's first k - 1 terminals) are computed;
+ * emv_batch_solve_tables computes them all. */
 int emv_batch_solve(emv_ctx *ctx, const emv_instance *inst, int32_t count,
                     int64_t *costs_out, emv_batch_stats *stats, void *stream);
 

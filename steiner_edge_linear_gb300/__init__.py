@@ -32,6 +32,7 @@ BATCH_CLASSES = 12
 TREE = 0x1
 TABLE = 0x2
 NOCHECK = 0x4
+ALL_ROWS = 0x8
 
 STATUS = {
     0: "EMV_OK", 1: "EMV_ERR_BAD_INPUT", 2: "EMV_ERR_PARSE", 3: "EMV_ERR_OOM", 4: "EMV_ERR_OVER_BUDGET",
@@ -426,8 +427,9 @@ class Solver:
             pass
 
     def solve(self, g: Csr, terminals: Optional[Sequence[int]] = None, tree: bool = False, table: bool = False,
-              check: bool = True, stream: Optional[int] = None) -> Result:
-        """erickson_monma_veinott on a host CSR (emv_solve)."""
+              check: bool = True, stream: Optional[int] = None, all_rows: bool = False) -> Result:
+        """erickson_monma_veinott on a host CSR (emv_solve).  all_rows fills
+        every row on the device even when no table is returned."""
         terms = np.ascontiguousarray(g.terminals if terminals is None else terminals, dtype=np.int32)
         k = int(terms.shape[0])
         res = _Result()
@@ -438,7 +440,8 @@ class Solver:
             res.tree_cap = g.n + 1
         if tab is not None:
             res.table = tab.ctypes.data
-        flags = (TREE if tree else 0) | (TABLE if table else 0) | (0 if check else NOCHECK)
+        flags = ((TREE if tree else 0) | (TABLE if table else 0) | (0 if check else NOCHECK) |
+                 (ALL_ROWS if all_rows else 0))
         cg = g.c_graph()
         _check(self._lib.emv_solve(self._ctx, ctypes.byref(cg), terms.ctypes.data, k, flags, ctypes.byref(res),
                                    stream))
@@ -446,8 +449,9 @@ class Solver:
         return Result(int(res.cost), tr, int(res.tree_weight), tab, _timing(res.timing))
 
     def solve_dev(self, n: int, arcs: int, row_ptr: int, col: int, w: int, terminals: Sequence[int],
-                  tree: bool = False, stream: Optional[int] = None) -> Result:
-        """emv_solve_dev on device pointers (e.g. torch tensors' data_ptr())."""
+                  tree: bool = False, stream: Optional[int] = None, all_rows: bool = False) -> Result:
+        """emv_solve_dev on device pointers (e.g. torch tensors' data_ptr());
+        all_rows as in solve."""
         terms = np.ascontiguousarray(terminals, dtype=np.int32)
         res = _Result()
         tree_buf = np.zeros((n + 1, 3), np.int32) if tree else None
@@ -456,7 +460,8 @@ class Solver:
             res.tree_cap = n + 1
         cg = _Graph(n, arcs, row_ptr, col, w)
         _check(self._lib.emv_solve_dev(self._ctx, ctypes.byref(cg), terms.ctypes.data, int(terms.shape[0]),
-                                       TREE if tree else 0, ctypes.byref(res), stream))
+                                       (TREE if tree else 0) | (ALL_ROWS if all_rows else 0), ctypes.byref(res),
+                                       stream))
         tr = tree_buf[:res.tree_count].copy() if tree_buf is not None else None
         return Result(int(res.cost), tr, int(res.tree_weight), None, _timing(res.timing))
 

@@ -95,11 +95,11 @@ int32_t batch_mw_max(int32_t n, int32_t k)
     return mw;
 }
 
-int32_t batch_mw_for(const emv_ctx *c, int32_t n, int32_t k)
+int32_t batch_mw_for(const emv_ctx *c, int32_t n, int32_t k, int32_t kt)
 {
     const int32_t cls = batch_class_of(n, k);
     const int32_t w = (cls >= 0 && cls < BATCH_CLASSES && c->tune_mw[cls] > 0) ? c->tune_mw[cls] : 1;
-    return std::min(batch_mw_max(n, k), pow2_floor(std::max(1, w)));
+    return std::min(batch_mw_max(n, kt), pow2_floor(std::max(1, w)));
 }
 
 int prepare_batch_subsets(emv_ctx *c, cudaStream_t st)
@@ -193,7 +193,7 @@ static int batch_solve(emv_ctx *c, const emv_instance *inst, int32_t count, int6
         return batch_work(inst[x].g.n, inst[x].k, inst[x].g.arcs) > batch_work(inst[y].g.n, inst[y].k, inst[y].g.arcs);
     });
     BatchPack pk;
-    int r = batch_pack(c, inst, order, 1, -1, pk);
+    int r = batch_pack(c, inst, order, tables_out != nullptr, pk);
     if (r) return r;
     r = batch_upload(c, pk, st);
     if (r) return r;
@@ -247,8 +247,7 @@ extern "C" int emv_batch_solve_tables(emv_ctx *c, const emv_instance *inst, int3
 
 // ---------------------------------------------------------------- packing
 
-int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &order, int32_t lo, int32_t hi,
-               BatchPack &pk)
+int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &order, bool whole, BatchPack &pk)
 {
     const int32_t count = (int32_t)order.size();
     pk.desc.resize((size_t)count);
@@ -263,11 +262,12 @@ int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> 
         std::memset(&d, 0, sizeof(d));
         d.n = I.g.n;
         d.k = I.k;
+        d.kt = whole ? I.k : table_terminals(I.k);
         d.rcap = batch_rcap_for(c, I.g.n, I.k);
-        d.mw = batch_mw_for(c, I.g.n, I.k);
+        d.mw = batch_mw_for(c, I.g.n, I.k, d.kt);
         d.orig = order[(size_t)j];
-        d.lo = lo;
-        d.hi = hi < 0 ? I.k : hi;
+        d.lo = 1;
+        d.hi = d.kt;
         pk.row_off[(size_t)j] = rows;
         pk.arc_off[(size_t)j] = arcs;
         pk.term_off[(size_t)j] = terms;
@@ -275,7 +275,7 @@ int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> 
         rows += I.g.n + 1;
         arcs += I.g.arcs;
         terms += I.k;
-        words += ((int64_t)I.g.n << I.k);
+        words += ((int64_t)I.g.n << d.kt);
         pk.rcap_used = std::max(pk.rcap_used, d.rcap);
         pk.cost_slots = std::max<int64_t>(pk.cost_slots, (int64_t)d.orig + 1);
     }
@@ -412,7 +412,7 @@ namespace {
 int time_sample(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &ids, cudaStream_t st, float &ms)
 {
     BatchPack pk;
-    int r = batch_pack(c, inst, ids, 1, -1, pk);
+    int r = batch_pack(c, inst, ids, false, pk);
     if (!r) r = batch_upload(c, pk, st);
     if (r) return r;
     BatchArgs a = batch_args(c, pk);
@@ -470,7 +470,7 @@ static int batch_autotune(emv_ctx *c, const emv_instance *inst, int32_t count, i
         }
         c->tune_rcap[cls] = best;
         int32_t best_mw = 1;
-        for (int32_t mw = 2; mw <= BATCH_MW_MAX && mw <= batch_mw_max(nmax, kmin); mw *= 2) {
+        for (int32_t mw = 2; mw <= BATCH_MW_MAX && mw <= batch_mw_max(nmax, table_terminals(kmin)); mw *= 2) {
             c->tune_mw[cls] = mw;
             float ms = 0;
             const int r = time_sample(c, inst, ids, st, ms);

@@ -197,7 +197,7 @@ __device__ bool batch_relax(const BatchArgs &a, int32_t *table, int32_t n, const
 // Runs levels [lo, hi] of one instance with the whole CTA.
 __device__ void batch_solve_one(const BatchArgs &a, const BatchInst &I, int32_t *S)
 {
-    const int32_t n = I.n, k = I.k;
+    const int32_t n = I.n, k = I.kt;
     int32_t *table = I.table;
     const int32_t *row_ptr = I.row_ptr;
     const int2 *adj = I.adj;
@@ -217,8 +217,8 @@ __device__ void batch_solve_one(const BatchArgs &a, const BatchInst &I, int32_t 
         if (!ok) atomicOr(a.err, (uint32_t)EMV_DEV_SWEEP_LIMIT);
         if (I.hi == k) {
             int64_t cost = INT64_MAX;
-            if (k >= 2) {
-                const int32_t x = table[(int64_t)((1 << (k - 1)) - 1) * n + terms[k - 1]];
+            if (I.k >= 2) {
+                const int32_t x = table[(int64_t)((1 << (I.k - 1)) - 1) * n + terms[I.k - 1]];
                 if (x < INF) cost = x;
             }
             a.costs[I.orig] = cost;

@@ -25,13 +25,13 @@ int32_t batch_class_of(int32_t n, int32_t k);
 int32_t batch_rcap_max(int32_t n);
 int32_t batch_rcap_for(const emv_ctx *c, int32_t n, int32_t k);
 int32_t batch_mw_max(int32_t n, int32_t k);
-int32_t batch_mw_for(const emv_ctx *c, int32_t n, int32_t k);
+int32_t batch_mw_for(const emv_ctx *c, int32_t n, int32_t k, int32_t kt);  // class of (n, k), rows of kt
 bool batch_fits(int32_t n, int32_t k);
 double batch_work(int32_t n, int32_t k, int64_t arcs);
 int prepare_batch_subsets(emv_ctx *c, cudaStream_t st);
 int batch_kernel_setup(emv_ctx *c);
-int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &order, int32_t lo, int32_t hi,
-               BatchPack &pk);
+// whole: solve the subsets of all terminals (the tables are wanted), else those the costs need.
+int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &order, bool whole, BatchPack &pk);
 int batch_upload(emv_ctx *c, BatchPack &pk, cudaStream_t st);
 emv::BatchArgs batch_args(emv_ctx *c, const BatchPack &pk);
 // max_blocks > 0 caps the persistent grid (the autotuner's samples).

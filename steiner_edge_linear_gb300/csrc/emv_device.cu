@@ -470,19 +470,24 @@ static int pack_and_check(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *ro
     return scan_status(*h, n);
 }
 
-// The DP proper on device data with packed arcs; fills the whole table.
+// The DP proper on device data with packed arcs over the first kt of the k
+// terminals (kt = k: the whole table; kt = k - 1: the rows of the subsets of
+// C = {t_0..t_{k-2}}, all that the cost d[C][t_{k-1}] and a tree traced back
+// from it read); fills those 2^kt rows.
 // With check set, a level-1 closure that left a vertex unreached (the graph
 // is not connected: the reference's table is undefined there, R:2077) makes
 // the solve EMV_ERR_DISCONNECTED; the table is then not meaningful.
-int run_dp(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32_t k, const int32_t *terms_host,
-           int32_t *table, int64_t ld, cudaStream_t st, int64_t *cost_out, emv_timing *tm, bool check)
+int run_dp(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32_t k_all, int32_t kt,
+           const int32_t *terms_host, int32_t *table, int64_t ld, cudaStream_t st, int64_t *cost_out, emv_timing *tm,
+           bool check)
 {
+    const int32_t k = kt;
     int r = prepare_subsets(c, k, st);
     if (!r) r = reserve_relax(c, n);
-    if (!r) r = dev_reserve(c->terms, sizeof(int32_t) * (size_t)k);
+    if (!r) r = dev_reserve(c->terms, sizeof(int32_t) * (size_t)k_all);
     if (r) return r;
     int32_t *d_terms = (int32_t *)c->terms.ptr;
-    CUDA_TRY(cudaMemcpyAsync(d_terms, terms_host, sizeof(int32_t) * (size_t)k, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(d_terms, terms_host, sizeof(int32_t) * (size_t)k_all, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemsetAsync(c->stat.ptr, 0, sizeof(DevStat), st));
     const uint32_t *xs = (const uint32_t *)c->kp->xs.ptr;
     int ev = 0;
@@ -563,9 +568,10 @@ int run_dp(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32
 
     // Cost d[C][q] (R:2137-2138) and the device status, then one host sync.
     int32_t *hp = (int32_t *)c->pinned;
-    if (k >= 2) {
-        const int64_t C = ((int64_t)1 << (k - 1)) - 1;
-        CUDA_TRY(cudaMemcpyAsync(hp, table + C * ld + terms_host[k - 1], sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    if (k_all >= 2) {
+        const int64_t C = ((int64_t)1 << (k_all - 1)) - 1;
+        CUDA_TRY(cudaMemcpyAsync(hp, table + C * ld + terms_host[k_all - 1], sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                 st));
     } else {
         hp[0] = INF;
     }
@@ -577,7 +583,7 @@ int run_dp(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32
     if (ds.err) return emv_dev_status_to_emv(ds.err);
     if (check && h_max[1] >= (uint32_t)INF)
         return emv_fail(EMV_ERR_DISCONNECTED, "graph: not connected (a vertex is unreachable from terminal 1)");
-    *cost_out = (k >= 2 && hp[0] < INF) ? (int64_t)hp[0] : INT64_MAX;
+    *cost_out = (k_all >= 2 && hp[0] < INF) ? (int64_t)hp[0] : INT64_MAX;
     if (tm) {
         float ms = 0;
         cudaEventElapsedTime(&ms, E[0], E[1]);
@@ -625,7 +631,7 @@ extern "C" int emv_kernel_dev(emv_ctx *c, int32_t n, int64_t arcs, const int32_t
     c->launches = 0;
     r = pack_and_check(c, n, arcs, d_row_ptr, d_col, d_w, true, st);
     if (r) return r;
-    return run_dp(c, n, d_row_ptr, (const int2 *)c->adj.ptr, k, terminals, d_table, ld, st, cost_out, nullptr, true);
+    return run_dp(c, n, d_row_ptr, (const int2 *)c->adj.ptr, k, k, terminals, d_table, ld, st, cost_out, nullptr, true);
 }
 
 // Runs the traceback kernel and reduces its edge list to a tree on the host.
@@ -710,12 +716,17 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
     int r = pack_and_check(c, n, arcs, row_ptr, col, w, check, st);
     if (r) return r;
     const int64_t ld = ((int64_t)n + 31) / 32 * 32;
-    const size_t tbytes = sizeof(int32_t) * (size_t)ld << k;
+    // Without a table to return, the rows of subsets that hold the last
+    // terminal are read by nothing: neither by the cost d[C][t_{k-1}] nor by
+    // the rows and the traceback below it.
+    const bool whole = ((flags & EMV_SOLVE_TABLE) && out->table) || (flags & EMV_SOLVE_ALL_ROWS);
+    const int32_t kt = whole ? k : table_terminals(k);
+    const size_t tbytes = sizeof(int32_t) * (size_t)ld << kt;
     r = dev_reserve(c->table, tbytes);
     if (r) return r;
     int32_t *table = (int32_t *)c->table.ptr;
     std::memset(&out->timing, 0, sizeof(out->timing));
-    r = run_dp(c, n, row_ptr, (const int2 *)c->adj.ptr, k, terms, table, ld, st, &out->cost, &out->timing, check);
+    r = run_dp(c, n, row_ptr, (const int2 *)c->adj.ptr, k, kt, terms, table, ld, st, &out->cost, &out->timing, check);
     if (r) return r;
     out->tree_count = 0;
     out->tree_weight = 0;

@@ -12,6 +12,11 @@
 // occupies xs[off[m], off[m + 1]).
 void subset_levels(int32_t k, std::vector<uint32_t> &xs, std::vector<int64_t> &off);
 
+// Terminals whose subsets a solve of k terminals needs when it returns no
+// table: the cost is d[C][t_{k-1}] with C = {t_0..t_{k-2}} (R:2137-2138), and a
+// row of the table depends only on the rows of its own subsets.
+inline int32_t table_terminals(int32_t k) { return k >= 2 ? k - 1 : k; }
+
 namespace emv {
 
 // Value widths of level m from the level maxima M[1..m-1] (M[j] = the largest

@@ -128,7 +128,7 @@ int stage_small(emv_server *s, Req *r, std::vector<int2> &adj)
     if (cudaMallocAsync((void **)&r->d_row, sizeof(int32_t) * ((size_t)r->n + 1), st) != cudaSuccess ||
         cudaMallocAsync((void **)&r->d_adj, sizeof(int2) * arcs, st) != cudaSuccess ||
         cudaMallocAsync((void **)&r->d_terms, sizeof(int32_t) * (size_t)r->k, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&r->d_table, sizeof(int32_t) * ((size_t)r->n << r->k), st) != cudaSuccess) {
+        cudaMallocAsync((void **)&r->d_table, sizeof(int32_t) * ((size_t)r->n << table_terminals(r->k)), st) != cudaSuccess) {
         cudaGetLastError();
         return emv_fail(EMV_ERR_OOM, "server: device allocation for request %lld", (long long)r->id);
     }
@@ -215,8 +215,9 @@ void scheduler(emv_server *s)
             d.table = r->d_table;
             d.n = r->n;
             d.k = r->k;
+            d.kt = table_terminals(r->k);
             d.rcap = batch_rcap_for(s->ctx_small, r->n, r->k);
-            d.mw = batch_mw_for(s->ctx_small, r->n, r->k);
+            d.mw = batch_mw_for(s->ctx_small, r->n, r->k, d.kt);
             d.orig = r->slot;
             d.lo = d.hi = r->next_level;
         }
@@ -258,7 +259,7 @@ void scheduler(emv_server *s)
             } else if (r->cancel) {
                 finish(s, r, EMV_ERR_CANCELLED, 0);
                 done = true;
-            } else if (r->next_level == r->k) {
+            } else if (r->next_level == table_terminals(r->k)) {
                 finish(s, r, EMV_OK, s->h_costs[r->slot]);
                 done = true;
             } else {

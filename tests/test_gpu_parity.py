@@ -459,3 +459,25 @@ def test_roofline_scale_solve(emv, orc, tmp_path):
                 assert (table[int(X) ^ (1 << b)].cpu().numpy() <= r).all()
     del table
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("n,degree,k,dup", [(64, 3, 1, False), (64, 3, 2, False), (300, 4, 3, False),
+                                            (301, 4, 6, True), (5000, 6, 9, False)])
+def test_calls_without_a_table_equal_whole_table_solves(emv, orc, solver, n, degree, k, dup):
+    """A call that returns no table computes the rows over the first k - 1
+    terminals only: its cost and tree are those of the whole-table solve,
+    also with a repeated terminal and for k = 1 and 2."""
+    inst = emv.StpInstance.regular(n, degree, 1, 50, k, 31 + k)
+    csr = emv.Csr.from_stp(inst)
+    terms = csr.terminals.copy()
+    if dup:
+        terms[-1] = terms[1]
+    csr = emv.Csr(csr.n, csr.row_ptr, csr.col, csr.w, terms)
+    _, want = orc.emv_table(csr.n, csr.row_ptr, csr.col, csr.w, csr.terminals, threads=8)
+    whole = solver.solve(csr, tree=True, table=True)
+    for res in (solver.solve(csr, tree=True), solver.solve(csr, tree=True, all_rows=True)):
+        assert res.cost == whole.cost == want
+        assert np.array_equal(res.tree, whole.tree) and res.tree_weight == whole.tree_weight
+    if k <= 10:
+        costs, _ = solver.batch_solve([csr])
+        assert int(costs[0]) == want
