@@ -41,6 +41,7 @@ SOURCES = [
     "emv_noalloc.cu",
     "emv_bin.cpp",
     "emv_plan.cpp",
+    "emv_resident.cu",
 ]
 CLI_SOURCES = ["cli.cpp"]
 GEN_SOURCES = ["gen_main.cpp", "emv_host.cpp"]

@@ -5,6 +5,7 @@
 //   erickson_monma_veinott  R:2141-2343  -> emv_solve / emv_solve_dev
 //   dijkstra (-dijkstra)    R:1762-1880, R:2454-2484 -> emv_sssp
 #include "emv_kernels.cuh"
+#include "emv_resident.h"
 #include "emv_solver.h"
 
 #include <algorithm>
@@ -128,7 +129,7 @@ extern "C" int emv_destroy(emv_ctx *c)
     cudaSetDevice(c->device);
     cudaDeviceSynchronize();
     for (DevBuf *b : {&c->ctrl, &c->stat, &c->lvlmax, &c->gscan, &c->shadow, &c->scratch, &c->act, &c->adj, &c->stamp, &c->terms, &c->g_row,
-                      &c->g_col, &c->g_w, &c->table, &c->tb_edges, &c->tb_out, &c->tb_work})
+                      &c->g_col, &c->g_w, &c->table, &c->tb_edges, &c->tb_out, &c->tb_work, &c->res_arcs, &c->res_out})
         dev_release(*b);
     for (KPlan *p : c->kplans) {
         if (!p) continue;
@@ -434,7 +435,7 @@ int launch_merge(emv_ctx *c, int32_t *table, int64_t ld, int32_t n, int32_t k, i
 // Status of a device CSR check: the same statuses, bound and messages as the
 // host check emv_graph_check, whose connectivity part comes from the level-1
 // closures instead (run_dp).
-static int scan_status(const GraphScan &s, int32_t n)
+int scan_status(const GraphScan &s, int32_t n)
 {
     if (s.bad & SCAN_BAD_ROWS) return emv_fail(EMV_ERR_BAD_INPUT, "graph: row_ptr not from 0 to arcs, non-decreasing");
     if (s.bad & SCAN_BAD_HEAD) return emv_fail(EMV_ERR_BAD_INPUT, "graph: arc head out of range");
@@ -629,14 +630,18 @@ extern "C" int emv_kernel_dev(emv_ctx *c, int32_t n, int64_t arcs, const int32_t
     CUDA_TRY(cudaSetDevice(c->device));
     cudaStream_t st = (cudaStream_t)stream;
     c->launches = 0;
+    ResidentPlan plan;
+    if (resident_plan(c, n, arcs, k, plan))
+        return run_resident(c, plan, n, arcs, d_row_ptr, d_col, d_w, terminals, k, k, d_table, ld, true, st, cost_out,
+                            nullptr);
     r = pack_and_check(c, n, arcs, d_row_ptr, d_col, d_w, true, st);
     if (r) return r;
     return run_dp(c, n, d_row_ptr, (const int2 *)c->adj.ptr, k, k, terminals, d_table, ld, st, cost_out, nullptr, true);
 }
 
 // Runs the traceback kernel and reduces its edge list to a tree on the host.
-int run_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32_t k, const int32_t *table,
-                  int64_t ld, cudaStream_t st, emv_result *out)
+int run_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32_t k, const int32_t *d_terms,
+                  const int32_t *table, int64_t ld, cudaStream_t st, emv_result *out)
 {
     const int32_t cap = std::max(64, 2 * n);
     int r = dev_reserve(c->tb_edges, sizeof(int32_t) * 3 * (size_t)cap);
@@ -653,7 +658,7 @@ int run_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj
     a.k = k;
     a.row_ptr = row_ptr;
     a.adj = adj;
-    a.terms = (const int32_t *)c->terms.ptr;
+    a.terms = d_terms;
     a.edges = (int32_t *)c->tb_edges.ptr;
     a.cap = cap;
     a.out = (int32_t *)c->tb_out.ptr;
@@ -713,8 +718,6 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
                     cudaStream_t st)
 {
     const bool check = !(flags & EMV_SOLVE_NOCHECK);
-    int r = pack_and_check(c, n, arcs, row_ptr, col, w, check, st);
-    if (r) return r;
     const int64_t ld = ((int64_t)n + 31) / 32 * 32;
     // Without a table to return, the rows of subsets that hold the last
     // terminal are read by nothing: neither by the cost d[C][t_{k-1}] nor by
@@ -722,16 +725,22 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
     const bool whole = ((flags & EMV_SOLVE_TABLE) && out->table) || (flags & EMV_SOLVE_ALL_ROWS);
     const int32_t kt = whole ? k : table_terminals(k);
     const size_t tbytes = sizeof(int32_t) * (size_t)ld << kt;
-    r = dev_reserve(c->table, tbytes);
+    ResidentPlan plan;
+    const bool resident = resident_plan(c, n, arcs, kt, plan);
+    int r = resident ? EMV_OK : pack_and_check(c, n, arcs, row_ptr, col, w, check, st);
+    if (!r) r = dev_reserve(c->table, tbytes);
     if (r) return r;
     int32_t *table = (int32_t *)c->table.ptr;
     std::memset(&out->timing, 0, sizeof(out->timing));
-    r = run_dp(c, n, row_ptr, (const int2 *)c->adj.ptr, k, kt, terms, table, ld, st, &out->cost, &out->timing, check);
+    r = resident ? run_resident(c, plan, n, arcs, row_ptr, col, w, terms, k, kt, table, ld, check, st, &out->cost,
+                                &out->timing)
+                 : run_dp(c, n, row_ptr, (const int2 *)c->adj.ptr, k, kt, terms, table, ld, st, &out->cost, &out->timing, check);
     if (r) return r;
     out->tree_count = 0;
     out->tree_weight = 0;
     if ((flags & EMV_SOLVE_TREE) && k >= 2) {
-        r = run_traceback(c, n, row_ptr, (const int2 *)c->adj.ptr, k, table, ld, st, out);
+        r = run_traceback(c, n, row_ptr, (const int2 *)c->adj.ptr, k,
+                          resident ? resident_terms(c) : (const int32_t *)c->terms.ptr, table, ld, st, out);
         if (r) return r;
     }
     if ((flags & EMV_SOLVE_TABLE) && out->table) {

@@ -1,0 +1,24 @@
+// emv_resident.h -- the one-launch solver of small instances (host side).
+#pragma once
+
+#include "emv_common.cuh"
+#include "emv_solver.h"
+
+constexpr int32_t RESIDENT_SMEM = 224 * 1024;
+
+struct ResidentPlan {
+    int blocks;              // CTAs
+    int32_t rows;            // rows of the widest level's largest share
+    int32_t mw;              // vertices of a merge block
+};
+
+bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, ResidentPlan &p);
+// The whole DP over the first kt of the k terminals, CSR check included;
+// fills the table's 2^kt rows (stride ld) and c->adj.
+int run_resident(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, const int32_t *row_ptr, const int32_t *col,
+                 const int32_t *w, const int32_t *terms, int32_t k, int32_t kt, int32_t *table, int64_t ld, bool check,
+                 cudaStream_t st, int64_t *cost_out, emv_timing *tm);
+// The terminals on the device after run_resident.
+const int32_t *resident_terms(const emv_ctx *c);
+// Status of a device CSR check (emv_device.cu).
+int scan_status(const emv::GraphScan &s, int32_t n);

@@ -78,6 +78,8 @@ struct emv_ctx {
     KPlan *kp = nullptr;           // plan of xs_k
     KPlan *kplans[EMV_MAX_K + 1] = {};  // plans of every k used so far
     bool merge_attr = false;
+    DevBuf res_arcs, res_out;        // one-launch solver: sliced arcs, control and result words
+    bool res_attr = false;
     int64_t launches = 0;
     // batched launch
     DevBuf bxs, bxs_off;           // subset lists of every k <= BATCH_KMAX

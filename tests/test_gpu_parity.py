@@ -481,3 +481,45 @@ def test_calls_without_a_table_equal_whole_table_solves(emv, orc, solver, n, deg
     if k <= 10:
         costs, _ = solver.batch_solve([csr])
         assert int(costs[0]) == want
+
+
+ONE_LAUNCH = {  # graph, k: the one-launch solver's edges
+    "one_slice": (("regular", 32, 3, 1, 9), 5),
+    "odd_n_many_rows": (("regular", 65, 4, 1, 50), 11),
+    "registers_two_pairs": (("regular", 1024, 4, 1, 1000), 6),
+    "pairs_past_the_registers": (("regular", 999, 10, 1, 100), 5),
+    "arcs_in_shared_memory": (("regular", 4096, 10, 1, 1024), 4),
+    "arcs_in_global_memory": (("regular", 12002, 8, 1, 100), 4),
+    "largest_weight_packed": (("regular", 1500, 4, 16383, 16383), 4),
+    "smallest_weight_not_packed": (("regular", 1500, 4, 16383, 16384), 4),
+    "hubs_only": (("clique", 200, 0, 1, 20000), 5),
+    "hubs_and_leaves": (("powlaw", 5000, 8, 1, 100), 6),
+    "most_vertices": (("regular", 29000, 4, 1, 30), 3),
+}
+
+
+@pytest.mark.parametrize("name", sorted(ONE_LAUNCH))
+def test_one_launch_solver_whole_table(emv, orc, solver, name):
+    """Small instances run as one launch: whole table against the oracle, from
+    host memory and into a caller's table of an odd stride."""
+    torch = pytest.importorskip("torch")
+    (kind, n, degree, wmin, wmax), k = ONE_LAUNCH[name]
+    if kind == "clique":
+        inst = emv.StpInstance.clique(n, wmin, wmax, k, 17)
+    elif kind == "powlaw":
+        inst = emv.StpInstance.powlaw(n, degree, -0.5, 8, wmin, wmax, k, 17)
+    else:
+        inst = emv.StpInstance.regular(n, degree, wmin, wmax, k, 17)
+    csr = emv.Csr.from_stp(inst)
+    want, want_cost = orc.emv_table(csr.n, csr.row_ptr, csr.col, csr.w, csr.terminals, threads=8)
+    res = solver.solve(csr, tree=True, table=True)
+    assert res.timing["relax_launches"] == 1
+    assert res.cost == want_cost and np.array_equal(res.table, want)
+    check_tree(csr.n, inst.edges, res.tree, csr.terminals, res.cost)
+    row, col, w = (torch.from_numpy(a).to("cuda:0") for a in (csr.row_ptr, csr.col, csr.w))
+    ld = csr.n + 3 - csr.n % 2
+    table = torch.full(((1 << k), ld), -7, dtype=torch.int32, device="cuda:0")
+    cost = solver.kernel_dev(csr.n, csr.arcs, row.data_ptr(), col.data_ptr(), w.data_ptr(), csr.terminals,
+                             table.data_ptr(), ld, torch.cuda.current_stream().cuda_stream)
+    got = table.cpu().numpy()
+    assert cost == want_cost and np.array_equal(got[:, :csr.n], want) and (got[:, csr.n:] == -7).all()
