@@ -7,6 +7,7 @@
 #include "emv_batch.cuh"
 #include "emv_solver.h"
 #include "emv_batch_host.h"
+#include "emv_resident.h"
 
 #include <algorithm>
 #include <atomic>
@@ -64,42 +65,77 @@ int32_t batch_class_of(int32_t n, int32_t k)
     return nb * 3 + kb;
 }
 
-// Largest rows-per-chunk whose vertex-major buffer fits the shared memory.
-int32_t batch_rcap_max(int32_t n)
-{
-    int32_t r = BATCH_RCAP_MAX;
-    while (r > 1 && (int64_t)n * batch_stride(r) * 4 > BATCH_SMEM_BYTES) r /= 2;
-    return r;
-}
-
 bool batch_fits(int32_t n, int32_t k)
 {
     return k >= 1 && k <= BATCH_KMAX && (int64_t)n * 2 * 4 <= BATCH_SMEM_BYTES &&
-           ((int64_t)32 << k) * 4 <= BATCH_SMEM_BYTES;
+           ((int64_t)32 << k) * 4 <= BATCH_SMEM_BYTES && resident_fits(n, k);
 }
 
-int32_t batch_rcap_for(const emv_ctx *c, int32_t n, int32_t k)
+BatchGraph batch_graph(const int32_t *row_ptr, const int32_t *w, int32_t n, int64_t arcs)
 {
-    const int32_t cap = batch_rcap_max(n);
-    const int32_t cls = batch_class_of(n, k);
-    int32_t r = (cls >= 0 && cls < BATCH_CLASSES && c->tune_rcap[cls] > 0) ? c->tune_rcap[cls] : 32;
-    return std::min(cap, pow2_floor(std::max(1, r)));
+    uint32_t most = 0;
+    for (int64_t e = 0; e < arcs; e++) most = std::max(most, (uint32_t)w[e]);
+    int64_t pairs = 0;
+    for (int32_t v0 = 0; v0 < n; v0 += 32) {
+        int32_t width = 0;
+        for (int32_t v = v0; v < std::min(n, v0 + 32); v++) {
+            const int32_t deg = row_ptr[v + 1] - row_ptr[v];
+            if (deg <= RES_HUB) width = std::max(width, (deg + 1) / 2);
+        }
+        pairs += width;
+    }
+    const bool narrow = most < RES_MAX_W;
+    return {narrow, pairs * 32 * (int64_t)(narrow ? sizeof(uint2) : sizeof(int4))};
 }
 
-// Largest merge block width (in 32-vertex columns) whose staged rows fit the
-// shared memory, and no wider than the instance.
-int32_t batch_mw_max(int32_t n, int32_t k)
+// Fitted to one-CTA solves (n = 128 .. 4096, kt = 7 .. 9): closures 0.68 ns an
+// arc and row, merges 0.016 ns a (subset pair, vertex), 15 us a level.
+double batch_work(int32_t n, int32_t kt, int64_t arcs, int32_t lo, int32_t hi)
 {
-    int32_t mw = BATCH_MW_MAX;
-    while (mw > 1 && (((int64_t)32 * mw << k) * 4 > BATCH_SMEM_BYTES || 32 * (mw / 2) >= n)) mw /= 2;
-    return mw;
+    const double all = 0.68e-3 * std::pow(2.0, kt) * (double)arcs + 0.016e-3 * std::pow(3.0, kt) * n;
+    return all * (hi - lo + 1) / kt + 15.0 * (hi - lo + 1);
 }
 
-int32_t batch_mw_for(const emv_ctx *c, int32_t n, int32_t k, int32_t kt)
+void batch_plan(const std::vector<double> &work, const std::vector<int64_t> &states, int32_t blocks, int32_t max_size,
+                std::vector<int32_t> &order, std::vector<int32_t> &size)
 {
-    const int32_t cls = batch_class_of(n, k);
-    const int32_t w = (cls >= 0 && cls < BATCH_CLASSES && c->tune_mw[cls] > 0) ? c->tune_mw[cls] : 1;
-    return std::min(batch_mw_max(n, kt), pow2_floor(std::max(1, w)));
+    const int32_t count = (int32_t)work.size();
+    double total = 0;
+    for (double w : work) total += w;
+    // A team large enough that the instance takes at most a third of the
+    // batch's fair time (and not below 100 us, where barriers take over), as
+    // far as every CTA still has about a thread's state of the widest level.
+    const double most = std::max(100.0, total / blocks * 0.35);
+    size.assign((size_t)count, 1);
+    for (int32_t i = 0; i < count; i++) {
+        int32_t g = 1;
+        while (2 * g <= max_size && 2 * g <= blocks && work[(size_t)i] / g > most &&
+               states[(size_t)i] > (int64_t)RES_THREADS * g)
+            g *= 2;
+        size[(size_t)i] = g;
+    }
+    order.resize((size_t)count);
+    for (int32_t i = 0; i < count; i++) order[(size_t)i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) {
+        if (size[(size_t)x] != size[(size_t)y]) return size[(size_t)x] > size[(size_t)y];
+        return work[(size_t)x] > work[(size_t)y];
+    });
+}
+
+void batch_shape(const emv_ctx *c, BatchInst &d)
+{
+    const int32_t cls = batch_class_of(d.n, d.k);
+    const int32_t rcap = c->tune_rcap[cls] > 0 ? pow2_floor(c->tune_rcap[cls]) : 0;
+    const int32_t most = (int32_t)((resident_max_rows(d.kt) + d.size - 1) / d.size);
+    d.rows = rcap > 0 ? std::min(most, rcap) : most;
+    d.mw = resident_merge_width(d.n, d.kt, d.size, c->tune_mw[cls] > 0 ? 32 * pow2_floor(c->tune_mw[cls]) : 0);
+    d.inv_slices = res_inv_slices(d.n);
+}
+
+int32_t batch_blocks(const emv_ctx *c, int64_t ctas, int32_t cap)
+{
+    const int32_t most = cap > 0 ? std::min(cap, c->batch_blocks) : c->batch_blocks;
+    return (int32_t)std::min<int64_t>(most, std::max<int64_t>(1, ctas));
 }
 
 int prepare_batch_subsets(emv_ctx *c, cudaStream_t st)
@@ -128,31 +164,29 @@ int prepare_batch_subsets(emv_ctx *c, cudaStream_t st)
 int batch_kernel_setup(emv_ctx *c)
 {
     if (c->batch_blocks > 0) return EMV_OK;
-    CUDA_TRY(cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, BATCH_SMEM_BYTES));
+    CUDA_TRY(cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, RESIDENT_SMEM));
     int per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch, BATCH_THREADS, BATCH_SMEM_BYTES));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch, RES_THREADS, RESIDENT_SMEM));
     c->batch_blocks = std::max(1, per_sm) * c->sms;
     return EMV_OK;
 }
 
-// Launches k_batch over `count` prepared descriptors (device arrays already set).
-int launch_batch(emv_ctx *c, const BatchArgs &args, int32_t count, cudaStream_t st, int32_t max_blocks)
+// Launches k_batch on `blocks` CTAs over prepared descriptors.  Teams wait for
+// their CTAs, so the launch is cooperative unless every team is a single CTA.
+int launch_batch(emv_ctx *c, const BatchArgs &args, int32_t blocks, cudaStream_t st)
 {
     int r = batch_kernel_setup(c);
     if (r) return r;
-    CUDA_TRY(cudaMemsetAsync(args.queue, 0, sizeof(uint32_t), st));
-    const int cap = max_blocks > 0 ? std::min(max_blocks, c->batch_blocks) : c->batch_blocks;
-    const int blocks = std::min(cap, std::max(1, count));
+    CUDA_TRY(cudaMemsetAsync(args.ctl, 0, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(blocks), st));
     BatchArgs a = args;
-    k_batch<<<blocks, BATCH_THREADS, BATCH_SMEM_BYTES, st>>>(a);
-    CUDA_TRY(cudaGetLastError());
+    void *p[] = {&a};
+    if (a.end[BATCH_SIZES - 2] > 0)
+        CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_batch, dim3((unsigned)blocks), dim3(RES_THREADS), p,
+                                             (size_t)RESIDENT_SMEM, st));
+    else
+        CUDA_TRY(cudaLaunchKernel((const void *)k_batch, dim3((unsigned)blocks), dim3(RES_THREADS), p,
+                                  (size_t)RESIDENT_SMEM, st));
     return EMV_OK;
-}
-
-// Estimated device work of one instance, for largest-first ordering.
-double batch_work(int32_t n, int32_t k, int64_t arcs)
-{
-    return std::pow(3.0, k) * n * 0.5 + std::pow(2.0, k) * (double)arcs * 6.0;
 }
 
 // emv_batch_solve and emv_batch_solve_tables: tables_out (or null) receives
@@ -186,36 +220,32 @@ static int batch_solve(emv_ctx *c, const emv_instance *inst, int32_t count, int6
     });
     for (int32_t i = 0; i < count; i++)
         if (bad[(size_t)i]) return emv_fail(bad[(size_t)i], "instance %d: %s", i, why[(size_t)i].c_str());
-    // Largest first, so the persistent CTAs finish together.
-    std::vector<int32_t> order((size_t)count);
-    for (int32_t i = 0; i < count; i++) order[(size_t)i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) {
-        return batch_work(inst[x].g.n, inst[x].k, inst[x].g.arcs) > batch_work(inst[y].g.n, inst[y].k, inst[y].g.arcs);
-    });
+    std::vector<int32_t> ids((size_t)count);
+    for (int32_t i = 0; i < count; i++) ids[(size_t)i] = i;
     BatchPack pk;
-    int r = batch_pack(c, inst, order, tables_out != nullptr, pk);
-    if (r) return r;
-    r = batch_upload(c, pk, st);
+    int r = batch_kernel_setup(c);
+    if (!r) r = batch_pack(c, inst, ids, tables_out != nullptr, 0, pk);
+    if (!r) r = batch_upload(c, pk, st);
     if (r) return r;
     CUDA_TRY(cudaEventRecord(c->ev[0], st));
     BatchArgs a = batch_args(c, pk);
-    // The queue reset and the persistent launch are replayed as one CUDA graph.
-    r = batch_graph_launch(c, a, count, st);
+    // The control reset and the persistent launch are replayed as one CUDA graph.
+    r = batch_graph_launch(c, a, pk.blocks, st);
     if (r) return r;
     CUDA_TRY(cudaEventRecord(c->ev[1], st));
     CUDA_TRY(cudaMemcpyAsync(costs_out, a.costs, sizeof(int64_t) * (size_t)count, cudaMemcpyDeviceToHost, st));
     uint32_t err = 0;
-    CUDA_TRY(cudaMemcpyAsync(&err, a.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(&err, a.ctl, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     if (err) return emv_dev_status_to_emv(err);
     if (tables_out) {
-        // instance order[j] ran in launch slot j; its table (ld = n) is at table_off[j]
         for (int32_t j = 0; j < count; j++) {
-            const int32_t i = order[(size_t)j];
+            const int32_t i = pk.desc[(size_t)j].orig;
             if (!tables_out[i]) continue;
-            const size_t words = (size_t)inst[i].g.n << inst[i].k;
-            CUDA_TRY(cudaMemcpyAsync(tables_out[i], (const int32_t *)c->b_table.ptr + pk.table_off[(size_t)j],
-                                     sizeof(int32_t) * words, cudaMemcpyDeviceToHost, st));
+            const size_t row = sizeof(int32_t) * (size_t)inst[i].g.n;
+            CUDA_TRY(cudaMemcpy2DAsync(tables_out[i], row, pk.desc[(size_t)j].table,
+                                       sizeof(int32_t) * (size_t)batch_ld(inst[i].g.n), row, (size_t)1 << inst[i].k,
+                                       cudaMemcpyDeviceToHost, st));
         }
         CUDA_TRY(cudaStreamSynchronize(st));
     }
@@ -247,27 +277,48 @@ extern "C" int emv_batch_solve_tables(emv_ctx *c, const emv_instance *inst, int3
 
 // ---------------------------------------------------------------- packing
 
-int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &order, bool whole, BatchPack &pk)
+int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &ids, bool whole, int32_t blocks,
+               BatchPack &pk)
 {
-    const int32_t count = (int32_t)order.size();
+    const int32_t count = (int32_t)ids.size();
+    std::vector<double> work((size_t)count);
+    std::vector<int64_t> states((size_t)count);
+    for (int32_t j = 0; j < count; j++) {
+        const emv_instance &I = inst[ids[(size_t)j]];
+        const int32_t kt = whole ? I.k : table_terminals(I.k);
+        work[(size_t)j] = batch_work(I.g.n, kt, I.g.arcs, 1, kt);
+        states[(size_t)j] = resident_max_rows(kt) * I.g.n;
+    }
+    std::vector<int32_t> order, size;
+    // a cap of `blocks` CTAs is a measurement of single-CTA teams
+    if (blocks > 0) {
+        size.assign((size_t)count, 1);
+        order.resize((size_t)count);
+        for (int32_t j = 0; j < count; j++) order[(size_t)j] = j;
+    } else {
+        batch_plan(work, states, c->batch_blocks, 1 << (BATCH_SIZES - 1), order, size);
+    }
     pk.desc.resize((size_t)count);
     pk.row_off.resize((size_t)count);
     pk.arc_off.resize((size_t)count);
     pk.term_off.resize((size_t)count);
     pk.table_off.resize((size_t)count);
-    int64_t rows = 0, arcs = 0, terms = 0, words = 0;
+    int64_t rows = 0, arcs = 0, terms = 0, words = 0, ctas = 0;
     for (int32_t j = 0; j < count; j++) {
-        const emv_instance &I = inst[order[(size_t)j]];
+        const int32_t id = ids[(size_t)order[(size_t)j]];
+        const emv_instance &I = inst[id];
         BatchInst &d = pk.desc[(size_t)j];
         std::memset(&d, 0, sizeof(d));
         d.n = I.g.n;
         d.k = I.k;
         d.kt = whole ? I.k : table_terminals(I.k);
-        d.rcap = batch_rcap_for(c, I.g.n, I.k);
-        d.mw = batch_mw_for(c, I.g.n, I.k, d.kt);
-        d.orig = order[(size_t)j];
+        d.size = size[(size_t)order[(size_t)j]];
+        batch_shape(c, d);
+        d.orig = id;
         d.lo = 1;
         d.hi = d.kt;
+        for (int32_t cl = 0; cl < BATCH_SIZES; cl++)
+            if (d.size >= 1 << (BATCH_SIZES - 1 - cl)) pk.end[cl] = j + 1;
         pk.row_off[(size_t)j] = rows;
         pk.arc_off[(size_t)j] = arcs;
         pk.term_off[(size_t)j] = terms;
@@ -275,10 +326,12 @@ int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> 
         rows += I.g.n + 1;
         arcs += I.g.arcs;
         terms += I.k;
-        words += ((int64_t)I.g.n << d.kt);
-        pk.rcap_used = std::max(pk.rcap_used, d.rcap);
+        words += (int64_t)batch_ld(I.g.n) << d.kt;
+        ctas += d.size;
+        pk.rcap_used = std::max(pk.rcap_used, d.rows);
         pk.cost_slots = std::max<int64_t>(pk.cost_slots, (int64_t)d.orig + 1);
     }
+    pk.blocks = batch_blocks(c, ctas, blocks);
     pk.rows = rows;
     pk.arcs = arcs;
     pk.terms = terms;
@@ -302,13 +355,18 @@ int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> 
     int2 *hadj = (int2 *)(hrow + rows);
     int32_t *hterm = (int32_t *)(hadj + arcs);
     BatchInst *hdesc = (BatchInst *)(((uintptr_t)(hterm + terms) + 15) & ~(uintptr_t)15);
+    std::vector<int64_t> arc_bytes((size_t)count);
     host_parallel_for(count, [&](int64_t j) {  // disjoint ranges of the staging buffer
-        const emv_instance &I = inst[order[(size_t)j]];
+        const emv_instance &I = inst[pk.desc[(size_t)j].orig];
+        const BatchGraph bg = batch_graph(I.g.row_ptr, I.g.w, I.g.n, I.g.arcs);
+        pk.desc[(size_t)j].narrow = bg.narrow;
+        arc_bytes[(size_t)j] = bg.arc_bytes;
         std::memcpy(hrow + pk.row_off[(size_t)j], I.g.row_ptr, sizeof(int32_t) * ((size_t)I.g.n + 1));
         int2 *ha = hadj + pk.arc_off[(size_t)j];
         for (int64_t e = 0; e < I.g.arcs; e++) ha[e] = make_int2(I.g.col[e], I.g.w[e]);
         std::memcpy(hterm + pk.term_off[(size_t)j], I.terminals, sizeof(int32_t) * (size_t)I.k);
     });
+    for (int64_t b : arc_bytes) pk.arc_bytes = std::max(pk.arc_bytes, b);
     std::memcpy(hdesc, pk.desc.data(), sizeof(BatchInst) * (size_t)count);
     pk.h_row = hrow;
     pk.h_adj = hadj;
@@ -327,7 +385,8 @@ int batch_upload(emv_ctx *c, BatchPack &pk, cudaStream_t st)
     // costs are written at index orig (the caller's instance index), which can
     // exceed the number of instances in this launch when it is a sample
     if (!r) r = dev_reserve(c->b_costs, sizeof(int64_t) * (size_t)std::max<int64_t>(pk.cost_slots, 1));
-    if (!r) r = dev_reserve(c->b_ctrl, 64);
+    if (!r) r = dev_reserve(c->b_ctrl, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(c->batch_blocks));
+    if (!r) r = dev_reserve(c->b_arcs, (size_t)batch_arc_stride(pk.arc_bytes) * (size_t)pk.blocks);
     if (!r) r = prepare_batch_subsets(c, st);
     if (r) return r;
     for (int32_t j = 0; j < pk.count; j++) {
@@ -345,32 +404,35 @@ int batch_upload(emv_ctx *c, BatchPack &pk, cudaStream_t st)
     CUDA_TRY(cudaMemcpyAsync(c->b_term.ptr, pk.h_term, sizeof(int32_t) * (size_t)pk.terms, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(c->b_desc.ptr, pk.h_desc, sizeof(BatchInst) * (size_t)pk.count, cudaMemcpyHostToDevice,
                              st));
-    CUDA_TRY(cudaMemsetAsync(c->b_ctrl.ptr, 0, 64, st));
     pk.t_upload_end = std::chrono::steady_clock::now();
     return EMV_OK;
 }
+
+int64_t batch_arc_stride(int64_t arc_bytes) { return std::max<int64_t>(256, (arc_bytes + 255) / 256 * 256); }
 
 BatchArgs batch_args(emv_ctx *c, const BatchPack &pk)
 {
     BatchArgs a;
     std::memset(&a, 0, sizeof(a));  // padding included: the graph cache compares bytes
     a.inst = (const BatchInst *)c->b_desc.ptr;
-    a.count = pk.count;
     a.xs = (const uint32_t *)c->bxs.ptr;
     a.xs_off = (const int32_t *)c->bxs_off.ptr;
     a.costs = (int64_t *)c->b_costs.ptr;
-    a.queue = (uint32_t *)c->b_ctrl.ptr;
-    a.err = (uint32_t *)c->b_ctrl.ptr + 8;
+    a.ctl = (uint32_t *)c->b_ctrl.ptr;
+    a.scratch = (char *)c->b_arcs.ptr;
+    a.scratch_stride = batch_arc_stride(pk.arc_bytes);
+    a.smem = RESIDENT_SMEM;
+    std::copy(pk.end, pk.end + BATCH_SIZES, a.end);
     return a;
 }
 
-// Captures {queue reset, persistent kernel} once per argument set and replays it.
-int batch_graph_launch(emv_ctx *c, const BatchArgs &a, int32_t count, cudaStream_t st)
+// Captures {control reset, persistent kernel} once per argument set and replays it.
+int batch_graph_launch(emv_ctx *c, const BatchArgs &a, int32_t blocks, cudaStream_t st)
 {
     int r = batch_kernel_setup(c);
     if (r) return r;
     static_assert(sizeof(BatchArgs) <= sizeof(c->bgraph_args), "graph key too small");
-    const bool same = c->bgraph_exec && std::memcmp(c->bgraph_args, &a, sizeof(a)) == 0;
+    const bool same = c->bgraph_exec && c->bgraph_blocks == blocks && std::memcmp(c->bgraph_args, &a, sizeof(a)) == 0;
     if (!same) {
         if (c->bgraph_exec) cudaGraphExecDestroy(c->bgraph_exec);
         c->bgraph_exec = nullptr;
@@ -379,7 +441,7 @@ int batch_graph_launch(emv_ctx *c, const BatchArgs &a, int32_t count, cudaStream
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            r = launch_batch(c, a, count, cap);
+            r = launch_batch(c, a, blocks, cap);
             e = cudaStreamEndCapture(cap, &g);
         }
         cudaStreamDestroy(cap);
@@ -396,6 +458,7 @@ int batch_graph_launch(emv_ctx *c, const BatchArgs &a, int32_t count, cudaStream
             return emv_fail(EMV_ERR_CUDA, "batch graph instantiate: %s", cudaGetErrorString(e));
         }
         std::memcpy(c->bgraph_args, &a, sizeof(a));
+        c->bgraph_blocks = blocks;
     }
     CUDA_TRY(cudaGraphLaunch(c->bgraph_exec, st));
     return EMV_OK;
@@ -412,15 +475,16 @@ namespace {
 int time_sample(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &ids, cudaStream_t st, float &ms)
 {
     BatchPack pk;
-    int r = batch_pack(c, inst, ids, false, pk);
+    const int32_t blocks = std::max<int32_t>(1, ((int32_t)ids.size() + 3) / 4);
+    int r = batch_kernel_setup(c);
+    if (!r) r = batch_pack(c, inst, ids, false, blocks, pk);
     if (!r) r = batch_upload(c, pk, st);
     if (r) return r;
     BatchArgs a = batch_args(c, pk);
-    const int32_t blocks = std::max<int32_t>(1, (pk.count + 3) / 4);
     ms = 1e30f;
     for (int rep = 0; rep < 3; rep++) {
         CUDA_TRY(cudaEventRecord(c->ev[0], st));
-        r = launch_batch(c, a, pk.count, st, blocks);
+        r = launch_batch(c, a, pk.blocks, st);
         if (r) return r;
         CUDA_TRY(cudaEventRecord(c->ev[1], st));
         CUDA_TRY(cudaStreamSynchronize(st));
@@ -470,7 +534,7 @@ static int batch_autotune(emv_ctx *c, const emv_instance *inst, int32_t count, i
         }
         c->tune_rcap[cls] = best;
         int32_t best_mw = 1;
-        for (int32_t mw = 2; mw <= BATCH_MW_MAX && mw <= batch_mw_max(nmax, table_terminals(kmin)); mw *= 2) {
+        for (int32_t mw = 2; mw <= BATCH_MW_MAX && 16 * mw < nmax && resident_merge_width(nmax, table_terminals(kmin), 1, 32 * mw) > 16 * mw; mw *= 2) {
             c->tune_mw[cls] = mw;
             float ms = 0;
             const int r = time_sample(c, inst, ids, st, ms);

@@ -12,6 +12,9 @@ struct BatchPack {
     std::vector<int64_t> row_off, arc_off, term_off, table_off;  // into the packed device buffers
     int64_t rows = 0, arcs = 0, terms = 0, table_words = 0;
     int32_t count = 0;
+    int32_t blocks = 0;                // CTAs of the launch
+    int32_t end[emv::BATCH_SIZES] = {};  // classes (BatchArgs::end)
+    int64_t arc_bytes = 0;             // largest sliced arcs
     int32_t rcap_used = 0;
     int64_t cost_slots = 0;            // entries the device cost array needs (max orig + 1)
     int32_t *h_row = nullptr;          // views into the pinned staging buffer
@@ -22,18 +25,32 @@ struct BatchPack {
 };
 
 int32_t batch_class_of(int32_t n, int32_t k);
-int32_t batch_rcap_max(int32_t n);
-int32_t batch_rcap_for(const emv_ctx *c, int32_t n, int32_t k);
-int32_t batch_mw_max(int32_t n, int32_t k);
-int32_t batch_mw_for(const emv_ctx *c, int32_t n, int32_t k, int32_t kt);  // class of (n, k), rows of kt
 bool batch_fits(int32_t n, int32_t k);
-double batch_work(int32_t n, int32_t k, int64_t arcs);
+// What the kernel needs to know of a host graph beyond its sizes.
+struct BatchGraph {
+    bool narrow;         // every weight fits a packed arc
+    int64_t arc_bytes;   // sliced arcs
+};
+BatchGraph batch_graph(const int32_t *row_ptr, const int32_t *w, int32_t n, int64_t arcs);
+// Estimated time (us) of levels lo..hi on one CTA.
+double batch_work(int32_t n, int32_t kt, int64_t arcs, int32_t lo, int32_t hi);
+// Team sizes (at most max_size) for a grid of `blocks` CTAs and the order by
+// class (then largest first): order[j] is the input's index, size[] by input index.
+void batch_plan(const std::vector<double> &work, const std::vector<int64_t> &states, int32_t blocks, int32_t max_size,
+                std::vector<int32_t> &order, std::vector<int32_t> &size);
+// Fills the fields that follow from n, k, kt and the team size.
+void batch_shape(const emv_ctx *c, emv::BatchInst &d);
 int prepare_batch_subsets(emv_ctx *c, cudaStream_t st);
 int batch_kernel_setup(emv_ctx *c);
-// whole: solve the subsets of all terminals (the tables are wanted), else those the costs need.
-int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &order, bool whole, BatchPack &pk);
+// whole: solve the subsets of all terminals (the tables are wanted), else
+// those the costs need.  blocks: CTAs of the launch that will take the pack.
+int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &ids, bool whole, int32_t blocks,
+               BatchPack &pk);
 int batch_upload(emv_ctx *c, BatchPack &pk, cudaStream_t st);
 emv::BatchArgs batch_args(emv_ctx *c, const BatchPack &pk);
-// max_blocks > 0 caps the persistent grid (the autotuner's samples).
-int launch_batch(emv_ctx *c, const emv::BatchArgs &a, int32_t count, cudaStream_t st, int32_t max_blocks = 0);
-int batch_graph_launch(emv_ctx *c, const emv::BatchArgs &a, int32_t count, cudaStream_t st);
+int launch_batch(emv_ctx *c, const emv::BatchArgs &a, int32_t blocks, cudaStream_t st);
+int batch_graph_launch(emv_ctx *c, const emv::BatchArgs &a, int32_t blocks, cudaStream_t st);
+// Bytes of BatchArgs::scratch for every CTA, from the largest sliced arcs.
+int64_t batch_arc_stride(int64_t arc_bytes);
+// CTAs for instances whose team sizes sum to ctas.
+int32_t batch_blocks(const emv_ctx *c, int64_t ctas, int32_t cap);

@@ -129,7 +129,9 @@ extern "C" int emv_destroy(emv_ctx *c)
     cudaSetDevice(c->device);
     cudaDeviceSynchronize();
     for (DevBuf *b : {&c->ctrl, &c->stat, &c->lvlmax, &c->gscan, &c->shadow, &c->scratch, &c->act, &c->adj, &c->stamp, &c->terms, &c->g_row,
-                      &c->g_col, &c->g_w, &c->table, &c->tb_edges, &c->tb_out, &c->tb_work, &c->res_arcs, &c->res_out})
+                      &c->g_col, &c->g_w, &c->table, &c->tb_edges, &c->tb_out, &c->tb_work, &c->res_arcs, &c->res_out,
+                      &c->bxs, &c->bxs_off, &c->b_row, &c->b_adj, &c->b_term, &c->b_desc, &c->b_table, &c->b_costs,
+                      &c->b_ctrl, &c->b_arcs})
         dev_release(*b);
     for (KPlan *p : c->kplans) {
         if (!p) continue;
@@ -140,6 +142,8 @@ extern "C" int emv_destroy(emv_ctx *c)
         if (c->ev[i]) cudaEventDestroy(c->ev[i]);
     for (int i = 0; i <= EMV_MAX_K; i++)
         if (c->evmax[i]) cudaEventDestroy(c->evmax[i]);
+    if (c->bgraph_exec) cudaGraphExecDestroy(c->bgraph_exec);
+    if (c->bstage) cudaFreeHost(c->bstage);
     if (c->pinned) cudaFreeHost(c->pinned);
     delete c;
     return EMV_OK;
@@ -631,7 +635,7 @@ extern "C" int emv_kernel_dev(emv_ctx *c, int32_t n, int64_t arcs, const int32_t
     cudaStream_t st = (cudaStream_t)stream;
     c->launches = 0;
     ResidentPlan plan;
-    if (resident_plan(c, n, arcs, k, plan))
+    if (resident_plan(c, n, k, plan))
         return run_resident(c, plan, n, arcs, d_row_ptr, d_col, d_w, terminals, k, k, d_table, ld, true, st, cost_out,
                             nullptr);
     r = pack_and_check(c, n, arcs, d_row_ptr, d_col, d_w, true, st);
@@ -726,7 +730,7 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
     const int32_t kt = whole ? k : table_terminals(k);
     const size_t tbytes = sizeof(int32_t) * (size_t)ld << kt;
     ResidentPlan plan;
-    const bool resident = resident_plan(c, n, arcs, kt, plan);
+    const bool resident = resident_plan(c, n, kt, plan);
     int r = resident ? EMV_OK : pack_and_check(c, n, arcs, row_ptr, col, w, check, st);
     if (!r) r = dev_reserve(c->table, tbytes);
     if (r) return r;

@@ -144,6 +144,12 @@ __device__ __forceinline__ int4 vadd(int4 a, int32_t w) { return make_int4(a.x +
 __device__ __forceinline__ bool vlt(int32_t a, int32_t b) { return a < b; }
 __device__ __forceinline__ bool vlt(int2 a, int2 b) { return a.x < b.x || a.y < b.y; }
 __device__ __forceinline__ bool vlt(int4 a, int4 b) { return a.x < b.x || a.y < b.y || a.z < b.z || a.w < b.w; }
+// min(a + w, c)
+__device__ __forceinline__ int4 vaddmin(int4 a, int32_t w, int4 c)
+{
+    return make_int4(__viaddmin_s32(a.x, w, c.x), __viaddmin_s32(a.y, w, c.y), __viaddmin_s32(a.z, w, c.z),
+                     __viaddmin_s32(a.w, w, c.w));
+}
 __device__ __forceinline__ int8v vmin(int8v x, int8v y) { return {vmin(x.a, y.a), vmin(x.b, y.b)}; }
 __device__ __forceinline__ int8v vadd(int8v x, int32_t w) { return {vadd(x.a, w), vadd(x.b, w)}; }
 __device__ __forceinline__ bool vlt(int8v x, int8v y) { return vlt(x.a, y.a) || vlt(x.b, y.b); }

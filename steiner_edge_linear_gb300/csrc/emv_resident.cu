@@ -8,33 +8,81 @@
 
 using namespace emv;
 
-// Whether a solve of n vertices over kt terminals' subsets runs as one
-// launch, and its shape.  The closure of a row needs about 7.4 bytes a vertex
-// of shared memory (distance, list entry, two marks, arc count), so n is at
-// most about 30 000.  Levels of more rows than SMs (kt >= 10) take turns on
-// them, and the record kernels, which read an arc once for 256 rows, are
-// faster from a few thousand vertices on.
-bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, ResidentPlan &p)
+namespace emv {
+
+// The whole solve: CSR check, arc slices, levels 1..kt.
+__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(ResArgs a)
 {
-    (void)arcs;
-    if (kt > RES_KMAX || (kt > 9 && n > 4096)) return false;
-    const int sms = c->relax_sm_cap > 0 && c->relax_sm_cap < c->sms ? c->relax_sm_cap : c->sms;
-    int64_t maxcnt = 1;
+    __shared__ ResShared sh;
+    ResTeam tm{a.out->bar, &a.out->err, (int32_t)blockIdx.x, (int32_t)gridDim.x, 0};
+    const int64_t first = (int64_t)blockIdx.x * RES_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * RES_THREADS;
+    const ResSmem sm = res_layout(a.inst.n, a.inst.kt, a.smem, a.xs, a.lvl[a.inst.kt + 1]);
+    if (threadIdx.x == 0) sh.ok = 1;  // before the barrier that first reads it
+    if (threadIdx.x < EMV_MAX_K) sh.terms[threadIdx.x] = a.terms[threadIdx.x];
+    if (threadIdx.x < RES_KMAX + 2) sh.lvl[threadIdx.x] = a.lvl[threadIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x < EMV_MAX_K) a.out->terms[threadIdx.x] = a.terms[threadIdx.x];
+    scan_csr(a.inst.row_ptr, a.inst.n, a.col, a.w, a.adj, a.arcs, &a.out->scan);
+    for (int64_t v = first; v < a.inst.n; v += stride) a.inst.table[v] = INF;  // row 0 (R:2243-2259)
+    if (!res_barrier(tm, sh)) return;
+    const uint32_t bad = __ldcg(&a.out->scan.bad), maxw = __ldcg(&a.out->scan.maxw);
+    if (a.check) {  // the host reads the same words and names the fault
+        if (bad) return;
+        const long long bound =
+            min((long long)(a.inst.n - 1) * (long long)maxw, (long long)(__ldcg(&a.out->scan.sumw) / 2));
+        if (bound >= INF) return;
+    }
+    res_solve(a.inst, tm, sm, sh, maxw < RES_MAX_W && !(bad & SCAN_BAD_WEIGHT), 1, a.inst.kt);
+}
+
+}  // namespace emv
+
+int64_t resident_max_rows(int32_t kt)
+{
+    int64_t most = 1;
     for (int32_t m = 1, x = 1; m <= kt; m++) {
         x = (int32_t)((int64_t)x * (kt - m + 1) / m);
-        maxcnt = std::max<int64_t>(maxcnt, x);
+        most = std::max<int64_t>(most, x);
     }
+    return most;
+}
+
+bool resident_fits(int32_t n, int32_t kt)
+{
+    if (kt > RES_KMAX || n > 32 * RES_THREADS) return false;
+    const int64_t big = RESIDENT_SMEM - res_fixed_smem(n, kt);
+    return res_state_bytes(n, 1) <= big && ((int64_t)16 << kt) + 4 * RES_ACC_WORDS <= big;  // a merge block of 4 vertices
+}
+
+int32_t resident_merge_width(int32_t n, int32_t kt, int32_t ctas, int32_t cap)
+{
+    const int64_t big = RESIDENT_SMEM - res_fixed_smem(n, kt);
+    int64_t wmax = std::min<int64_t>((big - 4 * RES_ACC_WORDS) / ((int64_t)16 << kt) * 4, (int64_t)(n + 3) / 4 * 4);
+    if (cap > 0) wmax = std::min<int64_t>(wmax, std::max<int64_t>(4, cap / 4 * 4));
+    const int64_t waves = (n + ctas * wmax - 1) / (ctas * wmax);
+    return (int32_t)std::min<int64_t>(wmax, ((n + ctas * waves - 1) / (ctas * waves) + 3) / 4 * 4);
+}
+
+uint32_t res_inv_slices(int32_t n)
+{
+    const uint64_t slices = ((uint64_t)n + 31) / 32;
+    return slices == 1 ? 0u : (uint32_t)((((uint64_t)1 << 32) + slices - 1) / slices);
+}
+
+// Whether a solve of n vertices over kt terminals' subsets runs as one
+// launch, and its shape.  The closure of a row needs about 7.3 bytes a vertex
+// of shared memory (distance, list entry, mark, arc count), so n is at most
+// about 31 000.  Levels of more rows than SMs (kt >= 10) take turns on them,
+// and the record kernels, which read an arc once for 256 rows, are faster
+// from a few thousand vertices on.
+bool resident_plan(const emv_ctx *c, int32_t n, int32_t kt, ResidentPlan &p)
+{
+    if (!resident_fits(n, kt) || (kt > 9 && n > 4096)) return false;
+    const int sms = c->relax_sm_cap > 0 && c->relax_sm_cap < c->sms ? c->relax_sm_cap : c->sms;
+    const int64_t maxcnt = resident_max_rows(kt);
     // a CTA for every 1024 states of the widest level
     p.blocks = (int)std::max<int64_t>(1, std::min<int64_t>(sms, (maxcnt * n + RES_THREADS - 1) / RES_THREADS));
     p.rows = (int32_t)((maxcnt + p.blocks - 1) / p.blocks);
-    const int64_t big = RESIDENT_SMEM - res_fixed_smem(n, kt);
-    const int64_t merge_min = ((int64_t)16 << kt) + 4 * RES_ACC_WORDS;  // blocks of 4 vertices
-    if (n > 32 * RES_THREADS || res_state_bytes(n, 1) > big || merge_min > big) return false;
-    // merge blocks: as few waves of blocks as the shared memory allows, and
-    // within them the narrowest blocks, so that every CTA has some
-    const int64_t wmax = std::min<int64_t>((big - 4 * RES_ACC_WORDS) / ((int64_t)16 << kt) * 4, (int64_t)(n + 3) / 4 * 4);
-    const int64_t waves = (n + p.blocks * wmax - 1) / (p.blocks * wmax);
-    p.mw = (int32_t)std::min<int64_t>(wmax, ((n + p.blocks * waves - 1) / (p.blocks * waves) + 3) / 4 * 4);
+    p.mw = resident_merge_width(n, kt, p.blocks, 0);
     return true;
 }
 
@@ -56,29 +104,34 @@ int run_resident(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, con
     }
     ResArgs a;
     std::memset(&a, 0, sizeof(a));
-    a.row_ptr = row_ptr;
+    ResInst &I = a.inst;
     a.col = col;
     a.w = w;
     a.adj = (int2 *)c->adj.ptr;
-    a.slices = c->res_arcs.ptr;
-    a.table = table;
     a.xs = (const uint32_t *)c->kp->xs.ptr;
     a.out = (ResOut *)c->res_out.ptr;
-    a.ld = ld;
     a.arcs = arcs;
-    a.n = n;
-    a.k = k;
-    a.kt = kt;
     a.check = check;
-    a.vec = ld % 4 == 0 && ((uintptr_t)table & 15) == 0;
-    a.want_rows = p.rows;
-    a.mw = p.mw;
     a.smem = RESIDENT_SMEM;
-    a.max_rounds = (c->sweep_limit > 0 && c->sweep_limit < (int64_t)n + 1) ? (int32_t)c->sweep_limit : n + 1;
-    const uint64_t slices = ((uint64_t)n + 31) / 32;
-    a.inv_slices = slices == 1 ? 0u : (uint32_t)((((uint64_t)1 << 32) + slices - 1) / slices);
-    for (int32_t m = 0; m <= kt + 1; m++) a.xs_off[m] = (int32_t)c->kp->xs_off[(size_t)m];
+    for (int32_t m = 0; m <= kt + 1; m++) a.lvl[m] = (int32_t)c->kp->xs_off[(size_t)m];
     for (int32_t t = 0; t < k; t++) a.terms[t] = terms[t];
+    I.row_ptr = row_ptr;
+    I.adj = a.adj;
+    I.slices = c->res_arcs.ptr;
+    I.table = table;
+    I.cost = &a.out->cost;
+    I.unreached = &a.out->unreached;
+    I.rounds = &a.out->rounds;
+    I.ns = a.out->ns;
+    I.ld = ld;
+    I.n = n;
+    I.k = k;
+    I.kt = kt;
+    I.vec = ld % 4 == 0 && ((uintptr_t)table & 15) == 0;
+    I.want_rows = p.rows;
+    I.mw = p.mw;
+    I.max_rounds = (c->sweep_limit > 0 && c->sweep_limit < (int64_t)n + 1) ? (int32_t)c->sweep_limit : n + 1;
+    I.inv_slices = res_inv_slices(n);
     CUDA_TRY(cudaMemsetAsync(a.out, 0, sizeof(ResOut), st));
     CUDA_TRY(cudaEventRecord(c->ev[0], st));
     void *args[] = {&a};
@@ -100,7 +153,7 @@ int run_resident(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, con
     if (h->err) return emv_dev_status_to_emv(h->err);
     if (check && h->unreached)
         return emv_fail(EMV_ERR_DISCONNECTED, "graph: not connected (a vertex is unreachable from terminal 1)");
-    *cost_out = (k >= 2 && h->cost < INF) ? (int64_t)h->cost : INT64_MAX;
+    *cost_out = k >= 2 ? h->cost : INT64_MAX;
     if (tm) {
         float ms = 0;
         cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]);

@@ -42,36 +42,64 @@ constexpr float RES_PULL_SHARE = 0.2f;   // a round after one that changed more 
 constexpr uint32_t RES_SPIN_LIMIT = 1u << 22;  // polls of an L2 word, over a second in all
 constexpr int RES_ACC_WORDS = 2 * RES_THREADS;  // merge minima of a level with at most half as many tasks as threads
 
-// Control and result words of one launch (zeroed before it).
+// One instance as the device functions below take it.
+struct ResInst {
+    const int32_t *row_ptr;
+    const int2 *adj;          // (head, weight) arcs
+    void *slices;             // sliced arcs (written here)
+    int32_t *table;           // 2^kt rows of stride ld
+    int64_t *cost;            // d[C][t_{k-1}], INT64_MAX without a value
+    uint32_t *unreached;      // if set: a level-1 closure left a vertex without a value
+    uint32_t *rounds;         // if set: += rounds of the closures (pull sweeps, push rounds)
+    unsigned long long *ns;   // if set: time of level 1, merges, relaxations (the first CTA's view)
+    int64_t ld;
+    int32_t n, k, kt;
+    int32_t vec;              // table rows are 16-byte aligned
+    int32_t want_rows;        // most rows of a closure
+    int32_t mw;               // vertices of a merge block (multiple of 4)
+    int32_t max_rounds;
+    uint32_t inv_slices;      // ceil(2^32 / slices), for slices > 1
+};
+
+// The CTAs that share an instance: all of them on the GPU at once.
+struct ResTeam {
+    uint32_t *bar;            // arrivals, on a line of its own, zero at first
+    uint32_t *err;            // EMV_DEV_* bits
+    int32_t rank, size;
+    uint32_t epoch;           // barriers passed
+};
+
+// A CTA's static shared memory.
+struct ResShared {
+    int ok;                   // 1 until the team failed
+    int32_t terms[EMV_MAX_K];
+    int32_t hubs[RES_WARPS];
+    int32_t lvl[RES_KMAX + 2];  // level m of the subset list: [lvl[m], lvl[m + 1])
+};
+
+// Control and result words of one k_resident launch (zeroed before it).
 struct ResOut {
-    uint32_t bar[32];        // arrivals of the grid barrier, on a line of its own
-    uint32_t err;            // EMV_DEV_* bits
-    uint32_t unreached;      // a level-1 closure left a vertex without a value
-    uint32_t hubs;           // a vertex has more than RES_HUB arcs
-    uint32_t rounds;         // pull sweeps and push rounds, summed over the CTAs' chunks
+    uint32_t bar[32];
+    uint32_t err;
+    uint32_t unreached;
+    uint32_t rounds;
+    uint32_t pad;
     GraphScan scan;
-    unsigned long long ns[3];  // level 1, merges, relaxations (CTA 0's view)
-    int32_t cost;            // d[C][t_{k-1}]
+    unsigned long long ns[3];
+    int64_t cost;
     int32_t terms[EMV_MAX_K];
 };
 
 struct ResArgs {
-    const int32_t *row_ptr, *col, *w;  // the CSR as given
-    int2 *adj;                // (head, weight) arcs (written here; read for hubs and by the traceback)
-    void *slices;             // sliced arcs (written here)
-    int32_t *table;           // 2^kt rows of stride ld
+    ResInst inst;
+    const int32_t *col, *w;   // the CSR as given
+    int2 *adj;                // (head, weight) arcs (written here; also read by the traceback)
     const uint32_t *xs;       // subsets by level
     ResOut *out;
-    int64_t ld, arcs;
-    int32_t n, k, kt;
+    int64_t arcs;
     int32_t check;            // leave after the CSR check found a fault
-    int32_t vec;              // table rows are 16-byte aligned
-    int32_t want_rows;        // rows of the widest level's largest share
-    int32_t mw;               // vertices of a merge block (multiple of 4)
     int32_t smem;             // dynamic shared memory
-    int32_t max_rounds;
-    uint32_t inv_slices;      // ceil(2^32 / slices), for slices > 1
-    int32_t xs_off[RES_KMAX + 2];
+    int32_t lvl[RES_KMAX + 2];
     int32_t terms[EMV_MAX_K];
 };
 
@@ -99,41 +127,40 @@ __device__ __forceinline__ volatile int32_t &res_i32(int32_t off)
 
 constexpr uint32_t RES_FAILED = 1u << 31;  // set in the barrier word when a CTA failed
 
-// Records an error and makes every CTA leave at its next barrier.
-__device__ __forceinline__ void res_fail(ResOut *out, uint32_t err, int *s_ok)
+// Records an error and makes every CTA of the team leave at its next barrier.
+__device__ __forceinline__ void res_fail(const ResTeam &t, uint32_t err, ResShared &sh)
 {
-    atomicOr(&out->err, err);
-    atomicOr(out->bar, RES_FAILED);
-    *(volatile int *)s_ok = 0;
+    atomicOr(t.err, err);
+    atomicOr(t.bar, RES_FAILED);
+    *(volatile int *)&sh.ok = 0;
 }
 
-// Barrier over the grid's CTAs (all resident: a cooperative launch, or one
-// CTA).  Arrivals only count up, so no word is reset.  Bounded: a CTA that
-// waits longer than RES_SPIN_LIMIT polls records the error; every CTA leaves
-// when it sees one (*s_ok is 1 until then).
-__device__ __forceinline__ bool res_barrier(ResOut *out, uint32_t &epoch, int *s_ok)
+// Barrier over the team's CTAs.  Arrivals only count up, so no word is reset.
+// Bounded: a CTA that waits longer than RES_SPIN_LIMIT polls records the
+// error; every CTA of the team leaves when it sees one.
+__device__ __forceinline__ bool res_barrier(ResTeam &t, ResShared &sh)
 {
     __syncthreads();
-    epoch++;
-    if (gridDim.x > 1) {
+    t.epoch++;
+    if (t.size > 1) {
         if (threadIdx.x == 0) {
-            const uint32_t target = epoch * gridDim.x;
+            const uint32_t target = t.epoch * (uint32_t)t.size;
             uint32_t spins = 0, seen;
             __threadfence();
-            atomicAdd(out->bar, 1u);
+            atomicAdd(t.bar, 1u);
             for (;;) {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(out->bar) : "memory");
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(t.bar) : "memory");
                 if ((seen & RES_FAILED) || (seen & ~RES_FAILED) >= target) break;
                 if (++spins > RES_SPIN_LIMIT) {
-                    res_fail(out, EMV_DEV_BARRIER_TIMEOUT, s_ok);
+                    res_fail(t, EMV_DEV_BARRIER_TIMEOUT, sh);
                     break;
                 }
             }
-            if (seen & RES_FAILED) *(volatile int *)s_ok = 0;
+            if (seen & RES_FAILED) *(volatile int *)&sh.ok = 0;
         }
         __syncthreads();
     }
-    return *(volatile int *)s_ok != 0;
+    return *(volatile int *)&sh.ok != 0;
 }
 
 __device__ __forceinline__ unsigned long long res_now()
@@ -166,10 +193,10 @@ __device__ __forceinline__ uint4 res_pairs(const uint4 *__restrict__ Sq, int32_t
     for (uint32_t p = p0; p < p1; p++) {
         const uint32_t Y = low | sub;
         const uint4 y = Sq[Y * Q], z = Sq[(X ^ Y) * Q];
-        a.x = min(a.x, y.x + z.x);
-        a.y = min(a.y, y.y + z.y);
-        a.z = min(a.z, y.z + z.z);
-        a.w = min(a.w, y.w + z.w);
+        a.x = __viaddmin_u32(y.x, z.x, a.x);
+        a.y = __viaddmin_u32(y.y, z.y, a.y);
+        a.z = __viaddmin_u32(y.z, z.z, a.z);
+        a.w = __viaddmin_u32(y.w, z.w, a.w);
         sub = (sub - rest) & rest;
     }
     return a;
@@ -178,39 +205,77 @@ __device__ __forceinline__ uint4 res_pairs(const uint4 *__restrict__ Sq, int32_t
 // Bytes of the merge's staged rows and of the minima of split pair lists.
 __host__ __device__ inline int32_t res_merge_bytes(int32_t mw, int32_t kt) { return ((4 * mw) << kt) + 4 * RES_ACC_WORDS; }
 
+// Finishes 4 merged vertices from v on of subset X: the arcs of the virtual
+// source (R:2099-2107; value(Y, d): vertex v + d of row Y) and the store.
+template <typename F>
+__device__ __forceinline__ void res_merged(const ResInst &a, const int32_t *terms, bool has_term, uint32_t X, int32_t v,
+                                           uint4 r, F value)
+{
+    if (has_term)
+        for (uint32_t bits = X; bits; bits &= bits - 1) {
+            const int ti = __ffs(bits) - 1, d = terms[ti] - v;
+            if (d < 0 || d >= 4) continue;
+            const uint32_t o = value(X ^ (1u << ti), d);
+            if (d == 0) r.x = o;
+            else if (d == 1) r.y = o;
+            else if (d == 2) r.z = o;
+            else r.w = o;
+        }
+    int32_t *dst = a.table + (int64_t)X * a.ld + v;
+    if (a.vec && v + 4 <= a.n) *reinterpret_cast<uint4 *>(dst) = r;
+    else {
+        if (v < a.n) dst[0] = (int32_t)r.x;
+        if (v + 1 < a.n) dst[1] = (int32_t)r.y;
+        if (v + 2 < a.n) dst[2] = (int32_t)r.z;
+        if (v + 3 < a.n) dst[3] = (int32_t)r.w;
+    }
+}
+
+// Four vertices of a table row from v on (INF past n).
+__device__ __forceinline__ int4 res_row4(const ResInst &a, uint32_t X, int32_t v)
+{
+    const int32_t *src = a.table + (int64_t)X * a.ld + v;
+    if (a.vec && v + 4 <= a.n) return __ldcg(reinterpret_cast<const int4 *>(src));
+    return make_int4(v < a.n ? __ldcg(src) : INF, v + 1 < a.n ? __ldcg(src + 1) : INF, v + 2 < a.n ? __ldcg(src + 2) : INF,
+                     v + 3 < a.n ? __ldcg(src + 3) : INF);
+}
+
 // Merge of level m for this CTA's vertex blocks, in the last res_merge_bytes
 // of the shared memory: 2^kt rows of mw words (row Y at Y * mw) and, after
-// them, the minima of split pair lists.
-__device__ void res_merge(const ResArgs &a, const ResSmem &sm, int32_t m, const int32_t *terms)
+// them, the minima of split pair lists.  (Blocks of half the width in two
+// halves of that space, the next staged while one is reduced: 280 against 212
+// us at n = 4000, kt = 11, and 5 % more time for 4096 mixed instances; level 2
+// read directly from the table, one pair a subset: the same.)
+__device__ __forceinline__ void res_merge(const ResInst &a, const ResTeam &tm, const ResSmem &sm, const ResShared &sh,
+                                          int32_t m)
 {
-    uint32_t *S = &res_at<uint32_t>(sm.end - res_merge_bytes(a.mw, a.kt));
     const uint16_t *xs = &res_at<uint16_t>(sm.xs);
-    const int32_t n = a.n, W = a.mw, Q = W / 4, tid = threadIdx.x;
-    const int32_t nlow = a.xs_off[m], cnt = a.xs_off[m + 1] - nlow;
+    const int32_t *terms = sh.terms;
+    const int32_t n = a.n, tid = threadIdx.x, kt = a.kt;
+    const int32_t nlow = sh.lvl[m], cnt = sh.lvl[m + 1] - nlow;
+    uint32_t *S = &res_at<uint32_t>(sm.end - res_merge_bytes(a.mw, kt));
+    uint32_t *acc = S + ((size_t)a.mw << kt);
+    const int32_t W = a.mw, Q = W / 4;
     const uint32_t npairs = (1u << (m - 1)) - 1;
     const int32_t tasks = cnt * Q;
     int32_t parts = 1;
     while (tasks * parts * 2 <= RES_THREADS && (uint32_t)parts * 2 <= npairs) parts *= 2;
-    uint32_t *acc = S + ((size_t)W << a.kt);
     const uint4 *S4 = reinterpret_cast<const uint4 *>(S);
-    for (int32_t v0 = blockIdx.x * W; v0 < n; v0 += gridDim.x * W) {
-        bool has_term = false;
-        for (int32_t t = 0; t < a.kt; t++) has_term |= terms[t] >= v0 && terms[t] < v0 + W;
+    for (int32_t v0 = tm.rank * W; v0 < n; v0 += tm.size * W) {
         for (int32_t i = tid; i < nlow * Q; i += RES_THREADS) {
-            const int32_t r = i / Q, q = i - r * Q;
+            const int32_t r = i / Q, q = i - r * Q, v = v0 + 4 * q;
             const uint32_t Y = xs[r];
-            const int32_t v = v0 + 4 * q;
-            const int32_t *src = a.table + (int64_t)Y * a.ld + v;
-            int4 x;
-            if (a.vec && v + 4 <= n) x = __ldcg(reinterpret_cast<const int4 *>(src));
-            else
-                x = make_int4(v < n ? __ldcg(src) : INF, v + 1 < n ? __ldcg(src + 1) : INF,
-                              v + 2 < n ? __ldcg(src + 2) : INF, v + 3 < n ? __ldcg(src + 3) : INF);
-            reinterpret_cast<int4 *>(S)[Y * Q + q] = x;
+            int4 *to = reinterpret_cast<int4 *>(S) + Y * Q + q;
+            // a row is ld >= n words: its last quad may hold words past n
+            if (a.vec && v < n) cp_async16(to, a.table + (int64_t)Y * a.ld + v);
+            else if (!a.vec) *to = res_row4(a, Y, v);
         }
         if (parts > 1)
             for (int32_t i = tid; i < cnt * W; i += RES_THREADS) acc[i] = (uint32_t)INF;
+        cp_async_wait_all();
         __syncthreads();
+        bool has_term = false;
+        for (int32_t t = 0; t < kt; t++) has_term |= terms[t] >= v0 && terms[t] < v0 + W;
         if (parts > 1) {
             for (int32_t t = tid; t < tasks * parts; t += RES_THREADS) {
                 const int32_t part = t / tasks, u = t - part * tasks, xi = u / Q, q = u - xi * Q;
@@ -227,26 +292,9 @@ __device__ void res_merge(const ResArgs &a, const ResSmem &sm, int32_t m, const 
         for (int32_t t = tid; t < tasks; t += RES_THREADS) {
             const int32_t xi = t / Q, q = t - xi * Q;
             const uint32_t X = xs[nlow + xi];
-            uint4 r = parts > 1 ? reinterpret_cast<const uint4 *>(acc)[t] : res_pairs(S4 + q, Q, X, 0, npairs);
-            const int32_t v = v0 + 4 * q;
-            if (has_term)  // arcs of the virtual source (R:2099-2107)
-                for (uint32_t bits = X; bits; bits &= bits - 1) {
-                    const int ti = __ffs(bits) - 1, d = terms[ti] - v;
-                    if (d < 0 || d >= 4) continue;
-                    const uint32_t o = S[(X ^ (1u << ti)) * W + 4 * q + d];
-                    if (d == 0) r.x = o;
-                    else if (d == 1) r.y = o;
-                    else if (d == 2) r.z = o;
-                    else r.w = o;
-                }
-            int32_t *dst = a.table + (int64_t)X * a.ld + v;
-            if (a.vec && v + 4 <= n) *reinterpret_cast<uint4 *>(dst) = r;
-            else {
-                if (v < n) dst[0] = (int32_t)r.x;
-                if (v + 1 < n) dst[1] = (int32_t)r.y;
-                if (v + 2 < n) dst[2] = (int32_t)r.z;
-                if (v + 3 < n) dst[3] = (int32_t)r.w;
-            }
+            const uint4 r = parts > 1 ? reinterpret_cast<const uint4 *>(acc)[t] : res_pairs(S4 + q, Q, X, 0, npairs);
+            res_merged(a, terms, has_term, X, v0 + 4 * q, r,
+                       [&](uint32_t Y, int d) { return S[Y * W + 4 * q + d]; });
         }
         __syncthreads();
     }
@@ -287,7 +335,7 @@ template <ResArcs SRC> struct ResGraph {
         int32_t off[2], w[2];
         unpack(x, off, w);
         const int32_t p = res_i32(row + off[0]), q = res_i32(row + off[1]);
-        return min(min(acc, p + w[0]), q + w[1]);
+        return __viaddmin_s32(q, w[1], __viaddmin_s32(p, w[0], acc));
     }
     static __device__ __forceinline__ void unpack(const T &x, int32_t (&off)[2], int32_t (&w)[2])
     {
@@ -305,10 +353,10 @@ template <ResArcs SRC> struct ResGraph {
     }
 };
 
-// wd / slices for a word index below 2^16.
-__device__ __forceinline__ int32_t res_div(const ResArgs &a, int32_t wd, int32_t slices)
+// wd / slices for a word index below 2^16 (inv: ResInst::inv_slices).
+__device__ __forceinline__ int32_t res_div(uint32_t inv, int32_t wd, int32_t slices)
 {
-    return slices == 1 ? wd : (int32_t)__umulhi((uint32_t)wd, a.inv_slices);
+    return slices == 1 ? wd : (int32_t)__umulhi((uint32_t)wd, inv);
 }
 
 // Closure of R rows in shared memory: states s = r * 32 * slices + v,
@@ -335,14 +383,15 @@ __device__ __forceinline__ int32_t res_div(const ResArgs &a, int32_t wd, int32_t
 // warp per vertex: one warp would otherwise walk all hubs of its run.
 // Returns false when max_rounds ran out; `rounds` counts barriers passed.
 template <ResArcs SRC>
-__device__ bool res_close(const ResArgs &a, const ResGraph<SRC> &g, bool has_hubs, int32_t R, bool level1, int32_t d,
+__device__ bool res_close(const ResInst &a, const ResGraph<SRC> &g, bool has_hubs, int32_t R, bool level1, int32_t d,
                           int32_t list, int32_t bm, int32_t *hub_cnt, int32_t &rounds)
 {
     using G = ResGraph<SRC>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1;
-    const int32_t slices = (a.n + 31) >> 5, words = R * slices;
-    auto row_of = [&](int32_t wd) -> int32_t { return R == 1 ? 0 : res_div(a, wd, slices); };
+    const int32_t slices = (a.n + 31) >> 5, words = R * slices, max_rounds = a.max_rounds;
+    const uint32_t inv = a.inv_slices;
+    auto row_of = [&](int32_t wd) -> int32_t { return R == 1 ? 0 : res_div(inv, wd, slices); };
     // this warp's words; its list holds at most their states
     const int32_t per = (words + RES_WARPS - 1) / RES_WARPS;
     const int32_t w0 = min(words, warp * per), w1 = min(words, w0 + per);
@@ -358,7 +407,7 @@ __device__ bool res_close(const ResArgs &a, const ResGraph<SRC> &g, bool has_hub
             for (int j = 0; j < 4; j++) x[j] = g.elem((first + min(j, max(width - 1, 0))) * 32 + lane);
             bool changed = false;
             do {
-                if (++rounds > a.max_rounds) return false;
+                if (++rounds > max_rounds) return false;
                 changed = false;
                 if (w0 < words && width > 0)
 #pragma unroll
@@ -403,7 +452,7 @@ __device__ bool res_close(const ResArgs &a, const ResGraph<SRC> &g, bool has_hub
     const int many = (int)(RES_THREADS * (1.0f - same));
     bool pull = !level1, any = true;
     for (;;) {
-        if (++rounds > a.max_rounds) return false;
+        if (++rounds > max_rounds) return false;
         if (pull) {
             int32_t hubs = 0;
             any = false;
@@ -533,27 +582,141 @@ __device__ bool res_close(const ResArgs &a, const ResGraph<SRC> &g, bool has_hub
 // Bytes of the states of R rows: distances, lists, the bitmap.
 __host__ __device__ inline int64_t res_state_bytes(int32_t n, int64_t R) { return (n + 31) / 32 * R * 196; }
 
+// Closure of nr <= R rows (R = 8, 16, .. 128) kept vertex by vertex: the R
+// distances of a vertex side by side, four to a lane, so that an arc is
+// decoded once for four rows and its head is read with 16-byte loads, which
+// meet the fewer bank conflicts the more rows lie together (none from 32 on,
+// where a quarter-warp reads 128 bytes).  A sweep takes every vertex, but for
+// a row and arc it needs a third of res_close's instructions, which outweighs
+// that res_close takes fewer states; used for shares of at least
+// RES_WIDE_MIN rows.  From 32 rows on, 16 bytes of padding per vertex keep the
+// transposing copies free of conflicts.  Returns false when max_rounds ran out.
+constexpr int RES_WIDE_SMALL = 8192;  // states
+constexpr int RES_WIDE_MIN = 6;
+constexpr int RES_WIDE_SMEM = 8;   // arcs stay in shared memory when this many rows fit beside them
+
+__host__ __device__ inline int32_t res_wide_words(int32_t R) { return R < 32 ? R : R + 4; }
+__host__ __device__ inline int64_t res_wide_bytes(int32_t n, int32_t R) { return (int64_t)n * res_wide_words(R) * 4; }
+
+template <ResArcs SRC>
+__device__ bool res_wide(const ResInst &a, const ResGraph<SRC> &g, int32_t R, int32_t nr, const uint16_t *xs, int32_t d,
+                         int32_t &rounds)
+{
+    using G = ResGraph<SRC>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int32_t n = a.n, slices = (n + 31) >> 5, scale = res_wide_words(R), stride = scale * 4, max_rounds = a.max_rounds;
+    const uint32_t inv = a.inv_slices;
+    const int64_t ld = a.ld;
+    int32_t *table = a.table;
+    // a warp moves four rows of one slice
+    auto each = [&](auto f) {
+#pragma unroll 2
+        for (int32_t i = warp; i < R / 4 * slices; i += RES_WARPS) {
+            const int32_t q = res_div(inv, i, slices), v = (i - q * slices) * 32 + lane;
+            if (v < n) f(4 * q, v, res_at<int4>(d + v * stride + 16 * q));
+        }
+    };
+    each([&](int32_t r, int32_t v, int4 &x) {
+        x.x = r < nr ? __ldcg(table + xs[r] * ld + v) : INF;
+        x.y = r + 1 < nr ? __ldcg(table + xs[r + 1] * ld + v) : INF;
+        x.z = r + 2 < nr ? __ldcg(table + xs[r + 2] * ld + v) : INF;
+        x.w = r + 3 < nr ? __ldcg(table + xs[r + 3] * ld + v) : INF;
+    });
+    __syncthreads();
+    const int lpv = R / 4, vpw = 32 / lpv;  // lanes of a vertex, vertices of a warp
+    const int32_t mine = d + (lane & (lpv - 1)) * 16, sub = lane / lpv;
+    bool changed;
+    rounds = 0;
+    do {
+        if (++rounds > max_rounds) return false;
+        changed = false;
+        for (int32_t v0 = warp * vpw; v0 < n; v0 += RES_WARPS * vpw) {
+            const int32_t v = v0 + sub, sl = v0 >> 5;
+            if (v >= n) continue;
+            int4 &own = res_at<int4>(mine + v * stride);
+            const int4 old = own;
+            int4 x = old;
+            int32_t e = res_i32(g.slice + 4 * sl);
+            const int32_t width = res_i32(g.slice + 4 * sl + 4) - e;
+            e = e * 32 + (v & 31);
+#pragma unroll 2
+            for (int32_t j = 0; j < width; j++) {
+                int32_t off[2], w[2];
+                G::unpack(g.elem(e + 32 * j), off, w);
+                const int4 p = res_at<int4>(mine + off[0] * scale), q = res_at<int4>(mine + off[1] * scale);
+                x = vaddmin(p, w[0], x);  // off counts 4 bytes a vertex, a record has 4 * scale
+                x = vaddmin(q, w[1], x);
+            }
+            if (vlt(x, old)) {
+                own = x;
+                changed = true;
+            }
+        }
+    } while (__syncthreads_or(changed));
+    each([&](int32_t r, int32_t v, int4 &x) {
+        if (r < nr) table[xs[r] * ld + v] = x.x;
+        if (r + 1 < nr) table[xs[r + 1] * ld + v] = x.y;
+        if (r + 2 < nr) table[xs[r + 2] * ld + v] = x.z;
+        if (r + 3 < nr) table[xs[r + 3] * ld + v] = x.w;
+    });
+    return true;
+}
+
+// Records of the next closure of a share with `left` rows: R rows vertex by
+// vertex (R <= cap), or 0 for res_close.
+__device__ __forceinline__ int32_t res_wide_rows(int32_t n, int32_t left, int32_t cap)
+{
+    if (cap < 8 || left < RES_WIDE_MIN) return 0;
+    int32_t R = 8;
+    while (R < cap && left > R) R *= 2;
+    // a quarter of the rows may be idle, more where latency outweighs the work
+    if (R > 8 && left * 4 < R * 3 && n * R > RES_WIDE_SMALL) R /= 2;
+    return R;
+}
+
 // Relaxation of this CTA's rows of level m, at most `rows` at a time, from
 // byte offset dyn of the shared memory.
 template <ResArcs SRC>
-__device__ void res_relax(const ResArgs &a, const ResGraph<SRC> &g, const ResSmem &sm, bool has_hubs, int32_t m,
-                          int32_t dyn, int32_t rows, const int32_t *terms, int32_t *hub_cnt, int *s_ok)
+__device__ void res_relax(const ResInst &a, const ResTeam &tm, const ResGraph<SRC> &g, const ResSmem &sm, ResShared &sh,
+                          bool has_hubs, int32_t m, int32_t dyn, int32_t rows, int32_t wide_cap)
 {
-    const int32_t n = a.n, slices = (n + 31) >> 5, np = slices * 32, cnt = a.xs_off[m + 1] - a.xs_off[m];
-    const int32_t rb = (int32_t)((int64_t)cnt * blockIdx.x / gridDim.x),
-                  re = (int32_t)((int64_t)cnt * (blockIdx.x + 1) / gridDim.x);
+    const int32_t *terms = sh.terms;
+    const int32_t n = a.n, slices = (n + 31) >> 5, np = slices * 32, cnt = sh.lvl[m + 1] - sh.lvl[m];
+    const int32_t rb = (int32_t)((int64_t)cnt * tm.rank / tm.size),
+                  re = (int32_t)((int64_t)cnt * (tm.rank + 1) / tm.size);
     const uint32_t C = (1u << (a.k - 1)) - 1;
     uint32_t rounds = 0;
-    for (int32_t r0 = rb; r0 < re; r0 += rows) {
-        const int32_t R = min(rows, re - r0), words = R * slices;
-        const uint16_t *xs = &res_at<uint16_t>(sm.xs) + a.xs_off[m] + r0;
+    for (int32_t r0 = rb, R; r0 < re; r0 += R) {
+        const uint16_t *xs = &res_at<uint16_t>(sm.xs) + sh.lvl[m] + r0;
+        const int32_t wide = m > 1 ? res_wide_rows(n, re - r0, wide_cap) : 0;
+        if (wide) {
+            R = min(wide, re - r0);
+            int32_t did = 0;
+            const bool ok = res_wide<SRC>(a, g, wide, R, xs, dyn, did);
+            rounds += did;
+            if (!ok) {
+                if (threadIdx.x == 0) res_fail(tm, EMV_DEV_SWEEP_LIMIT, sh);
+                __syncthreads();
+                break;
+            }
+            if (m == a.k - 1)
+                for (int32_t r = threadIdx.x; r < R; r += RES_THREADS)
+                    if (xs[r] == C) {
+                        const int32_t x = res_i32(dyn + (terms[a.k - 1] * res_wide_words(wide) + r) * 4);
+                        *a.cost = x < INF ? (int64_t)x : INT64_MAX;
+                    }
+            __syncthreads();
+            continue;
+        }
+        R = min(rows, re - r0);
+        const int32_t words = R * slices;
         int32_t *d = &res_at<int32_t>(dyn);
         uint32_t *bm = &res_at<uint32_t>(dyn + words * 128);
         // four states of a row at a time
         auto quads = [&](auto f) {
 #pragma unroll 2
             for (int32_t i = threadIdx.x; i < words * 8; i += RES_THREADS) {
-                const int32_t r = R == 1 ? 0 : res_div(a, i >> 3, slices);
+                const int32_t r = R == 1 ? 0 : res_div(a.inv_slices, i >> 3, slices);
                 const int32_t v = i * 4 - r * np;
                 f(i, v, a.table + (int64_t)xs[r] * a.ld + v);
             }
@@ -581,9 +744,9 @@ __device__ void res_relax(const ResArgs &a, const ResGraph<SRC> &g, const ResSme
             __syncthreads();
         }
         int32_t did = 0;
-        const bool ok = res_close<SRC>(a, g, has_hubs, R, m == 1, dyn, dyn + words * 132, dyn + words * 128, hub_cnt, did);
+        const bool ok = res_close<SRC>(a, g, has_hubs, R, m == 1, dyn, dyn + words * 132, dyn + words * 128, sh.hubs, did);
         rounds += did;
-        if (!ok && threadIdx.x == 0) res_fail(a.out, EMV_DEV_SWEEP_LIMIT, s_ok);
+        if (!ok && threadIdx.x == 0) res_fail(tm, EMV_DEV_SWEEP_LIMIT, sh);
         bool unreached = false;
         quads([&](int32_t i, int32_t v, int32_t *dst) {
             const int4 x = reinterpret_cast<const int4 *>(d)[i];
@@ -600,25 +763,28 @@ __device__ void res_relax(const ResArgs &a, const ResGraph<SRC> &g, const ResSme
                     unreached |= y[q] >= INF;
                 }
         });
-        if (m == 1 && unreached) a.out->unreached = 1;
+        if (m == 1 && unreached && a.unreached) *a.unreached = 1;
         if (m == a.k - 1)
             for (int32_t r = threadIdx.x; r < R; r += RES_THREADS)
-                if (xs[r] == C) a.out->cost = d[r * np + terms[a.k - 1]];
+                if (xs[r] == C) {
+                    const int32_t x = d[r * np + terms[a.k - 1]];
+                    *a.cost = x < INF ? (int64_t)x : INT64_MAX;
+                }
         __syncthreads();
         if (!ok) break;
     }
-    if (threadIdx.x == 0 && rounds) atomicAdd(&a.out->rounds, rounds);
+    if (threadIdx.x == 0 && rounds && a.rounds) atomicAdd(a.rounds, rounds);
 }
 
-// Levels 1..kt.  Arcs that the closures keep in shared memory are copied there
+// Levels lo..hi.  Arcs that the closures keep in shared memory are copied there
 // again for every level as far as the merge's staging overlaps them, between
 // the merge and the barrier after it.
 template <ResArcs SRC>
-__device__ void res_levels(const ResArgs &a, const ResSmem &sm, bool has_hubs, const int32_t *terms, int32_t *hub_cnt,
-                           uint32_t &epoch, int *s_ok)
+__device__ void res_levels(const ResInst &a, ResTeam &tm, const ResSmem &sm, ResShared &sh, bool has_hubs, int32_t lo,
+                           int32_t hi)
 {
     using T = typename ResElem<SRC>::T;
-    const bool clock = blockIdx.x == 0 && threadIdx.x == 0;
+    const bool clock = a.ns && tm.rank == 0 && threadIdx.x == 0;
     unsigned long long t0 = clock ? res_now() : 0;
     const int32_t slices = (a.n + 31) >> 5;
     const int32_t arc_bytes = SRC == ARCS_SMEM ? res_i32(sm.slice + 4 * slices) * 32 * (int32_t)sizeof(T) : 0;
@@ -629,27 +795,26 @@ __device__ void res_levels(const ResArgs &a, const ResSmem &sm, bool has_hubs, c
     // rows of a closure: what fits, and their states must fit 16 bits
     const int32_t rows = (int32_t)min(min((int64_t)a.want_rows, (int64_t)(65535 / (32 * slices))),
                                       (sm.end - dyn) / res_state_bytes(a.n, 1));
-    auto load_arcs = [&](int32_t from) {
-        for (int32_t i = from + threadIdx.x * 16; i < arc_bytes; i += RES_THREADS * 16)
+    int32_t wide_cap = has_hubs ? 0 : 128;
+    while (wide_cap >= 8 && (wide_cap > 2 * a.want_rows || res_wide_bytes(a.n, wide_cap) > sm.end - dyn)) wide_cap /= 2;
+    for (int32_t m = lo; m <= hi; m++) {
+        if (m > 1) res_merge(a, tm, sm, sh, m);
+        for (int32_t i = (m == lo ? 0 : keep) + threadIdx.x * 16; i < arc_bytes; i += RES_THREADS * 16)
             cp_async16(&res_at<int4>(sm.big + i), (const char *)a.slices + i);
-    };
-    for (int32_t m = 1; m <= a.kt; m++) {
-        if (m > 1) res_merge(a, sm, m, terms);
-        load_arcs(m > 1 ? keep : 0);
         if (m > 1) {
-            if (!res_barrier(a.out, epoch, s_ok)) break;
+            if (!res_barrier(tm, sh)) break;
             if (clock) {
                 const unsigned long long t = res_now();
-                a.out->ns[1] += t - t0;
+                a.ns[1] += t - t0;
                 t0 = t;
             }
         }
         cp_async_wait_all();  // made visible to the CTA by the barrier before the closure
-        res_relax<SRC>(a, g, sm, has_hubs, m, dyn, rows, terms, hub_cnt, s_ok);
-        if (m < a.kt && !res_barrier(a.out, epoch, s_ok)) break;
+        res_relax<SRC>(a, tm, g, sm, sh, has_hubs, m, dyn, rows, wide_cap);
+        if (m < hi && !res_barrier(tm, sh)) break;
         if (clock) {
             const unsigned long long t = res_now();
-            a.out->ns[m == 1 ? 0 : 2] += t - t0;
+            a.ns[m == 1 ? 0 : 2] += t - t0;
             t0 = t;
         }
     }
@@ -657,9 +822,11 @@ __device__ void res_levels(const ResArgs &a, const ResSmem &sm, bool has_hubs, c
 }
 
 // Widths of the slices in arc pairs, their prefix sums (sm.slice) and the
-// pairs of every vertex; needs at most RES_THREADS slices.
-__device__ void res_slice_starts(const ResArgs &a, const ResSmem &sm, int32_t *warp_sums)
+// pairs of every vertex; needs at most RES_THREADS slices.  Returns whether a
+// vertex has more than RES_HUB arcs.
+__device__ __forceinline__ bool res_slice_starts(const ResInst &a, const ResSmem &sm, int32_t *warp_sums)
 {
+    bool hub = false;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int32_t slices = (a.n + 31) >> 5;
     int32_t *slice = &res_at<int32_t>(sm.slice);
@@ -667,6 +834,7 @@ __device__ void res_slice_starts(const ResArgs &a, const ResSmem &sm, int32_t *w
         const int32_t v = i * 32 + lane;
         const int32_t deg = v < a.n ? __ldg(a.row_ptr + v + 1) - __ldg(a.row_ptr + v) : 0;
         const int32_t np = deg > RES_HUB ? 0 : (deg + 1) / 2;
+        hub |= deg > RES_HUB;
         res_at<uint8_t>(sm.pairs + v) = deg > RES_HUB ? RES_HUB_MARK : (uint8_t)np;
         const int32_t width = __reduce_max_sync(FULL, np);
         if (lane == 0) slice[i] = width;
@@ -685,83 +853,69 @@ __device__ void res_slice_starts(const ResArgs &a, const ResSmem &sm, int32_t *w
     before = __reduce_add_sync(FULL, before);
     if (threadIdx.x <= slices) slice[threadIdx.x] = before + pre - own;
     if (slices == RES_THREADS && threadIdx.x == RES_THREADS - 1) slice[slices] = before + pre;
-    __syncthreads();
+    return __syncthreads_or(hub) != 0;
 }
 
-// Writes the sliced arcs (a warp per slice, the grid's warps sharing them).
-template <ResArcs SRC> __device__ void res_pack(const ResArgs &a, const ResSmem &sm)
+// Writes the sliced arcs (a warp per slice, the team's warps sharing them).
+template <ResArcs SRC> __device__ void res_pack(const ResInst &a, const ResTeam &tm, const ResSmem &sm)
 {
     const int lane = threadIdx.x & 31;
     const int32_t slices = (a.n + 31) >> 5;
     const int32_t *slice = &res_at<int32_t>(sm.slice);
-    for (int32_t i = blockIdx.x * RES_WARPS + (threadIdx.x >> 5); i < slices; i += gridDim.x * RES_WARPS) {
+    for (int32_t i = tm.rank * RES_WARPS + (threadIdx.x >> 5); i < slices; i += tm.size * RES_WARPS) {
         const int32_t v = i * 32 + lane, p = res_at<uint8_t>(sm.pairs + v), np = p == RES_HUB_MARK ? 0 : p, width = slice[i + 1] - slice[i];
         const int32_t beg = np ? __ldg(a.row_ptr + v) : 0, deg = np ? __ldg(a.row_ptr + v + 1) - beg : 0;
         for (int32_t j = 0; j < width; j++) {
-            int32_t h[2], w[2];
+            int2 x[2];
 #pragma unroll
             for (int q = 0; q < 2; q++) {
-                const bool ok = 2 * j + q < deg;
-                h[q] = ok ? __ldg(a.col + beg + 2 * j + q) : v;
                 // a distance of at most INF plus INF - 1 stays below 2^31
-                w[q] = ok ? __ldg(a.w + beg + 2 * j + q) : SRC == ARCS_WIDE ? INF - 1 : (int32_t)RES_MAX_W - 1;
+                x[q] = make_int2(v, SRC == ARCS_WIDE ? INF - 1 : (int32_t)RES_MAX_W - 1);
+                if (2 * j + q < deg) x[q] = __ldcg(a.adj + beg + 2 * j + q);
             }
             const size_t at = (size_t)(slice[i] + j) * 32 + lane;
             if constexpr (SRC == ARCS_WIDE)
-                reinterpret_cast<int4 *>(a.slices)[at] = make_int4(4 * h[0], w[0], 4 * h[1], w[1]);
+                reinterpret_cast<int4 *>(a.slices)[at] = make_int4(4 * x[0].x, x[0].y, 4 * x[1].x, x[1].y);
             else
                 reinterpret_cast<uint2 *>(a.slices)[at] =
-                    make_uint2((uint32_t)h[0] << 2 | (uint32_t)w[0] << 18, (uint32_t)h[1] << 2 | (uint32_t)w[1] << 18);
+                    make_uint2((uint32_t)x[0].x << 2 | (uint32_t)x[0].y << 18, (uint32_t)x[1].x << 2 | (uint32_t)x[1].y << 18);
         }
     }
 }
 
-// The whole solve: CSR check and arc slices, then levels 1..kt.
-__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(ResArgs a)
+// The parts of `smem` bytes of dynamic shared memory, and the subset list in
+// its part (xs: the first level's; lvl[kt + 1] entries).
+__device__ __forceinline__ ResSmem res_layout(int32_t n, int32_t kt, int32_t smem, const uint32_t *xs, int32_t count)
 {
-    __shared__ int s_ok;
-    __shared__ int32_t s_terms[EMV_MAX_K];
-    __shared__ int32_t s_hubs[RES_WARPS];
-    uint32_t epoch = 0;
-    const int32_t slices = (a.n + 31) >> 5;
-    const int64_t first = (int64_t)blockIdx.x * RES_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * RES_THREADS;
     ResSmem sm;
     sm.xs = 0;
-    sm.slice = ((2 << a.kt) + 15) / 16 * 16;
-    sm.pairs = sm.slice + (4 * (slices + 1) + 15) / 16 * 16;
-    sm.big = res_fixed_smem(a.n, a.kt);
-    sm.end = a.smem;
-    if (threadIdx.x == 0) s_ok = 1;  // before the barrier that first reads it
-    for (int32_t i = threadIdx.x; i < a.xs_off[a.kt + 1]; i += RES_THREADS)
-        res_at<uint16_t>(sm.xs + 2 * i) = (uint16_t)__ldg(a.xs + i);
-    if (threadIdx.x < EMV_MAX_K) s_terms[threadIdx.x] = a.terms[threadIdx.x];
-    if (blockIdx.x == 0 && threadIdx.x < a.k) a.out->terms[threadIdx.x] = a.terms[threadIdx.x];
-    scan_csr(a.row_ptr, a.n, a.col, a.w, a.adj, a.arcs, &a.out->scan);
-    bool hub = false;
-    for (int64_t v = first; v < a.n; v += stride) {
-        a.table[v] = INF;  // row 0 (R:2243-2259)
-        hub |= a.row_ptr[v + 1] - a.row_ptr[v] > RES_HUB;
-    }
-    if (hub) a.out->hubs = 1;
-    if (!res_barrier(a.out, epoch, &s_ok)) return;
-    const uint32_t bad = __ldcg(&a.out->scan.bad), maxw = __ldcg(&a.out->scan.maxw);
-    if (a.check) {  // the host reads the same words and names the fault
-        if (bad) return;
-        const long long bound =
-            min((long long)(a.n - 1) * (long long)maxw, (long long)(__ldcg(&a.out->scan.sumw) / 2));
-        if (bound >= INF) return;
-    }
-    const bool has_hubs = __ldcg(&a.out->hubs) != 0;
-    res_slice_starts(a, sm, s_hubs);
-    const int64_t arc_bytes = (int64_t)res_i32(sm.slice + 4 * slices) * 32 * sizeof(uint2);
-    const bool narrow = maxw < RES_MAX_W && !(bad & SCAN_BAD_WEIGHT);
-    const bool in_smem = narrow && arc_bytes + res_state_bytes(a.n, 1) <= sm.end - sm.big;
-    if (narrow) res_pack<ARCS_PACKED>(a, sm);
-    else res_pack<ARCS_WIDE>(a, sm);
-    if (!res_barrier(a.out, epoch, &s_ok)) return;
-    if (in_smem) res_levels<ARCS_SMEM>(a, sm, has_hubs, s_terms, s_hubs, epoch, &s_ok);
-    else if (narrow) res_levels<ARCS_PACKED>(a, sm, has_hubs, s_terms, s_hubs, epoch, &s_ok);
-    else res_levels<ARCS_WIDE>(a, sm, has_hubs, s_terms, s_hubs, epoch, &s_ok);
+    sm.slice = ((2 << kt) + 15) / 16 * 16;
+    sm.pairs = sm.slice + (4 * ((n + 31) / 32 + 1) + 15) / 16 * 16;
+    sm.big = res_fixed_smem(n, kt);
+    sm.end = smem;
+    for (int32_t i = threadIdx.x; i < count; i += RES_THREADS)
+        res_at<uint16_t>(sm.xs + 2 * i) = (uint16_t)__ldg(xs + i);
+    return sm;
+}
+
+// Slices the arcs (narrow: every weight is below RES_MAX_W) and solves levels
+// lo..hi; returns when the CTA's part is done or the team failed.
+__device__ __forceinline__ void res_solve(const ResInst &a, ResTeam &tm, const ResSmem &sm, ResShared &sh, bool narrow,
+                                          int32_t lo, int32_t hi)
+{
+    const bool has_hubs = res_slice_starts(a, sm, sh.hubs);
+    const int64_t arc_bytes = (int64_t)res_i32(sm.slice + 4 * ((a.n + 31) >> 5)) * 32 * sizeof(uint2);
+    // arcs in shared memory, unless they would keep records of RES_WIDE_SMEM rows out of it
+    int64_t states = res_state_bytes(a.n, 1);
+    if (a.want_rows * 4 >= RES_WIDE_SMEM * 3 && !has_hubs && res_wide_bytes(a.n, RES_WIDE_SMEM) <= sm.end - sm.big)
+        states = max(states, res_wide_bytes(a.n, RES_WIDE_SMEM));
+    const bool in_smem = narrow && arc_bytes + states <= sm.end - sm.big;
+    if (narrow) res_pack<ARCS_PACKED>(a, tm, sm);
+    else res_pack<ARCS_WIDE>(a, tm, sm);
+    if (!res_barrier(tm, sh)) return;
+    if (in_smem) res_levels<ARCS_SMEM>(a, tm, sm, sh, has_hubs, lo, hi);
+    else if (narrow) res_levels<ARCS_PACKED>(a, tm, sm, sh, has_hubs, lo, hi);
+    else res_levels<ARCS_WIDE>(a, tm, sm, sh, has_hubs, lo, hi);
 }
 
 }  // namespace emv

@@ -12,7 +12,16 @@ struct ResidentPlan {
     int32_t mw;              // vertices of a merge block
 };
 
-bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, ResidentPlan &p);
+// Rows of the widest level of kt terminals' subsets.
+int64_t resident_max_rows(int32_t kt);
+// Whether the device functions of emv_resident.cuh can take the instance.
+bool resident_fits(int32_t n, int32_t kt);
+// Vertices of a merge block when `ctas` CTAs share the instance: as few waves
+// of blocks as the shared memory allows, and within them the narrowest blocks,
+// so that every CTA has some; cap > 0 bounds it.
+int32_t resident_merge_width(int32_t n, int32_t kt, int32_t ctas, int32_t cap);
+uint32_t res_inv_slices(int32_t n);
+bool resident_plan(const emv_ctx *c, int32_t n, int32_t kt, ResidentPlan &p);
 // The whole DP over the first kt of the k terminals, CSR check included;
 // fills the table's 2^kt rows (stride ld) and c->adj.
 int run_resident(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, const int32_t *row_ptr, const int32_t *col,

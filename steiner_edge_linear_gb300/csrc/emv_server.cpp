@@ -8,7 +8,7 @@
 // requests that arrive while others are on the GPU join at the next wave and
 // levels of different requests interleave.  Tables stay resident in HBM
 // across levels (stream-ordered allocations).  Requests too large for one
-// CTA (n above large_n, or k above the batched range) go to a second worker
+// team of CTAs (n above large_n, or k above the batched range) go to a second worker
 // that runs the multi-CTA solver on its own stream, concurrently with the
 // waves.  A wave block takes a whole SM, and a relaxation grid must be
 // resident at once, so while a large request runs with small ones resident
@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "emv_batch_host.h"
+#include "emv_resident.h"
 #include "emv_solver.h"
 
 using namespace emv;
@@ -51,6 +52,8 @@ struct Req {
     int state = Q_QUEUED;
     bool cancel = false;
     int32_t next_level = 1;
+    bool narrow = false;      // BatchGraph of the request
+    int64_t arc_bytes = 0;
     int32_t slot = -1;
     int64_t cost = 0;
     int status = EMV_OK;
@@ -87,12 +90,14 @@ struct emv_server {
     cudaStream_t st_small = nullptr, st_large = nullptr;
     // wave buffers
     std::vector<int32_t> free_slots;
-    DevBuf d_desc, d_costs, d_ctrl;
+    DevBuf d_desc, d_costs, d_ctrl, d_arcs;
     BatchInst *h_desc = nullptr;
     int64_t *h_costs = nullptr;
     int32_t cap_slots = 0;
     int32_t wave_sms = 0;                  // SMs the waves keep while a large request runs (0: no split)
     std::atomic<bool> large_sharing{false};  // a large solve runs on the other SMs
+    bool large_running = false;            // a large solve runs (mu)
+    bool wave_alone = false;               // a wave runs whose teams need the GPU to themselves (mu)
 };
 
 namespace {
@@ -128,7 +133,7 @@ int stage_small(emv_server *s, Req *r, std::vector<int2> &adj)
     if (cudaMallocAsync((void **)&r->d_row, sizeof(int32_t) * ((size_t)r->n + 1), st) != cudaSuccess ||
         cudaMallocAsync((void **)&r->d_adj, sizeof(int2) * arcs, st) != cudaSuccess ||
         cudaMallocAsync((void **)&r->d_terms, sizeof(int32_t) * (size_t)r->k, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&r->d_table, sizeof(int32_t) * ((size_t)r->n << table_terminals(r->k)), st) != cudaSuccess) {
+        cudaMallocAsync((void **)&r->d_table, sizeof(int32_t) * ((size_t)batch_ld(r->n) << table_terminals(r->k)), st) != cudaSuccess) {
         cudaGetLastError();
         return emv_fail(EMV_ERR_OOM, "server: device allocation for request %lld", (long long)r->id);
     }
@@ -205,8 +210,35 @@ void scheduler(emv_server *s)
             for (Req *r : s->resident) wave.push_back(r);
         }
         if (wave.empty()) continue;
+        // Beside a large solve the wave stays on its share of the SMs, with teams
+        // of one CTA; larger teams wait for their CTAs, as a relaxation grid does,
+        // so the large worker does not start while such a wave runs, and no such
+        // wave starts while a large request waits.
+        bool alone;
+        {
+            std::lock_guard<std::mutex> lk(s->mu);
+            alone = !s->large_running && s->queue_large.empty();
+            s->wave_alone = alone;
+        }
+        const int32_t cap = s->large_sharing.load() ? s->wave_sms : 0;
+        const int32_t most = batch_blocks(s->ctx_small, INT32_MAX, cap);
+        std::vector<double> work(wave.size());
+        std::vector<int64_t> states(wave.size());
         for (size_t j = 0; j < wave.size(); j++) {
-            Req *r = wave[j];
+            const Req *r = wave[j];
+            const int32_t kt = table_terminals(r->k), m = r->next_level;
+            work[j] = batch_work(r->n, kt, r->arcs, m, m);
+            int64_t rows = 1;
+            for (int32_t i = 1; i <= m; i++) rows = rows * (kt - i + 1) / i;
+            states[j] = rows * r->n;
+        }
+        std::vector<int32_t> order, size;
+        batch_plan(work, states, most, alone ? 1 << (BATCH_SIZES - 1) : 1, order, size);
+        BatchArgs a;
+        std::memset(&a, 0, sizeof(a));
+        int64_t ctas = 0, arc_bytes = 0;
+        for (size_t j = 0; j < wave.size(); j++) {
+            const Req *r = wave[(size_t)order[j]];
             BatchInst &d = s->h_desc[j];
             std::memset(&d, 0, sizeof(d));
             d.row_ptr = r->d_row;
@@ -216,40 +248,44 @@ void scheduler(emv_server *s)
             d.n = r->n;
             d.k = r->k;
             d.kt = table_terminals(r->k);
-            d.rcap = batch_rcap_for(s->ctx_small, r->n, r->k);
-            d.mw = batch_mw_for(s->ctx_small, r->n, r->k, d.kt);
+            d.size = size[(size_t)order[j]];
+            batch_shape(s->ctx_small, d);
+            d.narrow = r->narrow;
             d.orig = r->slot;
             d.lo = d.hi = r->next_level;
+            for (int32_t cl = 0; cl < BATCH_SIZES; cl++)
+                if (d.size >= 1 << (BATCH_SIZES - 1 - cl)) a.end[cl] = (int32_t)j + 1;
+            ctas += d.size;
+            arc_bytes = std::max(arc_bytes, r->arc_bytes);
         }
-        int st = EMV_OK;
-        BatchArgs a;
-        std::memset(&a, 0, sizeof(a));
+        const int32_t blocks = batch_blocks(s->ctx_small, ctas, cap);
         a.inst = (const BatchInst *)s->d_desc.ptr;
-        a.count = (int32_t)wave.size();
         a.xs = (const uint32_t *)s->ctx_small->bxs.ptr;
         a.xs_off = (const int32_t *)s->ctx_small->bxs_off.ptr;
         a.costs = (int64_t *)s->d_costs.ptr;
-        a.queue = (uint32_t *)s->d_ctrl.ptr;
-        a.err = (uint32_t *)s->d_ctrl.ptr + 8;
+        a.ctl = (uint32_t *)s->d_ctrl.ptr;
+        a.smem = RESIDENT_SMEM;
+        a.scratch_stride = batch_arc_stride(arc_bytes);
+        // grows when a request brings longer arc slices than any before
+        int st = dev_reserve(s->d_arcs, (size_t)a.scratch_stride * (size_t)batch_blocks(s->ctx_small, INT32_MAX, 0));
+        a.scratch = (char *)s->d_arcs.ptr;
         uint32_t err = 0;
-        if (cudaMemcpyAsync(s->d_desc.ptr, s->h_desc, sizeof(BatchInst) * wave.size(), cudaMemcpyHostToDevice,
+        if (!st && cudaMemcpyAsync(s->d_desc.ptr, s->h_desc, sizeof(BatchInst) * wave.size(), cudaMemcpyHostToDevice,
                             s->st_small) != cudaSuccess)
             st = emv_fail(EMV_ERR_CUDA, "server: descriptor upload");
-        // beside a large solve the wave stays on its share of the SMs
-        const int32_t wave_blocks = s->large_sharing.load() ? s->wave_sms : 0;
-        if (!st) st = launch_batch(s->ctx_small, a, a.count, s->st_small, wave_blocks);
+        if (!st) st = launch_batch(s->ctx_small, a, blocks, s->st_small);
         if (!st && cudaMemcpyAsync(s->h_costs, s->d_costs.ptr, sizeof(int64_t) * (size_t)s->cap_slots,
                                    cudaMemcpyDeviceToHost, s->st_small) != cudaSuccess)
             st = emv_fail(EMV_ERR_CUDA, "server: cost read");
-        if (!st && cudaMemcpyAsync(&err, a.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->st_small) != cudaSuccess)
+        if (!st && cudaMemcpyAsync(&err, a.ctl, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->st_small) != cudaSuccess)
             st = emv_fail(EMV_ERR_CUDA, "server: status read");
         if (!st && cudaStreamSynchronize(s->st_small) != cudaSuccess) {
             cudaGetLastError();
             st = emv_fail(EMV_ERR_CUDA, "server: wave failed");
         }
         if (!st && err) st = emv_dev_status_to_emv(err);
-        if (!st) cudaMemsetAsync(a.err, 0, sizeof(uint32_t), s->st_small);
         std::lock_guard<std::mutex> lk(s->mu);
+        s->wave_alone = false;
         s->stats.waves++;
         for (Req *r : wave) {
             bool done = false;
@@ -274,6 +310,7 @@ void scheduler(emv_server *s)
             }
         }
         s->cv_done.notify_all();
+        s->cv_work.notify_all();
     }
 }
 
@@ -286,12 +323,16 @@ void large_loop(emv_server *s)
             std::unique_lock<std::mutex> lk(s->mu);
             s->cv_work.wait(lk, [&] {
                 if (s->stop) return true;
-                if (s->queue_large.empty()) return false;
+                if (s->queue_large.empty() || s->wave_alone) return false;
                 return s->resident_bytes + s->queue_large.front()->bytes <= s->opts.hbm_budget_bytes ||
                        s->resident_count == 0;
             });
             if (s->stop && s->queue_large.empty()) return;
             if (s->queue_large.empty()) continue;
+            if (s->wave_alone) {  // stopping: the requests left are cancelled
+                s->cv_work.wait(lk, [&] { return !s->wave_alone; });
+                continue;
+            }
             r = s->queue_large.front();
             s->queue_large.pop_front();
             if (r->cancel) {
@@ -308,6 +349,7 @@ void large_loop(emv_server *s)
             const bool share = s->wave_sms > 0 && (!s->resident.empty() || !s->queue_small.empty());
             s->ctx_large->relax_sm_cap = share ? s->ctx_large->sms - s->wave_sms : 0;
             s->large_sharing = share;
+            s->large_running = true;
         }
         emv_graph g{r->n, r->arcs, r->row.data(), r->col.data(), r->w.data()};
         emv_result res;
@@ -315,6 +357,7 @@ void large_loop(emv_server *s)
         int st = emv_solve(s->ctx_large, &g, r->terms.data(), r->k, EMV_SOLVE_NOCHECK, &res, s->st_large);
         s->large_sharing = false;
         std::lock_guard<std::mutex> lk(s->mu);
+        s->large_running = false;
         s->resident_bytes -= r->bytes;
         s->resident_count--;
         finish(s, r, st, res.cost);
@@ -330,6 +373,7 @@ void server_free(emv_server *s)
     dev_release(s->d_desc);
     dev_release(s->d_costs);
     dev_release(s->d_ctrl);
+    dev_release(s->d_arcs);
     if (s->h_desc) cudaFreeHost(s->h_desc);
     if (s->h_costs) cudaFreeHost(s->h_costs);
     if (s->st_small) cudaStreamDestroy(s->st_small);
@@ -381,10 +425,11 @@ extern "C" int emv_server_create(emv_server **out, const emv_server_opts *opts)
     }
     st = dev_reserve(s->d_desc, sizeof(BatchInst) * (size_t)s->cap_slots);
     if (!st) st = dev_reserve(s->d_costs, sizeof(int64_t) * (size_t)s->cap_slots);
-    if (!st) st = dev_reserve(s->d_ctrl, 64);
     if (!st) st = prepare_batch_subsets(s->ctx_small, s->st_small);
     if (!st) st = batch_kernel_setup(s->ctx_small);
-    if (!st && cudaMemsetAsync(s->d_ctrl.ptr, 0, 64, s->st_small) != cudaSuccess) st = EMV_ERR_CUDA;
+    if (!st) st = dev_reserve(s->d_ctrl, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(s->ctx_small->batch_blocks));
+    // arc slices of up to 4096 vertices and 32 arcs each; longer ones grow it
+    if (!st) st = dev_reserve(s->d_arcs, (size_t)(4096 * 32 * 4) * (size_t)s->ctx_small->batch_blocks);
     // keep freed pool memory cached in the process (no release at stream syncs)
     cudaMemPool_t pool;
     if (!st && cudaDeviceGetDefaultMemPool(&pool, opts->device) == cudaSuccess) {
@@ -432,6 +477,11 @@ extern "C" int emv_server_submit(emv_server *s, const emv_graph *g, const int32_
     r->terms.assign(terminals, terminals + k);
     r->bytes = bytes;
     r->large = g->n >= s->opts.large_n || !batch_fits(g->n, k);
+    if (!r->large) {
+        const BatchGraph bg = batch_graph(g->row_ptr, g->w, g->n, g->arcs);
+        r->narrow = bg.narrow;
+        r->arc_bytes = bg.arc_bytes;
+    }
     r->t_submit = Clock::now();
     {
         std::lock_guard<std::mutex> lk(s->mu);

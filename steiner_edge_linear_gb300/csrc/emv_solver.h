@@ -85,11 +85,12 @@ struct emv_ctx {
     DevBuf bxs, bxs_off;           // subset lists of every k <= BATCH_KMAX
     bool bxs_ready = false;
     int batch_blocks = 0;
-    DevBuf b_row, b_adj, b_term, b_desc, b_table, b_costs, b_ctrl;
+    DevBuf b_row, b_adj, b_term, b_desc, b_table, b_costs, b_ctrl, b_arcs;
     void *bstage = nullptr;        // pinned staging of the packed batch
     size_t bstage_bytes = 0;
     cudaGraphExec_t bgraph_exec = nullptr;
     char bgraph_args[160] = {};    // BatchArgs of the captured graph
+    int32_t bgraph_blocks = 0;     // and its CTAs
     int32_t tune_rcap[BATCH_CLASSES] = {};
     int32_t tune_mw[BATCH_CLASSES] = {};  // merge vertex-block width per class (0: default 1)
 };

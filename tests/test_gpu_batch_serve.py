@@ -191,3 +191,24 @@ def test_autotune_first_on_fresh_context(emv):
         ref = [s.solve(g).cost for g in graphs[::25]]
     assert table.max() > 0
     assert list(costs[::25]) == ref
+
+
+@pytest.mark.parametrize("count", [1, 2, 7, 40])
+def test_batch_teams_whole_tables(emv, orc, count):
+    """Few instances are solved by teams of up to 128 CTAs, many by one CTA
+    each: whole tables against the oracle for a mix of sizes, an odd vertex
+    count, hubs and weights past the packed arcs."""
+    insts = [emv.StpInstance.regular(3001, 6, 1, 1000, 9, 1), emv.StpInstance.regular(70, 4, 1, 9, 1, 2),
+             emv.StpInstance.regular(1024, 4, 1, 20000, 7, 3), emv.StpInstance.clique(150, 1, 90, 6, 4),
+             emv.StpInstance.powlaw(900, 8, -0.5, 8, 1, 100, 8, 5), emv.StpInstance.regular(64, 3, 1, 9, 2, 6),
+             emv.StpInstance.regular(2000, 4, 1, 100, 10, 7)]
+    insts += [emv.StpInstance.mixed(99, i) for i in range(33)]
+    graphs = [emv.Csr.from_stp(i) for i in insts[:count]]
+    with emv.Solver(0) as s:
+        costs, _, tables = s.batch_solve(graphs, tables=True)
+        only, _ = s.batch_solve(graphs)
+    assert np.array_equal(costs, only)
+    for g, c, t in zip(graphs, costs, tables):
+        want, cost = orc.emv_table(g.n, g.row_ptr, g.col, g.w, g.terminals, threads=8)
+        assert np.array_equal(t, want)
+        assert c == (cost if g.k > 1 else (1 << 63) - 1)
