@@ -68,6 +68,10 @@ static const void *const relax_fns[RELAX_VARIANTS] = {
     (const void *)k_relax<2, true>, (const void *)k_relax<4, true>, (const void *)k_relax<5, true>,
     (const void *)k_relax<8, true>};
 
+// Level-1 kernels by record width (4, 8, 16 or 32 rows).
+static const void *const level1_fns[LEVEL1_VARIANTS] = {(const void *)k_level1<1>, (const void *)k_level1<2>,
+                                                        (const void *)k_level1<4>, (const void *)k_level1<8>};
+
 extern "C" int emv_create(emv_ctx **out, int32_t device)
 {
     if (!out) return emv_fail(EMV_ERR_BAD_INPUT, "null ctx pointer");
@@ -88,6 +92,11 @@ extern "C" int emv_create(emv_ctx **out, int32_t device)
         int per_sm = 0;
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, relax_fns[i], RELAX_THREADS, 0));
         c->relax_blocks_max[i] = std::max(1, per_sm) * c->sms;
+    }
+    for (int i = 0; i < LEVEL1_VARIANTS; i++) {
+        int per_sm = 0;
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, level1_fns[i], NARROW_THREADS, 0));
+        c->level1_blocks_max[i] = std::max(1, per_sm) * c->sms;
     }
     int st = dev_reserve(c->ctrl, sizeof(uint32_t) * C_WORDS);
     if (!st) st = dev_reserve(c->stat, sizeof(DevStat));
@@ -144,6 +153,7 @@ extern "C" int emv_destroy(emv_ctx *c)
         if (c->evmax[i]) cudaEventDestroy(c->evmax[i]);
     if (c->bgraph_exec) cudaGraphExecDestroy(c->bgraph_exec);
     if (c->bstage) cudaFreeHost(c->bstage);
+    if (c->h_dist) cudaFreeHost(c->h_dist);
     if (c->pinned) cudaFreeHost(c->pinned);
     delete c;
     return EMV_OK;
@@ -157,14 +167,18 @@ static int grid_for(int64_t work, int threads, int cap)
     return (int)std::max<int64_t>(1, std::min<int64_t>(g, cap));
 }
 
+static int32_t max_sweeps(const emv_ctx *c, int32_t n)
+{
+    return (c->sweep_limit > 0 && c->sweep_limit < (int64_t)n + 1) ? (int32_t)c->sweep_limit : n + 1;
+}
+
 // Launches the relaxation of one chunk of at most CHUNK_ROWS rows (2 *
 // CHUNK_ROWS with 16-bit records, which the caller takes only for rows whose
 // values are all at most 32767) as one cooperative, persistent kernel; the
-// record width follows the row count.  vmax (or null) receives the largest
-// value written.
+// record width follows the row count.
 int launch_relax(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n, int64_t ld, int32_t *table,
-                 const uint32_t *rows, int32_t nrows, const int32_t *terms, int32_t level1, cudaStream_t st,
-                 bool u16 = false, uint32_t *vmax = nullptr, uint16_t *shadow = nullptr, int64_t shadow_ld = 0)
+                 const uint32_t *rows, int32_t nrows, cudaStream_t st, bool u16 = false, uint16_t *shadow = nullptr,
+                 int64_t shadow_ld = 0)
 {
     RelaxArgs a;
     a.stamp = (int32_t *)c->stamp.ptr;
@@ -175,20 +189,17 @@ int launch_relax(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n,
     a.table = table;
     a.rows = rows;
     a.nrows = nrows;
-    a.terms = terms;
-    a.level1 = level1;
     a.scratch = (int32_t *)c->scratch.ptr;
     a.act0 = (uint8_t *)c->act.ptr;
     a.act1 = (uint8_t *)c->act.ptr + ((size_t)n + 255) / 256 * 256;
     a.ctrl = (uint32_t *)c->ctrl.ptr;
     a.stat = (DevStat *)c->stat.ptr;
-    a.max_sweeps = (c->sweep_limit > 0 && c->sweep_limit < (int64_t)n + 1) ? (int32_t)c->sweep_limit : n + 1;
+    a.max_sweeps = max_sweeps(c, n);
     // Dense sweeps pay off while almost every vertex has a changed neighbour:
     // with mean degree d and a fraction f of vertices changed, a vertex has none
     // with probability (1 - f)^d; take every vertex while that is below 10 %.
     const double deg = (double)c->relax_arcs / (double)n;
     a.dense_min = deg > 0 ? (int32_t)std::min<double>((double)n, (double)n * (1.0 - std::pow(0.1, 1.0 / deg))) : n;
-    a.vmax = vmax;
     a.shadow = shadow;
     a.shadow_ld = shadow_ld;
     const int32_t words = u16 ? (nrows + 1) / 2 : nrows;  // int32 words a vertex record needs
@@ -210,6 +221,45 @@ int launch_relax(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n,
     void *args[] = {&a};
     CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(RELAX_THREADS), args, 0, st));
     c->launches += 1;  // the kernel (the control-word memset is not a kernel)
+    return EMV_OK;
+}
+
+// Launches the single-source closures of rows[r] from terms[r] (device arrays,
+// at most 32) as one cooperative kernel; vmax (or null) receives the largest
+// value written.
+int launch_level1(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n, int64_t ld, int32_t *table,
+                  const uint32_t *rows, int32_t nrows, const int32_t *terms, cudaStream_t st, uint32_t *vmax = nullptr,
+                  uint16_t *shadow = nullptr, int64_t shadow_ld = 0, const GraphScan *scan = nullptr)
+{
+    const int vi = nrows <= 4 ? 0 : nrows <= 8 ? 1 : nrows <= 16 ? 2 : 3;
+    Level1Args a;
+    a.na.row_ptr = row_ptr;
+    a.na.n = n;
+    a.na.rec = (int4 *)c->scratch.ptr;
+    a.na.act0 = (uint8_t *)c->act.ptr;
+    a.na.act1 = (uint8_t *)c->act.ptr + ((size_t)n + 255) / 256 * 256;
+    a.na.ctrl = (uint32_t *)c->ctrl.ptr;
+    a.na.max_sweeps = max_sweeps(c, n);
+    a.na.dense_min = narrow_dense_min(n, c->relax_arcs);
+    a.adj = adj;
+    a.terms = terms;
+    a.rows = rows;
+    a.nrows = nrows;
+    a.table = table;
+    a.ld = ld;
+    a.vmax = vmax;
+    a.shadow = shadow;
+    a.shadow_ld = shadow_ld;
+    a.stat = (DevStat *)c->stat.ptr;
+    a.scan = scan;
+    const int vpb = narrow_vertices(1 << vi) * (NARROW_THREADS / 32);  // one group of vertices a warp
+    int bmax = c->level1_blocks_max[vi];
+    if (c->relax_sm_cap > 0 && c->relax_sm_cap < c->sms) bmax = std::max(1, bmax / c->sms * c->relax_sm_cap);
+    const int blocks = std::min(bmax, std::max(1, (n + vpb - 1) / vpb));
+    CUDA_TRY(cudaMemsetAsync(a.na.ctrl, 0, sizeof(uint32_t) * C_WORDS, st));
+    void *args[] = {&a};
+    CUDA_TRY(cudaLaunchCooperativeKernel(level1_fns[vi], dim3(blocks), dim3(NARROW_THREADS), args, 0, st));
+    c->launches += 1;
     return EMV_OK;
 }
 
@@ -527,8 +577,7 @@ int run_dp(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32
     CUDA_TRY(cudaMemsetAsync(d_max + 1, 0, sizeof(uint32_t), st));
 
     // Level 1: k single-source closures (R:1988-2031).
-    r = launch_relax(c, row_ptr, adj, n, ld, table, xs + c->kp->xs_off[1], k, d_terms, 1, st, false, d_max + 1,
-                     shadow, sld);
+    r = launch_level1(c, row_ptr, adj, n, ld, table, xs + c->kp->xs_off[1], k, d_terms, st, d_max + 1, shadow, sld);
     if (r) return r;
     CUDA_TRY(cudaEventRecord(E[ev++], st));  // 2: after level 1
     CUDA_TRY(cudaMemcpyAsync(h_max + 1, d_max + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -563,8 +612,7 @@ int run_dp(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32
         const int32_t chunk = relax_chunk_rows_level(c, n, u16, cnt);
         for (int64_t off = 0; off < cnt; off += chunk) {
             const int32_t rows = (int32_t)std::min<int64_t>(chunk, cnt - off);
-            r = launch_relax(c, row_ptr, adj, n, ld, table, xs + b + off, rows, d_terms, 0, st, u16, nullptr, shadow,
-                             sld);
+            r = launch_relax(c, row_ptr, adj, n, ld, table, xs + b + off, rows, st, u16, shadow, sld);
             if (r) return r;
             relax_launches++;
         }
@@ -636,7 +684,7 @@ extern "C" int emv_kernel_dev(emv_ctx *c, int32_t n, int64_t arcs, const int32_t
     c->launches = 0;
     ResidentPlan plan;
     if (resident_plan(c, n, k, plan))
-        return run_resident(c, plan, n, arcs, d_row_ptr, d_col, d_w, terminals, k, k, d_table, ld, true, st, cost_out,
+        return run_resident(c, plan, n, arcs, d_row_ptr, d_col, d_w, terminals, k, k, d_table, ld, true, true, st, cost_out,
                             nullptr);
     r = pack_and_check(c, n, arcs, d_row_ptr, d_col, d_w, true, st);
     if (r) return r;
@@ -736,7 +784,7 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
     if (r) return r;
     int32_t *table = (int32_t *)c->table.ptr;
     std::memset(&out->timing, 0, sizeof(out->timing));
-    r = resident ? run_resident(c, plan, n, arcs, row_ptr, col, w, terms, k, kt, table, ld, check, st, &out->cost,
+    r = resident ? run_resident(c, plan, n, arcs, row_ptr, col, w, terms, k, kt, table, ld, check, check, st, &out->cost,
                                 &out->timing)
                  : run_dp(c, n, row_ptr, (const int2 *)c->adj.ptr, k, kt, terms, table, ld, st, &out->cost, &out->timing, check);
     if (r) return r;
@@ -796,6 +844,9 @@ extern "C" int emv_solve_dev(emv_ctx *c, const emv_graph *d_g, const int32_t *te
                            (cudaStream_t)stream);
 }
 
+// Up to here one CTA's shared memory beats the whole GPU's sweeps.
+constexpr int32_t SSSP_RESIDENT_N = 8192;
+
 extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t *dist_out, float *ms_out, void *stream)
 {
     if (!c || !dist_out) return emv_fail(EMV_ERR_BAD_INPUT, "null argument");
@@ -806,37 +857,63 @@ extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t 
     cudaStream_t st = (cudaStream_t)stream;
     const int32_t n = g->n;
     const int64_t arcs = g->arcs;
+    // row 1 = {source}; rows of whole quads
+    const int64_t ld = ((int64_t)n + 3) / 4 * 4;
+    ResidentPlan plan;
+    const bool resident = n <= SSSP_RESIDENT_N && resident_plan(c, n, 1, plan);
     r = dev_reserve(c->g_row, sizeof(int32_t) * ((size_t)n + 1));
     if (!r) r = dev_reserve(c->g_col, sizeof(int32_t) * (size_t)std::max<int64_t>(arcs, 1));
     if (!r) r = dev_reserve(c->g_w, sizeof(int32_t) * (size_t)std::max<int64_t>(arcs, 1));
-    if (!r) r = dev_reserve(c->table, sizeof(int32_t) * 2 * (size_t)n);  // row 1 = {source}
-    if (!r) r = dev_reserve(c->terms, sizeof(int32_t));
+    if (!r) r = dev_reserve(c->table, sizeof(int32_t) * 2 * (size_t)ld);
     if (!r) r = prepare_subsets(c, 1, st);
-    if (!r) r = reserve_relax(c, n);
+    if (!r && !resident) r = reserve_relax(c, n);
+    if (!r && !resident) r = dev_reserve(c->terms, sizeof(int32_t));
+    if (!r && c->h_dist_n < n) {
+        if (c->h_dist) cudaFreeHost(c->h_dist);
+        c->h_dist = nullptr;
+        c->h_dist_n = 0;
+        if (cudaMallocHost((void **)&c->h_dist, sizeof(int32_t) * (size_t)n) != cudaSuccess) {
+            cudaGetLastError();
+            r = emv_fail(EMV_ERR_OOM, "pinned distances of %d vertices", n);
+        } else {
+            c->h_dist_n = n;
+        }
+    }
     if (r) return r;
     CUDA_TRY(cudaMemcpyAsync(c->g_row.ptr, g->row_ptr, sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, st));
     if (arcs > 0) {
         CUDA_TRY(cudaMemcpyAsync(c->g_col.ptr, g->col, sizeof(int32_t) * (size_t)arcs, cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(c->g_w.ptr, g->w, sizeof(int32_t) * (size_t)arcs, cudaMemcpyHostToDevice, st));
     }
-    CUDA_TRY(cudaMemcpyAsync(c->terms.ptr, &source, sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemsetAsync(c->stat.ptr, 0, sizeof(DevStat), st));
-    r = pack_and_check(c, n, arcs, (const int32_t *)c->g_row.ptr, (const int32_t *)c->g_col.ptr,
-                       (const int32_t *)c->g_w.ptr, true, st);
-    if (r) return r;
-    CUDA_TRY(cudaEventRecord(c->ev[0], st));
-    r = launch_relax(c, (const int32_t *)c->g_row.ptr, (const int2 *)c->adj.ptr, n, n, (int32_t *)c->table.ptr,
-                     (const uint32_t *)c->kp->xs.ptr, 1, (const int32_t *)c->terms.ptr, 1, st);
-    if (r) return r;
-    CUDA_TRY(cudaEventRecord(c->ev[1], st));
-    std::vector<int32_t> d((size_t)n);
-    CUDA_TRY(cudaMemcpyAsync(d.data(), (int32_t *)c->table.ptr + n, sizeof(int32_t) * (size_t)n,
-                             cudaMemcpyDeviceToHost, st));
-    DevStat ds;
-    CUDA_TRY(cudaMemcpyAsync(&ds, c->stat.ptr, sizeof(ds), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    if (ds.err) return emv_dev_status_to_emv(ds.err);
+    const int32_t *row = (const int32_t *)c->g_row.ptr, *col = (const int32_t *)c->g_col.ptr, *w = (const int32_t *)c->g_w.ptr;
+    int32_t *table = (int32_t *)c->table.ptr;
+    if (resident) {
+        int64_t cost;
+        r = run_resident(c, plan, n, arcs, row, col, w, &source, 1, 1, table, ld, true, false, st, &cost, nullptr);
+        if (r) return r;
+        CUDA_TRY(cudaMemcpyAsync(c->h_dist, table + ld, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+    } else {
+        CUDA_TRY(cudaMemcpyAsync(c->terms.ptr, &source, sizeof(int32_t), cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemsetAsync(c->stat.ptr, 0, sizeof(DevStat), st));
+        r = pack_and_check(c, n, arcs, row, col, w, false, st);
+        if (r) return r;
+        CUDA_TRY(cudaEventRecord(c->ev[0], st));
+        r = launch_level1(c, row, (const int2 *)c->adj.ptr, n, ld, table, (const uint32_t *)c->kp->xs.ptr, 1,
+                          (const int32_t *)c->terms.ptr, st, nullptr, nullptr, 0, (const GraphScan *)c->gscan.ptr);
+        if (r) return r;
+        CUDA_TRY(cudaEventRecord(c->ev[1], st));
+        GraphScan *hs = (GraphScan *)((char *)c->pinned + 1024);
+        DevStat *ds = (DevStat *)((char *)c->pinned + 1536);
+        CUDA_TRY(cudaMemcpyAsync(hs, c->gscan.ptr, sizeof(GraphScan), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaMemcpyAsync(ds, c->stat.ptr, sizeof(DevStat), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaMemcpyAsync(c->h_dist, table + ld, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        r = scan_status(*hs, n);
+        if (r) return r;
+        if (ds->err) return emv_dev_status_to_emv(ds->err);
+    }
     if (ms_out) cudaEventElapsedTime(ms_out, c->ev[0], c->ev[1]);
-    for (int32_t v = 0; v < n; v++) dist_out[v] = d[(size_t)v] >= INF ? INT64_MAX : (int64_t)d[(size_t)v];
+    for (int32_t v = 0; v < n; v++) dist_out[v] = c->h_dist[v] >= INF ? INT64_MAX : (int64_t)c->h_dist[v];
     return EMV_OK;
 }

@@ -13,7 +13,7 @@
 //                 subset merge of one level           R:2068-2107
 //   k_relax<VEC, U16>  multi-source closure of <= 32*VEC rows (64*VEC with
 //                 16-bit records; VEC = 1, 2, 4, 5, 8) R:2109-2130, R:1762-1880
-//                 (also the k level-1 SSSPs,          R:1988-2031)
+//   k_level1<LPV>  the k level-1 SSSPs, -dijkstra     R:1988-2031, R:2454-2484
 //   k_traceback   tree recovery by recomputation      R:1907-1944
 #pragma once
 
@@ -22,6 +22,7 @@
 
 #include "emv_common.cuh"
 #include "emv_device_util.cuh"
+#include "emv_narrow.cuh"
 
 namespace emv {
 
@@ -33,8 +34,6 @@ struct RelaxArgs {
     int32_t *table;
     const uint32_t *rows;   // subsets of this chunk
     int32_t nrows;          // <= 32 * VEC of the launch
-    const int32_t *terms;   // level-1 mode: row r is {r}, source terms[r]
-    int32_t level1;
     int32_t *scratch;       // vertex-major records, n * 32 * VEC int32
     uint8_t *act0;          // active flags, n bytes each
     uint8_t *act1;
@@ -44,7 +43,6 @@ struct RelaxArgs {
     int32_t *stamp;         // n: last sweep in which the vertex changed (-1 none)
     int32_t dense_min;      // a sweep after one with more changed vertices takes every vertex
     int32_t pull_all_min;   // a sweep after one with at least this many changed vertices reads no stamps
-    uint32_t *vmax;         // if set: atomicMax of every value phase C writes
     uint16_t *shadow;       // if set: phase C also writes min(value, 0xffff) to shadow[X * shadow_ld + v]
     int64_t shadow_ld;
 };
@@ -776,16 +774,14 @@ __device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok)
 }
 
 // Phase A of a relaxation chunk: rows -> vertex-major records (vertex v owns
-// 32*VEC int32 words, word e = row e; U16: word e = rows e | (e + 32*VEC) << 16);
-// in level-1 mode the rows are the k single-source initialisations.  A tile
-// is 32 vertices by all 32*VEC words, so a warp has all its row loads in
+// 32*VEC int32 words, word e = row e; U16: word e = rows e | (e + 32*VEC) << 16).
+// A tile is 32 vertices by all 32*VEC words, so a warp has all its row loads in
 // flight before one barrier.  Rows past the chunk's are INF (U16: 0, which
 // no sweep lowers).  Also resets the active flags and stamps.
 template <int VEC, bool U16>
 __device__ __forceinline__ int32_t relax_load_value(const RelaxArgs &a, int32_t row, int32_t v)
 {
     if (row >= a.nrows || v >= a.n) return U16 ? 0 : INF;
-    if (a.level1) return (v == __ldg(a.terms + row)) ? 0 : INF;
     return __ldcg(a.table + (int64_t)__ldg(a.rows + row) * a.ld + v);
 }
 
@@ -830,14 +826,13 @@ __device__ void relax_load_records(const RelaxArgs &a, int32_t (*tile)[33])
 }
 
 // Phase C: vertex-major records -> table rows, a whole 32-vertex tile at a
-// time; with a.vmax set, the largest value written goes to *a.vmax.
+// time.
 template <int VEC, bool U16>
 __device__ void relax_store_records(const RelaxArgs &a, int32_t (*tile)[33])
 {
     constexpr int R = 32 * VEC, NW = RELAX_THREADS / 32, PER = R / NW;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int32_t n = a.n, ntiles = (n + 31) >> 5, nrows = a.nrows;
-    uint32_t vmax = 0;
     // software pipeline: the next tile's record loads are in flight while
     // this tile's rows are written
     constexpr int VPW = 32 / NW;  // vertices of a tile per warp
@@ -881,14 +876,9 @@ __device__ void relax_store_records(const RelaxArgs &a, int32_t (*tile)[33])
                     const int64_t X = __ldg(a.rows + row);
                     a.table[X * a.ld + v] = (int32_t)word;
                     if (a.shadow) a.shadow[X * a.shadow_ld + v] = (uint16_t)min(word, 0xffffu);
-                    vmax = max(vmax, word);
                 }
             }
         __syncthreads();
-    }
-    if (a.vmax) {
-        vmax = __reduce_max_sync(FULL, vmax);
-        if (lane == 0) atomicMax(a.vmax, vmax);
     }
 }
 
@@ -913,6 +903,71 @@ __global__ void __launch_bounds__(RELAX_THREADS, 2) k_relax(RelaxArgs a)
     if (s < 0) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stat->sweeps, (unsigned long long)s);
     relax_store_records<VEC, U16>(a, tile);
+}
+
+// Single-source closures of up to 4 * LPV sources (level 1, R:1988-2031, and
+// the -dijkstra command): records of the sources' distances, sparse sweeps
+// from the sources' neighbours on (narrow_sweeps), records -> rows.
+struct Level1Args {
+    NarrowArgs na;
+    const int2 *adj;
+    const int32_t *terms;   // source of row r
+    const uint32_t *rows;   // table row of r
+    int32_t nrows;          // <= 4 * LPV
+    int32_t *table;
+    int64_t ld;
+    uint32_t *vmax;         // if set: atomicMax of every value written
+    uint16_t *shadow;       // if set: min(value, 0xffff) at shadow[row * shadow_ld + v]
+    int64_t shadow_ld;
+    DevStat *stat;
+    const GraphScan *scan;  // if set: the CSR's check; a faulty one is not read
+};
+
+template <int LPV>
+__global__ void __launch_bounds__(NARROW_THREADS, 2) k_level1(Level1Args a)
+{
+    __shared__ int s_ok;
+    if (a.scan && a.scan->bad) return;
+    const int32_t n = a.na.n;
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = first; i < (int64_t)n * LPV; i += stride) __stcg(a.na.rec + i, make_int4(INF, INF, INF, INF));
+    for (int64_t v = first; v < n; v += stride) a.na.act0[v] = a.na.act1[v] = 0;
+    if (!grid_barrier(a.na.ctrl, &s_ok)) {
+        if (threadIdx.x == 0) atomicOr(&a.stat->err, a.na.ctrl[C_ERR]);
+        return;
+    }
+    if (blockIdx.x == 0)  // a warp per source: its distance, and its neighbours take part in sweep 0
+        for (int32_t r = threadIdx.x >> 5; r < a.nrows; r += NARROW_THREADS / 32) {
+            const int32_t t = __ldg(a.terms + r);
+            if ((threadIdx.x & 31) == 0) __stcg(reinterpret_cast<int32_t *>(a.na.rec) + (int64_t)t * 4 * LPV + r, 0);
+            for (int32_t e = __ldg(a.na.row_ptr + t) + (threadIdx.x & 31); e < __ldg(a.na.row_ptr + t + 1); e += 32)
+                a.na.act0[__ldg(&a.adj[e].x)] = 1;
+        }
+    if (!grid_barrier(a.na.ctrl, &s_ok)) {
+        if (threadIdx.x == 0) atomicOr(&a.stat->err, a.na.ctrl[C_ERR]);
+        return;
+    }
+    const int32_t s = narrow_sweeps<LPV>(a.na, NarrowPacked{a.adj}, true, &a.stat->err, &s_ok);
+    if (s < 0) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stat->sweeps, (unsigned long long)s);
+    uint32_t vmax = 0;
+    for (int32_t g = 0; g < LPV && 4 * g < a.nrows; g++)
+        for (int64_t v = first; v < n; v += stride) {
+            const int4 x = __ldcg(a.na.rec + v * LPV + g);
+            const int32_t y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (4 * g + q < a.nrows) {
+                    const int64_t X = __ldg(a.rows + 4 * g + q);
+                    a.table[X * a.ld + v] = y[q];
+                    if (a.shadow) a.shadow[X * a.shadow_ld + v] = (uint16_t)min((uint32_t)y[q], 0xffffu);
+                    vmax = max(vmax, (uint32_t)y[q]);
+                }
+        }
+    if (a.vmax) {
+        vmax = __reduce_max_sync(FULL, vmax);
+        if ((threadIdx.x & 31) == 0) atomicMax(a.vmax, vmax);
+    }
 }
 
 // ------------------------------------------------------------- traceback

@@ -15,15 +15,19 @@
 // reader/reader-el.c:1762-1880 and 2109-2130), in a variant that reads the
 // CSR's col and w arrays as given instead of a packed copy:
 //   out[r][v] = min over u of init[r][u] + dist(u, v),  r < rows <= 32.
-// Each call first checks the CSR on the device (k_noalloc_scan) and returns
-// EMV_ERR_BAD_INPUT / EMV_ERR_OVERFLOW before the closure reads it; in the
-// closure a value plus a weight saturates at EMV_INF32 instead of wrapping,
-// and a finite candidate that saturates where no smaller one exists is
-// reported as EMV_ERR_OVERFLOW.
+// The kernel first checks the CSR and returns before the closure reads a
+// faulty one (EMV_ERR_BAD_INPUT / EMV_ERR_OVERFLOW).  Where the largest input
+// value plus the longest possible path stays below EMV_INF32 no sum can reach
+// it, and the closure runs on narrow records (emv_narrow.cuh); otherwise on
+// 128-byte ones, where a value plus a weight saturates at EMV_INF32 instead of
+// wrapping, and a finite candidate that saturates where no smaller one exists
+// is reported as EMV_ERR_OVERFLOW.
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 
 #include "emv_device_util.cuh"
+#include "emv_narrow.cuh"
 #include "emv_solver.h"
 
 using namespace emv;
@@ -38,9 +42,11 @@ constexpr size_t CTRL_OFF = REC_BYTES + 2 * FLAG_BYTES;
 constexpr size_t STAT_OFF = CTRL_OFF + (sizeof(uint32_t) * C_WORDS + 255) / 256 * 256;
 static_assert(CTRL_OFF % 128 == 0, "control words on their own lines");
 constexpr size_t SCAN_OFF = STAT_OFF + 64;
+constexpr size_t MAXV_OFF = STAT_OFF + 128;
 constexpr size_t NOALLOC_BYTES = STAT_OFF + 256;
-static_assert(SCAN_OFF + sizeof(GraphScan) <= NOALLOC_BYTES, "scan words inside the status area");
-constexpr int NOALLOC_THREADS = 512;
+static_assert(SCAN_OFF + sizeof(GraphScan) <= MAXV_OFF, "scan words inside the status area");
+constexpr int NOALLOC_THREADS = NARROW_THREADS;
+constexpr int NOALLOC_VARIANTS = 4;                // kernels by record width (4, 8, 16 or 32 rows)
 constexpr int MAX_DEVICES = 64;
 
 // The scratch of every call on this device: vertex-major records, two
@@ -49,7 +55,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
 std::mutex g_setup_mu;
 unsigned char *g_scratch_ptr[MAX_DEVICES] = {};
-int g_blocks[MAX_DEVICES] = {};
+int g_blocks[MAX_DEVICES][NOALLOC_VARIANTS] = {};
 
 struct NoallocArgs {
     const int32_t *row_ptr;
@@ -60,19 +66,16 @@ struct NoallocArgs {
     int64_t ld;
     int32_t n;
     int32_t rows;
+    int64_t arcs;
+    int32_t dense_min;
     int32_t *rec;
     uint8_t *act0;
     uint8_t *act1;
     uint32_t *ctrl;
     DevStat *stat;
+    GraphScan *scan;
+    uint32_t *maxv;  // largest finite input value
 };
-
-// The device check of the caller's CSR, into the scratch's status area.
-__global__ void k_noalloc_scan(const int32_t *__restrict__ row_ptr, int32_t n, const int32_t *__restrict__ col,
-                               const int32_t *__restrict__ w, int64_t arcs, GraphScan *__restrict__ scan)
-{
-    scan_csr(row_ptr, n, col, w, nullptr, arcs, scan);
-}
 
 // val + wt saturated at INF (wt is in [0, INF) after the scan, val <= INF);
 // *sat is set when a finite val saturated.
@@ -83,21 +86,18 @@ __device__ __forceinline__ int32_t sat_add(int32_t val, int32_t wt, bool *sat)
     return min(val, room) + wt;
 }
 
-// Same phases as k_relax<1>: rows -> records, frontier sweeps, records -> rows.
-__global__ void __launch_bounds__(NOALLOC_THREADS, 2) k_closure_noalloc(NoallocArgs a)
+// Closure on 128-byte records with saturating sums: rows -> records, frontier
+// sweeps, records -> rows.
+__device__ void noalloc_saturating(const NoallocArgs &a, int *ok_word)
 {
     __shared__ int32_t tile[32][33];
-    __shared__ int s_ok;
+    int &s_ok = *ok_word;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwb = blockDim.x >> 5;
     const int32_t n = a.n, ntiles = (n + 31) >> 5;
-    bool bad_value = false;
     for (int32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int32_t v = t * 32 + lane;
-        for (int r = warp; r < 32; r += nwb) {
-            const int32_t x = (r < a.rows && v < n) ? a.init[(int64_t)r * a.ld + v] : INF;
-            bad_value |= x > INF;
-            tile[r][lane] = min(x, INF);
-        }
+        for (int r = warp; r < 32; r += nwb)
+            tile[r][lane] = (r < a.rows && v < n) ? min(a.init[(int64_t)r * a.ld + v], INF) : INF;
         __syncthreads();
         for (int vv = warp; vv < 32; vv += nwb) {
             const int32_t v2 = t * 32 + vv;
@@ -109,7 +109,6 @@ __global__ void __launch_bounds__(NOALLOC_THREADS, 2) k_closure_noalloc(NoallocA
         a.act0[v] = 1;
         a.act1[v] = 0;
     }
-    if (__any_sync(FULL, bad_value) && lane == 0) atomicOr(&a.stat->err, (uint32_t)EMV_DEV_BAD_VALUE);
     bool overflow = false;
     if (!grid_barrier(a.ctrl, &s_ok)) {
         if (threadIdx.x == 0) atomicOr(&a.stat->err, a.ctrl[C_ERR]);
@@ -199,6 +198,59 @@ __global__ void __launch_bounds__(NOALLOC_THREADS, 2) k_closure_noalloc(NoallocA
     }
 }
 
+// The whole call: CSR check and largest input value, then the closure of rows
+// kept in records of 4 * LPV rows.
+template <int LPV> __global__ void __launch_bounds__(NOALLOC_THREADS, 2) k_closure_noalloc(NoallocArgs a)
+{
+    __shared__ int s_ok;
+    const int32_t n = a.n;
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    scan_csr(a.row_ptr, n, a.col, a.w, nullptr, a.arcs, a.scan);
+    bool bad_value = false;
+    uint32_t top = 0;
+    int4 *rec = reinterpret_cast<int4 *>(a.rec);
+    for (int g = 0; g < LPV; g++)  // four rows of a vertex a thread
+        for (int64_t v = first; v < n; v += stride) {
+            int32_t y[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                y[q] = 4 * g + q < a.rows ? a.init[(int64_t)(4 * g + q) * a.ld + v] : INF;  // d_out may be d_init
+                bad_value |= y[q] > INF;
+                if (y[q] < INF) top = max(top, (uint32_t)max(y[q], 0));
+            }
+            __stcg(rec + v * LPV + g, make_int4(y[0], y[1], y[2], y[3]));
+        }
+    top = __reduce_max_sync(FULL, top);
+    if ((threadIdx.x & 31) == 0 && top) atomicMax(a.maxv, top);
+    if (__any_sync(FULL, bad_value) && (threadIdx.x & 31) == 0) atomicOr(&a.stat->err, (uint32_t)EMV_DEV_BAD_VALUE);
+    for (int64_t v = first; v < n; v += stride) a.act0[v] = a.act1[v] = 0;
+    if (!grid_barrier(a.ctrl, &s_ok)) {
+        if (threadIdx.x == 0) atomicOr(&a.stat->err, a.ctrl[C_ERR]);
+        return;
+    }
+    if (__ldcg(&a.scan->bad) || __ldcg(&a.stat->err)) return;  // the host names the fault
+    // a path visits a vertex, and so an arc, once
+    const long long longest = min((long long)(n - 1) * (long long)__ldcg(&a.scan->maxw), (long long)__ldcg(&a.scan->sumw));
+    if ((long long)__ldcg(a.maxv) + longest >= INF) {
+        noalloc_saturating(a, &s_ok);
+        return;
+    }
+    const NarrowArgs na{a.row_ptr, n, rec, a.act0, a.act1, a.ctrl, n + 1, a.dense_min};
+    if (narrow_sweeps<LPV>(na, NarrowSplit{a.col, a.w}, false, &a.stat->err, &s_ok) < 0) return;
+    for (int g = 0; g < LPV; g++)
+        for (int64_t v = first; v < n; v += stride) {
+            const int4 x = __ldcg(rec + v * LPV + g);
+            const int32_t y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (4 * g + q < a.rows) a.out[(int64_t)(4 * g + q) * a.ld + v] = y[q];
+        }
+}
+
+const void *const noalloc_fns[NOALLOC_VARIANTS] = {
+    (const void *)k_closure_noalloc<1>, (const void *)k_closure_noalloc<2>, (const void *)k_closure_noalloc<4>,
+    (const void *)k_closure_noalloc<8>};
+
 // Per-device set-up, done once with that device current: the device address
 // of the scratch array (its host-side name is only a stand-in) and the
 // cooperative grid size.  No allocation happens here either.
@@ -218,14 +270,17 @@ int setup_device(int dev)
         cudaGetLastError();
         return emv_fail(EMV_ERR_CUDA, "scratch symbol address: %s", cudaGetErrorString(e));
     }
-    int per_sm = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_closure_noalloc, NOALLOC_THREADS, 0);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 0;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    for (int i = 0; e == cudaSuccess && i < NOALLOC_VARIANTS; i++) {
+        int per_sm = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, noalloc_fns[i], NOALLOC_THREADS, 0);
+        g_blocks[dev][i] = std::max(1, per_sm) * std::max(1, sms);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return emv_fail(EMV_ERR_CUDA, "occupancy query: %s", cudaGetErrorString(e));
     }
-    g_blocks[dev] = std::max(1, per_sm) * std::max(1, sms);
     g_scratch_ptr[dev] = (unsigned char *)p;
     return EMV_OK;
 }
@@ -265,6 +320,10 @@ extern "C" int emv_closure_noalloc(int32_t n, int64_t arcs, const int32_t *d_row
     a.ld = ld;
     a.n = n;
     a.rows = rows;
+    a.arcs = arcs;
+    a.dense_min = narrow_dense_min(n, arcs);
+    a.scan = (GraphScan *)(base + SCAN_OFF);
+    a.maxv = (uint32_t *)(base + MAXV_OFF);
     a.rec = (int32_t *)base;
     a.act0 = base + REC_BYTES;
     a.act1 = base + REC_BYTES + FLAG_BYTES;
@@ -273,26 +332,22 @@ extern "C" int emv_closure_noalloc(int32_t n, int64_t arcs, const int32_t *d_row
     // The array keeps the last call's contents: the barrier, status and check
     // words must start at zero (records and flags are rewritten by the kernel).
     CUDA_TRY(cudaMemsetAsync(base + CTRL_OFF, 0, NOALLOC_BYTES - CTRL_OFF, st));
-    // Check the CSR before the closure reads it (heads index the records).
-    GraphScan *d_scan = (GraphScan *)(base + SCAN_OFF), hs;
-    const int64_t scan_work = std::max<int64_t>(arcs, (int64_t)n + 1);
-    k_noalloc_scan<<<(unsigned)std::min<int64_t>(1024, (scan_work + 255) / 256), 256, 0, st>>>(d_row_ptr, n, d_col,
-                                                                                                  d_w, arcs, d_scan);
-    CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaMemcpyAsync(&hs, d_scan, sizeof(hs), cudaMemcpyDeviceToHost, st));
+    const int vi = rows <= 4 ? 0 : rows <= 8 ? 1 : rows <= 16 ? 2 : 3;
+    const int vpb = narrow_vertices(1 << vi) * (NOALLOC_THREADS / 32);  // one group of vertices a warp
+    const int blocks = std::min(g_blocks[dev][vi], std::max(1, (n + vpb - 1) / vpb));
+    void *args[] = {&a};
+    CUDA_TRY(cudaLaunchCooperativeKernel(noalloc_fns[vi], dim3(blocks), dim3(NOALLOC_THREADS), args, 0, st));
+    unsigned char words[MAXV_OFF - STAT_OFF];
+    CUDA_TRY(cudaMemcpyAsync(words, base + STAT_OFF, sizeof(words), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
+    DevStat ds;
+    GraphScan hs;
+    std::memcpy(&ds, words, sizeof(ds));
+    std::memcpy(&hs, words + (SCAN_OFF - STAT_OFF), sizeof(hs));
     if (hs.bad & SCAN_BAD_ROWS) return emv_fail(EMV_ERR_BAD_INPUT, "emv_closure_noalloc: row_ptr not from 0 to arcs, non-decreasing");
     if (hs.bad & SCAN_BAD_HEAD) return emv_fail(EMV_ERR_BAD_INPUT, "emv_closure_noalloc: arc head out of range");
     if (hs.bad & SCAN_BAD_WEIGHT) return emv_fail(EMV_ERR_BAD_INPUT, "emv_closure_noalloc: negative weight");
     if (hs.bad & SCAN_BIG_WEIGHT) return emv_fail(EMV_ERR_OVERFLOW, "emv_closure_noalloc: an arc weight reaches 2^30");
-    const int vpb = NOALLOC_THREADS;  // 32 vertices per warp
-    const int blocks = std::min(g_blocks[dev], std::max(1, (n + vpb - 1) / vpb));
-    void *args[] = {&a};
-    CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_closure_noalloc, dim3(blocks), dim3(NOALLOC_THREADS), args, 0,
-                                         st));
-    DevStat ds;
-    CUDA_TRY(cudaMemcpyAsync(&ds, a.stat, sizeof(ds), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
     if (ds.err) return emv_dev_status_to_emv(ds.err);
     return EMV_OK;
 }

@@ -90,7 +90,7 @@ const int32_t *resident_terms(const emv_ctx *c) { return ((const ResOut *)c->res
 
 int run_resident(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, const int32_t *row_ptr, const int32_t *col,
                  const int32_t *w, const int32_t *terms, int32_t k, int32_t kt, int32_t *table, int64_t ld, bool check,
-                 cudaStream_t st, int64_t *cost_out, emv_timing *tm)
+                 bool spanned, cudaStream_t st, int64_t *cost_out, emv_timing *tm)
 {
     int r = prepare_subsets(c, kt, st);
     if (!r) r = dev_reserve(c->adj, sizeof(int2) * (size_t)std::max<int64_t>(arcs, 1));
@@ -151,7 +151,7 @@ int run_resident(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, con
         if (r) return r;
     }
     if (h->err) return emv_dev_status_to_emv(h->err);
-    if (check && h->unreached)
+    if (spanned && h->unreached)
         return emv_fail(EMV_ERR_DISCONNECTED, "graph: not connected (a vertex is unreachable from terminal 1)");
     *cost_out = k >= 2 ? h->cost : INT64_MAX;
     if (tm) {

@@ -28,6 +28,7 @@ int dev_reserve(DevBuf &b, size_t bytes);
 void dev_release(DevBuf &b);
 
 constexpr int MAX_EVENTS = 64;
+constexpr int LEVEL1_VARIANTS = 4;  // level-1 kernels by record width (level1_fns)
 constexpr int RELAX_VARIANTS = 10;  // relaxation kernels by record width (relax_fns)
 constexpr int BATCH_CLASSES = 12;  // (n bucket 0..3) x (k bucket 0..2)
 
@@ -54,6 +55,7 @@ struct emv_ctx {
     int device = 0;
     int sms = 0;
     int relax_blocks_max[RELAX_VARIANTS] = {};  // cooperative grid of each relaxation kernel
+    int level1_blocks_max[LEVEL1_VARIANTS] = {};  // and of each level-1 kernel
     int relax_sm_cap = 0;          // > 0: relaxation grids sized for this many SMs (the server's large solves)
     int64_t l2_bytes = 0;
     int64_t sweep_limit = 0;       // relaxation sweeps per chunk, 0 = n + 1
@@ -72,6 +74,8 @@ struct emv_ctx {
     DevBuf g_row, g_col, g_w;      // device copy of a host CSR
     DevBuf table;                  // DP table of emv_solve
     DevBuf tb_edges, tb_out, tb_work;
+    int32_t *h_dist = nullptr;     // pinned distances of emv_sssp, h_dist_n of them
+    int32_t h_dist_n = 0;
     void *pinned = nullptr;        // small pinned host buffer for scalar reads
     cudaEvent_t ev[MAX_EVENTS] = {};
     int32_t xs_k = -1;             // k of the current plan

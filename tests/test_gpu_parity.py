@@ -523,3 +523,29 @@ def test_one_launch_solver_whole_table(emv, orc, solver, name):
                              table.data_ptr(), ld, torch.cuda.current_stream().cuda_stream)
     got = table.cpu().numpy()
     assert cost == want_cost and np.array_equal(got[:, :csr.n], want) and (got[:, csr.n:] == -7).all()
+
+
+@pytest.mark.parametrize("kind,n,degree,wmax", [("regular", 2, 1, 9), ("regular", 8192, 4, 1000), ("regular", 8193, 6, 100),
+                                                ("powlaw", 40000, 8, 100), ("regular", 100000, 20, 100)])
+def test_sssp_sizes_match_oracle(emv, orc, solver, kind, n, degree, wmax):
+    """Distances of one source on both sides of the one-launch solver's limit
+    and with hubs, a disconnected vertex included (INT64_MAX)."""
+    make = emv.StpInstance.powlaw if kind == "powlaw" else emv.StpInstance.regular
+    inst = make(n, degree, -0.5, 8, 1, wmax, 2, 8) if kind == "powlaw" else make(n + n * degree % 2, degree, 1, wmax, 2, 8)
+    alone = emv.StpInstance(inst.n + 1, inst.edges, inst.terminals)
+    for g in (emv.Csr.from_stp(inst), emv.Csr.from_stp(alone)):
+        for s in (0, g.n - 1):
+            d, _ = solver.sssp(g, s)
+            assert np.array_equal(d, orc.sssp(g.n, g.row_ptr, g.col, g.w, s))
+
+
+@pytest.mark.parametrize("k", [3, 6, 12])
+def test_level1_record_widths(emv, orc, solver, k):
+    """Level-1 records of 4, 8 and 16 rows in front of the record kernels
+    (a graph past the one-launch solver)."""
+    inst = emv.StpInstance.regular(33000, 4, 1, 1000, k, 77)
+    csr = emv.Csr.from_stp(inst)
+    res = solver.solve(csr, table=True)
+    for i, t in enumerate(csr.terminals):
+        d = orc.sssp(csr.n, csr.row_ptr, csr.col, csr.w, int(t))
+        assert np.array_equal(res.table[1 << i], d)

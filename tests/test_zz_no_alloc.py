@@ -192,3 +192,34 @@ def test_closure_noalloc_rejects_sizes_beyond_its_array(emv):
     assert ei.value.status == 1 and "exceed" in str(ei.value)
     with pytest.raises(emv.EmvError):
         emv.Solver.closure_noalloc(16, 10, p, p, p, p, 33, 16, p)
+
+
+@pytest.mark.parametrize("kind,n,degree,rows", [("regular", 64, 3, 1), ("regular", 1025, 4, 5), ("powlaw", 3000, 8, 9),
+                                                ("clique", 300, 0, 17), ("regular", 70001, 6, 4), ("regular", 2, 1, 32)])
+def test_closure_noalloc_record_widths(emv, orc, kind, n, degree, rows):
+    """Records of 4, 8, 16 and 32 rows, hubs of more arcs than a warp's lanes
+    take alone, and partial groups of vertices, against the oracle; negative
+    values too, and values whose longest possible path passes 2^30 (the
+    saturating records)."""
+    torch = pytest.importorskip("torch")
+    if kind == "clique":
+        inst = emv.StpInstance.clique(n, 1, 5000, 2, 3)
+    elif kind == "powlaw":
+        inst = emv.StpInstance.powlaw(n, degree, -0.5, 8, 1, 100, 2, 3)
+    else:
+        inst = emv.StpInstance.regular(n, degree, 1, 1000, 2, 3)
+    csr = emv.Csr.from_stp(inst)
+    n = csr.n
+    rng = np.random.default_rng(rows)
+    csr_t = _dev(torch, csr.row_ptr, csr.col, csr.w)
+    for offset in (0, -500, (1 << 30) - 2_000_000):
+        init = np.full((rows, n), emv.INF32, np.int32)
+        for r in range(rows):
+            seeds = rng.choice(n, size=min(n, 1 + r % 3), replace=False)
+            init[r, seeds] = offset + rng.integers(0, 900, size=seeds.size)
+        want = orc.closure(n, csr.row_ptr, csr.col, csr.w, init - min(offset, 0) * (init < emv.INF32))
+        want = np.where(want < emv.INF32, want + min(offset, 0), want)
+        (d_init,) = _dev(torch, init)
+        out = torch.full_like(d_init, -9)
+        _call(emv, torch, csr_t, n, csr.arcs, d_init, rows, n, out)
+        assert np.array_equal(out.cpu().numpy().astype(np.int64), want), offset
