@@ -32,6 +32,8 @@ struct GraphScan {
     uint32_t bad;             // SCAN_* bits
     uint32_t maxw;            // largest arc weight
     unsigned long long sumw;  // sum of the arc weights (both arcs of every edge)
+    uint32_t hubs;            // vertices of more than the caller's hub_min arcs (k_pack_scan)
+    uint32_t pad;
 };
 
 // Persistent device status of one solve (zeroed at solve start).

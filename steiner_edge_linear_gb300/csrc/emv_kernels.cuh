@@ -43,6 +43,9 @@ struct RelaxArgs {
     int32_t *stamp;         // n: last sweep in which the vertex changed (-1 none)
     int32_t dense_min;      // a sweep after one with more changed vertices takes every vertex
     int32_t pull_all_min;   // a sweep after one with at least this many changed vertices reads no stamps
+    const int32_t *hubs;    // HUBS: the nhubs vertices of more than hub_min arcs
+    int32_t nhubs;
+    int32_t hub_min;
     uint16_t *shadow;       // if set: phase C also writes min(value, 0xffff) to shadow[X * shadow_ld + v]
     int64_t shadow_ld;
 };
@@ -58,12 +61,15 @@ __global__ void k_fill(int32_t *__restrict__ p, int64_t count, int32_t value)
 // admission check of the device entry points; the reference reads only
 // well-formed STP, R:473-618): heads in [0, n), weights in [0, 2^30), row_ptr
 // from 0 to arcs and non-decreasing.  Reduces the largest weight and the
-// weight sum for the value bound.  *scan must be zero before the launch.
+// weight sum for the value bound, and lists the vertices of more than hub_min
+// arcs (in no particular order).  *scan must be zero before the launch.
 __global__ void k_pack_scan(const int32_t *__restrict__ row_ptr, int32_t n, const int32_t *__restrict__ col,
                             const int32_t *__restrict__ w, int2 *__restrict__ adj, int64_t arcs,
-                            GraphScan *__restrict__ scan)
+                            GraphScan *__restrict__ scan, int32_t hub_min, int32_t *__restrict__ hubs)
 {
     scan_csr(row_ptr, n, col, w, adj, arcs, scan);
+    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        if ((int64_t)row_ptr[v + 1] - row_ptr[v] > hub_min) hubs[atomicAdd(&scan->hubs, 1u)] = v;
 }
 
 // Subset merge of one level m (R:2068-2088) plus the terminal override of
@@ -495,7 +501,7 @@ __global__ void __launch_bounds__(1024) k_merge_stream16(int32_t *__restrict__ t
 // the warp's vertices; with flags_next, marks the neighbours of every changed
 // vertex for the next sweep.  Returns whether a record changed; counts the
 // changed vertices in *s_chg.
-template <int VEC, bool U16, int GROUP, int TASK_V>
+template <int VEC, bool U16, bool HUBS, int GROUP, int TASK_V>
 __device__ __forceinline__ bool relax_pass_all(const RelaxArgs &a, int32_t vbeg, int32_t vend, int32_t s,
                                                bool flags_next, uint8_t *cur, uint8_t *nxt, int2 *warcs,
                                                unsigned *s_chg)
@@ -507,9 +513,16 @@ __device__ __forceinline__ bool relax_pass_all(const RelaxArgs &a, int32_t vbeg,
         const int32_t v = base + lane;
         const bool mine = lane < TASK_V && v < vend;
         unsigned act = __ballot_sync(FULL, mine);
-        if (mine) cur[v] = 0;
         const int32_t rp0 = mine ? __ldg(a.row_ptr + v) : 0;
         const int32_t rp1 = mine ? __ldg(a.row_ptr + v + 1) : 0;
+        if (HUBS) {  // relax_hubs takes these
+            const bool hub = rp1 - rp0 > a.hub_min;
+            act &= ~__ballot_sync(FULL, hub);
+            if (mine && !hub) cur[v] = 0;
+            if (!act) continue;
+        } else if (mine) {
+            cur[v] = 0;
+        }
         int j = __ffs(act) - 1;
         act &= act - 1;
         int32_t beg = __shfl_sync(FULL, rp0, j), end = __shfl_sync(FULL, rp1, j);
@@ -574,7 +587,7 @@ __device__ __forceinline__ bool relax_pass_all(const RelaxArgs &a, int32_t vbeg,
 // vertices, stamps the arcs (unless pull_all).  A vertex is taken when its
 // flag in `flags` is set; with clear the flag is cleared first.  Returns
 // whether a record changed; counts changed vertices in *s_chg.
-template <int VEC, bool U16, int GROUP, int TASK_V>
+template <int VEC, bool U16, bool HUBS, int GROUP, int TASK_V>
 __device__ __forceinline__ bool relax_pass_sel(const RelaxArgs &a, int32_t vbeg, int32_t vend, int32_t s, bool dense,
                                                bool dense_next, bool pull_all, uint8_t *flags, bool clear,
                                                uint8_t *nxt, int2 *warcs, unsigned *s_chg)
@@ -586,12 +599,17 @@ __device__ __forceinline__ bool relax_pass_sel(const RelaxArgs &a, int32_t vbeg,
     for (int32_t base = vbeg; base < vend; base += TASK_V) {
         const int32_t v = base + lane;
         const bool mine = lane < TASK_V && v < vend;
-        const bool f = mine && (dense || __ldcg(flags + v) != 0);
+        bool f = mine && (dense || __ldcg(flags + v) != 0);
         unsigned act = __ballot_sync(FULL, f);
         if (!act) continue;
-        if (f && clear) flags[v] = 0;
         const int32_t rp0 = mine ? __ldg(a.row_ptr + v) : 0;
         const int32_t rp1 = mine ? __ldg(a.row_ptr + v + 1) : 0;
+        if (HUBS) {  // relax_hubs takes these
+            f = f && rp1 - rp0 <= a.hub_min;
+            act = __ballot_sync(FULL, f);
+        }
+        if (f && clear) flags[v] = 0;
+        if (HUBS && !act) continue;
         // first active vertex: bounds, first 32 arcs and their selection
         int j = __ffs(act) - 1;
         act &= act - 1;
@@ -669,6 +687,93 @@ __device__ __forceinline__ bool relax_pass_sel(const RelaxArgs &a, int32_t vbeg,
     return any;
 }
 
+// Stores a lane's share of a record into shared memory, in the record's layout.
+template <int VEC> __device__ __forceinline__ void part_st(int32_t *p, int lane, typename IVec<VEC>::T x)
+{
+    reinterpret_cast<typename IVec<VEC>::T *>(p)[lane] = x;
+}
+template <> __device__ __forceinline__ void part_st<5>(int32_t *p, int lane, int5v x)
+{
+    reinterpret_cast<int4 *>(p)[lane] = x.a;
+    p[128 + lane] = x.b;
+}
+
+// The sweep's share of the hubs (vertices of more than hub_min arcs): a block
+// takes every gridDim.x-th one, its warps 32 arcs each at a time, with the
+// selection of relax_pass_sel; the partial minima meet in shared memory
+// (part: 32 * VEC words a warp).  One warp walking a hub of 1000 arcs alone
+// bounded a sweep (45 us at n = 30 000, power-law degrees, against 18).
+template <int VEC, bool U16, int GROUP>
+__device__ __noinline__ bool relax_hubs(const RelaxArgs &a, int32_t s, bool dense, bool dense_next, bool pull_all,
+                                        uint8_t *cur, uint8_t *nxt, int2 *warcs, int32_t *part, unsigned *s_chg)
+{
+    using V = typename IVec<VEC>::T;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1;
+    bool any = false;
+    for (int32_t h = blockIdx.x; h < a.nhubs; h += gridDim.x) {
+        const int32_t v = __ldg(a.hubs + h);
+        const bool take = dense || __ldcg(cur + v) != 0;
+        __syncthreads();  // all have read the flag; the partial minima of the hub before are used
+        if (!take) continue;
+        if (threadIdx.x == 0) cur[v] = 0;
+        const int32_t beg = __ldg(a.row_ptr + v), end = __ldg(a.row_ptr + v + 1);
+        V acc = vsplat<V>(U16 ? -1 : INF);
+        for (int32_t e0 = beg + warp * 32; e0 < end; e0 += RELAX_THREADS) {
+            int2 arc = make_int2(0, 0);
+            bool pull = false;
+            if (e0 + lane < end) {
+                arc = __ldg(a.adj + e0 + lane);
+                pull = pull_all || __ldcg(a.stamp + arc.x) >= s - 1;
+            }
+            const unsigned sel = __ballot_sync(FULL, pull);
+            const int cnt = __popc(sel);
+            if (pull)
+                warcs[__popc(sel & lt)] =
+                    U16 ? make_int2(arc.x, (int32_t)(min((uint32_t)arc.y, 32768u) * 0x10001u)) : arc;
+            __syncwarp();
+            for (int i = 0; i < cnt; i += GROUP) {
+                V val[GROUP];
+                int32_t wt[GROUP];
+#pragma unroll
+                for (int g = 0; g < GROUP; g++) {
+                    const bool ok = i + g < cnt;
+                    const int2 aw = warcs[(i + g) & 31];
+                    wt[g] = ok ? aw.y : 0;
+                    val[g] = ok ? rec_ld<VEC>(a.scratch, aw.x, lane) : vsplat<V>(U16 ? -1 : INF);
+                }
+#pragma unroll
+                for (int g = 0; g < GROUP; g++) acc = U16 ? vaddmin16(val[g], wt[g], acc) : vmin(acc, vadd(val[g], wt[g]));
+            }
+            __syncwarp();
+        }
+        part_st<VEC>(part + warp * 32 * VEC, lane, acc);
+        __syncthreads();
+        bool dec = false;
+        if (threadIdx.x < 32 * VEC) {
+            int32_t *word = a.scratch + (int64_t)v * 32 * VEC + threadIdx.x;
+            const int32_t old = __ldcg(word);
+            int32_t x = old;
+            for (int w = 0; w < RELAX_THREADS / 32; w++) {
+                const int32_t p = part[w * 32 * VEC + threadIdx.x];
+                x = U16 ? (int32_t)__vminu2((uint32_t)x, (uint32_t)p) : min(x, p);
+            }
+            dec = x != old;
+            if (dec) __stcg(word, x);
+        }
+        if (__syncthreads_or(dec)) {
+            any = true;
+            if (threadIdx.x == 0) {
+                __stcg(a.stamp + v, s);
+                atomicAdd(s_chg, 1u);
+            }
+            if (!dense_next)
+                for (int32_t e = beg + threadIdx.x; e < end; e += RELAX_THREADS) nxt[__ldg(&a.adj[e].x)] = 1;
+        }
+    }
+    return any;
+}
+
 // Frontier sweeps over one chunk (phase B of k_relax).  A warp owns a
 // contiguous range of n / W vertices (W warps in the grid, so the shares
 // differ by one vertex at most) and takes them TASK_V at a time: it
@@ -689,8 +794,8 @@ __device__ __forceinline__ bool relax_pass_sel(const RelaxArgs &a, int32_t vbeg,
 // host takes them only when every value of the chunk's rows is at most
 // 32767; the arc weight is then clamped to 32768, so a value plus a weight
 // stays below 2^16, and a clamped sum (at least 32768) never beats a value.
-template <int VEC, bool U16>
-__device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok)
+template <int VEC, bool U16, bool HUBS>
+__device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok, int32_t *part)
 {
     constexpr int GROUP = VEC == 8 ? 2 : VEC >= 4 ? 4 : 8;  // gathers in flight per group
     constexpr int TASK_V = 8;
@@ -738,9 +843,9 @@ __device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok)
         }
         bool any = false;
         if (dense && pull_all)
-            any = relax_pass_all<VEC, U16, GROUP, TASK_V>(a, vbeg, vend, s, !dense_next, cur, nxt, warcs, &s_chg);
+            any = relax_pass_all<VEC, U16, HUBS, GROUP, TASK_V>(a, vbeg, vend, s, !dense_next, cur, nxt, warcs, &s_chg);
         else
-            any = relax_pass_sel<VEC, U16, GROUP, TASK_V>(a, vbeg, vend, s, dense, dense_next, pull_all, cur, true,
+            any = relax_pass_sel<VEC, U16, HUBS, GROUP, TASK_V>(a, vbeg, vend, s, dense, dense_next, pull_all, cur, true,
                                                           nxt, warcs, &s_chg);
         // A sparse sweep whose successor is sparse also takes, once, the vertices
         // already marked for the next sweep (marked by changes earlier in this
@@ -749,8 +854,9 @@ __device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok)
         // has made every change of this sweep visible, so a change this early
         // pass missed is still pulled there.
         if (!dense && !dense_next)
-            any |= relax_pass_sel<VEC, U16, GROUP, TASK_V>(a, vbeg, vend, s, false, dense_next, pull_all, nxt, false,
+            any |= relax_pass_sel<VEC, U16, HUBS, GROUP, TASK_V>(a, vbeg, vend, s, false, dense_next, pull_all, nxt, false,
                                                            nxt, warcs, &s_chg);
+        if (HUBS) any |= relax_hubs<VEC, U16, GROUP>(a, s, dense, dense_next, pull_all, cur, nxt, warcs, part, &s_chg);
         any = __syncthreads_or(any);
         if (threadIdx.x == 0) {
             if (any) vctrl[C_SLOT0 + s % 3] = 1;
@@ -889,17 +995,18 @@ __device__ void relax_store_records(const RelaxArgs &a, int32_t (*tile)[33])
 // bound), ending after a sweep that changes nothing; C. records -> rows.
 // Records and stamps are read with ld.global.cg (L2), never through a stale
 // L1 line.
-template <int VEC, bool U16 = false>
+template <int VEC, bool U16 = false, bool HUBS = false>
 __global__ void __launch_bounds__(RELAX_THREADS, 2) k_relax(RelaxArgs a)
 {
-    __shared__ int32_t tile[32 * VEC][33];  // 32 vertices by all words of the chunk's records
+    __shared__ __align__(16) int32_t tile[32 * VEC][33];  // 32 vertices by all words of the chunk's records
     __shared__ int s_ok;
     relax_load_records<VEC, U16>(a, tile);
     if (!grid_barrier(a.ctrl, &s_ok)) {
         if (threadIdx.x == 0) atomicOr(&a.stat->err, a.ctrl[C_ERR]);
         return;
     }
-    const int32_t s = relax_sweeps<VEC, U16>(a, &s_ok);
+    // the transposes' tile is free during the sweeps: 16 * 32 * VEC words of it hold the hubs' partial minima
+    const int32_t s = relax_sweeps<VEC, U16, HUBS>(a, &s_ok, &tile[0][0]);
     if (s < 0) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stat->sweeps, (unsigned long long)s);
     relax_store_records<VEC, U16>(a, tile);

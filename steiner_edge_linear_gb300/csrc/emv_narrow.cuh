@@ -19,7 +19,7 @@ namespace emv {
 
 constexpr int NARROW_THREADS = 512;
 constexpr int NARROW_AP1 = 4, NARROW_AP2 = 2, NARROW_AP4 = 2;
-constexpr int NARROW_HUB = 128;  // a vertex of more arcs is pulled by the whole warp
+constexpr int NARROW_HUB = 64;  // a vertex of more arcs is pulled by the whole warp
 
 // Arcs as packed pairs or as two arrays.
 struct NarrowPacked {

@@ -29,7 +29,7 @@ void dev_release(DevBuf &b);
 
 constexpr int MAX_EVENTS = 64;
 constexpr int LEVEL1_VARIANTS = 4;  // level-1 kernels by record width (level1_fns)
-constexpr int RELAX_VARIANTS = 10;  // relaxation kernels by record width (relax_fns)
+constexpr int RELAX_VARIANTS = 20;  // relaxation kernels by record width and hubs (relax_fns)
 constexpr int BATCH_CLASSES = 12;  // (n bucket 0..3) x (k bucket 0..2)
 
 // One launch of the streamed merge: subsets [x0, x0 + cnt) of a level, its
@@ -67,6 +67,8 @@ struct emv_ctx {
     DevBuf shadow;                 // 16-bit copy of the relaxed rows (the 16-bit merge's staging source)
     cudaEvent_t evmax[EMV_MAX_K + 1] = {};  // level m's maximum has reached the pinned buffer
     DevBuf scratch, act;           // vertex-major chunk buffer, active flags
+    DevBuf hubs;                   // vertices of many arcs of the graph being relaxed
+    int32_t relax_nhubs = 0;       // and their number
     DevBuf stamp;                  // per vertex: last sweep in which it changed
     DevBuf adj;                    // packed (col, w) arcs
     DevBuf gscan;                  // GraphScan of the last packed graph (device admission check)

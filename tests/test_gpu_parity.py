@@ -549,3 +549,20 @@ def test_level1_record_widths(emv, orc, solver, k):
     for i, t in enumerate(csr.terminals):
         d = orc.sssp(csr.n, csr.row_ptr, csr.col, csr.w, int(t))
         assert np.array_equal(res.table[1 << i], d)
+
+
+@pytest.mark.parametrize("n,k,wmax,bits", [(33000, 5, 100, 0), (33000, 7, 100, 0), (33000, 9, 5000, 0), (33000, 8, 100, 32),
+                                           (6000, 10, 8000, 0)])
+def test_hubs_in_the_record_kernels(emv, orc, n, k, wmax, bits):
+    """Power-law graphs past the one-launch solver: vertices of up to a thousand
+    arcs are relaxed by whole blocks, in every record width and both value
+    widths.  Whole table against the oracle."""
+    inst = emv.StpInstance.powlaw(n, 8, -0.5, 8, 1, wmax, k, 5)
+    csr = emv.Csr.from_stp(inst)
+    assert np.diff(csr.row_ptr).max() > 256
+    want, cost = orc.emv_table(csr.n, csr.row_ptr, csr.col, csr.w, csr.terminals, threads=16)
+    with emv.Solver(0) as s:
+        s.set_value_bits(bits)
+        for check in (True, False):
+            res = s.solve(csr, table=True, check=check)
+            assert res.cost == cost and np.array_equal(res.table, want)
