@@ -108,7 +108,7 @@ extern "C" int emv_create(emv_ctx **out, int32_t device)
     if (!st) st = dev_reserve(c->lvlmax, sizeof(uint32_t) * (EMV_MAX_K + 1));
     if (!st) st = dev_reserve(c->gscan, sizeof(GraphScan));
     if (!st) {
-        if (cudaMallocHost(&c->pinned, 4096) != cudaSuccess) { cudaGetLastError(); st = emv_fail(EMV_ERR_OOM, "pinned"); }
+        if (cudaMallocHost(&c->pinned, PINNED_BYTES) != cudaSuccess) { cudaGetLastError(); st = emv_fail(EMV_ERR_OOM, "pinned"); }
     }
     for (int i = 0; !st && i < MAX_EVENTS; i++)
         if (cudaEventCreate(&c->ev[i]) != cudaSuccess) st = emv_fail(EMV_ERR_CUDA, "event create");
@@ -142,8 +142,8 @@ extern "C" int emv_destroy(emv_ctx *c)
     if (!c) return EMV_OK;
     cudaSetDevice(c->device);
     cudaDeviceSynchronize();
-    for (DevBuf *b : {&c->ctrl, &c->stat, &c->lvlmax, &c->gscan, &c->shadow, &c->scratch, &c->act, &c->adj, &c->stamp, &c->hubs, &c->terms, &c->g_row,
-                      &c->g_col, &c->g_w, &c->table, &c->tb_edges, &c->tb_out, &c->tb_work, &c->res_arcs, &c->res_out,
+    for (DevBuf *b : {&c->ctrl, &c->stat, &c->lvlmax, &c->gscan, &c->shadow, &c->scratch, &c->act, &c->adj, &c->stamp, &c->hubs, &c->terms, &c->g_all,
+                      &c->table, &c->tb_edges, &c->tb_out, &c->tb_work, &c->res_arcs, &c->res_out,
                       &c->bxs, &c->bxs_off, &c->b_row, &c->b_adj, &c->b_term, &c->b_desc, &c->b_table, &c->b_costs,
                       &c->b_ctrl, &c->b_arcs})
         dev_release(*b);
@@ -158,6 +158,7 @@ extern "C" int emv_destroy(emv_ctx *c)
         if (c->evmax[i]) cudaEventDestroy(c->evmax[i]);
     if (c->bgraph_exec) cudaGraphExecDestroy(c->bgraph_exec);
     if (c->bstage) cudaFreeHost(c->bstage);
+    if (c->g_stage) cudaFreeHost(c->g_stage);
     if (c->h_dist) cudaFreeHost(c->h_dist);
     if (c->pinned) cudaFreeHost(c->pinned);
     delete c;
@@ -700,26 +701,36 @@ extern "C" int emv_kernel_dev(emv_ctx *c, int32_t n, int64_t arcs, const int32_t
     cudaStream_t st = (cudaStream_t)stream;
     c->launches = 0;
     ResidentPlan plan;
-    if (resident_plan(c, n, k, plan))
-        return run_resident(c, plan, n, arcs, d_row_ptr, d_col, d_w, terminals, k, k, d_table, ld, true, true, st, cost_out,
-                            nullptr);
+    if (resident_plan(c, n, k, plan)) {
+        r = resident_launch(c, plan, n, arcs, d_row_ptr, d_col, d_w, terminals, k, k, d_table, ld, true, st);
+        if (r) return r;
+        CUDA_TRY(cudaStreamSynchronize(st));
+        return resident_finish(c, n, k, true, true, cost_out, nullptr);
+    }
     r = pack_and_check(c, n, arcs, d_row_ptr, d_col, d_w, true, st);
     if (r) return r;
     return run_dp(c, n, d_row_ptr, (const int2 *)c->adj.ptr, k, k, terminals, d_table, ld, st, cost_out, nullptr, true);
 }
 
-// Runs the traceback kernel and reduces its edge list to a tree on the host.
-int run_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32_t k, const int32_t *d_terms,
-                  const int32_t *table, int64_t ld, cudaStream_t st, emv_result *out)
+// Words of the traceback's result that come back with its first copy.
+constexpr size_t TB_FIRST_EDGES = 1024;
+constexpr size_t TB_FIRST_WORDS = TB_HEAD + 3 * TB_FIRST_EDGES;
+static_assert(PINNED_TB + 4 * TB_FIRST_WORDS <= PINNED_BYTES, "traceback words fit the pinned buffer");
+
+// Enqueues the traceback and the copy of its head and first edges into the
+// pinned buffer.  skip_err, skip_bad (or null): device words that say, where
+// not 0, that there is nothing to trace.
+static int launch_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32_t k,
+                            const int32_t *d_terms, const int32_t *table, int64_t ld, const uint32_t *skip_err,
+                            const uint32_t *skip_bad, cudaStream_t st)
 {
     const int32_t cap = std::max(64, 2 * n);
-    int r = dev_reserve(c->tb_edges, sizeof(int32_t) * 3 * (size_t)cap);
-    if (!r) r = dev_reserve(c->tb_out, sizeof(int32_t) * 2);
+    const int32_t nchunks = cap / TB_CHUNK + TB_TASKS + 1;
+    int r = dev_reserve(c->tb_edges, sizeof(int32_t) * (TB_CHUNK * 3 + 1) * (size_t)nchunks);
+    if (!r) r = dev_reserve(c->tb_out, sizeof(int32_t) * (TB_HEAD + 3 * std::max<size_t>((size_t)cap, TB_FIRST_EDGES)));
     if (!r) r = dev_reserve(c->tb_work, sizeof(int32_t) * 3 * (size_t)n);
     if (r) return r;
     int32_t *work = (int32_t *)c->tb_work.ptr;
-    CUDA_TRY(cudaMemsetAsync(work + 2 * (size_t)n, 0xff, sizeof(int32_t) * (size_t)n, st));
-    CUDA_TRY(cudaMemsetAsync(c->tb_out.ptr, 0, sizeof(int32_t) * 2, st));
     TbArgs a;
     a.table = table;
     a.ld = ld;
@@ -728,42 +739,57 @@ int run_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj
     a.row_ptr = row_ptr;
     a.adj = adj;
     a.terms = d_terms;
-    a.edges = (int32_t *)c->tb_edges.ptr;
-    a.cap = cap;
+    a.skip_err = skip_err;
+    a.skip_bad = skip_bad;
+    a.chunks = (int32_t *)c->tb_edges.ptr;
+    a.next = a.chunks + (size_t)nchunks * TB_CHUNK * 3;
+    a.nchunks = nchunks;
     a.out = (int32_t *)c->tb_out.ptr;
+    a.cap = cap;
     a.queue = work;
     a.parent = work + n;
     a.stamp = work + 2 * (size_t)n;
     a.max_steps = 4 * n + 64 * k + 1024;
-    CUDA_TRY(cudaEventRecord(c->ev[MAX_EVENTS - 2], st));
-    k_traceback<<<1, 32, 0, st>>>(a);
+    k_traceback<<<1, 32 * TB_WARPS, 0, st>>>(a);
+    CUDA_TRY(cudaGetLastError());
     c->launches++;
-    CUDA_TRY(cudaEventRecord(c->ev[MAX_EVENTS - 1], st));
-    int32_t hout[2];
-    CUDA_TRY(cudaMemcpyAsync(hout, a.out, sizeof(hout), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, c->ev[MAX_EVENTS - 2], c->ev[MAX_EVENTS - 1]);
-    out->timing.traceback_ms = ms;
-    if (hout[1]) return emv_dev_status_to_emv((uint32_t)hout[1]);
-    std::vector<int32_t> e((size_t)hout[0] * 3);
-    if (hout[0] > 0)
-        CUDA_TRY(cudaMemcpy(e.data(), a.edges, sizeof(int32_t) * e.size(), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpyAsync((char *)c->pinned + PINNED_TB, a.out, sizeof(int32_t) * TB_FIRST_WORDS, cudaMemcpyDeviceToHost,
+                             st));
+    return EMV_OK;
+}
+
+// Reduces the edges of a finished traceback (the stream has been waited for)
+// to a tree.
+static int finish_traceback(emv_ctx *c, int32_t n, emv_result *out)
+{
+    const int32_t *head = (const int32_t *)((char *)c->pinned + PINNED_TB), *e = head + TB_HEAD;
+    const size_t edges = (size_t)head[0];
+    out->timing.traceback_ms = (float)(head[2] * 1e-6);
+    if (head[1]) return emv_dev_status_to_emv((uint32_t)head[1]);
+    std::vector<int32_t> all;
+    if (edges > TB_FIRST_EDGES) {
+        all.resize(3 * edges);
+        CUDA_TRY(cudaMemcpy(all.data(), (const int32_t *)c->tb_out.ptr + TB_HEAD, sizeof(int32_t) * all.size(),
+                            cudaMemcpyDeviceToHost));
+        e = all.data();
+    }
     // Keep a spanning forest of the emitted edges: duplicates and zero-weight
-    // cycles (possible only through zero-weight arcs) are dropped.
-    std::vector<int32_t> parent((size_t)n);
-    std::iota(parent.begin(), parent.end(), 0);
+    // cycles (possible only through zero-weight arcs) are dropped.  Vertices
+    // are their own parent (-1) until an edge touches them, and again after.
+    if (c->forest.size() < (size_t)n) c->forest.assign((size_t)n, -1);
+    std::vector<int32_t> &parent = c->forest;
     auto find = [&](int32_t x) {
-        while (parent[(size_t)x] != x) {
-            parent[(size_t)x] = parent[(size_t)parent[(size_t)x]];
-            x = parent[(size_t)x];
+        while (parent[(size_t)x] >= 0) {
+            const int32_t p = parent[(size_t)x];
+            if (parent[(size_t)p] >= 0) parent[(size_t)x] = parent[(size_t)p];
+            x = p;
         }
         return x;
     };
     int64_t count = 0, weight = 0;
-    for (int32_t i = 0; i < hout[0]; i++) {
-        int32_t u = e[(size_t)3 * i], v = e[(size_t)3 * i + 1], wt = e[(size_t)3 * i + 2];
-        int32_t ru = find(u), rv = find(v);
+    for (size_t i = 0; i < edges; i++) {
+        const int32_t u = e[3 * i], v = e[3 * i + 1], wt = e[3 * i + 2];
+        const int32_t ru = find(u), rv = find(v);
         if (ru == rv) continue;
         parent[(size_t)ru] = rv;
         if (out->tree && count < out->tree_cap) {
@@ -774,6 +800,7 @@ int run_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj
         count++;
         weight += wt;
     }
+    for (size_t i = 0; i < edges; i++) parent[(size_t)e[3 * i]] = parent[(size_t)e[3 * i + 1]] = -1;
     out->tree_count = count;
     out->tree_weight = weight;
     if (out->tree && count > out->tree_cap)
@@ -801,23 +828,76 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
     if (r) return r;
     int32_t *table = (int32_t *)c->table.ptr;
     std::memset(&out->timing, 0, sizeof(out->timing));
-    r = resident ? run_resident(c, plan, n, arcs, row_ptr, col, w, terms, k, kt, table, ld, check, check, st, &out->cost,
-                                &out->timing)
-                 : run_dp(c, n, row_ptr, (const int2 *)c->adj.ptr, k, kt, terms, table, ld, st, &out->cost, &out->timing, check);
-    if (r) return r;
     out->tree_count = 0;
     out->tree_weight = 0;
-    if ((flags & EMV_SOLVE_TREE) && k >= 2) {
-        r = run_traceback(c, n, row_ptr, (const int2 *)c->adj.ptr, k,
-                          resident ? resident_terms(c) : (const int32_t *)c->terms.ptr, table, ld, st, out);
+    const bool tree = (flags & EMV_SOLVE_TREE) && k >= 2;
+    if (resident) {  // one wait for the solve and its tree
+        r = resident_launch(c, plan, n, arcs, row_ptr, col, w, terms, k, kt, table, ld, check, st);
+        if (!r && tree) {
+            const ResidentWords d = resident_words(c);
+            r = launch_traceback(c, n, row_ptr, (const int2 *)c->adj.ptr, k, d.terms, table, ld, d.err, d.bad, st);
+        }
         if (r) return r;
+        CUDA_TRY(cudaStreamSynchronize(st));
+        r = resident_finish(c, n, k, check, check, &out->cost, &out->timing);
+    } else {
+        const int2 *adj = (const int2 *)c->adj.ptr;
+        r = run_dp(c, n, row_ptr, adj, k, kt, terms, table, ld, st, &out->cost, &out->timing, check);
+        if (!r && tree) {
+            r = launch_traceback(c, n, row_ptr, adj, k, (const int32_t *)c->terms.ptr, table, ld, nullptr, nullptr, st);
+            if (r) return r;
+            CUDA_TRY(cudaStreamSynchronize(st));
+        }
     }
+    if (!r && tree) r = finish_traceback(c, n, out);
+    if (r) return r;
     if ((flags & EMV_SOLVE_TABLE) && out->table) {
         CUDA_TRY(cudaMemcpy2DAsync(out->table, sizeof(int32_t) * (size_t)n, table, sizeof(int32_t) * (size_t)ld,
                                    sizeof(int32_t) * (size_t)n, (size_t)1 << k, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
     }
     out->timing.launches = c->launches;
+    return EMV_OK;
+}
+
+// Copies a host CSR to the device.  Graphs of up to GRAPH_STAGE_BYTES go through
+// one pinned buffer in one copy (three copies from pageable memory cost a
+// small solve 15 us); larger ones straight from the caller's arrays, which the
+// driver reads at 160-180 GB/s, close to the 200 GB/s from pinned memory.
+constexpr size_t GRAPH_STAGE_BYTES = 1 << 20;
+
+static int graph_to_device(emv_ctx *c, const emv_graph *g, cudaStream_t st, const int32_t **row, const int32_t **col,
+                           const int32_t **w)
+{
+    const size_t rows = (size_t)g->n + 1, arcs = (size_t)g->arcs;
+    const size_t col_at = (rows + 3) / 4 * 4, w_at = col_at + (arcs + 3) / 4 * 4, words = w_at + arcs;
+    int r = dev_reserve(c->g_all, sizeof(int32_t) * words);
+    if (r) return r;
+    int32_t *d = (int32_t *)c->g_all.ptr;
+    *row = d;
+    *col = d + col_at;
+    *w = d + w_at;
+    if (sizeof(int32_t) * words <= GRAPH_STAGE_BYTES && !c->g_stage &&
+        cudaMallocHost(&c->g_stage, GRAPH_STAGE_BYTES) != cudaSuccess) {
+        cudaGetLastError();
+        c->g_stage = nullptr;
+    }
+    if (sizeof(int32_t) * words <= GRAPH_STAGE_BYTES && c->g_stage) {
+        // every call waits for its stream before it returns, so the buffer is free
+        int32_t *h = (int32_t *)c->g_stage;
+        std::memcpy(h, g->row_ptr, sizeof(int32_t) * rows);
+        if (arcs > 0) {
+            std::memcpy(h + col_at, g->col, sizeof(int32_t) * arcs);
+            std::memcpy(h + w_at, g->w, sizeof(int32_t) * arcs);
+        }
+        CUDA_TRY(cudaMemcpyAsync(d, h, sizeof(int32_t) * words, cudaMemcpyHostToDevice, st));
+        return EMV_OK;
+    }
+    CUDA_TRY(cudaMemcpyAsync(d, g->row_ptr, sizeof(int32_t) * rows, cudaMemcpyHostToDevice, st));
+    if (arcs > 0) {
+        CUDA_TRY(cudaMemcpyAsync(d + col_at, g->col, sizeof(int32_t) * arcs, cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(d + w_at, g->w, sizeof(int32_t) * arcs, cudaMemcpyHostToDevice, st));
+    }
     return EMV_OK;
 }
 
@@ -832,19 +912,10 @@ extern "C" int emv_solve(emv_ctx *c, const emv_graph *g, const int32_t *terminal
     CUDA_TRY(cudaSetDevice(c->device));
     cudaStream_t st = (cudaStream_t)stream;
     c->launches = 0;
-    const int32_t n = g->n;
-    const int64_t arcs = g->arcs;
-    r = dev_reserve(c->g_row, sizeof(int32_t) * ((size_t)n + 1));
-    if (!r) r = dev_reserve(c->g_col, sizeof(int32_t) * (size_t)std::max<int64_t>(arcs, 1));
-    if (!r) r = dev_reserve(c->g_w, sizeof(int32_t) * (size_t)std::max<int64_t>(arcs, 1));
+    const int32_t *row, *col, *w;
+    r = graph_to_device(c, g, st, &row, &col, &w);
     if (r) return r;
-    CUDA_TRY(cudaMemcpyAsync(c->g_row.ptr, g->row_ptr, sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, st));
-    if (arcs > 0) {
-        CUDA_TRY(cudaMemcpyAsync(c->g_col.ptr, g->col, sizeof(int32_t) * (size_t)arcs, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(c->g_w.ptr, g->w, sizeof(int32_t) * (size_t)arcs, cudaMemcpyHostToDevice, st));
-    }
-    return solve_on_device(c, n, arcs, (const int32_t *)c->g_row.ptr, (const int32_t *)c->g_col.ptr,
-                           (const int32_t *)c->g_w.ptr, terminals, k, flags, out, st);
+    return solve_on_device(c, g->n, g->arcs, row, col, w, terminals, k, flags, out, st);
 }
 
 extern "C" int emv_solve_dev(emv_ctx *c, const emv_graph *d_g, const int32_t *terminals, int32_t k, int32_t flags,
@@ -878,10 +949,7 @@ extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t 
     const int64_t ld = ((int64_t)n + 3) / 4 * 4;
     ResidentPlan plan;
     const bool resident = n <= SSSP_RESIDENT_N && resident_plan(c, n, 1, plan);
-    r = dev_reserve(c->g_row, sizeof(int32_t) * ((size_t)n + 1));
-    if (!r) r = dev_reserve(c->g_col, sizeof(int32_t) * (size_t)std::max<int64_t>(arcs, 1));
-    if (!r) r = dev_reserve(c->g_w, sizeof(int32_t) * (size_t)std::max<int64_t>(arcs, 1));
-    if (!r) r = dev_reserve(c->table, sizeof(int32_t) * 2 * (size_t)ld);
+    r = dev_reserve(c->table, sizeof(int32_t) * 2 * (size_t)ld);
     if (!r) r = prepare_subsets(c, 1, st);
     if (!r && !resident) r = reserve_relax(c, n);
     if (!r && !resident) r = dev_reserve(c->terms, sizeof(int32_t));
@@ -897,19 +965,18 @@ extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t 
         }
     }
     if (r) return r;
-    CUDA_TRY(cudaMemcpyAsync(c->g_row.ptr, g->row_ptr, sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, st));
-    if (arcs > 0) {
-        CUDA_TRY(cudaMemcpyAsync(c->g_col.ptr, g->col, sizeof(int32_t) * (size_t)arcs, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(c->g_w.ptr, g->w, sizeof(int32_t) * (size_t)arcs, cudaMemcpyHostToDevice, st));
-    }
-    const int32_t *row = (const int32_t *)c->g_row.ptr, *col = (const int32_t *)c->g_col.ptr, *w = (const int32_t *)c->g_w.ptr;
+    const int32_t *row, *col, *w;
+    r = graph_to_device(c, g, st, &row, &col, &w);
+    if (r) return r;
     int32_t *table = (int32_t *)c->table.ptr;
     if (resident) {
         int64_t cost;
-        r = run_resident(c, plan, n, arcs, row, col, w, &source, 1, 1, table, ld, true, false, st, &cost, nullptr);
+        r = resident_launch(c, plan, n, arcs, row, col, w, &source, 1, 1, table, ld, true, st);
         if (r) return r;
         CUDA_TRY(cudaMemcpyAsync(c->h_dist, table + ld, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
+        r = resident_finish(c, n, 1, true, false, &cost, nullptr);
+        if (r) return r;
     } else {
         CUDA_TRY(cudaMemcpyAsync(c->terms.ptr, &source, sizeof(int32_t), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemsetAsync(c->stat.ptr, 0, sizeof(DevStat), st));

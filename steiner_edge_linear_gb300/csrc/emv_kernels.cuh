@@ -1079,16 +1079,22 @@ __global__ void __launch_bounds__(NARROW_THREADS, 2) k_level1(Level1Args a)
 
 // ------------------------------------------------------------- traceback
 
+// The bits of p, lowest first, at the set positions of mask.
 __device__ __forceinline__ uint32_t deposit_bits(uint32_t p, uint32_t mask)
 {
     uint32_t r = 0;
-    for (uint32_t b = 1; mask; b <<= 1) {
+    for (; p && mask; p >>= 1) {
         const uint32_t lowbit = mask & (0u - mask);
-        if (p & b) r |= lowbit;
+        if (p & 1u) r |= lowbit;
         mask ^= lowbit;
     }
     return r;
 }
+
+constexpr int TB_WARPS = 16;
+constexpr int TB_TASKS = 64;   // pieces of the tree: at most 2 (k - 1) - 1
+constexpr int TB_CHUNK = 64;   // edges of a chunk of a piece's list
+constexpr int TB_HEAD = 16;    // words before the edges of the result
 
 struct TbArgs {
     const int32_t *table;
@@ -1098,184 +1104,333 @@ struct TbArgs {
     const int32_t *row_ptr;
     const int2 *adj;
     const int32_t *terms;
-    int32_t *edges;     // 3 * cap
-    int32_t cap;
-    int32_t *out;       // [0] edge count, [1] status
+    const uint32_t *skip_err, *skip_bad;  // if set: words that are 0 where table and arcs may be read
+    int32_t *chunks;    // edge lists: chunks of TB_CHUNK edges of 3 words
+    int32_t *next;      // the chunk after each chunk
+    int32_t nchunks;
+    int32_t *out;       // TB_HEAD words ([0] edge count, [1] status, [2] ns), then the edges (3 words each)
+    int32_t cap;        // edges that fit
     int32_t *queue;     // n
     int32_t *parent;    // n
-    int32_t *stamp;     // n, -1 on entry
+    int32_t *stamp;     // n
     int32_t max_steps;
 };
 
-// Witness of d[X][v] (warp-collective, all lanes return the same):
+// Witness of d[X][v] = D (warp-collective, all lanes return the same):
 // 0 leaf (X = {i}, v = t_i); 1 split d[Y][v] + d[X\Y][v] = D (the lowest
-// pair index); 2 arc (u, v) of positive weight with d[X][u] + w = D;
-// 3 none of those (a zero-weight predecessor must exist).
-__device__ int tb_witness(const TbArgs &a, uint32_t X, int32_t v, int32_t D, uint32_t &Y, int32_t &u, int32_t &wt)
+// pair index; DY = d[Y][v]); 2 arc (u, v) of positive weight with d[X][u] + w
+// = D; 3 none of those (a zero-weight predecessor must exist).  [beg, end):
+// v's arcs, on return of 2 u's.  A step's time is its chain of dependent loads
+// (arc, value at its head), so the first 32 arcs are requested before the
+// pairs are looked at, and the bounds of a head's own arcs with its value.
+__device__ int tb_witness(const TbArgs &a, uint32_t X, int32_t v, int32_t D, int32_t &beg, int32_t &end, uint32_t &Y,
+                          int32_t &DY, int32_t &u, int32_t &wt)
 {
     const int lane = threadIdx.x & 31;
     const int pc = __popc(X);
     if (pc == 1 && v == __ldg(a.terms + (__ffs(X) - 1))) return 0;
+    const int32_t *row = a.table + (int64_t)X * a.ld;
+    int2 arc;
+    int32_t du = INF, ub = 0, ue = 0;
+    auto head = [&](int32_t e) {  // arc e, its head's value and arcs
+        du = INF;
+        if (e < end) {
+            arc = a.adj[e];
+            du = row[arc.x];
+            ub = a.row_ptr[arc.x];
+            ue = a.row_ptr[arc.x + 1];
+        }
+    };
+    head(beg + lane);
     if (pc >= 2) {
         const uint32_t low = X & (0u - X), rest = X ^ low;
         const uint32_t npairs = (1u << __popc(rest)) - 1;
-        for (uint32_t base = 0; base < npairs; base += 32) {
-            const uint32_t p = base + lane;
-            bool ok = false;
-            uint32_t y = 0;
-            if (p < npairs) {
-                y = low | deposit_bits(p, rest);
-                const int32_t x1 = a.table[(int64_t)y * a.ld + v];
-                const int32_t x2 = a.table[(int64_t)(X ^ y) * a.ld + v];
-                ok = x1 < INF && x2 < INF && x1 + x2 == D;
+        const uint32_t mine = deposit_bits((uint32_t)lane, rest);  // the pair index's low five bits
+        uint32_t high = rest;                                      // positions of its other bits
+        for (int i = 0; i < 5; i++) high &= high - 1;
+        for (uint32_t base = 0; base < npairs; base += 128) {
+            uint32_t y[4];
+            int32_t x1[4], x2[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                x1[q] = x2[q] = INF;
+                if (base + 32 * q >= npairs) continue;
+                const bool ok = base + 32 * q + lane < npairs;
+                y[q] = low | (ok ? mine : 0u) | deposit_bits((base >> 5) + q, high);
+                if (!ok) continue;
+                x1[q] = a.table[(int64_t)y[q] * a.ld + v];
+                x2[q] = a.table[(int64_t)(X ^ y[q]) * a.ld + v];
             }
-            const unsigned bal = __ballot_sync(FULL, ok);
-            if (bal) {
-                Y = __shfl_sync(FULL, y, __ffs(bal) - 1);
-                return 1;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const unsigned bal = __ballot_sync(FULL, x1[q] < INF && x2[q] < INF && x1[q] + x2[q] == D);
+                if (bal) {
+                    Y = __shfl_sync(FULL, y[q], __ffs(bal) - 1);
+                    DY = __shfl_sync(FULL, x1[q], __ffs(bal) - 1);
+                    return 1;
+                }
             }
         }
     }
-    const int32_t beg = a.row_ptr[v], end = a.row_ptr[v + 1];
-    for (int32_t e0 = beg; e0 < end; e0 += 32) {
-        const int32_t e = e0 + lane;
-        bool ok = false;
-        int2 arc = make_int2(0, 0);
-        if (e < end) {
-            arc = a.adj[e];
-            if (arc.y > 0) {
-                const int32_t du = a.table[(int64_t)X * a.ld + arc.x];
-                ok = du < INF && du + arc.y == D;
-            }
-        }
-        const unsigned bal = __ballot_sync(FULL, ok);
+    for (int32_t e0 = beg;;) {
+        const unsigned bal = __ballot_sync(FULL, du < INF && arc.y > 0 && du + arc.y == D);
         if (bal) {
             const int src = __ffs(bal) - 1;
             u = __shfl_sync(FULL, arc.x, src);
             wt = __shfl_sync(FULL, arc.y, src);
+            beg = __shfl_sync(FULL, ub, src);
+            end = __shfl_sync(FULL, ue, src);
             return 2;
         }
+        e0 += 32;
+        if (e0 >= end) return 3;
+        head(e0 + lane);
     }
-    return 3;
 }
 
-// Tree recovery from the finished table (one warp).  Starts at (C, q) and
+// A piece of the tree: the walk from (X, v) along arcs of row X to a leaf or to
+// a split into kid (X \ Y) and kid + 1 (Y).
+struct TbTask {
+    uint32_t X;
+    int32_t v, D;
+    int32_t first, count;  // its edges
+    int32_t kid;           // -1: a leaf
+    int32_t ready;
+};
+
+// Tree recovery from the finished table (one block).  Starts at (C, q) and
 // repeatedly explains d[X][v] by a leaf, a split into (Y, v) and (X\Y, v),
 // or an arc (v, u) into (X, u) -- the decisions the reference records in b_v
 // (R:2081-2084, R:2122-2128) and walks in backtrack() (R:1907-1932), found
-// here by recomputation instead of a 2x-table predecessor store.  A run of
-// zero-weight arcs is resolved by a breadth-first search inside the set of
-// vertices with the same value, so zero-weight cycles cannot loop.
-__global__ void __launch_bounds__(32) k_traceback(TbArgs a)
+// here by recomputation instead of a 2x-table predecessor store.  Every piece
+// between two splits is walked by a warp of its own (one warp for the whole
+// tree: 83 us at n = 4096, k = 10, a chain of 67 steps; the pieces together
+// are as long as the longest way from the root), into its own edge list; the
+// lists are then laid out in the order of the depth-first walk that visits
+// X \ Y first.  A run of zero-weight arcs is resolved by a breadth-first
+// search inside the set of vertices with the same value, so zero-weight
+// cycles cannot loop; its arrays serve one warp at a time.
+__global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(TbArgs a)
 {
-    __shared__ uint32_t stX[TB_STACK];
-    __shared__ int32_t stV[TB_STACK];
-    const int lane = threadIdx.x & 31;
-    int sp = 0, cnt = 0, walk = 0, steps = 0;
-    uint32_t status = 0;
-    if (a.k >= 2) {
-        if (lane == 0) {
-            stX[0] = (1u << (a.k - 1)) - 1;
-            stV[0] = a.terms[a.k - 1];
-        }
-        sp = 1;
+    __shared__ TbTask task[TB_TASKS];
+    __shared__ int s_alloc, s_next, s_done, s_chunk, s_lock, s_walk;
+    __shared__ uint32_t s_status;
+    __shared__ int32_t s_order[TB_TASKS], s_at[TB_TASKS], s_pieces;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((a.skip_err && *a.skip_err) || (a.skip_bad && *a.skip_bad)) {
+        if (threadIdx.x < TB_HEAD) a.out[threadIdx.x] = 0;
+        return;
     }
-    __syncwarp();
-    while (sp > 0) {
-        if (++steps > a.max_steps) { status |= EMV_DEV_TB_STEPS; break; }
-        const uint32_t X = stX[sp - 1];
-        const int32_t v = stV[sp - 1];
-        sp--;
-        __syncwarp();
-        const int32_t D = a.table[(int64_t)X * a.ld + v];
-        uint32_t Y = 0;
-        int32_t u = 0, wt = 0;
-        const int kind = tb_witness(a, X, v, D, Y, u, wt);
-        if (kind == 0) continue;
-        if (kind == 1) {
-            if (sp + 2 > TB_STACK) { status |= EMV_DEV_TB_OVERFLOW; break; }
-            if (lane == 0) {
-                stX[sp] = Y; stV[sp] = v;
-                stX[sp + 1] = X ^ Y; stV[sp + 1] = v;
-            }
-            sp += 2;
-            __syncwarp();
-            continue;
+    unsigned long long t0 = 0;
+    if (threadIdx.x == 0) {
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+        s_next = s_done = s_chunk = s_lock = s_walk = 0;
+        s_alloc = a.k >= 2;
+        s_status = 0;
+        if (a.k >= 2) {
+            TbTask &t = task[0];
+            t.X = (1u << (a.k - 1)) - 1;
+            t.v = a.terms[a.k - 1];
+            t.D = a.table[(int64_t)t.X * a.ld + t.v];
+            t.ready = 1;
         }
-        if (kind == 2) {
-            if (cnt >= a.cap || sp + 1 > TB_STACK) { status |= EMV_DEV_TB_OVERFLOW; break; }
-            if (lane == 0) {
-                a.edges[3 * cnt] = v; a.edges[3 * cnt + 1] = u; a.edges[3 * cnt + 2] = wt;
-                stX[sp] = X; stV[sp] = u;
-            }
-            cnt++;
-            sp++;
-            __syncwarp();
-            continue;
-        }
-        // Zero-weight run: BFS over arcs of weight 0 between vertices of value D.
-        walk++;
-        if (lane == 0) {
-            a.queue[0] = v;
-            a.parent[v] = -1;
-            a.stamp[v] = walk;
-        }
-        __syncwarp();
-        int32_t head = 0, tail = 1, target = -1;
-        while (head < tail) {
-            const int32_t x = *(volatile int32_t *)(a.queue + head);
-            head++;
-            if (x != v) {
-                uint32_t Y2;
-                int32_t u2, w2;
-                if (tb_witness(a, X, x, D, Y2, u2, w2) != 3) { target = x; break; }
-            }
-            const int32_t beg = a.row_ptr[x], end = a.row_ptr[x + 1];
-            for (int32_t e0 = beg; e0 < end; e0 += 32) {
-                const int32_t e = e0 + lane;
-                bool add = false;
-                int32_t y = 0;
-                if (e < end) {
-                    const int2 arc = a.adj[e];
-                    y = arc.x;
-                    if (arc.y == 0 && a.table[(int64_t)X * a.ld + y] == D)
-                        add = atomicExch(a.stamp + y, walk) != walk;
+        for (int i = a.k >= 2; i < TB_TASKS; i++) task[i].ready = 0;
+    }
+    __syncthreads();
+    int32_t steps = 0;
+    for (;;) {
+        // claim a piece; a warp that finds none for long leaves the rest to the others
+        int mine = -1;
+        if (lane == 0)
+            for (int spins = 0; spins < (1 << 20); spins++) {
+                const int h = *(volatile int *)&s_next;
+                if (h < min(*(volatile int *)&s_alloc, TB_TASKS) && *(volatile int *)&task[h].ready) {
+                    if (atomicCAS(&s_next, h, h + 1) == h) {
+                        mine = h;
+                        break;
+                    }
+                } else if (*(volatile int *)&s_done >= *(volatile int *)&s_alloc || *(volatile uint32_t *)&s_status) {
+                    break;
                 }
-                const unsigned bal = __ballot_sync(FULL, add);
-                if (add) {
-                    const int pos = tail + __popc(bal & ((1u << lane) - 1));
-                    a.queue[pos] = y;
-                    a.parent[y] = x;
-                }
-                tail += __popc(bal);
-                __syncwarp();
             }
-        }
-        if (target < 0) { status |= EMV_DEV_TB_NO_WITNESS; break; }
-        int32_t z = target, emitted = 0;
-        bool ovf = false;
-        if (lane == 0) {
-            while (z != v) {
+        mine = __shfl_sync(FULL, mine, 0);
+        if (mine < 0) break;
+        const uint32_t X = task[mine].X;
+        int32_t v = task[mine].v, D = task[mine].D;
+        int32_t beg = a.row_ptr[v], end = a.row_ptr[v + 1];
+        int32_t count = 0, first = -1, chunk = -1, kid = -1;
+        uint32_t fail = 0;
+        auto add_edge = [&](int32_t x, int32_t y, int32_t w) {  // lane 0's arguments
+            if (count % TB_CHUNK == 0) {
+                int c = 0;
+                if (lane == 0) c = atomicAdd(&s_chunk, 1);
+                c = __shfl_sync(FULL, c, 0);
+                if (c >= a.nchunks) {
+                    fail = EMV_DEV_TB_OVERFLOW;
+                    return;
+                }
+                if (lane == 0 && chunk >= 0) a.next[chunk] = c;
+                if (first < 0) first = c;
+                chunk = c;
+            }
+            if (lane == 0) {
+                int32_t *e = a.chunks + ((int64_t)chunk * TB_CHUNK + count % TB_CHUNK) * 3;
+                e[0] = x;
+                e[1] = y;
+                e[2] = w;
+            }
+            count++;
+        };
+        while (!fail) {
+            if (++steps > a.max_steps) {
+                fail = EMV_DEV_TB_STEPS;
+                break;
+            }
+            uint32_t Y = 0;
+            int32_t DY = 0, u = 0, wt = 0;
+            const int kind = tb_witness(a, X, v, D, beg, end, Y, DY, u, wt);
+            if (kind == 0) break;
+            if (kind == 1) {
+                if (lane == 0) kid = atomicAdd(&s_alloc, 2);
+                kid = __shfl_sync(FULL, kid, 0);
+                if (kid + 2 > TB_TASKS) {
+                    fail = EMV_DEV_TB_OVERFLOW;
+                    break;
+                }
+                if (lane < 2) {
+                    TbTask &t = task[kid + lane];
+                    t.X = lane ? Y : X ^ Y;
+                    t.v = v;
+                    t.D = lane ? DY : D - DY;
+                    __threadfence_block();
+                    *(volatile int *)&t.ready = 1;
+                }
+                break;
+            }
+            if (kind == 2) {
+                add_edge(v, u, wt);
+                v = u;
+                D -= wt;
+                continue;
+            }
+            // Zero-weight run: BFS over arcs of weight 0 between vertices of value D.
+            int walk = 0;
+            if (lane == 0) {
+                int spins = 0;
+                while (atomicCAS(&s_lock, 0, 1) != 0 && ++spins < (1 << 24)) {}
+                walk = spins < (1 << 24) ? ++s_walk : -1;
+            }
+            walk = __shfl_sync(FULL, walk, 0);
+            if (walk < 0) {
+                fail = EMV_DEV_TB_STEPS;
+                break;
+            }
+            if (walk == 1)  // the first run of this launch clears the stamps
+                for (int32_t i = lane; i < a.n; i += 32) a.stamp[i] = 0;
+            __syncwarp();
+            if (lane == 0) {
+                a.queue[0] = v;
+                a.parent[v] = -1;
+                a.stamp[v] = walk;
+            }
+            __syncwarp();
+            int32_t head = 0, tail = 1, target = -1;
+            while (head < tail) {
+                const int32_t x = *(volatile int32_t *)(a.queue + head);
+                head++;
+                if (x != v) {
+                    uint32_t Y2;
+                    int32_t d2, u2, w2, xb = a.row_ptr[x], xe = a.row_ptr[x + 1];
+                    if (tb_witness(a, X, x, D, xb, xe, Y2, d2, u2, w2) != 3) {
+                        target = x;
+                        break;
+                    }
+                }
+                const int32_t xb = a.row_ptr[x], xe = a.row_ptr[x + 1];
+                for (int32_t e0 = xb; e0 < xe; e0 += 32) {
+                    const int32_t e = e0 + lane;
+                    bool add = false;
+                    int32_t y = 0;
+                    if (e < xe) {
+                        const int2 arc = a.adj[e];
+                        y = arc.x;
+                        if (arc.y == 0 && a.table[(int64_t)X * a.ld + y] == D) add = atomicExch(a.stamp + y, walk) != walk;
+                    }
+                    const unsigned bal = __ballot_sync(FULL, add);
+                    if (add) {
+                        const int pos = tail + __popc(bal & ((1u << lane) - 1));
+                        a.queue[pos] = y;
+                        a.parent[y] = x;
+                    }
+                    tail += __popc(bal);
+                    __syncwarp();
+                }
+            }
+            if (target < 0) fail = EMV_DEV_TB_NO_WITNESS;
+            for (int32_t z = target; !fail && z != v;) {
                 const int32_t p = *(volatile int32_t *)(a.parent + z);
-                if (cnt + emitted >= a.cap) { ovf = true; break; }
-                a.edges[3 * (cnt + emitted)] = z;
-                a.edges[3 * (cnt + emitted) + 1] = p;
-                a.edges[3 * (cnt + emitted) + 2] = 0;
-                emitted++;
+                add_edge(z, p, 0);
                 z = p;
             }
+            if (!fail) {
+                v = target;
+                beg = a.row_ptr[v];
+                end = a.row_ptr[v + 1];
+            }
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) atomicExch(&s_lock, 0);
         }
-        emitted = __shfl_sync(FULL, emitted, 0);
-        ovf = __shfl_sync(FULL, (int)ovf, 0) != 0;
-        cnt += emitted;
-        if (ovf || sp + 1 > TB_STACK) { status |= EMV_DEV_TB_OVERFLOW; break; }
-        if (lane == 0) { stX[sp] = X; stV[sp] = target; }
-        sp++;
+        if (lane == 0) {
+            task[mine].first = first;
+            task[mine].count = count;
+            task[mine].kid = kid;
+            if (fail) atomicOr(&s_status, fail);
+            __threadfence_block();
+            atomicAdd(&s_done, 1);
+        }
         __syncwarp();
     }
-    if (lane == 0) {
-        a.out[0] = cnt;
-        a.out[1] = (int32_t)status;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {  // the pieces in depth-first order and where their edges go
+        int32_t total = 0, pieces = 0, sp = 0;
+        int32_t stack[TB_TASKS];
+        if (!s_status && s_done < s_alloc) s_status = EMV_DEV_TB_STEPS;
+        if (!s_status && a.k >= 2) stack[sp++] = 0;
+        while (sp > 0) {
+            const int32_t t = stack[--sp];
+            s_order[pieces] = t;
+            s_at[pieces++] = total;
+            total += task[t].count;
+            if (task[t].kid >= 0) {
+                stack[sp++] = task[t].kid + 1;
+                stack[sp++] = task[t].kid;
+            }
+        }
+        if (total > a.cap) {
+            s_status |= EMV_DEV_TB_OVERFLOW;
+            pieces = 0;
+        }
+        s_pieces = pieces;
+        a.out[0] = s_status ? 0 : total;
+        a.out[1] = (int32_t)s_status;
+    }
+    __syncthreads();
+    for (int p = warp; p < s_pieces; p += TB_WARPS) {
+        const TbTask &t = task[s_order[p]];
+        int32_t *dst = a.out + TB_HEAD + (int64_t)s_at[p] * 3;
+        for (int32_t i = 0, c = t.first; i < t.count; i += TB_CHUNK) {
+            const int32_t words = min(TB_CHUNK, t.count - i) * 3;
+            for (int32_t w = lane; w < words; w += 32)
+                dst[(int64_t)i * 3 + w] = __ldcg(a.chunks + (int64_t)c * TB_CHUNK * 3 + w);
+            c = __ldcg(a.next + c);
+        }
+    }
+    if (threadIdx.x == 0) {
+        unsigned long long t1;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+        a.out[2] = (int32_t)min(t1 - t0, 2000000000ull);
     }
 }
 

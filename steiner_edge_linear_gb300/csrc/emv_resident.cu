@@ -86,11 +86,15 @@ bool resident_plan(const emv_ctx *c, int32_t n, int32_t kt, ResidentPlan &p)
     return true;
 }
 
-const int32_t *resident_terms(const emv_ctx *c) { return ((const ResOut *)c->res_out.ptr)->terms; }
+ResidentWords resident_words(const emv_ctx *c)
+{
+    const ResOut *o = (const ResOut *)c->res_out.ptr;
+    return {o->terms, &o->err, &o->scan.bad};
+}
 
-int run_resident(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, const int32_t *row_ptr, const int32_t *col,
-                 const int32_t *w, const int32_t *terms, int32_t k, int32_t kt, int32_t *table, int64_t ld, bool check,
-                 bool spanned, cudaStream_t st, int64_t *cost_out, emv_timing *tm)
+int resident_launch(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, const int32_t *row_ptr,
+                    const int32_t *col, const int32_t *w, const int32_t *terms, int32_t k, int32_t kt, int32_t *table,
+                    int64_t ld, bool check, cudaStream_t st)
 {
     int r = prepare_subsets(c, kt, st);
     if (!r) r = dev_reserve(c->adj, sizeof(int2) * (size_t)std::max<int64_t>(arcs, 1));
@@ -142,12 +146,16 @@ int run_resident(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, con
         CUDA_TRY(cudaLaunchKernel((const void *)k_resident, dim3(1), dim3(RES_THREADS), args, (size_t)RESIDENT_SMEM, st));
     c->launches++;
     CUDA_TRY(cudaEventRecord(c->ev[1], st));
-    ResOut *h = (ResOut *)((char *)c->pinned + 2048);
-    static_assert(sizeof(ResOut) <= 2048, "result words fit the pinned buffer");
-    CUDA_TRY(cudaMemcpyAsync(h, a.out, sizeof(ResOut), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    static_assert(PINNED_RES + sizeof(ResOut) <= PINNED_TB, "result words fit the pinned buffer");
+    CUDA_TRY(cudaMemcpyAsync((char *)c->pinned + PINNED_RES, a.out, sizeof(ResOut), cudaMemcpyDeviceToHost, st));
+    return EMV_OK;
+}
+
+int resident_finish(emv_ctx *c, int32_t n, int32_t k, bool check, bool spanned, int64_t *cost_out, emv_timing *tm)
+{
+    const ResOut *h = (const ResOut *)((char *)c->pinned + PINNED_RES);
     if (check) {
-        r = scan_status(h->scan, n);
+        const int r = scan_status(h->scan, n);
         if (r) return r;
     }
     if (h->err) return emv_dev_status_to_emv(h->err);

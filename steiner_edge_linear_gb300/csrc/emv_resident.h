@@ -22,13 +22,20 @@ bool resident_fits(int32_t n, int32_t kt);
 int32_t resident_merge_width(int32_t n, int32_t kt, int32_t ctas, int32_t cap);
 uint32_t res_inv_slices(int32_t n);
 bool resident_plan(const emv_ctx *c, int32_t n, int32_t kt, ResidentPlan &p);
-// The whole DP over the first kt of the k terminals, CSR check included (with
-// spanned set, a vertex that no terminal reaches is EMV_ERR_DISCONNECTED);
-// fills the table's 2^kt rows (stride ld) and c->adj.
-int run_resident(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, const int32_t *row_ptr, const int32_t *col,
-                 const int32_t *w, const int32_t *terms, int32_t k, int32_t kt, int32_t *table, int64_t ld, bool check,
-                 bool spanned, cudaStream_t st, int64_t *cost_out, emv_timing *tm);
-// The terminals on the device after run_resident.
-const int32_t *resident_terms(const emv_ctx *c);
+// Enqueues the whole DP over the first kt of the k terminals, CSR check
+// included, and the copy of its result words; fills the table's 2^kt rows
+// (stride ld) and c->adj.
+int resident_launch(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, const int32_t *row_ptr,
+                    const int32_t *col, const int32_t *w, const int32_t *terms, int32_t k, int32_t kt, int32_t *table,
+                    int64_t ld, bool check, cudaStream_t st);
+// Status, cost and times once the stream has been waited for (with spanned
+// set, a vertex that no terminal reaches is EMV_ERR_DISCONNECTED).
+int resident_finish(emv_ctx *c, int32_t n, int32_t k, bool check, bool spanned, int64_t *cost_out, emv_timing *tm);
+// Device words of the launch: the terminals, the error word, the CSR check's.
+struct ResidentWords {
+    const int32_t *terms;
+    const uint32_t *err, *bad;
+};
+ResidentWords resident_words(const emv_ctx *c);
 // Status of a device CSR check (emv_device.cu).
 int scan_status(const emv::GraphScan &s, int32_t n);

@@ -28,6 +28,8 @@ int dev_reserve(DevBuf &b, size_t bytes);
 void dev_release(DevBuf &b);
 
 constexpr int MAX_EVENTS = 64;
+// emv_ctx::pinned: scalars of run_dp, then the one-launch solver's and the traceback's results
+constexpr size_t PINNED_RES = 2048, PINNED_TB = 4096, PINNED_BYTES = 32768;
 constexpr int LEVEL1_VARIANTS = 4;  // level-1 kernels by record width (level1_fns)
 constexpr int RELAX_VARIANTS = 20;  // relaxation kernels by record width and hubs (relax_fns)
 constexpr int BATCH_CLASSES = 12;  // (n bucket 0..3) x (k bucket 0..2)
@@ -73,12 +75,14 @@ struct emv_ctx {
     DevBuf adj;                    // packed (col, w) arcs
     DevBuf gscan;                  // GraphScan of the last packed graph (device admission check)
     DevBuf terms;                  // terminals
-    DevBuf g_row, g_col, g_w;      // device copy of a host CSR
+    DevBuf g_all;                  // device copy of a host CSR (row_ptr, col, w)
+    void *g_stage = nullptr;       // pinned staging of small host CSRs
     DevBuf table;                  // DP table of emv_solve
     DevBuf tb_edges, tb_out, tb_work;
+    std::vector<int32_t> forest;   // union-find of the tree's edges, -1 between calls
     int32_t *h_dist = nullptr;     // pinned distances of emv_sssp, h_dist_n of them
     int32_t h_dist_n = 0;
-    void *pinned = nullptr;        // small pinned host buffer for scalar reads
+    void *pinned = nullptr;        // small pinned host buffer for scalar reads, PINNED_BYTES
     cudaEvent_t ev[MAX_EVENTS] = {};
     int32_t xs_k = -1;             // k of the current plan
     KPlan *kp = nullptr;           // plan of xs_k

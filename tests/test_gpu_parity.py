@@ -566,3 +566,25 @@ def test_hubs_in_the_record_kernels(emv, orc, n, k, wmax, bits):
         for check in (True, False):
             res = s.solve(csr, table=True, check=check)
             assert res.cost == cost and np.array_equal(res.table, want)
+
+
+@pytest.mark.parametrize("n,wmin,wmax,k", [(64, 1, 9, 2), (500, 0, 1, 9), (2000, 0, 2, 12), (40000, 0, 3, 6)])
+def test_traceback_pieces_and_zero_weight_runs(emv, orc, solver, n, wmin, wmax, k):
+    """The pieces of a tree are walked by different warps; runs of zero-weight
+    arcs share one set of search arrays between them.  Valid trees of the
+    optimal weight, the same on every call."""
+    csr = emv.Csr.from_stp(inst := emv.StpInstance.regular(n, 4, wmin, wmax, k, 3))
+    first = solver.solve(csr, tree=True)
+    check_tree(csr.n, inst.edges, first.tree, csr.terminals, first.cost)
+    again = solver.solve(csr, tree=True, all_rows=True)
+    assert again.cost == first.cost and again.tree_weight == first.tree_weight
+
+
+def test_traceback_of_a_long_path(emv, solver):
+    """More edges than come back with the first copy."""
+    n = 5000
+    edges = np.stack([np.arange(n - 1), np.arange(1, n), np.ones(n - 1, np.int64)], axis=1).astype(np.int64)
+    inst = emv.StpInstance(n, edges, np.array([0, 2500, n - 1], np.int64))
+    res = solver.solve(emv.Csr.from_stp(inst), tree=True)
+    assert res.cost == n - 1
+    check_tree(n, edges, res.tree, inst.terminals, res.cost)
