@@ -18,6 +18,8 @@
 #include <thread>
 #include <vector>
 
+constexpr int32_t BATCH_CUT_MIN = 768;
+
 namespace {
 
 // f(i) for i in [0, count) on up to 16 host threads (chunks of 16 indices).
@@ -189,6 +191,21 @@ int launch_batch(emv_ctx *c, const BatchArgs &args, int32_t blocks, cudaStream_t
     return EMV_OK;
 }
 
+// Where a batch is cut into two launches: behind the instances of teams and at
+// least half of the work, so that the host checks and packs the other (smaller)
+// instances while these run.  Packing takes about a fifth of the time that
+// the packed instances run, so a batch of a few hundred gains nothing.
+static int32_t batch_cut(const BatchOrder &ord)
+{
+    const int32_t count = (int32_t)ord.ids.size();
+    if (count < BATCH_CUT_MIN) return count;
+    double total = 0, part = 0;
+    for (double w : ord.work) total += w;
+    int32_t cut = 0;
+    while (cut < count && (ord.size[(size_t)cut] > 1 || part < 0.5 * total)) part += ord.work[(size_t)cut++];
+    return count - cut < BATCH_CUT_MIN / 2 ? count : cut;
+}
+
 // emv_batch_solve and emv_batch_solve_tables: tables_out (or null) receives
 // the finished table of every instance whose entry is not null.
 static int batch_solve(emv_ctx *c, const emv_instance *inst, int32_t count, int64_t *costs_out,
@@ -200,64 +217,119 @@ static int batch_solve(emv_ctx *c, const emv_instance *inst, int32_t count, int6
     CUDA_TRY(cudaSetDevice(c->device));
     cudaStream_t st = (cudaStream_t)stream;
     const auto t0 = std::chrono::steady_clock::now();
-    // Admission checks of every instance, in parallel on the host; the first
-    // failing instance (lowest index) is reported.
+    // Admission checks: sizes first (the layout follows from them), the arrays
+    // when an instance is packed; the failing instance of the lowest index is
+    // reported.
     std::vector<int> bad((size_t)count, 0);
     std::vector<std::string> why((size_t)count);
-    host_parallel_for(count, [&](int64_t i) {
+    auto noted = [&](int64_t i, int r) {
+        if (r) {
+            bad[(size_t)i] = r;
+            why[(size_t)i] = emv_last_error();
+        }
+        return r == 0;
+    };
+    auto check_sizes = [&](int64_t i) {
         const emv_instance &I = inst[i];
         int r = emv_graph_validate(&I.g);
         if (!r && !batch_fits(I.g.n, I.k))
             r = emv_fail(EMV_ERR_BAD_INPUT, "n = %d, k = %d outside the batched range (k <= %d)", I.g.n, I.k, BATCH_KMAX);
         if (!r && !I.terminals) r = emv_fail(EMV_ERR_BAD_INPUT, "null terminals");
+        return noted(i, r);
+    };
+    auto check_arrays = [&](int64_t i) {
+        const emv_instance &I = inst[i];
+        int r = EMV_OK;
         for (int32_t t = 0; !r && t < I.k; t++)
             if (I.terminals[t] < 0 || I.terminals[t] >= I.g.n) r = emv_fail(EMV_ERR_BAD_INPUT, "terminal out of range");
         if (!r) r = emv_graph_check(&I.g, nullptr);
-        if (r) {
-            bad[(size_t)i] = r;
-            why[(size_t)i] = emv_last_error();
-        }
-    });
-    for (int32_t i = 0; i < count; i++)
-        if (bad[(size_t)i]) return emv_fail(bad[(size_t)i], "instance %d: %s", i, why[(size_t)i].c_str());
+        return noted(i, r);
+    };
+    auto first_bad = [&]() {
+        for (int32_t i = 0; i < count; i++)
+            if (bad[(size_t)i]) return emv_fail(bad[(size_t)i], "instance %d: %s", i, why[(size_t)i].c_str());
+        return (int)EMV_OK;
+    };
+    bool sizes_ok = true;
+    for (int32_t i = 0; i < count; i++) sizes_ok &= check_sizes(i);
+    if (!sizes_ok) {  // an instance before it may fail the other checks
+        host_parallel_for(count, [&](int64_t i) {
+            if (!bad[(size_t)i]) check_arrays(i);
+        });
+        return first_bad();
+    }
+    int r = batch_kernel_setup(c);
+    if (!r) r = dev_reserve(c->b_costs, sizeof(int64_t) * (size_t)count);
+    if (!r && !c->bstream) {
+        CUDA_TRY(cudaStreamCreateWithFlags(&c->bstream, cudaStreamNonBlocking));
+        for (cudaEvent_t &e : c->bev) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    if (r) return r;
+    const bool whole = tables_out != nullptr;
     std::vector<int32_t> ids((size_t)count);
     for (int32_t i = 0; i < count; i++) ids[(size_t)i] = i;
-    BatchPack pk;
-    int r = batch_kernel_setup(c);
-    if (!r) r = batch_pack(c, inst, ids, tables_out != nullptr, 0, pk);
-    if (!r) r = batch_upload(c, pk, st);
-    if (r) return r;
-    CUDA_TRY(cudaEventRecord(c->ev[0], st));
-    BatchArgs a = batch_args(c, pk);
-    // The control reset and the persistent launch are replayed as one CUDA graph.
-    r = batch_graph_launch(c, a, pk.blocks, st);
-    if (r) return r;
-    CUDA_TRY(cudaEventRecord(c->ev[1], st));
-    CUDA_TRY(cudaMemcpyAsync(costs_out, a.costs, sizeof(int64_t) * (size_t)count, cudaMemcpyDeviceToHost, st));
-    uint32_t err = 0;
-    CUDA_TRY(cudaMemcpyAsync(&err, a.ctl, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    if (err) return emv_dev_status_to_emv(err);
-    if (tables_out) {
-        for (int32_t j = 0; j < count; j++) {
-            const int32_t i = pk.desc[(size_t)j].orig;
-            if (!tables_out[i]) continue;
-            const size_t row = sizeof(int32_t) * (size_t)inst[i].g.n;
-            CUDA_TRY(cudaMemcpy2DAsync(tables_out[i], row, pk.desc[(size_t)j].table,
-                                       sizeof(int32_t) * (size_t)batch_ld(inst[i].g.n), row, (size_t)1 << inst[i].k,
-                                       cudaMemcpyDeviceToHost, st));
+    const BatchOrder ord = batch_order(c, inst, ids, whole, 0);
+    const int32_t cut = batch_cut(ord);
+    BatchPack pk[BATCH_LANES];
+    BatchArgs a[BATCH_LANES];
+    const int lanes = cut < count ? 2 : 1;
+    CUDA_TRY(cudaEventRecord(c->bev[0], st));  // the second lane starts behind the caller's work too
+    int status = EMV_OK;
+    bool failed = false;
+    auto check = [&](int32_t i) { return check_arrays(i); };
+    for (int l = 0; l < lanes && !status && !failed; l++) {
+        cudaStream_t ls = l ? c->bstream : st;
+        pk[l].lane = l;
+        status = batch_layout(c, inst, ord, l ? cut : 0, l ? count : cut, whole, 0, pk[l]);
+        if (!status) status = batch_fill(c, inst, pk[l], check);
+        for (const BatchInst &d : pk[l].desc) failed |= bad[(size_t)d.orig] != 0;
+        if (status || failed) break;
+        if (l) CUDA_TRY(cudaStreamWaitEvent(ls, c->bev[0], 0));
+        status = batch_upload(c, pk[l], ls);
+        if (status) break;
+        a[l] = batch_args(c, pk[l]);
+        if (l == 0) CUDA_TRY(cudaEventRecord(c->ev[0], st));
+        // The control reset and the persistent launch are replayed as one CUDA graph.
+        status = batch_graph_launch(c, l, a[l], pk[l].blocks, ls);
+        if (!status && l) {
+            CUDA_TRY(cudaEventRecord(c->bev[1], ls));
+            CUDA_TRY(cudaStreamWaitEvent(st, c->bev[1], 0));
         }
+    }
+    if (status || failed) {
+        if (failed && lanes == 2 && pk[1].desc.empty())  // the second part was not looked at yet
+            host_parallel_for(count - cut, [&](int64_t j) { check_arrays(ord.ids[(size_t)(cut + j)]); });
+        CUDA_TRY(cudaStreamSynchronize(c->bstream));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        return failed ? first_bad() : status;
+    }
+    CUDA_TRY(cudaEventRecord(c->ev[1], st));
+    CUDA_TRY(cudaMemcpyAsync(costs_out, c->b_costs.ptr, sizeof(int64_t) * (size_t)count, cudaMemcpyDeviceToHost, st));
+    uint32_t err[BATCH_LANES] = {};
+    for (int l = 0; l < lanes; l++)
+        CUDA_TRY(cudaMemcpyAsync(&err[l], a[l].ctl, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    if (err[0] | err[1]) return emv_dev_status_to_emv(err[0] | err[1]);
+    if (tables_out) {
+        for (int l = 0; l < lanes; l++)
+            for (const BatchInst &d : pk[l].desc) {
+                const int32_t i = d.orig;
+                if (!tables_out[i]) continue;
+                const size_t row = sizeof(int32_t) * (size_t)inst[i].g.n;
+                CUDA_TRY(cudaMemcpy2DAsync(tables_out[i], row, d.table, sizeof(int32_t) * (size_t)batch_ld(inst[i].g.n), row,
+                                           (size_t)1 << inst[i].k, cudaMemcpyDeviceToHost, st));
+            }
         CUDA_TRY(cudaStreamSynchronize(st));
     }
     if (stats) {
         float ms = 0;
         cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]);
         stats->total_ms = ms;
-        stats->upload_ms = (float)std::chrono::duration<double, std::milli>(pk.t_upload_end - t0).count();
+        stats->upload_ms = (float)std::chrono::duration<double, std::milli>(pk[lanes - 1].t_upload_end - t0).count();
         stats->work_items = count;
-        stats->table_bytes = pk.table_words * 4;
+        stats->table_bytes = (pk[0].table_words + pk[1].table_words) * 4;
         stats->merge_tile = 32;
-        stats->relax_rows = pk.rcap_used;
+        stats->relax_rows = std::max(pk[0].rcap_used, pk[1].rcap_used);
     }
     return EMV_OK;
 }
@@ -277,8 +349,8 @@ extern "C" int emv_batch_solve_tables(emv_ctx *c, const emv_instance *inst, int3
 
 // ---------------------------------------------------------------- packing
 
-int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &ids, bool whole, int32_t blocks,
-               BatchPack &pk)
+BatchOrder batch_order(const emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &ids, bool whole,
+                       int32_t blocks)
 {
     const int32_t count = (int32_t)ids.size();
     std::vector<double> work((size_t)count);
@@ -289,15 +361,27 @@ int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> 
         work[(size_t)j] = batch_work(I.g.n, kt, I.g.arcs, 1, kt);
         states[(size_t)j] = resident_max_rows(kt) * I.g.n;
     }
-    std::vector<int32_t> order, size;
-    // a cap of `blocks` CTAs is a measurement of single-CTA teams
+    std::vector<int32_t> order, size((size_t)count, 1);
     if (blocks > 0) {
-        size.assign((size_t)count, 1);
         order.resize((size_t)count);
         for (int32_t j = 0; j < count; j++) order[(size_t)j] = j;
     } else {
         batch_plan(work, states, c->batch_blocks, 1 << (BATCH_SIZES - 1), order, size);
     }
+    BatchOrder o;
+    for (int32_t j : order) {
+        o.ids.push_back(ids[(size_t)j]);
+        o.size.push_back(size[(size_t)j]);
+        o.work.push_back(work[(size_t)j]);
+    }
+    return o;
+}
+
+int batch_layout(emv_ctx *c, const emv_instance *inst, const BatchOrder &ord, int32_t from, int32_t to, bool whole,
+                 int32_t blocks, BatchPack &pk)
+{
+    const int32_t count = to - from;
+    BatchLane &L = c->blane[pk.lane];
     pk.desc.resize((size_t)count);
     pk.row_off.resize((size_t)count);
     pk.arc_off.resize((size_t)count);
@@ -305,14 +389,14 @@ int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> 
     pk.table_off.resize((size_t)count);
     int64_t rows = 0, arcs = 0, terms = 0, words = 0, ctas = 0;
     for (int32_t j = 0; j < count; j++) {
-        const int32_t id = ids[(size_t)order[(size_t)j]];
+        const int32_t id = ord.ids[(size_t)(from + j)];
         const emv_instance &I = inst[id];
         BatchInst &d = pk.desc[(size_t)j];
         std::memset(&d, 0, sizeof(d));
         d.n = I.g.n;
         d.k = I.k;
         d.kt = whole ? I.k : table_terminals(I.k);
-        d.size = size[(size_t)order[(size_t)j]];
+        d.size = ord.size[(size_t)(from + j)];
         batch_shape(c, d);
         d.orig = id;
         d.lo = 1;
@@ -337,73 +421,85 @@ int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> 
     pk.terms = terms;
     pk.table_words = words;
     pk.count = count;
-    // Host staging (pinned, reused): row_ptr | adj | terms | desc
+    // Host staging (pinned, reused): adj | row_ptr | terms | desc
     const size_t bytes = sizeof(int32_t) * (size_t)rows + sizeof(int2) * (size_t)arcs + sizeof(int32_t) * (size_t)terms +
                          sizeof(BatchInst) * (size_t)count + 64;
-    if (c->bstage_bytes < bytes) {
-        if (c->bstage) cudaFreeHost(c->bstage);
-        c->bstage = nullptr;
-        c->bstage_bytes = 0;
-        if (cudaMallocHost(&c->bstage, bytes) != cudaSuccess) {
+    if (L.stage_bytes < bytes) {
+        if (L.stage) cudaFreeHost(L.stage);
+        L.stage = nullptr;
+        L.stage_bytes = 0;
+        const size_t want = bytes + bytes / 4;  // the next batch of this kind is a little larger or smaller
+        if (cudaMallocHost(&L.stage, want) != cudaSuccess) {
             cudaGetLastError();
-            return emv_fail(EMV_ERR_OOM, "pinned staging of %zu bytes", bytes);
+            return emv_fail(EMV_ERR_OOM, "pinned staging of %zu bytes", want);
         }
-        c->bstage_bytes = bytes;
+        L.stage_bytes = want;
     }
-    char *p = (char *)c->bstage;
-    int32_t *hrow = (int32_t *)p;
-    int2 *hadj = (int2 *)(hrow + rows);
-    int32_t *hterm = (int32_t *)(hadj + arcs);
-    BatchInst *hdesc = (BatchInst *)(((uintptr_t)(hterm + terms) + 15) & ~(uintptr_t)15);
-    std::vector<int64_t> arc_bytes((size_t)count);
-    host_parallel_for(count, [&](int64_t j) {  // disjoint ranges of the staging buffer
-        const emv_instance &I = inst[pk.desc[(size_t)j].orig];
+    pk.h_adj = (int2 *)L.stage;
+    pk.h_row = (int32_t *)(pk.h_adj + arcs);
+    pk.h_term = pk.h_row + rows;
+    pk.h_desc = (BatchInst *)(((uintptr_t)(pk.h_term + terms) + 15) & ~(uintptr_t)15);
+    return EMV_OK;
+}
+
+int batch_fill(emv_ctx *c, const emv_instance *inst, BatchPack &pk, const std::function<bool(int32_t)> &check)
+{
+    (void)c;
+    std::vector<int64_t> arc_bytes((size_t)pk.count);
+    host_parallel_for(pk.count, [&](int64_t j) {  // disjoint ranges of the staging buffer
+        const int32_t id = pk.desc[(size_t)j].orig;
+        if (check && !check(id)) return;
+        const emv_instance &I = inst[id];
         const BatchGraph bg = batch_graph(I.g.row_ptr, I.g.w, I.g.n, I.g.arcs);
         pk.desc[(size_t)j].narrow = bg.narrow;
         arc_bytes[(size_t)j] = bg.arc_bytes;
-        std::memcpy(hrow + pk.row_off[(size_t)j], I.g.row_ptr, sizeof(int32_t) * ((size_t)I.g.n + 1));
-        int2 *ha = hadj + pk.arc_off[(size_t)j];
+        std::memcpy(pk.h_row + pk.row_off[(size_t)j], I.g.row_ptr, sizeof(int32_t) * ((size_t)I.g.n + 1));
+        int2 *ha = pk.h_adj + pk.arc_off[(size_t)j];
         for (int64_t e = 0; e < I.g.arcs; e++) ha[e] = make_int2(I.g.col[e], I.g.w[e]);
-        std::memcpy(hterm + pk.term_off[(size_t)j], I.terminals, sizeof(int32_t) * (size_t)I.k);
+        std::memcpy(pk.h_term + pk.term_off[(size_t)j], I.terminals, sizeof(int32_t) * (size_t)I.k);
     });
     for (int64_t b : arc_bytes) pk.arc_bytes = std::max(pk.arc_bytes, b);
-    std::memcpy(hdesc, pk.desc.data(), sizeof(BatchInst) * (size_t)count);
-    pk.h_row = hrow;
-    pk.h_adj = hadj;
-    pk.h_term = hterm;
-    pk.h_desc = hdesc;
     return EMV_OK;
+}
+
+// dev_reserve with a quarter to spare when a buffer grows (exactly what is
+// needed where that does not fit): batches of one kind differ a little in
+// size, and a larger one would free and allocate gigabytes again.
+static int reserve_more(DevBuf &b, size_t bytes)
+{
+    if (b.bytes >= bytes) return EMV_OK;
+    return dev_reserve(b, bytes + bytes / 4) == EMV_OK ? (int)EMV_OK : dev_reserve(b, bytes);
 }
 
 int batch_upload(emv_ctx *c, BatchPack &pk, cudaStream_t st)
 {
-    int r = dev_reserve(c->b_row, sizeof(int32_t) * (size_t)pk.rows);
-    if (!r) r = dev_reserve(c->b_adj, sizeof(int2) * (size_t)std::max<int64_t>(pk.arcs, 1));
-    if (!r) r = dev_reserve(c->b_term, sizeof(int32_t) * (size_t)std::max<int64_t>(pk.terms, 1));
-    if (!r) r = dev_reserve(c->b_desc, sizeof(BatchInst) * (size_t)pk.count);
-    if (!r) r = dev_reserve(c->b_table, sizeof(int32_t) * (size_t)pk.table_words);
+    BatchLane &L = c->blane[pk.lane];
+    int r = reserve_more(L.row, sizeof(int32_t) * (size_t)pk.rows);
+    if (!r) r = reserve_more(L.adj, sizeof(int2) * (size_t)std::max<int64_t>(pk.arcs, 1));
+    if (!r) r = reserve_more(L.term, sizeof(int32_t) * (size_t)std::max<int64_t>(pk.terms, 1));
+    if (!r) r = reserve_more(L.desc, sizeof(BatchInst) * (size_t)pk.count);
+    if (!r) r = reserve_more(L.table, sizeof(int32_t) * (size_t)pk.table_words);
     // costs are written at index orig (the caller's instance index), which can
-    // exceed the number of instances in this launch when it is a sample
+    // exceed the number of instances in this launch when it is a part or a sample
     if (!r) r = dev_reserve(c->b_costs, sizeof(int64_t) * (size_t)std::max<int64_t>(pk.cost_slots, 1));
-    if (!r) r = dev_reserve(c->b_ctrl, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(c->batch_blocks));
-    if (!r) r = dev_reserve(c->b_arcs, (size_t)batch_arc_stride(pk.arc_bytes) * (size_t)pk.blocks);
+    if (!r) r = dev_reserve(L.ctrl, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(c->batch_blocks));
+    if (!r) r = reserve_more(L.arcs, (size_t)batch_arc_stride(pk.arc_bytes) * (size_t)pk.blocks);
     if (!r) r = prepare_batch_subsets(c, st);
     if (r) return r;
     for (int32_t j = 0; j < pk.count; j++) {
-        BatchInst &d = pk.h_desc[j];
+        BatchInst &d = pk.desc[(size_t)j];
         if (d.orig < 0 || d.orig >= pk.cost_slots) return emv_fail(EMV_ERR_INTERNAL, "batch: cost slot out of range");
-        d.row_ptr = (const int32_t *)c->b_row.ptr + pk.row_off[(size_t)j];
-        d.adj = (const int2 *)c->b_adj.ptr + pk.arc_off[(size_t)j];
-        d.terms = (const int32_t *)c->b_term.ptr + pk.term_off[(size_t)j];
-        d.table = (int32_t *)c->b_table.ptr + pk.table_off[(size_t)j];
-        pk.desc[(size_t)j] = d;
+        d.row_ptr = (const int32_t *)L.row.ptr + pk.row_off[(size_t)j];
+        d.adj = (const int2 *)L.adj.ptr + pk.arc_off[(size_t)j];
+        d.terms = (const int32_t *)L.term.ptr + pk.term_off[(size_t)j];
+        d.table = (int32_t *)L.table.ptr + pk.table_off[(size_t)j];
+        pk.h_desc[j] = d;
     }
-    CUDA_TRY(cudaMemcpyAsync(c->b_row.ptr, pk.h_row, sizeof(int32_t) * (size_t)pk.rows, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(L.row.ptr, pk.h_row, sizeof(int32_t) * (size_t)pk.rows, cudaMemcpyHostToDevice, st));
     if (pk.arcs > 0)
-        CUDA_TRY(cudaMemcpyAsync(c->b_adj.ptr, pk.h_adj, sizeof(int2) * (size_t)pk.arcs, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(c->b_term.ptr, pk.h_term, sizeof(int32_t) * (size_t)pk.terms, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(c->b_desc.ptr, pk.h_desc, sizeof(BatchInst) * (size_t)pk.count, cudaMemcpyHostToDevice,
-                             st));
+        CUDA_TRY(cudaMemcpyAsync(L.adj.ptr, pk.h_adj, sizeof(int2) * (size_t)pk.arcs, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(L.term.ptr, pk.h_term, sizeof(int32_t) * (size_t)pk.terms, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(L.desc.ptr, pk.h_desc, sizeof(BatchInst) * (size_t)pk.count, cudaMemcpyHostToDevice, st));
     pk.t_upload_end = std::chrono::steady_clock::now();
     return EMV_OK;
 }
@@ -414,12 +510,13 @@ BatchArgs batch_args(emv_ctx *c, const BatchPack &pk)
 {
     BatchArgs a;
     std::memset(&a, 0, sizeof(a));  // padding included: the graph cache compares bytes
-    a.inst = (const BatchInst *)c->b_desc.ptr;
+    const BatchLane &L = c->blane[pk.lane];
+    a.inst = (const BatchInst *)L.desc.ptr;
     a.xs = (const uint32_t *)c->bxs.ptr;
     a.xs_off = (const int32_t *)c->bxs_off.ptr;
     a.costs = (int64_t *)c->b_costs.ptr;
-    a.ctl = (uint32_t *)c->b_ctrl.ptr;
-    a.scratch = (char *)c->b_arcs.ptr;
+    a.ctl = (uint32_t *)L.ctrl.ptr;
+    a.scratch = (char *)L.arcs.ptr;
     a.scratch_stride = batch_arc_stride(pk.arc_bytes);
     a.smem = RESIDENT_SMEM;
     std::copy(pk.end, pk.end + BATCH_SIZES, a.end);
@@ -427,15 +524,16 @@ BatchArgs batch_args(emv_ctx *c, const BatchPack &pk)
 }
 
 // Captures {control reset, persistent kernel} once per argument set and replays it.
-int batch_graph_launch(emv_ctx *c, const BatchArgs &a, int32_t blocks, cudaStream_t st)
+int batch_graph_launch(emv_ctx *c, int32_t lane, const BatchArgs &a, int32_t blocks, cudaStream_t st)
 {
+    BatchLane &L = c->blane[lane];
     int r = batch_kernel_setup(c);
     if (r) return r;
-    static_assert(sizeof(BatchArgs) <= sizeof(c->bgraph_args), "graph key too small");
-    const bool same = c->bgraph_exec && c->bgraph_blocks == blocks && std::memcmp(c->bgraph_args, &a, sizeof(a)) == 0;
+    static_assert(sizeof(BatchArgs) <= sizeof(L.graph_args), "graph key too small");
+    const bool same = L.graph && L.graph_blocks == blocks && std::memcmp(L.graph_args, &a, sizeof(a)) == 0;
     if (!same) {
-        if (c->bgraph_exec) cudaGraphExecDestroy(c->bgraph_exec);
-        c->bgraph_exec = nullptr;
+        if (L.graph) cudaGraphExecDestroy(L.graph);
+        L.graph = nullptr;
         cudaStream_t cap;
         CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
         cudaGraph_t g = nullptr;
@@ -450,17 +548,17 @@ int batch_graph_launch(emv_ctx *c, const BatchArgs &a, int32_t blocks, cudaStrea
             cudaGetLastError();
             return emv_fail(EMV_ERR_CUDA, "batch graph capture: %s", cudaGetErrorString(e));
         }
-        e = cudaGraphInstantiate(&c->bgraph_exec, g, 0);
+        e = cudaGraphInstantiate(&L.graph, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) {
             cudaGetLastError();
-            c->bgraph_exec = nullptr;
+            L.graph = nullptr;
             return emv_fail(EMV_ERR_CUDA, "batch graph instantiate: %s", cudaGetErrorString(e));
         }
-        std::memcpy(c->bgraph_args, &a, sizeof(a));
-        c->bgraph_blocks = blocks;
+        std::memcpy(L.graph_args, &a, sizeof(a));
+        L.graph_blocks = blocks;
     }
-    CUDA_TRY(cudaGraphLaunch(c->bgraph_exec, st));
+    CUDA_TRY(cudaGraphLaunch(L.graph, st));
     return EMV_OK;
 }
 
@@ -477,7 +575,11 @@ int time_sample(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t>
     BatchPack pk;
     const int32_t blocks = std::max<int32_t>(1, ((int32_t)ids.size() + 3) / 4);
     int r = batch_kernel_setup(c);
-    if (!r) r = batch_pack(c, inst, ids, false, blocks, pk);
+    if (!r) {
+        const BatchOrder ord = batch_order(c, inst, ids, false, blocks);
+        r = batch_layout(c, inst, ord, 0, (int32_t)ids.size(), false, blocks, pk);
+    }
+    if (!r) r = batch_fill(c, inst, pk, nullptr);
     if (!r) r = batch_upload(c, pk, st);
     if (r) return r;
     BatchArgs a = batch_args(c, pk);

@@ -2,12 +2,14 @@
 #pragma once
 
 #include <chrono>
+#include <functional>
 #include <vector>
 
 #include "emv_batch_types.h"
 #include "emv_solver.h"
 
 struct BatchPack {
+    int32_t lane = 0;                  // emv_ctx::blane
     std::vector<emv::BatchInst> desc;  // in launch order
     std::vector<int64_t> row_off, arc_off, term_off, table_off;  // into the packed device buffers
     int64_t rows = 0, arcs = 0, terms = 0, table_words = 0;
@@ -42,14 +44,25 @@ void batch_plan(const std::vector<double> &work, const std::vector<int64_t> &sta
 void batch_shape(const emv_ctx *c, emv::BatchInst &d);
 int prepare_batch_subsets(emv_ctx *c, cudaStream_t st);
 int batch_kernel_setup(emv_ctx *c);
-// whole: solve the subsets of all terminals (the tables are wanted), else
-// those the costs need.  blocks: CTAs of the launch that will take the pack.
-int batch_pack(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &ids, bool whole, int32_t blocks,
-               BatchPack &pk);
+// Team sizes and launch order of the instances ids[] (blocks > 0: single-CTA
+// teams in the given order, for a launch of that many CTAs).  whole: solve the
+// subsets of all terminals (the tables are wanted), else those the costs need.
+struct BatchOrder {
+    std::vector<int32_t> ids, size;  // in launch order
+    std::vector<double> work;
+};
+BatchOrder batch_order(const emv_ctx *c, const emv_instance *inst, const std::vector<int32_t> &ids, bool whole,
+                       int32_t blocks);
+// Lays out entries [from, to) of an order for one launch, and reserves staging.
+int batch_layout(emv_ctx *c, const emv_instance *inst, const BatchOrder &ord, int32_t from, int32_t to, bool whole,
+                 int32_t blocks, BatchPack &pk);
+// Fills the staging from the instances; check(i) is called for each before it
+// is read and says whether to.
+int batch_fill(emv_ctx *c, const emv_instance *inst, BatchPack &pk, const std::function<bool(int32_t)> &check);
 int batch_upload(emv_ctx *c, BatchPack &pk, cudaStream_t st);
 emv::BatchArgs batch_args(emv_ctx *c, const BatchPack &pk);
 int launch_batch(emv_ctx *c, const emv::BatchArgs &a, int32_t blocks, cudaStream_t st);
-int batch_graph_launch(emv_ctx *c, const emv::BatchArgs &a, int32_t blocks, cudaStream_t st);
+int batch_graph_launch(emv_ctx *c, int32_t lane, const emv::BatchArgs &a, int32_t blocks, cudaStream_t st);
 // Bytes of BatchArgs::scratch for every CTA, from the largest sliced arcs.
 int64_t batch_arc_stride(int64_t arc_bytes);
 // CTAs for instances whose team sizes sum to ctas.

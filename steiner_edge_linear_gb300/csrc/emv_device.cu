@@ -144,8 +144,7 @@ extern "C" int emv_destroy(emv_ctx *c)
     cudaDeviceSynchronize();
     for (DevBuf *b : {&c->ctrl, &c->stat, &c->lvlmax, &c->gscan, &c->shadow, &c->scratch, &c->act, &c->adj, &c->stamp, &c->hubs, &c->terms, &c->g_all,
                       &c->table, &c->tb_edges, &c->tb_out, &c->tb_work, &c->res_arcs, &c->res_out,
-                      &c->bxs, &c->bxs_off, &c->b_row, &c->b_adj, &c->b_term, &c->b_desc, &c->b_table, &c->b_costs,
-                      &c->b_ctrl, &c->b_arcs})
+                      &c->bxs, &c->bxs_off, &c->b_costs})
         dev_release(*b);
     for (KPlan *p : c->kplans) {
         if (!p) continue;
@@ -156,8 +155,14 @@ extern "C" int emv_destroy(emv_ctx *c)
         if (c->ev[i]) cudaEventDestroy(c->ev[i]);
     for (int i = 0; i <= EMV_MAX_K; i++)
         if (c->evmax[i]) cudaEventDestroy(c->evmax[i]);
-    if (c->bgraph_exec) cudaGraphExecDestroy(c->bgraph_exec);
-    if (c->bstage) cudaFreeHost(c->bstage);
+    for (BatchLane &L : c->blane) {
+        for (DevBuf *b : {&L.row, &L.adj, &L.term, &L.desc, &L.table, &L.ctrl, &L.arcs}) dev_release(*b);
+        if (L.graph) cudaGraphExecDestroy(L.graph);
+        if (L.stage) cudaFreeHost(L.stage);
+    }
+    for (cudaEvent_t e : c->bev)
+        if (e) cudaEventDestroy(e);
+    if (c->bstream) cudaStreamDestroy(c->bstream);
     if (c->g_stage) cudaFreeHost(c->g_stage);
     if (c->h_dist) cudaFreeHost(c->h_dist);
     if (c->pinned) cudaFreeHost(c->pinned);

@@ -53,6 +53,18 @@ struct KPlan {
     std::vector<std::vector<StreamGroup>> mstream_groups;  // per level (none = not streamed)
 };
 
+// Buffers of one launch of the batched kernel.  A large batch runs as two
+// launches, so that the host packs the second while the first is on the GPU.
+constexpr int BATCH_LANES = 2;
+struct BatchLane {
+    DevBuf row, adj, term, desc, table, ctrl, arcs;
+    void *stage = nullptr;         // pinned staging of the packed instances
+    size_t stage_bytes = 0;
+    cudaGraphExec_t graph = nullptr;
+    char graph_args[160] = {};     // BatchArgs of the captured graph
+    int32_t graph_blocks = 0;      // and its CTAs
+};
+
 struct emv_ctx {
     int device = 0;
     int sms = 0;
@@ -95,12 +107,10 @@ struct emv_ctx {
     DevBuf bxs, bxs_off;           // subset lists of every k <= BATCH_KMAX
     bool bxs_ready = false;
     int batch_blocks = 0;
-    DevBuf b_row, b_adj, b_term, b_desc, b_table, b_costs, b_ctrl, b_arcs;
-    void *bstage = nullptr;        // pinned staging of the packed batch
-    size_t bstage_bytes = 0;
-    cudaGraphExec_t bgraph_exec = nullptr;
-    char bgraph_args[160] = {};    // BatchArgs of the captured graph
-    int32_t bgraph_blocks = 0;     // and its CTAs
+    BatchLane blane[BATCH_LANES];
+    DevBuf b_costs;                // by the caller's instance index
+    cudaStream_t bstream = nullptr;  // of the second lane
+    cudaEvent_t bev[2] = {};       // the caller's stream reached, the second lane done
     int32_t tune_rcap[BATCH_CLASSES] = {};
     int32_t tune_mw[BATCH_CLASSES] = {};  // merge vertex-block width per class (0: default 1)
 };

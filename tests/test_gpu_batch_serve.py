@@ -212,3 +212,28 @@ def test_batch_teams_whole_tables(emv, orc, count):
         want, cost = orc.emv_table(g.n, g.row_ptr, g.col, g.w, g.terminals, threads=8)
         assert np.array_equal(t, want)
         assert c == (cost if g.k > 1 else (1 << 63) - 1)
+
+
+def test_batch_in_two_launches(emv):
+    """A large batch is packed and launched in two parts: costs equal single
+    solves in the caller's order, a faulty instance of either part is reported
+    by its index (the lowest one), and the context solves again."""
+    graphs = [emv.Csr.from_stp(emv.StpInstance.mixed(5, i, nmin=64, nmax=400, kmin=4, kmax=7)) for i in range(900)]
+    with emv.Solver(0) as s:
+        costs, st = s.batch_solve(graphs)
+        again, _ = s.batch_solve(graphs)
+        assert np.array_equal(costs, again) and st["work_items"] == 900
+        for i in range(0, 900, 75):
+            assert s.solve(graphs[i]).cost == costs[i]
+        order = sorted(range(900), key=lambda i: -(graphs[i].n * 3 ** graphs[i].k))
+        for faulty in ([order[0]], [order[-1]], [order[-1], order[0]], [17, 800, 400]):
+            bad = list(graphs)
+            for i in faulty:
+                g = graphs[i]
+                col = g.col.copy()
+                col[3] = g.n
+                bad[i] = emv.Csr(g.n, g.row_ptr, col, g.w, g.terminals)
+            with pytest.raises(emv.EmvError) as ei:
+                s.batch_solve(bad)
+            assert ei.value.status == 1 and f"instance {min(faulty)}:" in str(ei.value)
+        assert np.array_equal(s.batch_solve(graphs)[0], costs)
