@@ -142,7 +142,7 @@ extern "C" int emv_destroy(emv_ctx *c)
     if (!c) return EMV_OK;
     cudaSetDevice(c->device);
     cudaDeviceSynchronize();
-    for (DevBuf *b : {&c->ctrl, &c->stat, &c->lvlmax, &c->gscan, &c->shadow, &c->scratch, &c->act, &c->adj, &c->stamp, &c->hubs, &c->terms, &c->g_all,
+    for (DevBuf *b : {&c->ctrl, &c->stat, &c->lvlmax, &c->gscan, &c->shadow, &c->scratch, &c->act, &c->adj, &c->mark, &c->hubs, &c->terms, &c->g_all,
                       &c->table, &c->tb_edges, &c->tb_out, &c->tb_work, &c->res_arcs, &c->res_out,
                       &c->bxs, &c->bxs_off, &c->b_costs})
         dev_release(*b);
@@ -199,7 +199,8 @@ int launch_relax(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n,
                  int64_t shadow_ld = 0)
 {
     RelaxArgs a;
-    a.stamp = (int32_t *)c->stamp.ptr;
+    a.mark = (int2 *)c->mark.ptr;
+    a.high = (int32_t *)(a.mark + n);
     a.row_ptr = row_ptr;
     a.adj = adj;
     a.n = n;
@@ -221,13 +222,7 @@ int launch_relax(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n,
     a.shadow = shadow;
     a.shadow_ld = shadow_ld;
     const int32_t words = u16 ? (nrows + 1) / 2 : nrows;  // int32 words a vertex record needs
-    // Without stamps a sweep pulls every arc, also from heads that did not
-    // change: worth it once most heads changed while the records are L2 hits
-    // (from 75 % of the vertices), only at 97 % when they stream from HBM.
     const int wi = words <= 32 ? 0 : words <= 64 ? 1 : words <= 128 ? 2 : words <= 160 ? 3 : 4;
-    const int64_t rec_words = (int64_t)32 * (wi == 3 ? 5 : 1 << (wi < 3 ? wi : 3));
-    const bool resident = (int64_t)n * rec_words * 4 <= c->l2_bytes * 3 / 4;
-    a.pull_all_min = n - n / (resident ? 4 : 32);
     const int vi = wi + (u16 ? 5 : 0) + (c->relax_nhubs > 0 ? 10 : 0);
     a.hubs = (const int32_t *)c->hubs.ptr;
     a.nhubs = c->relax_nhubs;
@@ -296,7 +291,7 @@ int reserve_relax(emv_ctx *c, int32_t n)
     const size_t npad = ((size_t)n + 31) / 32 * 32;
     int st = dev_reserve(c->scratch, npad * CHUNK_ROWS * sizeof(int32_t));
     if (!st) st = dev_reserve(c->act, 2 * (((size_t)n + 255) / 256 * 256));
-    if (!st) st = dev_reserve(c->stamp, sizeof(int32_t) * (size_t)n);
+    if (!st) st = dev_reserve(c->mark, (sizeof(int2) + sizeof(int32_t)) * (size_t)n);
     return st;
 }
 

@@ -40,9 +40,9 @@ struct RelaxArgs {
     uint32_t *ctrl;         // C_WORDS words
     DevStat *stat;
     int32_t max_sweeps;
-    int32_t *stamp;         // n: last sweep in which the vertex changed (-1 none)
+    int2 *mark;             // n: last sweep in which the vertex changed (-1 none), lowest excess of its record
+    int32_t *high;          // n: highest excess of its record
     int32_t dense_min;      // a sweep after one with more changed vertices takes every vertex
-    int32_t pull_all_min;   // a sweep after one with at least this many changed vertices reads no stamps
     const int32_t *hubs;    // HUBS: the nhubs vertices of more than hub_min arcs
     int32_t nhubs;
     int32_t hub_min;
@@ -493,198 +493,248 @@ __global__ void __launch_bounds__(1024) k_merge_stream16(int32_t *__restrict__ t
     if (threadIdx.x == 0) atomicMax(level_max, s_max);
 }
 
-// A sweep that takes every vertex and pulls every arc (sweep 0, and the
-// sweeps after one that changed most vertices): the task loop of
-// relax_sweeps with the selection fixed at compile time -- no flag or stamp
-// reads, every arc of a vertex compacted -- so the compiler keeps none of the
-// other paths' state live around the gathers.  Clears this sweep's flags of
-// the warp's vertices; with flags_next, marks the neighbours of every changed
-// vertex for the next sweep.  Returns whether a record changed; counts the
-// changed vertices in *s_chg.
-template <int VEC, bool U16, bool HUBS, int GROUP, int TASK_V>
-__device__ __forceinline__ bool relax_pass_all(const RelaxArgs &a, int32_t vbeg, int32_t vend, int32_t s,
-                                               bool flags_next, uint8_t *cur, uint8_t *nxt, int2 *warcs,
-                                               unsigned *s_chg)
+// ------------------------------------------------------------ excesses
+//
+// Most arcs of a record cannot improve any of its rows: an arc (u, w) of v is
+// of use only where d_X[u] + w < d_X[v] for some row X, and random weights are
+// often as long as the distances' differences.  The excess of row X at a
+// vertex is d_X - c_X with any constant c_X; with the lowest excess low[u] and
+// the highest high[v] over the record's rows, low[u] + w >= high[v] rules the
+// arc out for all of them, without its 512-byte gather.  c_X is the row's mean
+// over 32 vertices spread over the graph, which brings the rows of a record
+// close together.  An arc is ruled out until u changes again: high[v] only
+// falls, and a change of u stamps it anew.
+// Visited arcs of a closure's 13 sweeps, per arc: 13.0 -> 4.6 at n = 10^5,
+// degree 20, weights to 100 (2.0 would be enough); 14.6 -> 11.9 at n = 2^17,
+// degree 8, weights to 1000 (5.6).  More bounds a vertex, one for each part of
+// the rows, rule out little more: 4.4 and 11.5 with 4, 4.1 and 11.0 with 16.
+
+// Minus c_X of every row in the record's layout, as it enters the highest
+// (neg) and the lowest (neg + 32 * VEC) excess.  Rows past the chunk's get
+// what leaves the one as low and the other as high as can be.
+template <int VEC, bool U16> __device__ __forceinline__ void relax_offsets(const RelaxArgs &a, int32_t *neg)
 {
-    using V = typename IVec<VEC>::T;
-    const int lane = threadIdx.x & 31;
-    bool any = false;
-    for (int32_t base = vbeg; base < vend; base += TASK_V) {
-        const int32_t v = base + lane;
-        const bool mine = lane < TASK_V && v < vend;
-        unsigned act = __ballot_sync(FULL, mine);
-        const int32_t rp0 = mine ? __ldg(a.row_ptr + v) : 0;
-        const int32_t rp1 = mine ? __ldg(a.row_ptr + v + 1) : 0;
-        if (HUBS) {  // relax_hubs takes these
-            const bool hub = rp1 - rp0 > a.hub_min;
-            act &= ~__ballot_sync(FULL, hub);
-            if (mine && !hub) cur[v] = 0;
-            if (!act) continue;
-        } else if (mine) {
-            cur[v] = 0;
-        }
-        int j = __ffs(act) - 1;
-        act &= act - 1;
-        int32_t beg = __shfl_sync(FULL, rp0, j), end = __shfl_sync(FULL, rp1, j);
-        int2 arc = beg + lane < end ? __ldg(a.adj + beg + lane) : make_int2(0, 0);
-        for (;;) {
-            const int32_t vv = base + j;
-            const V old = rec_ld<VEC>(a.scratch, vv, lane);
-            V acc = old;
-            for (int32_t e0 = beg;;) {
-                const int cnt = min(32, end - e0);
-                // the arcs in this warp's slots (U16: clamped weight in both halves)
-                if (lane < cnt)
-                    warcs[lane] = U16 ? make_int2(arc.x, (int32_t)(min((uint32_t)arc.y, 32768u) * 0x10001u)) : arc;
-                __syncwarp();
-                for (int i = 0; i < cnt; i += GROUP) {
-                    V val[GROUP];
-                    int32_t wt[GROUP];
-#pragma unroll
-                    for (int g = 0; g < GROUP; g++) {
-                        const bool ok = i + g < cnt;
-                        const int2 aw = warcs[(i + g) & 31];  // slots past cnt hold stale arcs: not used
-                        wt[g] = ok ? aw.y : 0;
-                        val[g] = ok ? rec_ld<VEC>(a.scratch, aw.x, lane) : vsplat<V>(U16 ? -1 : INF);
-                    }
-#pragma unroll
-                    for (int g = 0; g < GROUP; g++)
-                        acc = U16 ? vaddmin16(val[g], wt[g], acc) : vmin(acc, vadd(val[g], wt[g]));
-                }
-                __syncwarp();
-                e0 += 32;
-                if (e0 >= end) break;
-                arc = e0 + lane < end ? __ldg(a.adj + e0 + lane) : make_int2(0, 0);  // high degree: next 32 arcs
-            }
-            // the next vertex of the task before finishing this one
-            const int32_t cbeg = beg, cend = end;
-            const bool more = act != 0;
-            if (more) {
-                j = __ffs(act) - 1;
-                act &= act - 1;
-                beg = __shfl_sync(FULL, rp0, j);
-                end = __shfl_sync(FULL, rp1, j);
-                arc = beg + lane < end ? __ldg(a.adj + beg + lane) : make_int2(0, 0);
-            }
-            const bool dec = U16 ? vne(acc, old) : vlt(acc, old);
-            if (dec) rec_st<VEC>(a.scratch, vv, lane, acc);
-            if (__ballot_sync(FULL, dec)) {
-                any = true;
-                if (lane == 0) {
-                    __stcg(a.stamp + vv, s);
-                    atomicAdd(s_chg, 1u);
-                }
-                if (flags_next)
-                    for (int32_t e = cbeg + lane; e < cend; e += 32) nxt[__ldg(&a.adj[e].x)] = 1;
-            }
-            if (!more) break;
+    constexpr int R = 32 * VEC, NW = RELAX_THREADS / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t v = (int64_t)a.n * lane / 32;
+#pragma unroll 4
+    for (int r = warp; r < (U16 ? 2 * R : R); r += NW) {
+        const bool real = r < a.nrows;
+        const int32_t x = real ? __ldcg(a.table + (int64_t)__ldg(a.rows + r) * a.ld + v) : 0;
+        const int32_t c = __reduce_add_sync(FULL, x >> 5) + (__reduce_add_sync(FULL, x & 31) >> 5);
+        if (lane) continue;
+        if (U16) {
+            reinterpret_cast<int16_t *>(neg)[2 * (r % R) + r / R] = (int16_t)(real ? -c : -32768);
+            reinterpret_cast<int16_t *>(neg + R)[2 * (r % R) + r / R] = (int16_t)(real ? -c : 32767);
+        } else {
+            neg[r] = real ? -c : (int32_t)0x80000000;
+            neg[R + r] = real ? -c : INF - 1;
         }
     }
-    return any;
 }
 
-// The other sweeps: flags (or, in a dense sweep, every vertex) select the
-// vertices, stamps the arcs (unless pull_all).  A vertex is taken when its
-// flag in `flags` is set; with clear the flag is cleared first.  Returns
+// x: highest, y: lowest excess of some words of a record.  16-bit values are
+// at most 32767 here, so a difference of two fits 16 bits.
+template <bool U16> __device__ __forceinline__ int2 excess_none()
+{
+    return U16 ? make_int2((int32_t)0x80008000, 0x7fff7fff) : make_int2((int32_t)0x80000000, 0x7fffffff);
+}
+template <bool U16> __device__ __forceinline__ int2 excess_word(int2 b, int32_t d, int32_t nh, int32_t nl)
+{
+    if (U16)
+        return make_int2((int32_t)__viaddmax_s16x2((uint32_t)d, (uint32_t)nh, (uint32_t)b.x),
+                         (int32_t)__viaddmin_s16x2((uint32_t)d, (uint32_t)nl, (uint32_t)b.y));
+    return make_int2(__viaddmax_s32(d, nh, b.x), __viaddmin_s32(d, nl, b.y));
+}
+// Over the warp.
+template <bool U16> __device__ __forceinline__ int2 excess_reduce(int2 b)
+{
+    if (U16) b = make_int2(max((int32_t)(int16_t)b.x, b.x >> 16), min((int32_t)(int16_t)b.y, b.y >> 16));
+    return make_int2(__reduce_max_sync(FULL, b.x), __reduce_min_sync(FULL, b.y));
+}
+// Of a record held by a warp (the lanes' shares; rec_ld's layout).
+template <int VEC, bool U16>
+__device__ __forceinline__ int2 excess_of(typename IVec<VEC>::T x, const int32_t *neg, int lane)
+{
+    const int32_t *w = reinterpret_cast<const int32_t *>(&x);
+    int2 b = excess_none<U16>();
+    if constexpr (VEC >= 4) {
+#pragma unroll
+        for (int q = 0; q + 4 <= VEC; q += 4) {
+            const int at = VEC == 8 ? 8 * lane + q : 4 * lane;
+            const int4 h = *reinterpret_cast<const int4 *>(neg + at), l = *reinterpret_cast<const int4 *>(neg + 32 * VEC + at);
+            b = excess_word<U16>(b, w[q], h.x, l.x);
+            b = excess_word<U16>(b, w[q + 1], h.y, l.y);
+            b = excess_word<U16>(b, w[q + 2], h.z, l.z);
+            b = excess_word<U16>(b, w[q + 3], h.w, l.w);
+        }
+        if constexpr (VEC == 5) b = excess_word<U16>(b, w[4], neg[128 + lane], neg[160 + 128 + lane]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < VEC; q++)
+            b = excess_word<U16>(b, w[q], neg[VEC * lane + q], neg[32 * VEC + VEC * lane + q]);
+    }
+    return excess_reduce<U16>(b);
+}
+
+constexpr int RELAX_LIST = 128;             // at most 64 new entries beside 2 * GROUP - 1 waiting ones
+constexpr int32_t RELAX_SELF = -1;          // in place of a weight: the vertex's own record
+// A warp's working memory in shared memory.
+struct RelaxWarp {
+    int4 win[32];             // the window's vertices with arcs: vertex, first arc minus start, start, highest excess
+    int4 list[RELAX_LIST / 2];  // ring of records to read, two an element: an arc (head, weight), or (vertex, RELAX_SELF)
+};
+
+// A pass over the warp's vertices.  Flags (or, in a dense sweep, every vertex)
+// select the vertices, stamps and excesses the arcs.  A vertex is taken when
+// its flag in `flags` is set; with clear the flag is cleared first.  Returns
 // whether a record changed; counts changed vertices in *s_chg.
-template <int VEC, bool U16, bool HUBS, int GROUP, int TASK_V>
-__device__ __forceinline__ bool relax_pass_sel(const RelaxArgs &a, int32_t vbeg, int32_t vend, int32_t s, bool dense,
-                                               bool dense_next, bool pull_all, uint8_t *flags, bool clear,
-                                               uint8_t *nxt, int2 *warcs, unsigned *s_chg)
+//
+// The arcs of up to 32 taken vertices are looked at one after another, 32 at a
+// time whatever their vertices, two steps ahead: while the arcs of one step are
+// selected, the marks of the next and the arcs after those are on their way.
+// Selected arcs go to a ring, after an entry for the vertex's own record where
+// they are its first, and GROUP records of the ring are always being read: the
+// loads of a vertex do not wait for those of the vertex before.  (A vertex at
+// a time, with the next one's arcs and marks requested early, a sweep at n =
+// 10^5 was bound by its chain of dependent loads: 46 us, 2.2 us a vertex.)
+template <int VEC, bool U16, bool HUBS, int GROUP>
+__device__ __forceinline__ bool relax_pass(const RelaxArgs &a, int32_t vbeg, int32_t vend, int32_t s, bool dense,
+                                           bool dense_next, uint8_t *flags, bool clear, uint8_t *nxt, RelaxWarp &ws,
+                                           const int32_t *neg, unsigned *s_chg)
 {
     using V = typename IVec<VEC>::T;
     const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1;
-    bool any = false;
-    for (int32_t base = vbeg; base < vend; base += TASK_V) {
+    const unsigned lt = (1u << lane) - 1, le = lt << 1 | 1u;
+    V val[GROUP], acc = vsplat<V>(0), old = acc;
+    int32_t cur = 0, done = 0, made = 0;  // vertex being reduced; entries used, entries listed
+    unsigned changed = 0;
+#pragma unroll
+    for (int g = 0; g < GROUP; g++) val[g] = acc;
+    auto finish = [&]() {
+        const bool dec = U16 ? vne(acc, old) : vlt(acc, old);
+        if (!__ballot_sync(FULL, dec)) return;
+        if (dec) rec_st<VEC>(a.scratch, cur, lane, acc);
+        const int2 b = excess_of<VEC, U16>(acc, neg, lane);
+        if (lane == 0) {
+            __stcg(a.mark + cur, make_int2(s, b.y));
+            __stcg(a.high + cur, b.x);
+        }
+        changed++;
+        if (!dense_next) {
+            const int32_t end = __ldg(a.row_ptr + cur + 1);
+            for (int32_t e = __ldg(a.row_ptr + cur) + lane; e < end; e += 32) nxt[__ldg(&a.adj[e].x)] = 1;
+        }
+    };
+    int2 *list = reinterpret_cast<int2 *>(ws.list);
+    // the GROUP entries from k (a multiple of GROUP) on
+    auto fetch = [&](int32_t k) {
+        const int4 *e = ws.list + (k & (RELAX_LIST - 1)) / 2;
+#pragma unroll
+        for (int g = 0; g < GROUP; g += 2) {
+            const int4 x = e[g / 2];
+            val[g] = rec_ld<VEC>(a.scratch, x.x, lane);
+            val[g + 1] = rec_ld<VEC>(a.scratch, x.z, lane);
+        }
+    };
+    auto use = [&](int32_t vertex, int32_t weight, const V &x) {
+        if (weight == RELAX_SELF) {
+            finish();
+            cur = vertex;
+            old = acc = x;
+        } else {
+            acc = U16 ? vaddmin16(x, weight, acc) : vmin(acc, vadd(x, weight));
+        }
+    };
+    // uses all entries but the last GROUP to 2 * GROUP - 1, the first GROUP of which are being read
+    auto drain = [&]() {
+        while (made - done >= 2 * GROUP) {
+            const int4 *now = ws.list + (done & (RELAX_LIST - 1)) / 2;
+            const int4 *then = ws.list + ((done + GROUP) & (RELAX_LIST - 1)) / 2;
+#pragma unroll
+            for (int g = 0; g < GROUP; g += 2) {
+                const int4 e = now[g / 2], next = then[g / 2];
+                use(e.x, e.y, val[g]);
+                val[g] = rec_ld<VEC>(a.scratch, next.x, lane);
+                use(e.z, e.w, val[g + 1]);
+                val[g + 1] = rec_ld<VEC>(a.scratch, next.z, lane);
+            }
+            done += GROUP;
+        }
+    };
+    auto listed = [&](int32_t count) {
+        __syncwarp();
+        if (made < GROUP && made + count >= GROUP) fetch(0);
+        made += count;
+        drain();
+        __syncwarp();
+    };
+    for (int32_t base = vbeg; base < vend; base += 32) {
         const int32_t v = base + lane;
-        const bool mine = lane < TASK_V && v < vend;
+        const bool mine = v < vend;
         bool f = mine && (dense || __ldcg(flags + v) != 0);
-        unsigned act = __ballot_sync(FULL, f);
-        if (!act) continue;
+        if (!__any_sync(FULL, f)) continue;
         const int32_t rp0 = mine ? __ldg(a.row_ptr + v) : 0;
         const int32_t rp1 = mine ? __ldg(a.row_ptr + v + 1) : 0;
-        if (HUBS) {  // relax_hubs takes these
-            f = f && rp1 - rp0 <= a.hub_min;
-            act = __ballot_sync(FULL, f);
-        }
+        const int32_t hv = mine ? __ldcg(a.high + v) : 0;
+        if (HUBS) f = f && rp1 - rp0 <= a.hub_min;  // relax_hubs takes the others
         if (f && clear) flags[v] = 0;
-        if (HUBS && !act) continue;
-        // first active vertex: bounds, first 32 arcs and their selection
-        int j = __ffs(act) - 1;
-        act &= act - 1;
-        int32_t beg = __shfl_sync(FULL, rp0, j), end = __shfl_sync(FULL, rp1, j);
-        int2 arc = make_int2(0, 0);
-        bool pull = false;
-        if (beg + lane < end) {
-            arc = __ldg(a.adj + beg + lane);
-            pull = pull_all || __ldcg(a.stamp + arc.x) >= s - 1;
-        }
-        for (;;) {
-            const int32_t vv = base + j;
-            const V old = rec_ld<VEC>(a.scratch, vv, lane);
-            V acc = old;
-            for (int32_t e0 = beg;;) {
-                const unsigned sel = __ballot_sync(FULL, pull);
-                const int cnt = __popc(sel);
-                // selected arcs compacted in this warp's slots (U16: clamped weight in both halves)
-                if (pull)
-                    warcs[__popc(sel & lt)] =
-                        U16 ? make_int2(arc.x, (int32_t)(min((uint32_t)arc.y, 32768u) * 0x10001u)) : arc;
-                __syncwarp();
-                for (int i = 0; i < cnt; i += GROUP) {
-                    V val[GROUP];
-                    int32_t wt[GROUP];
+        const int32_t deg = f ? rp1 - rp0 : 0;
+        int32_t start = deg;
 #pragma unroll
-                    for (int g = 0; g < GROUP; g++) {
-                        const bool ok = i + g < cnt;
-                        const int2 aw = warcs[(i + g) & 31];  // slots past cnt hold stale arcs: not used
-                        wt[g] = ok ? aw.y : 0;
-                        val[g] = ok ? rec_ld<VEC>(a.scratch, aw.x, lane) : vsplat<V>(U16 ? -1 : INF);
-                    }
-#pragma unroll
-                    for (int g = 0; g < GROUP; g++)
-                        acc = U16 ? vaddmin16(val[g], wt[g], acc) : vmin(acc, vadd(val[g], wt[g]));
-                }
-                __syncwarp();
-                e0 += 32;
-                if (e0 >= end) break;
-                pull = false;  // high-degree vertex: next 32 arcs
-                if (e0 + lane < end) {
-                    arc = __ldg(a.adj + e0 + lane);
-                    pull = pull_all || __ldcg(a.stamp + arc.x) >= s - 1;
-                }
-            }
-            // prefetch the next active vertex before finishing this one
-            const int32_t cbeg = beg, cend = end;
-            const bool more = act != 0;
-            if (more) {
-                j = __ffs(act) - 1;
-                act &= act - 1;
-                beg = __shfl_sync(FULL, rp0, j);
-                end = __shfl_sync(FULL, rp1, j);
-                pull = false;
-                arc = make_int2(0, 0);
-                if (beg + lane < end) {
-                    arc = __ldg(a.adj + beg + lane);
-                    pull = pull_all || __ldcg(a.stamp + arc.x) >= s - 1;
-                }
-            }
-            const bool dec = U16 ? vne(acc, old) : vlt(acc, old);
-            if (dec) rec_st<VEC>(a.scratch, vv, lane, acc);
-            if (__ballot_sync(FULL, dec)) {
-                any = true;
-                if (lane == 0) {
-                    __stcg(a.stamp + vv, s);
-                    atomicAdd(s_chg, 1u);
-                }
-                if (!dense_next)
-                    for (int32_t e = cbeg + lane; e < cend; e += 32) nxt[__ldg(&a.adj[e].x)] = 1;
-            }
-            if (!more) break;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t t = __shfl_up_sync(FULL, start, o);
+            if (lane >= o) start += t;
         }
+        const int32_t total = __shfl_sync(FULL, start, 31);
+        start -= deg;
+        const unsigned some = __ballot_sync(FULL, deg > 0);
+        if (deg > 0) ws.win[__popc(some & lt)] = make_int4(v, rp0 - start, start, hv);
+        __syncwarp();
+        int32_t before = -1;  // the last vertex whose arcs start before the step
+        auto request = [&](int32_t p0, int32_t &rank, int2 &arc) {
+            const unsigned at = (unsigned)(start - p0);
+            const unsigned starts = __reduce_or_sync(FULL, deg > 0 && at < 32 ? 1u << at : 0u);
+            rank = before + __popc(starts & le);
+            before += __popc(starts);
+            arc = p0 + lane < total ? __ldg(a.adj + ws.win[rank].y + p0 + lane) : make_int2(0, 0);
+        };
+        int32_t rank0 = 0, rank1 = 0, last = -1;  // last: the vertex of the last own entry
+        int2 arc0, arc1 = make_int2(0, 0);
+        request(0, rank0, arc0);
+        int2 mark0 = __ldcg(a.mark + arc0.x);
+        if (total > 32) request(32, rank1, arc1);
+        for (int32_t p0 = 0; p0 < total; p0 += 32) {
+            const int4 w = ws.win[rank0];
+            const bool pull = p0 + lane < total && mark0.x >= s - 1 && arc0.y + mark0.y < w.w;
+            const unsigned sel = __ballot_sync(FULL, pull);
+            // U16: clamped weight in both halves
+            const int2 entry = U16 ? make_int2(arc0.x, (int32_t)(min((uint32_t)arc0.y, 32768u) * 0x10001u)) : arc0;
+            const int32_t rank = rank0;
+            arc0 = arc1;
+            rank0 = rank1;
+            if (p0 + 32 < total) mark0 = __ldcg(a.mark + arc0.x);
+            if (p0 + 64 < total) request(p0 + 64, rank1, arc1);
+            if (!sel) continue;
+            const unsigned first = __ballot_sync(FULL, pull && rank != last && !(sel & lt & ~0u << max(w.z - p0, 0)));
+            const int32_t at = made + __popc(sel & lt) + __popc(first & le);
+            if (pull) list[at & (RELAX_LIST - 1)] = entry;
+            if (first >> lane & 1u) list[(at - 1) & (RELAX_LIST - 1)] = make_int2(w.x, RELAX_SELF);
+            last = __shfl_sync(FULL, rank, 31 - __clz(sel));
+            listed(__popc(sel) + __popc(first));
+        }
+        __syncwarp();
     }
-    return any;
+    if (made) {
+        // entries that change nothing (a vertex's own record again) until the last one is used
+        const int32_t more = (-made & (GROUP - 1)) + 2 * GROUP;
+        const int32_t any = list[(made - 1) & (RELAX_LIST - 1)].x;
+        __syncwarp();
+        if (lane < more) list[(made + lane) & (RELAX_LIST - 1)] = make_int2(any, RELAX_SELF);
+        listed(more);
+    }
+    if (lane == 0 && changed) atomicAdd(s_chg, changed);
+    return changed != 0;
 }
 
 // Stores a lane's share of a record into shared memory, in the record's layout.
@@ -700,13 +750,14 @@ template <> __device__ __forceinline__ void part_st<5>(int32_t *p, int lane, int
 
 // The sweep's share of the hubs (vertices of more than hub_min arcs): a block
 // takes every gridDim.x-th one, its warps 32 arcs each at a time, with the
-// selection of relax_pass_sel; the partial minima meet in shared memory
+// selection of relax_pass; the partial minima meet in shared memory
 // (part: 32 * VEC words a warp).  One warp walking a hub of 1000 arcs alone
 // bounded a sweep (45 us at n = 30 000, power-law degrees, against 18).
 template <int VEC, bool U16, int GROUP>
-__device__ __noinline__ bool relax_hubs(const RelaxArgs &a, int32_t s, bool dense, bool dense_next, bool pull_all,
-                                        uint8_t *cur, uint8_t *nxt, int2 *warcs, int32_t *part, unsigned *s_chg)
+__device__ __noinline__ bool relax_hubs(const RelaxArgs &a, int32_t s, bool dense, bool dense_next, uint8_t *cur,
+                                        uint8_t *nxt, int2 *warcs, int32_t *part, const int32_t *neg, unsigned *s_chg)
 {
+    __shared__ int2 s_excess[VEC];
     using V = typename IVec<VEC>::T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1;
@@ -714,6 +765,7 @@ __device__ __noinline__ bool relax_hubs(const RelaxArgs &a, int32_t s, bool dens
     for (int32_t h = blockIdx.x; h < a.nhubs; h += gridDim.x) {
         const int32_t v = __ldg(a.hubs + h);
         const bool take = dense || __ldcg(cur + v) != 0;
+        const int32_t high = __ldcg(a.high + v);
         __syncthreads();  // all have read the flag; the partial minima of the hub before are used
         if (!take) continue;
         if (threadIdx.x == 0) cur[v] = 0;
@@ -724,7 +776,8 @@ __device__ __noinline__ bool relax_hubs(const RelaxArgs &a, int32_t s, bool dens
             bool pull = false;
             if (e0 + lane < end) {
                 arc = __ldg(a.adj + e0 + lane);
-                pull = pull_all || __ldcg(a.stamp + arc.x) >= s - 1;
+                const int2 m = __ldcg(a.mark + arc.x);
+                pull = m.x >= s - 1 && arc.y + m.y < high;
             }
             const unsigned sel = __ballot_sync(FULL, pull);
             const int cnt = __popc(sel);
@@ -760,11 +813,17 @@ __device__ __noinline__ bool relax_hubs(const RelaxArgs &a, int32_t s, bool dens
             }
             dec = x != old;
             if (dec) __stcg(word, x);
+            const int2 b = excess_reduce<U16>(
+                excess_word<U16>(excess_none<U16>(), x, neg[threadIdx.x], neg[32 * VEC + threadIdx.x]));
+            if (lane == 0) s_excess[warp] = b;
         }
         if (__syncthreads_or(dec)) {
             any = true;
             if (threadIdx.x == 0) {
-                __stcg(a.stamp + v, s);
+                int2 b = s_excess[0];
+                for (int q = 1; q < VEC; q++) b = make_int2(max(b.x, s_excess[q].x), min(b.y, s_excess[q].y));
+                __stcg(a.mark + v, make_int2(s, b.y));
+                __stcg(a.high + v, b.x);
                 atomicAdd(s_chg, 1u);
             }
             if (!dense_next)
@@ -776,17 +835,13 @@ __device__ __noinline__ bool relax_hubs(const RelaxArgs &a, int32_t s, bool dens
 
 // Frontier sweeps over one chunk (phase B of k_relax).  A warp owns a
 // contiguous range of n / W vertices (W warps in the grid, so the shares
-// differ by one vertex at most) and takes them TASK_V at a time: it
-// reads their active flags and CSR bounds with one load each, and
-// for every active vertex pulls min over its arcs (u, w) of rec[u] + w with
-// coalesced 128*VEC-byte gathers -- only from heads stamped as changed in the
-// previous sweep (a head that last changed earlier was already pulled when
-// that change marked this vertex active).  The selected arcs of a window are
-// compacted into the warp's shared-memory slots, so the gather loop reads one
-// (head, weight) pair per arc instead of searching the selection mask.  The
-// arcs and stamps of the next active vertex are requested before the current
-// one's record is stored.  Sweeps that take every vertex and pull every arc
-// run relax_pass_all, the others relax_pass_sel.  Only the owner writes a
+// differ by one vertex at most; half of them dealt out in windows of 4 or 8 to
+// whoever is done: 6 % slower, the windows' first loads cost more than the
+// wait for the last warp); for every active vertex it pulls min over its
+// arcs (u, w) of rec[u] + w with coalesced 128*VEC-byte gathers -- only from
+// heads stamped as changed in the previous sweep (a head that last changed
+// earlier was already pulled when that change marked this vertex active), and
+// of those only the arcs that the excesses leave.  Only the owner writes a
 // record and values only decrease, so no atomics are needed.  Returns the
 // number of sweeps, or -1 after an error (recorded).
 //
@@ -795,18 +850,15 @@ __device__ __noinline__ bool relax_hubs(const RelaxArgs &a, int32_t s, bool dens
 // 32767; the arc weight is then clamped to 32768, so a value plus a weight
 // stays below 2^16, and a clamped sum (at least 32768) never beats a value.
 template <int VEC, bool U16, bool HUBS>
-__device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok, int32_t *part)
+__device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok, RelaxWarp *warps, int32_t *part, const int32_t *neg)
 {
-    constexpr int GROUP = VEC == 8 ? 2 : VEC >= 4 ? 4 : 8;  // gathers in flight per group
-    constexpr int TASK_V = 8;
+    constexpr int GROUP = VEC == 8 ? 2 : 4;  // gathers in flight
     const int32_t n = a.n;
     const int32_t gw = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int32_t nwg = (int32_t)((gridDim.x * blockDim.x) >> 5);
-    // each warp owns a contiguous range of n / (warps) vertices, scanned TASK_V at a time
     const int32_t vbeg = (int32_t)((int64_t)n * gw / nwg), vend = (int32_t)((int64_t)n * (gw + 1) / nwg);
     volatile uint32_t *vctrl = a.ctrl;
-    __shared__ int2 s_arcs[RELAX_THREADS / 32][32];
-    int2 *warcs = s_arcs[threadIdx.x >> 5];
+    RelaxWarp &ws = warps[threadIdx.x >> 5];
     __shared__ unsigned s_chg;
     // read by thread 0 after each sweep's barrier: [0] the sweep changed a
     // record, [1] its changed count, [2] the count of the sweep before
@@ -835,18 +887,11 @@ __device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok, int32_t *part)
                                       ? (uint32_t)((uint64_t)prev_chg * prev_chg / prev2_chg)
                                       : prev_chg;
         const bool dense_next = pred_chg > (uint32_t)a.dense_min;
-        // after a sweep that changed most vertices, pull every arc without reading stamps
-        const bool pull_all = prev_chg >= (uint32_t)a.pull_all_min;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             vctrl[C_SLOT0 + (s + 1) % 3] = 0;
             vctrl[C_CNT0 + (s + 1) % 4] = 0;
         }
-        bool any = false;
-        if (dense && pull_all)
-            any = relax_pass_all<VEC, U16, HUBS, GROUP, TASK_V>(a, vbeg, vend, s, !dense_next, cur, nxt, warcs, &s_chg);
-        else
-            any = relax_pass_sel<VEC, U16, HUBS, GROUP, TASK_V>(a, vbeg, vend, s, dense, dense_next, pull_all, cur, true,
-                                                          nxt, warcs, &s_chg);
+        bool any = relax_pass<VEC, U16, HUBS, GROUP>(a, vbeg, vend, s, dense, dense_next, cur, true, nxt, ws, neg, &s_chg);
         // A sparse sweep whose successor is sparse also takes, once, the vertices
         // already marked for the next sweep (marked by changes earlier in this
         // sweep), so a change travels two arcs per sweep in the frontier's tail.
@@ -854,9 +899,9 @@ __device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok, int32_t *part)
         // has made every change of this sweep visible, so a change this early
         // pass missed is still pulled there.
         if (!dense && !dense_next)
-            any |= relax_pass_sel<VEC, U16, HUBS, GROUP, TASK_V>(a, vbeg, vend, s, false, dense_next, pull_all, nxt, false,
-                                                           nxt, warcs, &s_chg);
-        if (HUBS) any |= relax_hubs<VEC, U16, GROUP>(a, s, dense, dense_next, pull_all, cur, nxt, warcs, part, &s_chg);
+            any |= relax_pass<VEC, U16, HUBS, GROUP>(a, vbeg, vend, s, false, dense_next, nxt, false, nxt, ws, neg, &s_chg);
+        if (HUBS) any |= relax_hubs<VEC, U16, GROUP>(a, s, dense, dense_next, cur, nxt, reinterpret_cast<int2 *>(ws.list),
+                                                    part, neg, &s_chg);
         any = __syncthreads_or(any);
         if (threadIdx.x == 0) {
             if (any) vctrl[C_SLOT0 + s % 3] = 1;
@@ -883,7 +928,7 @@ __device__ int32_t relax_sweeps(const RelaxArgs &a, int *s_ok, int32_t *part)
 // 32*VEC int32 words, word e = row e; U16: word e = rows e | (e + 32*VEC) << 16).
 // A tile is 32 vertices by all 32*VEC words, so a warp has all its row loads in
 // flight before one barrier.  Rows past the chunk's are INF (U16: 0, which
-// no sweep lowers).  Also resets the active flags and stamps.
+// no sweep lowers).  Also sets the active flags, stamps and excesses.
 template <int VEC, bool U16>
 __device__ __forceinline__ int32_t relax_load_value(const RelaxArgs &a, int32_t row, int32_t v)
 {
@@ -892,7 +937,7 @@ __device__ __forceinline__ int32_t relax_load_value(const RelaxArgs &a, int32_t 
 }
 
 template <int VEC, bool U16>
-__device__ void relax_load_records(const RelaxArgs &a, int32_t (*tile)[33])
+__device__ void relax_load_records(const RelaxArgs &a, int32_t (*tile)[33], int32_t *neg)
 {
     constexpr int R = 32 * VEC, NW = RELAX_THREADS / 32, PER = R / NW;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -909,6 +954,7 @@ __device__ void relax_load_records(const RelaxArgs &a, int32_t (*tile)[33])
         }
     };
     if (blockIdx.x < ntiles) fetch(blockIdx.x);
+    relax_offsets<VEC, U16>(a, neg);
     for (int32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
 #pragma unroll
         for (int q = 0; q < PER; q++)
@@ -918,16 +964,25 @@ __device__ void relax_load_records(const RelaxArgs &a, int32_t (*tile)[33])
         if (t + (int32_t)gridDim.x < ntiles) fetch(t + gridDim.x);
         for (int vv = warp; vv < 32; vv += NW) {
             const int32_t v2 = t * 32 + vv;
-            if (v2 < n)
+            if (v2 >= n) break;
+            int2 b = excess_none<U16>();
 #pragma unroll
-                for (int g = 0; g < VEC; g++) __stcg(a.scratch + (int64_t)v2 * R + g * 32 + lane, tile[g * 32 + lane][vv]);
+            for (int g = 0; g < VEC; g++) {
+                const int32_t x = tile[g * 32 + lane][vv];
+                __stcg(a.scratch + (int64_t)v2 * R + g * 32 + lane, x);
+                b = excess_word<U16>(b, x, neg[g * 32 + lane], neg[R + g * 32 + lane]);
+            }
+            b = excess_reduce<U16>(b);
+            if (lane == 0) {
+                __stcg(a.mark + v2, make_int2(-1, b.y));
+                __stcg(a.high + v2, b.x);
+            }
         }
         __syncthreads();
     }
     for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         a.act0[v] = 1;
         a.act1[v] = 0;
-        a.stamp[v] = -1;
     }
 }
 
@@ -998,15 +1053,21 @@ __device__ void relax_store_records(const RelaxArgs &a, int32_t (*tile)[33])
 template <int VEC, bool U16 = false, bool HUBS = false>
 __global__ void __launch_bounds__(RELAX_THREADS, 2) k_relax(RelaxArgs a)
 {
-    __shared__ __align__(16) int32_t tile[32 * VEC][33];  // 32 vertices by all words of the chunk's records
+    // the transposes' tile (32 vertices by all words of the chunk's records);
+    // during the sweeps the warps' working memory and the hubs' partial minima
+    constexpr int TILE = 32 * VEC * 33, WARPS = RELAX_THREADS / 32 * (int)sizeof(RelaxWarp) / 4;
+    constexpr int SWEEP = WARPS + (HUBS ? RELAX_THREADS / 32 * 32 * VEC : 0);
+    __shared__ __align__(16) int32_t mem[TILE > SWEEP ? TILE : SWEEP];
+    int32_t(*tile)[33] = reinterpret_cast<int32_t(*)[33]>(mem);
+    __shared__ __align__(16) int32_t neg[2 * 32 * VEC];  // relax_offsets
     __shared__ int s_ok;
-    relax_load_records<VEC, U16>(a, tile);
+    relax_load_records<VEC, U16>(a, tile, neg);
     if (!grid_barrier(a.ctrl, &s_ok)) {
         if (threadIdx.x == 0) atomicOr(&a.stat->err, a.ctrl[C_ERR]);
         return;
     }
-    // the transposes' tile is free during the sweeps: 16 * 32 * VEC words of it hold the hubs' partial minima
-    const int32_t s = relax_sweeps<VEC, U16, HUBS>(a, &s_ok, &tile[0][0]);
+    const int32_t s =
+        relax_sweeps<VEC, U16, HUBS>(a, &s_ok, reinterpret_cast<RelaxWarp *>(mem), mem + WARPS, neg);
     if (s < 0) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stat->sweeps, (unsigned long long)s);
     relax_store_records<VEC, U16>(a, tile);

@@ -83,7 +83,7 @@ struct emv_ctx {
     DevBuf scratch, act;           // vertex-major chunk buffer, active flags
     DevBuf hubs;                   // vertices of many arcs of the graph being relaxed
     int32_t relax_nhubs = 0;       // and their number
-    DevBuf stamp;                  // per vertex: last sweep in which it changed
+    DevBuf mark;                   // per vertex: last sweep in which it changed, lowest and highest excess
     DevBuf adj;                    // packed (col, w) arcs
     DevBuf gscan;                  // GraphScan of the last packed graph (device admission check)
     DevBuf terms;                  // terminals

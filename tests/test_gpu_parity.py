@@ -588,3 +588,46 @@ def test_traceback_of_a_long_path(emv, solver):
     res = solver.solve(emv.Csr.from_stp(inst), tree=True)
     assert res.cost == n - 1
     check_tree(n, edges, res.tree, inst.terminals, res.cost)
+
+
+RECORD_CLOSURES = {
+    # kind: n, degree, wmin, wmax, k, value bits
+    "one warp": (33, 4, 1, 9, 12, 0),
+    "zero weights": (64, 4, 0, 0, 12, 0),
+    "long arcs": (6001, 20, 1, 100, 12, 0),
+    "short arcs": (5000, 21, 90, 100, 12, 0),
+    "long arcs 32 bits": (6001, 20, 1, 100, 12, 32),
+    "values above 16 bits": (3000, 10, 1, 100000, 12, 0),
+    "several windows a warp": (200002, 3, 1, 1000, 4, 0),
+}
+
+
+@pytest.mark.parametrize("kind", sorted(RECORD_CLOSURES))
+def test_arcs_ruled_out_by_the_excesses(emv, orc, kind):
+    """Record closures skip arcs that no row of a record can use: whole table
+    against the oracle where few and where most arcs are skipped."""
+    n, degree, wmin, wmax, k, bits = RECORD_CLOSURES[kind]
+    csr = emv.Csr.from_stp(emv.StpInstance.regular(n, degree, wmin, wmax, k, 11))
+    want, cost = orc.emv_table(csr.n, csr.row_ptr, csr.col, csr.w, csr.terminals, threads=16)
+    with emv.Solver(0) as s:
+        s.set_value_bits(bits)
+        res = s.solve(csr, table=True)
+        assert res.timing["relax_launches"] > 1
+        assert res.cost == cost and np.array_equal(res.table, want)
+
+
+@pytest.mark.parametrize("k", [3, 12])
+def test_record_closures_with_unreached_and_isolated_vertices(emv, orc, solver, k):
+    """Weights above 32768 beside 16-bit distances, a component without a
+    terminal and vertices without arcs: values of a row may be unreached."""
+    rng = np.random.default_rng(3)
+    n = 20040
+    a = emv.StpInstance.regular(20000, 4, 1, 40, k, 2)
+    heavy = np.stack([rng.integers(0, 10000, 3000), rng.integers(10000, 20000, 3000), rng.integers(30000, 70000, 3000)], axis=1)
+    far = np.stack([np.arange(20000, 20029), np.arange(20001, 20030), np.full(29, 7)], axis=1)
+    for edges, lost in ((np.concatenate([a.edges, heavy]), 0), (np.concatenate([a.edges, heavy, far]), 40)):
+        inst = emv.StpInstance(n if lost else 20000, edges.astype(np.int64), a.terminals)
+        csr = emv.Csr.from_stp(inst)
+        want, cost = orc.emv_table(csr.n, csr.row_ptr, csr.col, csr.w, csr.terminals, threads=16)
+        res = solver.solve(csr, table=True, check=not lost)
+        assert res.cost == cost and np.array_equal(res.table, want)
