@@ -73,9 +73,9 @@ static const void *const relax_fns[RELAX_VARIANTS] = {
     (const void *)k_relax<2, true, true>,  (const void *)k_relax<4, true, true>,  (const void *)k_relax<5, true, true>,
     (const void *)k_relax<8, true, true>};
 
-// Level-1 kernels by record width (4, 8, 16 or 32 rows).
-static const void *const level1_fns[LEVEL1_VARIANTS] = {(const void *)k_level1<1>, (const void *)k_level1<2>,
-                                                        (const void *)k_level1<4>, (const void *)k_level1<8>};
+// Narrow-record kernels by width (4, 8, 16 or 32 rows).
+static const void *const narrow_fns[NARROW_VARIANTS] = {(const void *)k_narrow<1>, (const void *)k_narrow<2>,
+                                                        (const void *)k_narrow<4>, (const void *)k_narrow<8>};
 
 extern "C" int emv_create(emv_ctx **out, int32_t device)
 {
@@ -98,10 +98,10 @@ extern "C" int emv_create(emv_ctx **out, int32_t device)
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, relax_fns[i], RELAX_THREADS, 0));
         c->relax_blocks_max[i] = std::max(1, per_sm) * c->sms;
     }
-    for (int i = 0; i < LEVEL1_VARIANTS; i++) {
+    for (int i = 0; i < NARROW_VARIANTS; i++) {
         int per_sm = 0;
-        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, level1_fns[i], NARROW_THREADS, 0));
-        c->level1_blocks_max[i] = std::max(1, per_sm) * c->sms;
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, narrow_fns[i], NARROW_THREADS, 0));
+        c->narrow_blocks_max[i] = std::max(1, per_sm) * c->sms;
     }
     int st = dev_reserve(c->ctrl, sizeof(uint32_t) * C_WORDS);
     if (!st) st = dev_reserve(c->stat, sizeof(DevStat));
@@ -185,6 +185,14 @@ static int grid_for(int64_t work, int threads, int cap)
 // against 2.50 at n = 10^5).
 static int32_t relax_hub_min(int32_t n, int64_t arcs) { return (int32_t)std::max<int64_t>(64, 4 * arcs / n); }
 
+// Chunks of at most this many rows are closed on narrow records, several
+// vertices a warp, instead of 128-byte records, a vertex a warp: n = 2^17,
+// degree 8, k = 7 (chunks of 21, 7 and 1 rows) 1.99 -> 1.57 ms of relaxation,
+// n = 10^5, degree 20, k = 12 (12 and 1) 9.93 -> 9.80.  With hubs only a single
+// row, whose sweeps are nearly all barrier: narrow records leave a hub to one
+// warp (n = 30 000, power-law degrees, k = 10, a chunk of 10 rows: 2.36 -> 2.52).
+constexpr int32_t RELAX_NARROW = 32;
+
 static int32_t max_sweeps(const emv_ctx *c, int32_t n)
 {
     return (c->sweep_limit > 0 && c->sweep_limit < (int64_t)n + 1) ? (int32_t)c->sweep_limit : n + 1;
@@ -240,15 +248,16 @@ int launch_relax(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n,
     return EMV_OK;
 }
 
-// Launches the single-source closures of rows[r] from terms[r] (device arrays,
-// at most 32) as one cooperative kernel; vmax (or null) receives the largest
-// value written.
-int launch_level1(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n, int64_t ld, int32_t *table,
+// Launches the closures of at most 32 rows as one cooperative kernel: the
+// single-source distances of terms[r] in rows[r] (device arrays), or, with
+// terms null, the closures of the rows as they are; vmax (or null) receives the
+// largest value written.
+int launch_narrow(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n, int64_t ld, int32_t *table,
                   const uint32_t *rows, int32_t nrows, const int32_t *terms, cudaStream_t st, uint32_t *vmax = nullptr,
                   uint16_t *shadow = nullptr, int64_t shadow_ld = 0, const GraphScan *scan = nullptr)
 {
     const int vi = nrows <= 4 ? 0 : nrows <= 8 ? 1 : nrows <= 16 ? 2 : 3;
-    Level1Args a;
+    NarrowLaunch a;
     a.na.row_ptr = row_ptr;
     a.na.n = n;
     a.na.rec = (int4 *)c->scratch.ptr;
@@ -269,12 +278,12 @@ int launch_level1(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n
     a.stat = (DevStat *)c->stat.ptr;
     a.scan = scan;
     const int vpb = narrow_vertices(1 << vi) * (NARROW_THREADS / 32);  // one group of vertices a warp
-    int bmax = c->level1_blocks_max[vi];
+    int bmax = c->narrow_blocks_max[vi];
     if (c->relax_sm_cap > 0 && c->relax_sm_cap < c->sms) bmax = std::max(1, bmax / c->sms * c->relax_sm_cap);
     const int blocks = std::min(bmax, std::max(1, (n + vpb - 1) / vpb));
     CUDA_TRY(cudaMemsetAsync(a.na.ctrl, 0, sizeof(uint32_t) * C_WORDS, st));
     void *args[] = {&a};
-    CUDA_TRY(cudaLaunchCooperativeKernel(level1_fns[vi], dim3(blocks), dim3(NARROW_THREADS), args, 0, st));
+    CUDA_TRY(cudaLaunchCooperativeKernel(narrow_fns[vi], dim3(blocks), dim3(NARROW_THREADS), args, 0, st));
     c->launches += 1;
     return EMV_OK;
 }
@@ -594,7 +603,7 @@ int run_dp(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32
     CUDA_TRY(cudaMemsetAsync(d_max + 1, 0, sizeof(uint32_t), st));
 
     // Level 1: k single-source closures (R:1988-2031).
-    r = launch_level1(c, row_ptr, adj, n, ld, table, xs + c->kp->xs_off[1], k, d_terms, st, d_max + 1, shadow, sld);
+    r = launch_narrow(c, row_ptr, adj, n, ld, table, xs + c->kp->xs_off[1], k, d_terms, st, d_max + 1, shadow, sld);
     if (r) return r;
     CUDA_TRY(cudaEventRecord(E[ev++], st));  // 2: after level 1
     CUDA_TRY(cudaMemcpyAsync(h_max + 1, d_max + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -630,7 +639,9 @@ int run_dp(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32
         const int32_t chunk = relax_chunk_rows_level(c, n, u16, cnt);
         for (int64_t off = 0; off < cnt; off += chunk) {
             const int32_t rows = (int32_t)std::min<int64_t>(chunk, cnt - off);
-            r = launch_relax(c, row_ptr, adj, n, ld, table, xs + b + off, rows, st, u16, shadow, sld);
+            if (rows <= (c->relax_nhubs > 0 ? 1 : RELAX_NARROW))
+                r = launch_narrow(c, row_ptr, adj, n, ld, table, xs + b + off, rows, nullptr, st, nullptr, shadow, sld);
+            else r = launch_relax(c, row_ptr, adj, n, ld, table, xs + b + off, rows, st, u16, shadow, sld);
             if (r) return r;
             relax_launches++;
         }
@@ -983,7 +994,7 @@ extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t 
         r = pack_and_check(c, n, arcs, row, col, w, false, st);
         if (r) return r;
         CUDA_TRY(cudaEventRecord(c->ev[0], st));
-        r = launch_level1(c, row, (const int2 *)c->adj.ptr, n, ld, table, (const uint32_t *)c->kp->xs.ptr, 1,
+        r = launch_narrow(c, row, (const int2 *)c->adj.ptr, n, ld, table, (const uint32_t *)c->kp->xs.ptr, 1,
                           (const int32_t *)c->terms.ptr, st, nullptr, nullptr, 0, (const GraphScan *)c->gscan.ptr);
         if (r) return r;
         CUDA_TRY(cudaEventRecord(c->ev[1], st));

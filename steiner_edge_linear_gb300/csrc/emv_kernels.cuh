@@ -13,7 +13,8 @@
 //                 subset merge of one level           R:2068-2107
 //   k_relax<VEC, U16>  multi-source closure of <= 32*VEC rows (64*VEC with
 //                 16-bit records; VEC = 1, 2, 4, 5, 8) R:2109-2130, R:1762-1880
-//   k_level1<LPV>  the k level-1 SSSPs, -dijkstra     R:1988-2031, R:2454-2484
+//   k_narrow<LPV>  closures of at most 32 rows: the    R:1988-2031, R:2109-2130,
+//                  k level-1 SSSPs, -dijkstra, ...     R:2454-2484
 //   k_traceback   tree recovery by recomputation      R:1907-1944
 #pragma once
 
@@ -1078,13 +1079,13 @@ __global__ void __launch_bounds__(RELAX_THREADS, 2) k_relax(RelaxArgs a)
     relax_store_records<VEC, U16>(a, tile);
 }
 
-// Single-source closures of up to 4 * LPV sources (level 1, R:1988-2031, and
-// the -dijkstra command): records of the sources' distances, sparse sweeps
-// from the sources' neighbours on (narrow_sweeps), records -> rows.
-struct Level1Args {
+// Closures of up to 4 * LPV rows on narrow records: from sources (level 1,
+// R:1988-2031, and the -dijkstra command), with sparse sweeps from the sources'
+// neighbours on, or of merged rows (R:2109-2130).
+struct NarrowLaunch {
     NarrowArgs na;
     const int2 *adj;
-    const int32_t *terms;   // source of row r
+    const int32_t *terms;   // source of row r, or null: closures of the rows as they are
     const uint32_t *rows;   // table row of r
     int32_t nrows;          // <= 4 * LPV
     int32_t *table;
@@ -1097,30 +1098,41 @@ struct Level1Args {
 };
 
 template <int LPV>
-__global__ void __launch_bounds__(NARROW_THREADS, 2) k_level1(Level1Args a)
+__global__ void __launch_bounds__(NARROW_THREADS, 2) k_narrow(NarrowLaunch a)
 {
     __shared__ int s_ok;
     if (a.scan && a.scan->bad) return;
     const int32_t n = a.na.n;
     const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = first; i < (int64_t)n * LPV; i += stride) __stcg(a.na.rec + i, make_int4(INF, INF, INF, INF));
+    if (a.terms) {
+        for (int64_t i = first; i < (int64_t)n * LPV; i += stride) __stcg(a.na.rec + i, make_int4(INF, INF, INF, INF));
+    } else {
+        for (int32_t g = 0; g < LPV; g++)  // four rows of a vertex a thread
+            for (int64_t v = first; v < n; v += stride) {
+                int32_t y[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    y[q] = 4 * g + q < a.nrows ? __ldcg(a.table + (int64_t)__ldg(a.rows + 4 * g + q) * a.ld + v) : INF;
+                __stcg(a.na.rec + v * LPV + g, make_int4(y[0], y[1], y[2], y[3]));
+            }
+    }
     for (int64_t v = first; v < n; v += stride) a.na.act0[v] = a.na.act1[v] = 0;
     if (!grid_barrier(a.na.ctrl, &s_ok)) {
         if (threadIdx.x == 0) atomicOr(&a.stat->err, a.na.ctrl[C_ERR]);
         return;
     }
-    if (blockIdx.x == 0)  // a warp per source: its distance, and its neighbours take part in sweep 0
+    if (a.terms && blockIdx.x == 0)  // a warp per source: its distance, and its neighbours take part in sweep 0
         for (int32_t r = threadIdx.x >> 5; r < a.nrows; r += NARROW_THREADS / 32) {
             const int32_t t = __ldg(a.terms + r);
             if ((threadIdx.x & 31) == 0) __stcg(reinterpret_cast<int32_t *>(a.na.rec) + (int64_t)t * 4 * LPV + r, 0);
             for (int32_t e = __ldg(a.na.row_ptr + t) + (threadIdx.x & 31); e < __ldg(a.na.row_ptr + t + 1); e += 32)
                 a.na.act0[__ldg(&a.adj[e].x)] = 1;
         }
-    if (!grid_barrier(a.na.ctrl, &s_ok)) {
+    if (a.terms && !grid_barrier(a.na.ctrl, &s_ok)) {
         if (threadIdx.x == 0) atomicOr(&a.stat->err, a.na.ctrl[C_ERR]);
         return;
     }
-    const int32_t s = narrow_sweeps<LPV>(a.na, NarrowPacked{a.adj}, true, &a.stat->err, &s_ok);
+    const int32_t s = narrow_sweeps<LPV>(a.na, NarrowPacked{a.adj}, a.terms != nullptr, &a.stat->err, &s_ok);
     if (s < 0) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stat->sweeps, (unsigned long long)s);
     uint32_t vmax = 0;

@@ -30,7 +30,7 @@ void dev_release(DevBuf &b);
 constexpr int MAX_EVENTS = 64;
 // emv_ctx::pinned: scalars of run_dp, then the one-launch solver's and the traceback's results
 constexpr size_t PINNED_RES = 2048, PINNED_TB = 4096, PINNED_BYTES = 32768;
-constexpr int LEVEL1_VARIANTS = 4;  // level-1 kernels by record width (level1_fns)
+constexpr int NARROW_VARIANTS = 4;  // narrow-record kernels by width (narrow_fns)
 constexpr int RELAX_VARIANTS = 20;  // relaxation kernels by record width and hubs (relax_fns)
 constexpr int BATCH_CLASSES = 12;  // (n bucket 0..3) x (k bucket 0..2)
 
@@ -69,7 +69,7 @@ struct emv_ctx {
     int device = 0;
     int sms = 0;
     int relax_blocks_max[RELAX_VARIANTS] = {};  // cooperative grid of each relaxation kernel
-    int level1_blocks_max[LEVEL1_VARIANTS] = {};  // and of each level-1 kernel
+    int narrow_blocks_max[NARROW_VARIANTS] = {};  // and of each narrow-record kernel
     int relax_sm_cap = 0;          // > 0: relaxation grids sized for this many SMs (the server's large solves)
     int64_t l2_bytes = 0;
     int64_t sweep_limit = 0;       // relaxation sweeps per chunk, 0 = n + 1

@@ -631,3 +631,16 @@ def test_record_closures_with_unreached_and_isolated_vertices(emv, orc, solver, 
         want, cost = orc.emv_table(csr.n, csr.row_ptr, csr.col, csr.w, csr.terminals, threads=16)
         res = solver.solve(csr, table=True, check=not lost)
         assert res.cost == cost and np.array_equal(res.table, want)
+
+
+@pytest.mark.parametrize("n,degree,wmax,k,bits", [(9001, 5, 50, 12, 0), (20011, 6, 10000, 7, 0), (20011, 20, 100, 9, 32),
+                                                  (160001, 4, 1000, 5, 0)])
+def test_levels_of_few_rows_on_narrow_records(emv, orc, n, degree, wmax, k, bits):
+    """Levels of 1 to 36 rows: merged rows closed on narrow records of every
+    width, beside wider levels that read their 16-bit copies."""
+    csr = emv.Csr.from_stp(emv.StpInstance.regular(n + n * degree % 2, degree, 1, wmax, k, 4))
+    want, cost = orc.emv_table(csr.n, csr.row_ptr, csr.col, csr.w, csr.terminals, threads=16)
+    with emv.Solver(0) as s:
+        s.set_value_bits(bits)
+        res = s.solve(csr, table=True)
+        assert res.cost == cost and np.array_equal(res.table, want)
