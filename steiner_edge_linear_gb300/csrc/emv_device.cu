@@ -148,7 +148,9 @@ extern "C" int emv_destroy(emv_ctx *c)
         dev_release(*b);
     for (KPlan *p : c->kplans) {
         if (!p) continue;
-        for (DevBuf *b : {&p->xs, &p->mpairs, &p->movr, &p->mstream_data, &p->mstream_phases}) dev_release(*b);
+        for (DevBuf *b : {&p->xs, &p->mpairs, &p->movr, &p->mstream_data, &p->mstream_phases, &p->mblock_data,
+                          &p->mblock_phases})
+            dev_release(*b);
         delete p;
     }
     for (int i = 0; i < MAX_EVENTS; i++)
@@ -358,6 +360,46 @@ int plan_stream_merge(emv_ctx *c, int32_t k, cudaStream_t st)
     return EMV_OK;
 }
 
+// Plans the block merge of every level of k and uploads it.
+// From BLOCK_KMIN on, where a level has pairs enough (n = 4 * 10^5, k = 6: 1.34 ->
+// 0.92 ms of merges); every level up to BLOCK_KMAX fits.
+constexpr int32_t BLOCK_KMIN = 6, BLOCK_KMAX = 12;
+// The ring of staged rows holds two phases, or less where it and the minima
+// would take more than this many rows: the rest of the memory is L1, which
+// serves the plan (n = 2^17, k = 11: 2.58 ms with 1600, 2.42 with 1280).
+constexpr int64_t BLOCK_SMEM_ROWS = 1280;
+static int plan_block_merge(emv_ctx *c, int32_t k, cudaStream_t st)
+{
+    c->kp->mblock_levels.assign((size_t)k + 2, {});
+    if (k < BLOCK_KMIN || k > BLOCK_KMAX) return EMV_OK;
+    std::vector<uint32_t> data;
+    std::vector<HostBlockLevel> plan;
+    plan_block_levels(k, BLOCK_LOW, c->kp->xs_host, c->kp->xs_off, STREAM_SMEM_BYTES, data, plan);
+    int r = dev_reserve(c->kp->mblock_data, sizeof(uint32_t) * std::max<size_t>(1, data.size()));
+    if (r) return r;
+    const uint32_t *base = (const uint32_t *)c->kp->mblock_data.ptr;
+    std::vector<BlockPhase> phases;
+    for (int32_t m = 3; m <= k; m++) {
+        const HostBlockLevel &L = plan[(size_t)m];
+        BlockLevel &to = c->kp->mblock_levels[(size_t)m];
+        to.phase_off = (int64_t)phases.size();
+        to.nphase = (int64_t)L.phases.size();
+        to.rows = L.rows;
+        to.split = L.split;
+        for (const HostBlockPhase &P : L.phases)
+            phases.push_back({base + P.warps_at, base + P.units_at, base + P.words_at, (int32_t)P.y0, (int32_t)P.ny,
+                              (int32_t)P.z0, (int32_t)P.nz});
+    }
+    r = dev_reserve(c->kp->mblock_phases, sizeof(BlockPhase) * std::max<size_t>(1, phases.size()));
+    if (r) return r;
+    CUDA_TRY(cudaMemcpyAsync(c->kp->mblock_data.ptr, data.data(), sizeof(uint32_t) * data.size(), cudaMemcpyHostToDevice,
+                             st));
+    CUDA_TRY(cudaMemcpyAsync(c->kp->mblock_phases.ptr, phases.data(), sizeof(BlockPhase) * phases.size(),
+                             cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    return EMV_OK;
+}
+
 static int build_plan(emv_ctx *c, int32_t k, cudaStream_t st);
 
 int prepare_subsets(emv_ctx *c, int32_t k, cudaStream_t st)
@@ -375,7 +417,8 @@ int prepare_subsets(emv_ctx *c, int32_t k, cudaStream_t st)
     c->xs_k = -1;
     const int r0 = build_plan(c, k, st);
     if (r0) {
-        for (DevBuf *b : {&plan->xs, &plan->mpairs, &plan->movr, &plan->mstream_data, &plan->mstream_phases})
+        for (DevBuf *b : {&plan->xs, &plan->mpairs, &plan->movr, &plan->mstream_data, &plan->mstream_phases,
+                          &plan->mblock_data, &plan->mblock_phases})
             dev_release(*b);
         delete plan;
         c->kp = nullptr;
@@ -395,6 +438,7 @@ static int build_plan(emv_ctx *c, int32_t k, cudaStream_t st)
     CUDA_TRY(cudaMemcpyAsync(c->kp->xs.ptr, c->kp->xs_host.data(), sizeof(uint32_t) * c->kp->xs_host.size(),
                              cudaMemcpyHostToDevice, st));
     r = plan_stream_merge(c, k, st);
+    if (!r) r = plan_block_merge(c, k, st);
     if (r) return r;
     // Pair and override slot lists of the staged-all-rows merge, for the levels
     // the streamed merge has no plan for (level order).
@@ -465,6 +509,8 @@ int launch_merge(emv_ctx *c, int32_t *table, int64_t ld, int32_t n, int32_t k, i
                                       STREAM_SMEM_BYTES));
         CUDA_TRY(cudaFuncSetAttribute((const void *)k_merge_stream16, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       STREAM_SMEM_BYTES));
+        for (const void *f : {(const void *)k_merge_block<false>, (const void *)k_merge_block<true>})
+            CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, STREAM_SMEM_BYTES));
         c->merge_attr = true;
     }
     const int64_t nstage = c->kp->xs_off[(size_t)m];
@@ -479,7 +525,20 @@ int launch_merge(emv_ctx *c, int32_t *table, int64_t ld, int32_t n, int32_t k, i
         // 16-bit staging reads int2 pairs of vertices: even stride and base
         u16 = u16 && ld % 2 == 0 && ((uintptr_t)table & 7) == 0;
         c->merge16_last = u16;
-        for (const StreamGroup &g : c->kp->mstream_groups[(size_t)m]) {
+        const BlockLevel &L = c->kp->mblock_levels[(size_t)m];
+        if (L.nphase > 0) {
+            const int32_t cnt = (int32_t)(c->kp->xs_off[(size_t)m + 1] - b);
+            const int64_t acc = (u16 && L.split ? 2 : 1) * cnt;
+            const int64_t ring = std::max(L.rows, std::min(2 * L.rows, BLOCK_SMEM_ROWS - acc));
+            const size_t smem = 128 * (size_t)(acc + ring);
+            const BlockPhase *pg = (const BlockPhase *)c->kp->mblock_phases.ptr + L.phase_off;
+            const unsigned blocks = (unsigned)std::min(u16 ? (n + 63) / 64 : (n + 31) / 32, c->sms);
+            auto *fn = u16 ? k_merge_block<true> : k_merge_block<false>;
+            fn<<<blocks, 32 * BLOCK_WARPS, smem, st>>>(table, ld, n, (const uint32_t *)c->kp->xs.ptr, (int32_t)b, cnt, pg,
+                                                       (int32_t)L.nphase, L.split, (int32_t)ring, d_terms, k,
+                                                       (uint32_t *)c->lvlmax.ptr + m, shadow, shadow_ld);
+            e = cudaGetLastError();
+        } else for (const StreamGroup &g : c->kp->mstream_groups[(size_t)m]) {
             const uint32_t *xg = (const uint32_t *)c->kp->xs.ptr + b + g.x0;
             const MergePhase *pg = (const MergePhase *)c->kp->mstream_phases.ptr + g.phase_off;
             if (u16)

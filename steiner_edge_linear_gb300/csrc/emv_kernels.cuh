@@ -9,7 +9,7 @@
 //   k_fill        f_v = INF                          R:2243-2259
 //   k_pack_scan   (col, w) arcs packed as int2        R:794-826 (adjacency fill)
 //                 and the device CSR checked
-//   k_merge, k_merge_smem, k_merge_stream, k_merge_stream16
+//   k_merge, k_merge_smem, k_merge_stream, k_merge_stream16, k_merge_block
 //                 subset merge of one level           R:2068-2107
 //   k_relax<VEC, U16>  multi-source closure of <= 32*VEC rows (64*VEC with
 //                 16-bit records; VEC = 1, 2, 4, 5, 8) R:2109-2130, R:1762-1880
@@ -20,10 +20,12 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <type_traits>
 
 #include "emv_common.cuh"
 #include "emv_device_util.cuh"
 #include "emv_narrow.cuh"
+#include "emv_plan.h"
 
 namespace emv {
 
@@ -488,6 +490,271 @@ __global__ void __launch_bounds__(1024) k_merge_stream16(int32_t *__restrict__ t
                 vmax = max(vmax, a0);
             }
         }
+    vmax = __reduce_max_sync(FULL, vmax);
+    if (lane == 0) atomicMax(&s_max, vmax);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(level_max, s_max);
+}
+
+// ---------------------------------------------------------- block merge
+//
+// Merge of a level whose phases' rows and minima fit shared memory (k <= 12).
+// The streamed merge reads two staged rows for every pair: it is bound by
+// shared-memory wavefronts, 2 a pair and 64 vertices.  Here the terminals are
+// split, X = (Xh, Xl) with B low bits, and a warp reduces all subsets of one Xh
+// together: for a split Yh, Xh \ Yh of the high bits it loads the rows of every
+// Yl of a bits and every Zl of c bits once (C(B, a) + C(B, c) rows) and forms
+// the C(B, a) * C(B - a, c) pairs of disjoint ones in registers, 0.84 loads a
+// pair at k = 12, B = 5 (1.1 with B = 4: 4.75 against 4.11 ms at n = 10^5, k =
+// 12; 3 % less at k = 8).  A row is a word a lane: 64 vertices of 16-bit values, or 32
+// vertices.  Merge of k_merge_stream16 -> here: n = 10^5, k = 12 6.0 -> 4.1 ms,
+// n = 2^17, k = 11 3.4 -> 2.4, n = 2^20, k = 10 13.1 -> 9.1 (and 32-bit values, n
+// = 30 000, k = 10: 0.85 -> 0.70).  Bound: instruction issue (55 % of the peak)
+// and, in the levels of few subsets, the latency of the staged rows.
+// Units are dealt out to the warps by cost on the host; where the
+// memory allows a minimum per vertex and subset, a unit's words lie with
+// several warps (shared-memory atomicMin), else a unit belongs to one.
+struct BlockPhase {
+    const uint32_t *warps, *units, *words;  // HostBlockPhase
+    int32_t y0, ny, z0, nz;
+};
+
+// The i-th number of a bits, and the number of smaller ones with as many bits.
+__host__ __device__ constexpr int bits_nth(int a, int i)
+{
+    for (int s = 0;; s++) {
+        int c = 0;
+        for (int b = s; b; b &= b - 1) c++;
+        if (c == a && i-- == 0) return s;
+    }
+}
+__host__ __device__ constexpr int bits_rank(int x)
+{
+    int a = 0, r = 0;
+    for (int b = x; b; b &= b - 1) a++;
+    for (int s = 0; s < x; s++) {
+        int c = 0;
+        for (int b = s; b; b &= b - 1) c++;
+        r += c == a;
+    }
+    return r;
+}
+__host__ __device__ constexpr int choose(int n, int r)
+{
+    int x = 1;
+    for (int i = 0; i < r; i++) x = x * (n - i) / (i + 1);
+    return x;
+}
+template <int N, int I = 0, typename F> __device__ __forceinline__ void static_for(F f)
+{
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        static_for<N, I + 1>(f);
+    }
+}
+
+template <bool U16> __device__ __forceinline__ uint32_t block_addmin(uint32_t y, uint32_t z, uint32_t acc)
+{
+    return U16 ? addmin16(y, z, acc) : __viaddmin_u32(y, z, acc);
+}
+
+// The pairs of all Yl of A bits with all Zl of C bits; Y, Z: this lane's word of the first rows.
+template <int B, int A, int C, bool U16>
+__device__ __forceinline__ void block_pairs(uint32_t (&acc)[choose(B, A + C)], const uint32_t *Y, const uint32_t *Z)
+{
+    uint32_t y[choose(B, A)], z[choose(B, C)];
+#pragma unroll
+    for (int i = 0; i < choose(B, A); i++) y[i] = Y[32 * i];
+#pragma unroll
+    for (int i = 0; i < choose(B, C); i++) z[i] = Z[32 * i];
+    static_for<choose(B, A)>([&](auto i) {
+        static_for<choose(B, C)>([&](auto j) {
+            constexpr int a = bits_nth(A, i.value), c = bits_nth(C, j.value);
+            if constexpr ((a & c) == 0) {
+                constexpr int o = bits_rank(a | c);
+                acc[o] = block_addmin<U16>(y[i.value], z[j.value], acc[o]);
+            }
+        });
+    });
+}
+
+// One unit of subsets with Q low bits: S, M: this lane's word of the first
+// staged row and of the unit's first minimum.
+template <int B, int Q, bool U16>
+__device__ __forceinline__ void block_unit(const uint32_t *S, uint32_t *M, bool split, const uint4 &h, uint32_t n45,
+                                           const uint32_t *__restrict__ words)
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t acc[choose(B, Q)];
+#pragma unroll
+    for (int o = 0; o < choose(B, Q); o++) acc[o] = U16 ? 0xffffffffu : (uint32_t)INF;
+    // a lane holds every 32nd word (the plan's are followed by 32 that are not used)
+    const uint32_t *w = words + h.y + lane;
+    uint32_t mine = __ldg(w);
+    int32_t d = 0;
+    static_for<Q + 1>([&](auto a) {
+        constexpr int A = a.value;
+        const uint32_t n2 = A < 2 ? h.z : A < 4 ? h.w : n45;
+        for (int32_t left = (int32_t)(A % 2 ? n2 >> 16 : n2 & 0xffffu); left > 0; left--) {
+            const uint32_t x = __shfl_sync(FULL, mine, d & 31);
+            block_pairs<B, A, Q - A, U16>(acc, S + (x & 0xffffu) * 32, S + (x >> 16) * 32);
+            if ((++d & 31) == 0) mine = __ldg(w += 32);
+        }
+    });
+#pragma unroll
+    for (int o = 0; o < choose(B, Q); o++) {
+        if (!U16) atomicMin(M + 32 * o, acc[o]);
+        else if (split) {  // vertices 2 * lane and 2 * lane + 1: words lane and 32 + lane
+            atomicMin(M + 64 * o, acc[o] & 0xffffu);
+            atomicMin(M + 64 * o + 32, acc[o] >> 16);
+        } else M[32 * o] = __vminu2(M[32 * o], acc[o]);
+    }
+}
+
+// Merge of a level of cnt subsets xs[x0..] (R:2068-2107); U16: see
+// k_merge_stream16 for the values' bounds and the shadow.  A persistent block
+// goes through vertex blocks and phases; the rest of the shared memory is a
+// ring of `ring` staged rows, and the rows of the next steps are copied, as far
+// as they fit, while this one is reduced.  (A block per vertex block, whose
+// phases wait for their copies: n = 2^20, k = 10 11.3 ms, now 9.1.)
+template <bool U16>
+__global__ void __launch_bounds__(32 * BLOCK_WARPS, 1)
+    k_merge_block(int32_t *__restrict__ table, int64_t ld, int32_t n, const uint32_t *__restrict__ xs, int32_t x0,
+                  int32_t cnt, const BlockPhase *__restrict__ phases, int32_t nphase, bool split, int32_t ring,
+                  const int32_t *__restrict__ terms, int32_t k, uint32_t *__restrict__ level_max,
+                  const uint16_t *__restrict__ shadow, int64_t sld)
+{
+    extern __shared__ __align__(16) uint32_t sm[];
+    constexpr int NV = U16 ? 64 : 32, NW = BLOCK_WARPS, B = BLOCK_LOW;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int acc_words = U16 && split ? 64 : 32;  // per subset
+    const uint32_t none = U16 ? 0xffffffffu : (uint32_t)INF;
+    uint32_t *S0 = sm + (size_t)cnt * acc_words;
+    const int32_t nblocks = (n + NV - 1) / NV;
+    __shared__ uint32_t s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    for (int32_t i = threadIdx.x; i < cnt * acc_words; i += 32 * NW) sm[i] = none;
+    // copies the rows of a phase and vertex block to S (asynchronously, but for 16-bit values without a shadow)
+    auto stage = [&](int32_t vb, const BlockPhase &P, uint32_t *S) {
+        const int32_t v0 = vb * NV, va = v0 + (U16 ? 2 * lane : lane), nrows = P.ny + P.nz;
+        for (int32_t c0 = warp * 32; c0 < nrows; c0 += NW * 32) {
+            const int32_t i = c0 + lane, nr = min(32, nrows - c0);
+            const uint32_t myr = i < nrows ? __ldg(xs + (i < P.ny ? P.y0 + i : P.z0 + i - P.ny)) : 0u;
+            if (U16 && shadow) {
+                // eight lanes copy a row, all of a warp's rows in flight;
+                // vertices past n are read but never stored
+                const int sub = lane >> 3, sl = lane & 7;
+                for (int32_t j0 = 0; j0 < nr; j0 += 4) {
+                    const int32_t j = j0 + sub;
+                    const uint32_t r = __shfl_sync(FULL, myr, j & 31);
+                    if (j < nr) cp_async16(S + (c0 + j) * 32 + sl * 4, shadow + (int64_t)r * sld + v0 + sl * 8);
+                }
+            } else if (U16) {
+                for (int32_t j0 = 0; j0 < nr; j0 += 16) {
+                    int2 x[16];
+#pragma unroll
+                    for (int u = 0; u < 16; u++) {
+                        const uint32_t r = __shfl_sync(FULL, myr, (j0 + u) & 31);
+                        const int32_t *row = table + (int64_t)r * ld;
+                        x[u] = make_int2(-1, -1);
+                        if (j0 + u < nr) {
+                            if (v0 + NV <= n) x[u] = __ldg(reinterpret_cast<const int2 *>(row + v0) + lane);
+                            else if (va < n) x[u] = make_int2(__ldg(row + va), va + 1 < n ? __ldg(row + va + 1) : -1);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 16; u++)
+                        if (j0 + u < nr) S[(c0 + j0 + u) * 32 + lane] = pack16(x[u]);
+                }
+            } else {
+                for (int32_t j = 0; j < nr; j++) {
+                    const uint32_t r = __shfl_sync(FULL, myr, j);
+                    if (va < n) cp_async4(S + (c0 + j) * 32 + lane, table + (int64_t)r * ld + va);
+                    else S[(c0 + j) * 32 + lane] = (uint32_t)INF;
+                }
+            }
+        }
+        cp_async_commit();
+    };
+    uint32_t vmax = 0;  // largest value written: the relaxation's record width follows it
+    // steps staged but not reduced yet; next step to stage; the ring's end and
+    // the rows it holds (with those left out before its end)
+    int32_t ahead = 0, nvb = blockIdx.x, nph = 0, end = 0, held = 0, from = 0;
+    for (int32_t vb = blockIdx.x; vb < nblocks; vb += gridDim.x) {
+        for (int32_t ph = 0; ph < nphase; ph++) {
+            if (ahead == 0) end = held = from = 0;
+            while (ahead < 4 && nvb < nblocks) {
+                const int32_t need = phases[nph].ny + phases[nph].nz;
+                const bool wrap = end + need > ring;
+                const int32_t take = need + (wrap ? ring - end : 0);
+                if (held + take > ring) break;
+                if (wrap) end = 0;
+                stage(nvb, phases[nph], S0 + (size_t)end * 32);
+                end += need;
+                held += take;
+                ahead++;
+                if (++nph == nphase) {
+                    nph = 0;
+                    nvb += gridDim.x;
+                }
+            }
+            const int32_t here = phases[ph].ny + phases[ph].nz;
+            if (from + here > ring) {
+                held -= ring - from;
+                from = 0;
+            }
+            uint32_t *S = S0 + (size_t)from * 32;
+            from += here;
+            held -= here;  // free after this step
+            cp_async_wait_but(--ahead);
+            __syncthreads();
+            const uint32_t *warps = phases[ph].warps, *units = phases[ph].units, *words = phases[ph].words;
+            const uint32_t u1 = __ldg(warps + warp + 1);
+            for (uint32_t u = __ldg(warps + warp); u < u1; u++) {
+                const uint4 h = __ldg(reinterpret_cast<const uint4 *>(units) + 2 * u);
+                const uint32_t n45 = __ldg(units + 8 * u + 4);
+                uint32_t *M = sm + (h.x & 0xffffu) * acc_words + lane;
+                const uint32_t q = h.x >> 16;
+                static_for<B + 1>([&](auto Q) {
+                    if (q == Q.value) block_unit<B, Q.value, U16>(S + lane, M, split, h, n45, words);
+                });
+            }
+            __syncthreads();
+        }
+        const int32_t v0 = vb * NV, va = v0 + (U16 ? 2 * lane : lane);
+        bool has_term = false;
+        for (int t = 0; t < k; t++) {
+            const int32_t tv = __ldg(terms + t);
+            has_term |= tv >= v0 && tv < v0 + NV;
+        }
+        for (int32_t xi = warp; xi < cnt; xi += NW) {
+            const uint32_t X = __ldg(xs + x0 + xi);
+            uint32_t *M = sm + xi * acc_words + lane;
+            uint32_t a0 = M[0], a1 = 0;
+            M[0] = none;  // for the next vertex block
+            if (U16) {
+                a1 = split ? M[32] : a0 >> 16;
+                if (split) M[32] = none;
+                a0 &= 0xffffu;
+            }
+            if (va >= n) continue;
+            if (has_term)
+                for (uint32_t bits = X; bits; bits &= bits - 1) {
+                    const int t = __ffs(bits) - 1;
+                    const int32_t tv = __ldg(terms + t);
+                    if (tv == va) a0 = (uint32_t)table[(int64_t)(X ^ (1u << t)) * ld + va];
+                    if (U16 && tv == va + 1) a1 = (uint32_t)table[(int64_t)(X ^ (1u << t)) * ld + va + 1];
+                }
+            int32_t *dst = table + (int64_t)X * ld + va;
+            if (U16 && va + 1 < n) {
+                *reinterpret_cast<int2 *>(dst) = make_int2((int32_t)a0, (int32_t)a1);
+                vmax = max(vmax, max(a0, a1));
+            } else {
+                *dst = (int32_t)a0;
+                vmax = max(vmax, a0);
+            }
+        }
+    }
     vmax = __reduce_max_sync(FULL, vmax);
     if (lane == 0) atomicMax(&s_max, vmax);
     __syncthreads();

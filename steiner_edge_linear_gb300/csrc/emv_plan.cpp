@@ -186,4 +186,123 @@ void plan_stream_levels(int32_t k, const std::vector<uint32_t> &xs, const std::v
     }
 }
 
+void plan_block_levels(int32_t k, int32_t low, const std::vector<uint32_t> &xs, const std::vector<int64_t> &off,
+                       int64_t smem_bytes, std::vector<uint32_t> &data, std::vector<HostBlockLevel> &plan)
+{
+    plan.assign((size_t)k + 2, {});
+    data.clear();
+    const int32_t high = k - low;
+    if (high < 1) return;
+    std::vector<uint32_t> rank((size_t)1 << k, 0);  // position within its level
+    for (int32_t m = 1; m <= k; m++)
+        for (int64_t i = off[(size_t)m]; i < off[(size_t)m + 1]; i++) rank[xs[(size_t)i]] = (uint32_t)(i - off[(size_t)m]);
+    auto choose = [](int32_t a, int32_t b) {
+        int64_t r = 1;
+        for (int32_t i = 0; i < b; i++) r = r * (a - i) / (i + 1);
+        return b < 0 || b > a ? (int64_t)0 : r;
+    };
+    auto first = [&](uint32_t h, int32_t a) { return rank[h << low | ((1u << a) - 1)]; };
+    struct Part {
+        uint32_t acc;
+        int32_t q;
+        int64_t cost;
+        std::vector<uint32_t> words[6];
+    };
+    for (int32_t m = 3; m <= k; m++) {
+        auto count = [&](int32_t j) { return off[(size_t)j + 1] - off[(size_t)j]; };
+        HostBlockLevel L;
+        for (int32_t j = 1; 2 * j <= m; j++) L.rows = std::max(L.rows, count(j) + (2 * j == m ? 0 : count(m - j)));
+        const int64_t budget = smem_bytes / 128;
+        if (count(m) + L.rows > budget) continue;
+        // room to stage a phase beside another comes before shared minima
+        L.split = 2 * count(m) + 2 * L.rows <= budget ||
+                  (count(m) + 2 * L.rows > budget && 2 * count(m) + L.rows <= budget);
+        for (int32_t j = 1; 2 * j <= m; j++) {
+            const bool same = 2 * j == m;
+            HostBlockPhase P{off[(size_t)j], count(j), same ? 0 : off[(size_t)(m - j)], same ? 0 : count(m - j), 0, 0, 0};
+            std::vector<Part> parts;
+            int64_t total = 0;
+            auto cost = [&](int32_t a, int32_t c) {
+                return 4 + choose(low, a) + choose(low, c) + choose(low, a) * choose(low - a, c);
+            };
+            for (uint32_t X = 0; X < 1u << high; X++) {
+                const int32_t p = __builtin_popcount(X), q = m - p;
+                if (q < 0 || q > low) continue;
+                Part part{first(X, q), q, 0, {}};
+                for (int32_t a = 0; a <= std::min(q, j); a++) {
+                    const int32_t yh = j - a;
+                    if (yh > p) continue;
+                    for (uint32_t Y = X;; Y = (Y - 1) & X) {
+                        // one of {Y, X \ Y} of equal sizes: the one with X's lowest high bit
+                        if (__builtin_popcount(Y) == yh && !(same && X && !(Y & X & (0u - X)))) {
+                            const uint32_t z = first(X ^ Y, q - a) + (uint32_t)(same ? 0 : P.ny);
+                            part.words[a].push_back(first(Y, a) | z << 16);
+                            part.cost += cost(a, q - a);
+                        }
+                        if (!Y) break;
+                    }
+                }
+                if (!part.cost) continue;
+                total += part.cost;
+                parts.push_back(std::move(part));
+            }
+            if (L.split) {  // parts of at most one and a half warps' share (of a third: 8 % slower, unit by unit overhead)
+                const int64_t want = std::max<int64_t>(60, total * 3 / (2 * BLOCK_WARPS));
+                std::vector<Part> cut;
+                for (const Part &u : parts) {
+                    Part part{u.acc, u.q, 0, {}};
+                    for (int32_t a = 0; a <= u.q; a++)
+                        for (uint32_t w : u.words[a]) {
+                            part.words[a].push_back(w);
+                            part.cost += cost(a, u.q - a);
+                            if (part.cost >= want) {
+                                cut.push_back(part);
+                                part = Part{u.acc, u.q, 0, {}};
+                            }
+                        }
+                    if (part.cost) cut.push_back(part);
+                }
+                parts.swap(cut);
+            }
+            std::stable_sort(parts.begin(), parts.end(), [](const Part &a, const Part &b) { return a.cost > b.cost; });
+            std::vector<std::vector<const Part *>> warp(BLOCK_WARPS);
+            int64_t load[BLOCK_WARPS] = {};
+            for (const Part &u : parts) {
+                const size_t w = (size_t)(std::min_element(load, load + BLOCK_WARPS) - load);
+                warp[w].push_back(&u);
+                load[w] += u.cost + 3 * choose(low, u.q) + 15;
+            }
+            P.warps_at = data.size();
+            uint32_t units = 0;
+            for (auto &w : warp) {
+                // the warps run the same code at about the same time
+                std::stable_sort(w.begin(), w.end(), [](const Part *a, const Part *b) { return a->q > b->q; });
+                data.push_back(units);
+                units += (uint32_t)w.size();
+            }
+            data.push_back(units);
+            while (data.size() % 4) data.push_back(0);
+            P.units_at = data.size();
+            uint32_t at = 0;
+            for (const auto &w : warp)
+                for (const Part *u : w) {
+                    uint32_t n[6];
+                    for (int a = 0; a < 6; a++) n[a] = (uint32_t)u->words[a].size();
+                    for (uint32_t x : {u->acc | (uint32_t)u->q << 16, at, n[0] | n[1] << 16, n[2] | n[3] << 16,
+                                       n[4] | n[5] << 16, 0u, 0u, 0u})
+                        data.push_back(x);
+                    for (int a = 0; a < 6; a++) at += n[a];
+                }
+            P.words_at = data.size();
+            for (const auto &w : warp)
+                for (const Part *u : w)
+                    for (int a = 0; a < 6; a++) data.insert(data.end(), u->words[a].begin(), u->words[a].end());
+            data.insert(data.end(), 32, 0u);  // a warp reads 32 words at a time
+            data.insert(data.end(), 32, 0u);
+            L.phases.push_back(P);
+        }
+        plan[(size_t)m] = L;
+    }
+}
+
 }  // namespace emv

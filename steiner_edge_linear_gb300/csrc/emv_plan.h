@@ -63,4 +63,29 @@ int64_t stream_acc_rows(int64_t g);
 void plan_stream_levels(int32_t k, const std::vector<uint32_t> &xs, const std::vector<int64_t> &off,
                         int64_t smem_bytes, std::vector<uint32_t> &data, std::vector<std::vector<HostGroup>> &plan);
 
+// Block merge of a level: the terminals are split into the low bits `low` and
+// the others, X = (Xh, Xl).  A unit is one Xh, whose subsets of the level, Xl of
+// q = m - |Xh| bits, are neighbours in level order; in phase j it has one word
+// (posY | posZ << 16) for every Yh of Xh and a = j - |Yh|: the staged positions
+// of the first Y = (Yh, any a bits) and the first Z = (Xh \ Yh, any q - a bits),
+// the others following in order.  Each word stands for the pairs of every
+// disjoint Yl, Zl.  A unit in the plan data is 8 words: first accumulator | q <<
+// 16, its first word, and the counts of its words by a (16 bits each).
+constexpr int BLOCK_WARPS = 32;
+struct HostBlockPhase {
+    int64_t y0, ny, z0, nz;          // staged rows: subsets [y0, y0 + ny) and [z0, z0 + nz) of the level order
+    size_t warps_at, units_at;       // first unit of every warp (BLOCK_WARPS + 1 words); 16-byte aligned units
+    size_t words_at;
+};
+struct HostBlockLevel {
+    int64_t rows = 0;                // most staged rows of a phase (0: no plan)
+    bool split = false;              // a unit's words may lie with several warps (shared minima)
+    std::vector<HostBlockPhase> phases;
+};
+constexpr int32_t BLOCK_LOW = 5;     // low bits
+// Plans every level 3..k whose minima (one 128-byte row a subset, two where
+// 16-bit minima are shared) and phases fit smem_bytes.
+void plan_block_levels(int32_t k, int32_t low, const std::vector<uint32_t> &xs, const std::vector<int64_t> &off,
+                       int64_t smem_bytes, std::vector<uint32_t> &data, std::vector<HostBlockLevel> &plan);
+
 }  // namespace emv

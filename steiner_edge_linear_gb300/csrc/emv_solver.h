@@ -40,6 +40,12 @@ struct StreamGroup {
     int64_t x0, cnt, phase_off, nphase, smem;
 };
 
+// The block merge of a level.
+struct BlockLevel {
+    int64_t phase_off = 0, nphase = 0, rows = 0;
+    bool split = false;
+};
+
 // Everything the DP needs per k, built once per k and context: the subsets by
 // level, the pair and override slots of the staged-all-rows merge and the
 // streamed merge's groups and phases.
@@ -51,6 +57,8 @@ struct KPlan {
     std::vector<int64_t> mpair_base, movr_base;  // per level
     DevBuf mstream_data, mstream_phases;
     std::vector<std::vector<StreamGroup>> mstream_groups;  // per level (none = not streamed)
+    DevBuf mblock_data, mblock_phases;
+    std::vector<BlockLevel> mblock_levels;                 // per level (nphase 0 = no block merge)
 };
 
 // Buffers of one launch of the batched kernel.  A large batch runs as two
