@@ -771,7 +771,7 @@ extern "C" int emv_kernel_dev(emv_ctx *c, int32_t n, int64_t arcs, const int32_t
     cudaStream_t st = (cudaStream_t)stream;
     c->launches = 0;
     ResidentPlan plan;
-    if (resident_plan(c, n, k, plan)) {
+    if (resident_plan(c, n, arcs, k, false, plan)) {
         r = resident_launch(c, plan, n, arcs, d_row_ptr, d_col, d_w, terminals, k, k, d_table, ld, true, st);
         if (r) return r;
         CUDA_TRY(cudaStreamSynchronize(st));
@@ -892,7 +892,7 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
     const int32_t kt = whole ? k : table_terminals(k);
     const size_t tbytes = sizeof(int32_t) * (size_t)ld << kt;
     ResidentPlan plan;
-    const bool resident = resident_plan(c, n, kt, plan);
+    const bool resident = resident_plan(c, n, arcs, kt, (flags & EMV_SOLVE_TABLE) && out->table, plan);
     int r = resident ? EMV_OK : pack_and_check(c, n, arcs, row_ptr, col, w, check, st);
     if (!r) r = dev_reserve(c->table, tbytes);
     if (r) return r;
@@ -1018,7 +1018,7 @@ extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t 
     // row 1 = {source}; rows of whole quads
     const int64_t ld = ((int64_t)n + 3) / 4 * 4;
     ResidentPlan plan;
-    const bool resident = n <= SSSP_RESIDENT_N && resident_plan(c, n, 1, plan);
+    const bool resident = n <= SSSP_RESIDENT_N && resident_plan(c, n, 0, 1, false, plan);  // the bound on n is the measured one
     r = dev_reserve(c->table, sizeof(int32_t) * 2 * (size_t)ld);
     if (!r) r = prepare_subsets(c, 1, st);
     if (!r && !resident) r = reserve_relax(c, n);

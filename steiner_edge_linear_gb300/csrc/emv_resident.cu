@@ -71,12 +71,20 @@ uint32_t res_inv_slices(int32_t n)
 // Whether a solve of n vertices over kt terminals' subsets runs as one
 // launch, and its shape.  The closure of a row needs about 7.3 bytes a vertex
 // of shared memory (distance, list entry, mark, arc count), so n is at most
-// about 31 000.  Levels of more rows than SMs (kt >= 10) take turns on them,
-// and the record kernels, which read an arc once for 256 rows, are faster
-// from a few thousand vertices on.
-bool resident_plan(const emv_ctx *c, int32_t n, int32_t kt, ResidentPlan &p)
+// about 31 000.  Levels of more rows than SMs (kt >= 10) take turns on them, and
+// arcs that do not fit shared memory are read again in every sweep, while the
+// record kernels read an arc once for 256 rows.  Kernel times here and there:
+// degree 8, kt = 10: n = 5800 0.62 and 1.57 ms, 12 000 1.15 and 1.83, 20 011 1.86
+// and 2.07; kt = 11, n = 12 000 2.05 and 2.84; degree 20, kt = 9: n = 10 000 1.13
+// and 1.57, 16 000 1.68 and 1.66, 20 011 2.08 and 1.89.
+// host_table: the call copies the table to the host.  Past 2^22 cells that copy
+// outweighs the solve, and such calls keep the kernels whose value widths
+// emv_timing reports.
+constexpr int64_t RESIDENT_MAX_ARCS = 300000;
+bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, bool host_table, ResidentPlan &p)
 {
-    if (!resident_fits(n, kt) || (kt > 9 && n > 4096)) return false;
+    if (!resident_fits(n, kt) || arcs > RESIDENT_MAX_ARCS) return false;
+    if (kt > 9 && n > 4096 && (n > 16384 || (host_table && (int64_t)n << kt > 1 << 22))) return false;
     const int sms = c->relax_sm_cap > 0 && c->relax_sm_cap < c->sms ? c->relax_sm_cap : c->sms;
     const int64_t maxcnt = resident_max_rows(kt);
     // a CTA for every 1024 states of the widest level

@@ -21,7 +21,7 @@ bool resident_fits(int32_t n, int32_t kt);
 // so that every CTA has some; cap > 0 bounds it.
 int32_t resident_merge_width(int32_t n, int32_t kt, int32_t ctas, int32_t cap);
 uint32_t res_inv_slices(int32_t n);
-bool resident_plan(const emv_ctx *c, int32_t n, int32_t kt, ResidentPlan &p);
+bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, bool host_table, ResidentPlan &p);
 // Enqueues the whole DP over the first kt of the k terminals, CSR check
 // included, and the copy of its result words; fills the table's 2^kt rows
 // (stride ld) and c->adj.

@@ -644,3 +644,21 @@ def test_levels_of_few_rows_on_narrow_records(emv, orc, n, degree, wmax, k, bits
         s.set_value_bits(bits)
         res = s.solve(csr, table=True)
         assert res.cost == cost and np.array_equal(res.table, want)
+
+
+@pytest.mark.parametrize("n,degree,k", [(5001, 8, 10), (9000, 6, 11), (16384, 3, 10), (16385, 4, 10), (15002, 20, 9),
+                                        (14998, 20, 7)])
+def test_one_launch_limits_on_caller_tables(emv, orc, solver, n, degree, k):
+    """Both sides of the one-launch solver's limits on vertices and arcs from 10
+    terminals on: whole caller table and the cost-only solve."""
+    torch = pytest.importorskip("torch")
+    csr = emv.Csr.from_stp(emv.StpInstance.regular(n + n * degree % 2, degree, 1, 200, k, 23))
+    want, want_cost = orc.emv_table(csr.n, csr.row_ptr, csr.col, csr.w, csr.terminals, threads=16)
+    row, col, w = (torch.from_numpy(a).to("cuda:0") for a in (csr.row_ptr, csr.col, csr.w))
+    ld = csr.n + 3 - csr.n % 2
+    table = torch.full(((1 << k), ld), -7, dtype=torch.int32, device="cuda:0")
+    cost = solver.kernel_dev(csr.n, csr.arcs, row.data_ptr(), col.data_ptr(), w.data_ptr(), csr.terminals,
+                             table.data_ptr(), ld, torch.cuda.current_stream().cuda_stream)
+    got = table.cpu().numpy()
+    assert cost == want_cost and np.array_equal(got[:, :csr.n], want) and (got[:, csr.n:] == -7).all()
+    assert solver.solve(csr, tree=True).cost == want_cost
