@@ -532,7 +532,9 @@ int launch_merge(emv_ctx *c, int32_t *table, int64_t ld, int32_t n, int32_t k, i
             const int64_t ring = std::max(L.rows, std::min(2 * L.rows, BLOCK_SMEM_ROWS - acc));
             const size_t smem = 128 * (size_t)(acc + ring);
             const BlockPhase *pg = (const BlockPhase *)c->kp->mblock_phases.ptr + L.phase_off;
-            const unsigned blocks = (unsigned)std::min(u16 ? (n + 63) / 64 : (n + 31) / 32, c->sms);
+            // one block an SM, of those this context may take: a block that waits for an SM would double the time
+            const int sms = c->relax_sm_cap > 0 && c->relax_sm_cap < c->sms ? c->relax_sm_cap : c->sms;
+            const unsigned blocks = (unsigned)std::min(u16 ? (n + 63) / 64 : (n + 31) / 32, sms);
             auto *fn = u16 ? k_merge_block<true> : k_merge_block<false>;
             fn<<<blocks, 32 * BLOCK_WARPS, smem, st>>>(table, ld, n, (const uint32_t *)c->kp->xs.ptr, (int32_t)b, cnt, pg,
                                                        (int32_t)L.nphase, L.split, (int32_t)ring, d_terms, k,
