@@ -347,7 +347,7 @@ def run_single(args, dist: Dist, cfg: dict = SINGLE, cfg_name: str = SINGLE_NAME
         alg = rows * relax_bytes_per_row(n, m)
         unit_note = f"12n+16m+4(n+1) bytes per row closure x {rows} rows"
     else:
-        kname, kms, launches_k = ("k_merge_stream16" if cfg is SINGLE else "merge"), merge_ms, k - 1
+        kname, kms, launches_k = ("k_merge_block" if cfg is SINGLE else "merge"), merge_ms, k - 1
         alg = merge_bytes(n, k)
         unit_note = "12 bytes per (X,Y,v) triple x n(3^k-2^(k+1)+1)"
     achieved = alg / (kms / 1000.0) / 1e9

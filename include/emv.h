@@ -172,8 +172,9 @@ int emv_destroy(emv_ctx *ctx);
  * usable: a latency bound for callers that prefer an error to an unusually
  * long solve.  No reference counterpart (its Dijkstra has no budget). */
 int emv_set_sweep_limit(emv_ctx *ctx, int64_t limit);
-/* Width of the DP values inside the kernels of the context's later solves:
- * 0 (the default) stages a level's merge rows as 16-bit values when every
+/* Width of the DP values inside the kernels of the context's later solves
+ * (a small instance, solved in one launch, and batches always use 32 bits): 0
+ * (the default) stages a level's merge rows as 16-bit values when every
  * sum of two of them is provably at most 65533, and relaxes a level with
  * 16-bit records when its values are provably at most 32767 (twice the rows
  * per chunk at the same bytes); 32 always keeps 32 bits.  With 0 the context
@@ -182,7 +183,9 @@ int emv_set_sweep_limit(emv_ctx *ctx, int64_t limit);
  * reference counterpart (it works on the int32 table directly). */
 int emv_set_value_bits(emv_ctx *ctx, int32_t bits);
 
-/* Per-phase device times of the last solve (CUDA events, ms). */
+/* Per-phase device times of the last solve (CUDA events, ms; of a solve in one
+ * launch, as its first block saw them, with relax_launches = 1 and relax_sweeps
+ * the rounds of its closures summed over the blocks). */
 typedef struct emv_timing {
     float zero_ms;        /* table fill, R:2243-2259                     */
     float level1_ms;      /* k single-source closures, R:1988-2031       */
@@ -192,7 +195,7 @@ typedef struct emv_timing {
     float kernel_ms;      /* level1 + merge + relax                      */
     int64_t relax_sweeps; /* frontier sweeps summed over chunks          */
     int64_t launches;     /* kernel launches issued by the solve         */
-    int64_t relax16_levels; /* levels relaxed with 16-bit records        */
+    int64_t relax16_levels; /* levels whose values allow 16-bit records  */
     int64_t merge16_levels; /* levels merged from 16-bit staged rows     */
     int64_t relax_launches; /* relaxation launches, level 1 included      */
 } emv_timing;
@@ -306,7 +309,8 @@ typedef struct emv_batch_stats {
 
 /* Solves many independent instances (no counterpart in the reference, which
  * runs one instance per process): one persistent, CUDA-graph-captured launch
- * whose teams of 1 to 128 CTAs take instances from device queues.  costs_out
+ * (two for a large batch, the second packed while the first runs) whose teams
+ * of 1 to 128 CTAs take instances from device queues.  costs_out
  * gets one int64 per instance.  Only the rows that the costs depend on (the
  * subsets of each instance's first k - 1 terminals) are computed;
  * emv_batch_solve_tables computes them all. */
