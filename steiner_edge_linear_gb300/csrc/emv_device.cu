@@ -362,12 +362,8 @@ int plan_stream_merge(emv_ctx *c, int32_t k, cudaStream_t st)
 
 // Plans the block merge of every level of k and uploads it.
 // From BLOCK_KMIN on, where a level has pairs enough (n = 4 * 10^5, k = 6: 1.34 ->
-// 0.92 ms of merges); every level up to BLOCK_KMAX fits.
+// 0.68 ms of merges); every level up to BLOCK_KMAX fits.
 constexpr int32_t BLOCK_KMIN = 6, BLOCK_KMAX = 12;
-// The ring of staged rows holds two phases, or less where it and the minima
-// would take more than this many rows: the rest of the memory is L1, which
-// serves the plan (n = 2^17, k = 11: 2.58 ms with 1600, 2.42 with 1280).
-constexpr int64_t BLOCK_SMEM_ROWS = 1280;
 static int plan_block_merge(emv_ctx *c, int32_t k, cudaStream_t st)
 {
     c->kp->mblock_levels.assign((size_t)k + 2, {});

@@ -507,10 +507,10 @@ __global__ void __launch_bounds__(1024) k_merge_stream16(int32_t *__restrict__ t
 // the C(B, a) * C(B - a, c) pairs of disjoint ones in registers, 0.84 loads a
 // pair at k = 12, B = 5 (1.1 with B = 4: 4.75 against 4.11 ms at n = 10^5, k =
 // 12; 3 % less at k = 8).  A row is a word a lane: 64 vertices of 16-bit values, or 32
-// vertices.  Merge of k_merge_stream16 -> here: n = 10^5, k = 12 6.0 -> 4.1 ms,
-// n = 2^17, k = 11 3.4 -> 2.4, n = 2^20, k = 10 13.1 -> 9.1 (and 32-bit values, n
-// = 30 000, k = 10: 0.85 -> 0.70).  Bound: instruction issue (55 % of the peak)
-// and, in the levels of few subsets, the latency of the staged rows.
+// vertices.  Merge of k_merge_stream16 -> here: n = 10^5, k = 12 6.0 -> 3.9 ms,
+// n = 2^17, k = 11 3.4 -> 2.1, n = 2^20, k = 10 13.1 -> 6.7 (and 32-bit values, n
+// = 30 000, k = 10: 0.85 -> 0.52).  Bound: instruction issue (55 to 60 % of the
+// peak) and, in the levels of few subsets, the latency of the staged rows.
 // Units are dealt out to the warps by cost on the host; where the
 // memory allows a minimum per vertex and subset, a unit's words lie with
 // several warps (shared-memory atomicMin), else a unit belongs to one.
@@ -616,7 +616,7 @@ __device__ __forceinline__ void block_unit(const uint32_t *S, uint32_t *M, bool 
 // goes through vertex blocks and phases; the rest of the shared memory is a
 // ring of `ring` staged rows, and the rows of the next steps are copied, as far
 // as they fit, while this one is reduced.  (A block per vertex block, whose
-// phases wait for their copies: n = 2^20, k = 10 11.3 ms, now 9.1.)
+// phases, a size each, wait for their copies: n = 2^20, k = 10 11.3 ms, 9.1 so.)
 template <bool U16>
 __global__ void __launch_bounds__(32 * BLOCK_WARPS, 1)
     k_merge_block(int32_t *__restrict__ table, int64_t ld, int32_t n, const uint32_t *__restrict__ xs, int32_t x0,

@@ -210,16 +210,31 @@ void plan_block_levels(int32_t k, int32_t low, const std::vector<uint32_t> &xs, 
     };
     for (int32_t m = 3; m <= k; m++) {
         auto count = [&](int32_t j) { return off[(size_t)j + 1] - off[(size_t)j]; };
+        auto rows = [&](int32_t j) { return count(j) + (2 * j == m ? 0 : count(m - j)); };
         HostBlockLevel L;
-        for (int32_t j = 1; 2 * j <= m; j++) L.rows = std::max(L.rows, count(j) + (2 * j == m ? 0 : count(m - j)));
+        for (int32_t j = 1; 2 * j <= m; j++) L.rows = std::max(L.rows, rows(j));
         const int64_t budget = smem_bytes / 128;
         if (count(m) + L.rows > budget) continue;
-        // room to stage a phase beside another comes before shared minima
-        L.split = 2 * count(m) + 2 * L.rows <= budget ||
-                  (count(m) + 2 * L.rows > budget && 2 * count(m) + L.rows <= budget);
-        for (int32_t j = 1; 2 * j <= m; j++) {
-            const bool same = 2 * j == m;
-            HostBlockPhase P{off[(size_t)j], count(j), same ? 0 : off[(size_t)(m - j)], same ? 0 : count(m - j), 0, 0, 0};
+        // few subsets have too few units to keep every warp busy
+        L.split = count(m) <= 240 && 2 * count(m) + L.rows <= budget;
+        // A phase takes j0..j1: as many neighbouring sizes as the memory holds (at
+        // least one), so that a unit's pairs are formed in few phases.  Room for
+        // the copies of the next phase is worth less: n = 2^20, k = 10 9.2 ms of
+        // merges with a phase a size, 7.4 where two phases fit, 6.7 so.
+        const int64_t fits = budget - (L.split ? 2 : 1) * count(m);
+        for (int32_t j0 = 1, j1; 2 * j0 <= m; j0 = j1 + 1) {
+            int64_t all = rows(j0);
+            for (j1 = j0; 2 * (j1 + 1) <= m && all + rows(j1 + 1) <= fits; j1++) all += rows(j1 + 1);
+            const int32_t zl = 2 * j1 == m ? j1 + 1 : m - j1;  // sizes zl..m - j0 beside j0..j1
+            HostBlockPhase P{off[(size_t)j0], off[(size_t)j1 + 1] - off[(size_t)j0], off[(size_t)zl],
+                             off[(size_t)(m - j0) + 1] - off[(size_t)zl], 0, 0, 0};
+            if (P.nz <= 0) P.z0 = P.nz = 0;
+            L.rows = std::max(L.rows, P.ny + P.nz);
+            auto staged = [&](uint32_t h, int32_t a) {  // position of the first row of h and any a low bits
+                const int32_t size = __builtin_popcount(h) + a;
+                const int64_t at = off[(size_t)size] + first(h, a);
+                return (uint32_t)(size <= j1 ? at - P.y0 : P.ny + at - P.z0);
+            };
             std::vector<Part> parts;
             int64_t total = 0;
             auto cost = [&](int32_t a, int32_t c) {
@@ -229,19 +244,16 @@ void plan_block_levels(int32_t k, int32_t low, const std::vector<uint32_t> &xs, 
                 const int32_t p = __builtin_popcount(X), q = m - p;
                 if (q < 0 || q > low) continue;
                 Part part{first(X, q), q, 0, {}};
-                for (int32_t a = 0; a <= std::min(q, j); a++) {
-                    const int32_t yh = j - a;
-                    if (yh > p) continue;
+                for (int32_t a = 0; a <= q; a++)
                     for (uint32_t Y = X;; Y = (Y - 1) & X) {
+                        const int32_t j = __builtin_popcount(Y) + a;
                         // one of {Y, X \ Y} of equal sizes: the one with X's lowest high bit
-                        if (__builtin_popcount(Y) == yh && !(same && X && !(Y & X & (0u - X)))) {
-                            const uint32_t z = first(X ^ Y, q - a) + (uint32_t)(same ? 0 : P.ny);
-                            part.words[a].push_back(first(Y, a) | z << 16);
+                        if (j >= j0 && j <= j1 && !(2 * j == m && X && !(Y & X & (0u - X)))) {
+                            part.words[a].push_back(staged(Y, a) | staged(X ^ Y, q - a) << 16);
                             part.cost += cost(a, q - a);
                         }
                         if (!Y) break;
                     }
-                }
                 if (!part.cost) continue;
                 total += part.cost;
                 parts.push_back(std::move(part));
