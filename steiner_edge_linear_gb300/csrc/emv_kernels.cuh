@@ -1440,6 +1440,7 @@ constexpr int TB_WARPS = 16;
 constexpr int TB_TASKS = 64;   // pieces of the tree: at most 2 (k - 1) - 1
 constexpr int TB_CHUNK = 64;   // edges of a chunk of a piece's list
 constexpr int TB_HEAD = 16;    // words before the edges of the result
+constexpr int32_t TB_WAIT = 1 << 22;  // polls for the search arrays while their holder makes no progress (over 0.4 s)
 
 struct TbArgs {
     const int32_t *table;
@@ -1554,11 +1555,14 @@ struct TbTask {
 // lists are then laid out in the order of the depth-first walk that visits
 // X \ Y first.  A run of zero-weight arcs is resolved by a breadth-first
 // search inside the set of vertices with the same value, so zero-weight
-// cycles cannot loop; its arrays serve one warp at a time.
+// cycles cannot loop; its arrays serve one warp at a time, and the others wait
+// as long as that search goes on (each visits a vertex once, so it ends): it
+// may take in the whole graph, a chain of dependent loads per vertex, and up to
+// k - 2 pieces stand behind it.
 __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(TbArgs a)
 {
     __shared__ TbTask task[TB_TASKS];
-    __shared__ int s_alloc, s_next, s_done, s_chunk, s_lock, s_walk;
+    __shared__ int s_alloc, s_next, s_done, s_chunk, s_lock, s_walk, s_beat;
     __shared__ uint32_t s_status;
     __shared__ int32_t s_order[TB_TASKS], s_at[TB_TASKS], s_pieces;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1569,7 +1573,7 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(TbArgs a)
     unsigned long long t0 = 0;
     if (threadIdx.x == 0) {
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-        s_next = s_done = s_chunk = s_lock = s_walk = 0;
+        s_next = s_done = s_chunk = s_lock = s_walk = s_beat = 0;
         s_alloc = a.k >= 2;
         s_status = 0;
         if (a.k >= 2) {
@@ -1661,9 +1665,18 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(TbArgs a)
             // Zero-weight run: BFS over arcs of weight 0 between vertices of value D.
             int walk = 0;
             if (lane == 0) {
-                int spins = 0;
-                while (atomicCAS(&s_lock, 0, 1) != 0 && ++spins < (1 << 24)) {}
-                walk = spins < (1 << 24) ? ++s_walk : -1;
+                int beat = -1;
+                for (int32_t spins = 0; spins < TB_WAIT;) {
+                    if (atomicCAS(&s_lock, 0, 1) == 0) {
+                        walk = ++s_walk;
+                        break;
+                    }
+                    const int now = *(volatile int *)&s_beat;
+                    spins = now == beat ? spins + 1 : 0;
+                    beat = now;
+                    __nanosleep(100);
+                }
+                if (!walk) walk = -1;
             }
             walk = __shfl_sync(FULL, walk, 0);
             if (walk < 0) {
@@ -1683,6 +1696,7 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(TbArgs a)
             while (head < tail) {
                 const int32_t x = *(volatile int32_t *)(a.queue + head);
                 head++;
+                if (lane == 0) ++*(volatile int *)&s_beat;
                 if (x != v) {
                     uint32_t Y2;
                     int32_t d2, u2, w2, xb = a.row_ptr[x], xe = a.row_ptr[x + 1];
@@ -1715,6 +1729,7 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(TbArgs a)
             for (int32_t z = target; !fail && z != v;) {
                 const int32_t p = *(volatile int32_t *)(a.parent + z);
                 add_edge(z, p, 0);
+                if (lane == 0) ++*(volatile int *)&s_beat;
                 z = p;
             }
             if (!fail) {

@@ -662,3 +662,12 @@ def test_one_launch_limits_on_caller_tables(emv, orc, solver, n, degree, k):
     got = table.cpu().numpy()
     assert cost == want_cost and np.array_equal(got[:, :csr.n], want) and (got[:, csr.n:] == -7).all()
     assert solver.solve(csr, tree=True).cost == want_cost
+
+
+def test_traceback_waits_for_long_zero_weight_searches(emv, solver):
+    """All weights 0: every piece of the tree is one search over a large part of
+    the graph, and the pieces queue for the search's arrays for seconds."""
+    csr = emv.Csr.from_stp(inst := emv.StpInstance.regular(1 << 19, 4, 0, 0, 12, 3))
+    res = solver.solve(csr, tree=True)
+    assert res.cost == 0 and res.tree_weight == 0
+    check_tree(csr.n, inst.edges, res.tree, csr.terminals, 0)
