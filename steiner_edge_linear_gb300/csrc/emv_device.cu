@@ -786,11 +786,11 @@ constexpr size_t TB_FIRST_WORDS = TB_HEAD + 3 * TB_FIRST_EDGES;
 static_assert(PINNED_TB + 4 * TB_FIRST_WORDS <= PINNED_BYTES, "traceback words fit the pinned buffer");
 
 // Enqueues the traceback and the copy of its head and first edges into the
-// pinned buffer.  skip_err, skip_bad (or null): device words that say, where
+// pinned buffer.  skip_err, skip_refused (or null): device words that say, where
 // not 0, that there is nothing to trace.
 static int launch_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32_t k,
                             const int32_t *d_terms, const int32_t *table, int64_t ld, const uint32_t *skip_err,
-                            const uint32_t *skip_bad, cudaStream_t st)
+                            const uint32_t *skip_refused, cudaStream_t st)
 {
     const int32_t cap = std::max(64, 2 * n);
     const int32_t nchunks = cap / TB_CHUNK + TB_TASKS + 1;
@@ -808,7 +808,7 @@ static int launch_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const
     a.adj = adj;
     a.terms = d_terms;
     a.skip_err = skip_err;
-    a.skip_bad = skip_bad;
+    a.skip_refused = skip_refused;
     a.chunks = (int32_t *)c->tb_edges.ptr;
     a.next = a.chunks + (size_t)nchunks * TB_CHUNK * 3;
     a.nchunks = nchunks;
@@ -903,7 +903,7 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
         r = resident_launch(c, plan, n, arcs, row_ptr, col, w, terms, k, kt, table, ld, check, st);
         if (!r && tree) {
             const ResidentWords d = resident_words(c);
-            r = launch_traceback(c, n, row_ptr, (const int2 *)c->adj.ptr, k, d.terms, table, ld, d.err, d.bad, st);
+            r = launch_traceback(c, n, row_ptr, (const int2 *)c->adj.ptr, k, d.terms, table, ld, d.err, d.refused, st);
         }
         if (r) return r;
         CUDA_TRY(cudaStreamSynchronize(st));

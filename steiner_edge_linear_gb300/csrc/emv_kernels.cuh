@@ -1450,7 +1450,7 @@ struct TbArgs {
     const int32_t *row_ptr;
     const int2 *adj;
     const int32_t *terms;
-    const uint32_t *skip_err, *skip_bad;  // if set: words that are 0 where table and arcs may be read
+    const uint32_t *skip_err, *skip_refused;  // if set: words that are 0 where table and arcs may be read
     int32_t *chunks;    // edge lists: chunks of TB_CHUNK edges of 3 words
     int32_t *next;      // the chunk after each chunk
     int32_t nchunks;
@@ -1566,7 +1566,7 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(TbArgs a)
     __shared__ uint32_t s_status;
     __shared__ int32_t s_order[TB_TASKS], s_at[TB_TASKS], s_pieces;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if ((a.skip_err && *a.skip_err) || (a.skip_bad && *a.skip_bad)) {
+    if ((a.skip_err && *a.skip_err) || (a.skip_refused && *a.skip_refused)) {
         if (threadIdx.x < TB_HEAD) a.out[threadIdx.x] = 0;
         return;
     }

@@ -26,10 +26,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(ResArgs a)
     if (!res_barrier(tm, sh)) return;
     const uint32_t bad = __ldcg(&a.out->scan.bad), maxw = __ldcg(&a.out->scan.maxw);
     if (a.check) {  // the host reads the same words and names the fault
-        if (bad) return;
         const long long bound =
             min((long long)(a.inst.n - 1) * (long long)maxw, (long long)(__ldcg(&a.out->scan.sumw) / 2));
-        if (bound >= INF) return;
+        if (bad || bound >= INF) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) a.out->refused = 1;
+            return;
+        }
     }
     res_solve(a.inst, tm, sm, sh, maxw < RES_MAX_W && !(bad & SCAN_BAD_WEIGHT), 1, a.inst.kt);
 }
@@ -97,7 +99,7 @@ bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, bool h
 ResidentWords resident_words(const emv_ctx *c)
 {
     const ResOut *o = (const ResOut *)c->res_out.ptr;
-    return {o->terms, &o->err, &o->scan.bad};
+    return {o->terms, &o->err, &o->refused};
 }
 
 int resident_launch(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, const int32_t *row_ptr,

@@ -83,7 +83,7 @@ struct ResOut {
     uint32_t err;
     uint32_t unreached;
     uint32_t rounds;
-    uint32_t pad;
+    uint32_t refused;         // the CSR check found a fault: no row was filled
     GraphScan scan;
     unsigned long long ns[3];
     int64_t cost;

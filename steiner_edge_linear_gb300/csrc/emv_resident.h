@@ -31,10 +31,11 @@ int resident_launch(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, 
 // Status, cost and times once the stream has been waited for (with spanned
 // set, a vertex that no terminal reaches is EMV_ERR_DISCONNECTED).
 int resident_finish(emv_ctx *c, int32_t n, int32_t k, bool check, bool spanned, int64_t *cost_out, emv_timing *tm);
-// Device words of the launch: the terminals, the error word, the CSR check's.
+// Device words of the launch: the terminals, and two that are 0 where the table
+// has been filled (the error word, and whether the CSR check refused the graph).
 struct ResidentWords {
     const int32_t *terms;
-    const uint32_t *err, *bad;
+    const uint32_t *err, *refused;
 };
 ResidentWords resident_words(const emv_ctx *c);
 // Status of a device CSR check (emv_device.cu).

@@ -6,6 +6,7 @@ valid Steiner tree of real edges whose weight equals the cost.
 """
 import os
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -671,3 +672,25 @@ def test_traceback_waits_for_long_zero_weight_searches(emv, solver):
     res = solver.solve(csr, tree=True)
     assert res.cost == 0 and res.tree_weight == 0
     check_tree(csr.n, inst.edges, res.tree, csr.terminals, 0)
+
+
+def test_refused_one_launch_solve_traces_nothing(emv, solver):
+    """A small graph whose value bound reaches 2^30 is refused without a walk
+    through the table: with a tree requested the refusal takes no longer than
+    half of the walk through the rows that the solve before it left there."""
+    n = 20000
+    edges = np.stack([np.arange(n - 1), np.arange(1, n), np.ones(n - 1, np.int64)], axis=1).astype(np.int64)
+    good = emv.Csr.from_stp(emv.StpInstance(n, edges, np.array([0, n - 1, n - 2], np.int64)))
+    far = edges.copy()
+    far[[5, 6], 2] = 2**30 - 1
+    bad = emv.Csr.from_stp(emv.StpInstance(n, far, good.terminals.astype(np.int64)))
+    walk = solver.solve(good, tree=True).timing["traceback_ms"]
+    assert walk > 4.0
+    for _ in range(3):
+        solver.solve(good)
+        t0 = time.perf_counter()
+        with pytest.raises(emv.EmvError) as ei:
+            solver.solve(bad, tree=True)
+        took = 1e3 * (time.perf_counter() - t0)
+        assert ei.value.status == 8
+        assert took < walk / 2
