@@ -22,7 +22,6 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(ResArgs a)
     if (threadIdx.x < RES_KMAX + 2) sh.lvl[threadIdx.x] = a.lvl[threadIdx.x];
     if (blockIdx.x == 0 && threadIdx.x < EMV_MAX_K) a.out->terms[threadIdx.x] = a.terms[threadIdx.x];
     scan_csr(a.inst.row_ptr, a.inst.n, a.col, a.w, a.adj, a.arcs, &a.out->scan);
-    for (int64_t v = first; v < a.inst.n; v += stride) a.inst.table[v] = INF;  // row 0 (R:2243-2259)
     if (!res_barrier(tm, sh)) return;
     const uint32_t bad = __ldcg(&a.out->scan.bad), maxw = __ldcg(&a.out->scan.maxw);
     if (a.check) {  // the host reads the same words and names the fault
@@ -33,6 +32,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(ResArgs a)
             return;
         }
     }
+    // row 0 (R:2243-2259), which no level reads; after the check: a refused call leaves the caller's table as it is
+    for (int64_t v = first; v < a.inst.n; v += stride) a.inst.table[v] = INF;
     res_solve(a.inst, tm, sm, sh, maxw < RES_MAX_W && !(bad & SCAN_BAD_WEIGHT), 1, a.inst.kt);
 }
 

@@ -694,3 +694,20 @@ def test_refused_one_launch_solve_traces_nothing(emv, solver):
         took = 1e3 * (time.perf_counter() - t0)
         assert ei.value.status == 8
         assert took < walk / 2
+
+
+@pytest.mark.parametrize("n", [300, 40000])
+def test_refused_graphs_leave_the_callers_table_alone(emv, solver, n):
+    """emv_kernel_dev on a graph that its check refuses writes no cell."""
+    torch = pytest.importorskip("torch")
+    g = emv.Csr.from_stp(emv.StpInstance.regular(n, 4, 1, 9, 4, 5))
+    table = torch.full((1 << 4, n), -7, dtype=torch.int32, device="cuda:0")
+    for array, value, status in (("col", n, 1), ("w", -1, 1), ("w", 2**30 - 1, 8)):
+        arrays = {name: getattr(g, name).copy() for name in ("row_ptr", "col", "w")}
+        arrays[array][10:14] = value
+        row, col, w = (torch.from_numpy(arrays[x]).to("cuda:0") for x in ("row_ptr", "col", "w"))
+        with pytest.raises(emv.EmvError) as ei:
+            solver.kernel_dev(n, g.arcs, row.data_ptr(), col.data_ptr(), w.data_ptr(), g.terminals, table.data_ptr(), n,
+                              torch.cuda.current_stream().cuda_stream)
+        assert ei.value.status == status
+        assert bool((table == -7).all())
