@@ -785,19 +785,29 @@ constexpr size_t TB_FIRST_EDGES = 1024;
 constexpr size_t TB_FIRST_WORDS = TB_HEAD + 3 * TB_FIRST_EDGES;
 static_assert(PINNED_TB + 4 * TB_FIRST_WORDS <= PINNED_BYTES, "traceback words fit the pinned buffer");
 
-// Enqueues the traceback and the copy of its head and first edges into the
-// pinned buffer.  skip_err, skip_refused (or null): device words that say, where
-// not 0, that there is nothing to trace.
+static int32_t traceback_cap(int32_t n) { return std::max(64, 2 * n); }
+static int32_t traceback_chunks(int32_t n) { return traceback_cap(n) / TB_CHUNK + TB_TASKS + 1; }
+
+// Buffers of a traceback, to be had before anything of the solve is enqueued
+// that would still run when a failed call returns.
+static int reserve_traceback(emv_ctx *c, int32_t n)
+{
+    int r = dev_reserve(c->tb_edges, sizeof(int32_t) * (TB_CHUNK * 3 + 1) * (size_t)traceback_chunks(n));
+    if (!r)
+        r = dev_reserve(c->tb_out,
+                        sizeof(int32_t) * (TB_HEAD + 3 * std::max<size_t>((size_t)traceback_cap(n), TB_FIRST_EDGES)));
+    if (!r) r = dev_reserve(c->tb_work, sizeof(int32_t) * 3 * (size_t)n);
+    return r;
+}
+
+// Enqueues the traceback (its buffers are reserved) and the copy of its head
+// and first edges into the pinned buffer.  skip_err, skip_refused (or null):
+// device words that say, where not 0, that there is nothing to trace.
 static int launch_traceback(emv_ctx *c, int32_t n, const int32_t *row_ptr, const int2 *adj, int32_t k,
                             const int32_t *d_terms, const int32_t *table, int64_t ld, const uint32_t *skip_err,
                             const uint32_t *skip_refused, cudaStream_t st)
 {
-    const int32_t cap = std::max(64, 2 * n);
-    const int32_t nchunks = cap / TB_CHUNK + TB_TASKS + 1;
-    int r = dev_reserve(c->tb_edges, sizeof(int32_t) * (TB_CHUNK * 3 + 1) * (size_t)nchunks);
-    if (!r) r = dev_reserve(c->tb_out, sizeof(int32_t) * (TB_HEAD + 3 * std::max<size_t>((size_t)cap, TB_FIRST_EDGES)));
-    if (!r) r = dev_reserve(c->tb_work, sizeof(int32_t) * 3 * (size_t)n);
-    if (r) return r;
+    const int32_t cap = traceback_cap(n), nchunks = traceback_chunks(n);
     int32_t *work = (int32_t *)c->tb_work.ptr;
     TbArgs a;
     a.table = table;
@@ -899,6 +909,8 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
     out->tree_count = 0;
     out->tree_weight = 0;
     const bool tree = (flags & EMV_SOLVE_TREE) && k >= 2;
+    if (tree) r = reserve_traceback(c, n);
+    if (r) return r;
     if (resident) {  // one wait for the solve and its tree
         r = resident_launch(c, plan, n, arcs, row_ptr, col, w, terms, k, kt, table, ld, check, st);
         if (!r && tree) {

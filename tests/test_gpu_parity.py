@@ -4,6 +4,7 @@ The bar is bit-exact: the whole int32 DP table and the cost equal the
 oracle's on the same instance and the reference's golden hashes; the tree is a
 valid Steiner tree of real edges whose weight equals the cost.
 """
+import ctypes
 import os
 import subprocess
 import time
@@ -711,3 +712,34 @@ def test_refused_graphs_leave_the_callers_table_alone(emv, solver, n):
                               torch.cuda.current_stream().cuda_stream)
         assert ei.value.status == status
         assert bool((table == -7).all())
+
+
+def test_out_of_memory_for_the_tree_leaves_no_work_behind(emv):
+    """A one-launch solve that cannot have the traceback's buffers fails before
+    it enqueues anything: the caller may free its arrays on return."""
+    torch = pytest.importorskip("torch")
+    cudart = ctypes.CDLL("libcudart.so")
+    cudart.cudaMalloc.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_size_t]
+    cudart.cudaFree.argtypes = [ctypes.c_void_p]
+    g = emv.Csr.from_stp(emv.StpInstance.regular(24000, 4, 1, 9, 10, 5))
+    stream = torch.cuda.Stream()
+    held = []
+    with emv.Solver(0) as s:
+        want = s.solve(g, stream=stream.cuda_stream).cost
+        size = 1 << 36
+        while size >= 1 << 16:
+            p = ctypes.c_void_p()
+            if cudart.cudaMalloc(ctypes.byref(p), size) == 0:
+                held.append(p)
+            else:
+                cudart.cudaGetLastError()
+                size >>= 1
+        try:
+            with pytest.raises(emv.EmvError) as ei:
+                s.solve(g, tree=True, stream=stream.cuda_stream)
+            idle = stream.query()
+        finally:
+            for p in held:
+                cudart.cudaFree(p)
+        assert ei.value.status == 3 and idle
+        assert s.solve(g, tree=True, stream=stream.cuda_stream).cost == want
