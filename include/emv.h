@@ -170,7 +170,9 @@ int emv_destroy(emv_ctx *ctx);
  * default, is the Bellman-Ford bound n + 1, which no closure reaches).  A solve
  * that hits a smaller cap returns EMV_ERR_TIMEOUT and leaves the context
  * usable: a latency bound for callers that prefer an error to an unusually
- * long solve.  No reference counterpart (its Dijkstra has no budget). */
+ * long solve.  Closures that sweep more lightly (few rows, or a small instance
+ * solved in one launch) may take three times the cap.  No reference counterpart
+ * (its Dijkstra has no budget). */
 int emv_set_sweep_limit(emv_ctx *ctx, int64_t limit);
 /* Width of the DP values inside the kernels of the context's later solves
  * (a small instance, solved in one launch, and batches always use 32 bits): 0

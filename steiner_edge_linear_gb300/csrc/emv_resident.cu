@@ -145,7 +145,7 @@ int resident_launch(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, 
     I.vec = ld % 4 == 0 && ((uintptr_t)table & 15) == 0;
     I.want_rows = p.rows;
     I.mw = p.mw;
-    I.max_rounds = (c->sweep_limit > 0 && c->sweep_limit < (int64_t)n + 1) ? (int32_t)c->sweep_limit : n + 1;
+    I.max_rounds = max_sweeps(c, n, SWEEP_RATE);
     I.inv_slices = res_inv_slices(n);
     CUDA_TRY(cudaMemsetAsync(a.out, 0, sizeof(ResOut), st));
     CUDA_TRY(cudaEventRecord(c->ev[0], st));

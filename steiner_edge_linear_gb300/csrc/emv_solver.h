@@ -125,5 +125,7 @@ struct emv_ctx {
 
 int prepare_subsets(emv_ctx *c, int32_t k, cudaStream_t st);
 int reserve_relax(emv_ctx *c, int32_t n);
+constexpr int32_t SWEEP_RATE = 3;  // sweeps of narrow records, or rounds in one launch, for one of k_relax
+int32_t max_sweeps(const emv_ctx *c, int32_t n, int32_t rate);
 int32_t relax_chunk_rows(const emv_ctx *c, int32_t n, bool u16);
 int32_t relax_chunk_rows_level(const emv_ctx *c, int32_t n, bool u16, int64_t cnt);

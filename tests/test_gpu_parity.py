@@ -743,3 +743,25 @@ def test_out_of_memory_for_the_tree_leaves_no_work_behind(emv):
                 cudart.cudaFree(p)
         assert ei.value.status == 3 and idle
         assert s.solve(g, tree=True, stream=stream.cuda_stream).cost == want
+
+
+@pytest.mark.parametrize("side,limit", [(100, 110), (200, 210), (316, 340)])
+def test_sweep_limit_holds_for_long_frontiers(emv, side, limit):
+    """Grids need about a sweep of the record kernels for a row of vertices;
+    closures that move a change by one arc a sweep take twice as many within
+    the same cap."""
+    at = np.arange(side * side).reshape(side, side)
+    ends = np.concatenate([np.stack([at[:, :-1].ravel(), at[:, 1:].ravel()], 1),
+                           np.stack([at[:-1].ravel(), at[1:].ravel()], 1)])
+    w = np.random.default_rng(side + 77).integers(1, 101 if side > 300 else 11, len(ends))
+    terms = np.random.default_rng(1).choice(side * side, size=5, replace=False)
+    csr = emv.Csr.from_stp(emv.StpInstance(side * side, np.concatenate([ends, w[:, None]], 1), terms.astype(np.int64)))
+    with emv.Solver(0) as s:
+        want, dist = s.solve(csr).cost, s.sssp(csr, 1)[0]
+        s.set_sweep_limit(limit)
+        assert s.solve(csr).cost == want
+        assert np.array_equal(s.sssp(csr, 1)[0], dist)
+        s.set_sweep_limit(limit // 8)
+        with pytest.raises(emv.EmvError) as ei:
+            s.solve(csr)
+        assert ei.value.status == 5
