@@ -1019,8 +1019,13 @@ extern "C" int emv_solve_dev(emv_ctx *c, const emv_graph *d_g, const int32_t *te
                            (cudaStream_t)stream);
 }
 
-// Up to here one CTA's shared memory beats the whole GPU's sweeps.
+// Up to here one CTA's shared memory beats the whole GPU's sweeps: one CTA
+// reads all arcs in every dense round.  Calls by one launch and by narrow
+// records, random graphs of n vertices and arcs: 300, 88 000 0.16 and 0.20 ms;
+// 1000, 120 000 0.28 and 0.21; 4000, 100 000 0.239 and 0.239; 8192, 80 000 0.23 and
+// 0.22; 8192, 500 000 0.92 and 0.32; grid of 90 x 90 0.38 and 0.95.
 constexpr int32_t SSSP_RESIDENT_N = 8192;
+constexpr int64_t SSSP_RESIDENT_ARCS = 100000;
 
 extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t *dist_out, float *ms_out, void *stream)
 {
@@ -1035,7 +1040,8 @@ extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t 
     // row 1 = {source}; rows of whole quads
     const int64_t ld = ((int64_t)n + 3) / 4 * 4;
     ResidentPlan plan;
-    const bool resident = n <= SSSP_RESIDENT_N && resident_plan(c, n, 0, 1, false, plan);  // the bound on n is the measured one
+    const bool resident =
+        n <= SSSP_RESIDENT_N && arcs <= SSSP_RESIDENT_ARCS && resident_plan(c, n, arcs, 1, false, plan);
     r = dev_reserve(c->table, sizeof(int32_t) * 2 * (size_t)ld);
     if (!r) r = prepare_subsets(c, 1, st);
     if (!r && !resident) r = reserve_relax(c, n);

@@ -765,3 +765,21 @@ def test_sweep_limit_holds_for_long_frontiers(emv, side, limit):
         with pytest.raises(emv.EmvError) as ei:
             s.solve(csr)
         assert ei.value.status == 5
+
+
+def test_sssp_of_many_arcs_takes_the_whole_gpu(emv, orc, solver):
+    """One CTA does not read all arcs of a dense graph: its kernel takes no more
+    than twice the time of the same graph with leaves past the one-launch limit."""
+    n, m = 8192, 500000
+    rng = np.random.default_rng(n)
+    ends = rng.integers(0, n, (m, 2))
+    ends = np.concatenate([ends[ends[:, 0] != ends[:, 1]], np.stack([np.arange(n - 1), np.arange(1, n)], 1)])
+    leaves = np.arange(n, 8200)
+    more = np.concatenate([ends, np.stack([leaves % n, leaves], 1)])
+    ms = []
+    for count, e in ((n, ends), (8200, more)):
+        w = rng.integers(1, 51, len(e))
+        g = emv.Csr.from_stp(emv.StpInstance(count, np.concatenate([e, w[:, None]], 1), np.array([0], np.int64)))
+        assert np.array_equal(solver.sssp(g, 1)[0], orc.sssp(g.n, g.row_ptr, g.col, g.w, 1))
+        ms.append(min(solver.sssp(g, 1)[1] for _ in range(5)))
+    assert ms[0] < 2 * ms[1]
