@@ -74,19 +74,32 @@ uint32_t res_inv_slices(int32_t n)
 // Whether a solve of n vertices over kt terminals' subsets runs as one
 // launch, and its shape.  The closure of a row needs about 7.3 bytes a vertex
 // of shared memory (distance, list entry, mark, arc count), so n is at most
-// about 31 000.  Levels of more rows than SMs (kt >= 10) take turns on them, and
-// arcs that do not fit shared memory are read again in every sweep, while the
-// record kernels read an arc once for 256 rows.  Kernel times here and there:
-// degree 8, kt = 10: n = 5800 0.62 and 1.57 ms, 12 000 1.15 and 1.83, 20 011 1.86
-// and 2.07; kt = 11, n = 12 000 2.05 and 2.84; degree 20, kt = 9: n = 10 000 1.13
-// and 1.57, 16 000 1.68 and 1.66, 20 011 2.08 and 1.89.
+// about 31 000.  A row is closed by one CTA, and arcs that do not fit shared
+// memory are read again in every round, while the record kernels read an arc
+// once for 256 rows and have the whole GPU for a level of few rows; the more
+// rows a level has, the more CTAs close some.  Whole calls into a device table,
+// one launch and record kernels in ms, k = 3 and k = 9:
+//   n = 8000, degree 36     0.49  0.48    1.36  1.62
+//   n = 20 000, degree 8    0.43  0.48    1.30  1.68
+//   n = 20 000, degree 12   0.49  0.43    1.47  1.65
+//   n = 30 000, degree 4    0.51  0.53    1.56  1.75
+//   n = 30 000, degree 8    0.60  0.48    1.86  1.83
+// and with irregular degrees and weights past the packed arcs (twice the bytes)
+//   n = 30 000, degree 8    0.94  0.47    2.91  2.14
+// Levels of more rows than SMs (kt >= 10) take turns on them and read the arcs
+// again each time: kernel times here and there, degree 8, kt = 10: n = 5800 0.62
+// and 1.57 ms, 12 000 1.15 and 1.83, 20 011 1.86 and 2.07; kt = 11, n = 12 000 2.05
+// and 2.84; calls, kt = 10: n = 12 000, degree 20 1.82 and 1.93, 14 000 2.08 and
+// 1.99; kt = 11: n = 16 384, degree 10 3.07 and 3.02, 14 000, degree 20 3.63 and
+// 3.11 (irregular degrees 3.72 and 3.03, 4.55 and 3.22).
 // host_table: the call copies the table to the host.  Past 2^22 cells that copy
 // outweighs the solve, and such calls keep the kernels whose value widths
 // emv_timing reports.
 constexpr int64_t RESIDENT_MAX_ARCS = 300000;
 bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, bool host_table, ResidentPlan &p)
 {
-    if (!resident_fits(n, kt) || arcs > RESIDENT_MAX_ARCS) return false;
+    const int64_t most = kt <= 9 ? 270000 + 9000 * kt : 320000 - 80000 * (kt - 10);
+    if (!resident_fits(n, kt) || arcs > RESIDENT_MAX_ARCS || arcs + 5 * (int64_t)n > most) return false;
     if (kt > 9 && n > 4096 && (n > 16384 || (host_table && (int64_t)n << kt > 1 << 22))) return false;
     const int sms = c->relax_sm_cap > 0 && c->relax_sm_cap < c->sms ? c->relax_sm_cap : c->sms;
     const int64_t maxcnt = resident_max_rows(kt);

@@ -783,3 +783,17 @@ def test_sssp_of_many_arcs_takes_the_whole_gpu(emv, orc, solver):
         assert np.array_equal(solver.sssp(g, 1)[0], orc.sssp(g.n, g.row_ptr, g.col, g.w, 1))
         ms.append(min(solver.sssp(g, 1)[1] for _ in range(5)))
     assert ms[0] < 2 * ms[1]
+
+
+@pytest.mark.parametrize("n,degree,k,wmax,one", [(20011, 8, 9, 100, True), (24000, 12, 5, 100, False), (30000, 4, 4, 100, True),
+                                                 (30000, 8, 4, 100, False), (20000, 14, 8, 30000, False),
+                                                 (4000, 20, 11, 100, True), (4000, 60, 12, 100, False)])
+def test_one_launch_for_as_many_arcs_as_it_reads_faster(emv, orc, solver, n, degree, k, wmax, one):
+    """Both sides of the line on vertices, arcs and terminals up to which a
+    small solve runs in one launch."""
+    csr = emv.Csr.from_stp(emv.StpInstance.regular(n + n * degree % 2, degree, 1, wmax, k, 29))
+    want, cost = orc.emv_table(csr.n, csr.row_ptr, csr.col, csr.w, csr.terminals, threads=16)
+    for table in (False, True):
+        res = solver.solve(csr, table=table)
+        assert res.cost == cost and (res.timing["relax_launches"] == 1) == one
+    assert np.array_equal(res.table, want)
