@@ -318,8 +318,10 @@ constexpr int32_t MERGE_SMEM_KMAX = 15;  // staged slots must fit 16 bits
 
 constexpr int32_t STREAM_SMEM_BYTES = 224 * 1024;
 
-// Plans the streamed merge of every level of k on the host (emv_plan.cpp)
-// and uploads the plan data and the per-launch phase descriptors.
+// Plans the streamed merge of the levels of k that have no block merge, on the
+// host (emv_plan.cpp), and uploads the plan data and the per-launch phase
+// descriptors.  (Of all levels: 24 of the 30 ms of a context's first solve, n =
+// 2000, k = 12.)
 int plan_stream_merge(emv_ctx *c, int32_t k, cudaStream_t st)
 {
     const std::vector<uint32_t> &xs = c->kp->xs_host;
@@ -328,7 +330,9 @@ int plan_stream_merge(emv_ctx *c, int32_t k, cudaStream_t st)
     if (k > MERGE_SMEM_KMAX) return EMV_OK;
     std::vector<uint32_t> data;
     std::vector<std::vector<HostGroup>> plan;
-    plan_stream_levels(k, xs, off, STREAM_SMEM_BYTES, data, plan);
+    std::vector<bool> block;
+    for (const BlockLevel &L : c->kp->mblock_levels) block.push_back(L.nphase > 0);
+    plan_stream_levels(k, xs, off, STREAM_SMEM_BYTES, data, plan, block);
     if (data.empty()) return EMV_OK;
     int r = dev_reserve(c->kp->mstream_data, sizeof(uint32_t) * data.size());
     if (r) return r;
@@ -440,11 +444,11 @@ static int build_plan(emv_ctx *c, int32_t k, cudaStream_t st)
     if (r) return r;
     CUDA_TRY(cudaMemcpyAsync(c->kp->xs.ptr, c->kp->xs_host.data(), sizeof(uint32_t) * c->kp->xs_host.size(),
                              cudaMemcpyHostToDevice, st));
-    r = plan_stream_merge(c, k, st);
-    if (!r) r = plan_block_merge(c, k, st);
+    r = plan_block_merge(c, k, st);
+    if (!r) r = plan_stream_merge(c, k, st);
     if (r) return r;
     // Pair and override slot lists of the staged-all-rows merge, for the levels
-    // the streamed merge has no plan for (level order).
+    // the others have no plan for (level order).
     c->kp->mpair_base.assign((size_t)k + 2, 0);
     c->kp->movr_base.assign((size_t)k + 2, 0);
     std::vector<uint32_t> pairs, ovr;
@@ -454,7 +458,7 @@ static int build_plan(emv_ctx *c, int32_t k, cudaStream_t st)
         for (int32_t m = 2; m <= k; m++) {
             c->kp->mpair_base[(size_t)m] = (int64_t)pairs.size();
             c->kp->movr_base[(size_t)m] = (int64_t)ovr.size();
-            if (!c->kp->mstream_groups[(size_t)m].empty()) continue;
+            if (c->kp->mblock_levels[(size_t)m].nphase > 0 || !c->kp->mstream_groups[(size_t)m].empty()) continue;
             for (int64_t i = c->kp->xs_off[(size_t)m]; i < c->kp->xs_off[(size_t)m + 1]; i++) {
                 const uint32_t X = c->kp->xs_host[(size_t)i];
                 const uint32_t low = X & (0u - X), rest = X ^ low;
@@ -520,15 +524,15 @@ int launch_merge(emv_ctx *c, int32_t *table, int64_t ld, int32_t n, int32_t k, i
     cudaError_t e = cudaSuccess;
     c->merge16_last = false;
     c->launches++;
-    if (k <= MERGE_SMEM_KMAX && !c->kp->mstream_groups[(size_t)m].empty()) {
-        // the streamed merge records the level's largest value (other kernels leave it unknown)
+    const BlockLevel &L = c->kp->mblock_levels[(size_t)m];
+    if (L.nphase > 0 || !c->kp->mstream_groups[(size_t)m].empty()) {
+        // these merges record the level's largest value (other kernels leave it unknown)
         CUDA_TRY(cudaMemsetAsync((uint32_t *)c->lvlmax.ptr + m, 0, sizeof(uint32_t), st));
         const int64_t b = c->kp->xs_off[(size_t)m];
-        c->launches += (int64_t)c->kp->mstream_groups[(size_t)m].size() - 1;
+        if (L.nphase == 0) c->launches += (int64_t)c->kp->mstream_groups[(size_t)m].size() - 1;
         // 16-bit staging reads int2 pairs of vertices: even stride and base
         u16 = u16 && ld % 2 == 0 && ((uintptr_t)table & 7) == 0;
         c->merge16_last = u16;
-        const BlockLevel &L = c->kp->mblock_levels[(size_t)m];
         if (L.nphase > 0) {
             const int32_t cnt = (int32_t)(c->kp->xs_off[(size_t)m + 1] - b);
             const int64_t acc = (u16 && L.split ? 2 : 1) * cnt;

@@ -149,7 +149,8 @@ bool plan_level(const std::vector<uint32_t> &xs, const std::vector<int64_t> &off
 }  // namespace
 
 void plan_stream_levels(int32_t k, const std::vector<uint32_t> &xs, const std::vector<int64_t> &off,
-                        int64_t smem_bytes, std::vector<uint32_t> &data, std::vector<std::vector<HostGroup>> &plan)
+                        int64_t smem_bytes, std::vector<uint32_t> &data, std::vector<std::vector<HostGroup>> &plan,
+                        const std::vector<bool> &skip)
 {
     std::vector<uint32_t> rank((size_t)1 << k, 0);  // position within its level
     for (int32_t m = 1; m <= k; m++)
@@ -160,6 +161,7 @@ void plan_stream_levels(int32_t k, const std::vector<uint32_t> &xs, const std::v
     data.clear();
     plan.assign((size_t)k + 2, {});
     for (int32_t m = 2; m <= k; m++) {
+        if ((size_t)m < skip.size() && skip[(size_t)m]) continue;
         const int64_t cnt = off[(size_t)m + 1] - off[(size_t)m];
         int64_t best_cost = -1;
         for (int64_t gx : {cnt, (int64_t)1024, (int64_t)768, (int64_t)512, (int64_t)384, (int64_t)256, (int64_t)128}) {

@@ -58,10 +58,12 @@ struct HostGroup {
 int64_t stream_acc_rows(int64_t g);
 
 // Plans every level 2..k into data (all offsets relative to its start, blocks
-// read as uint4 16-byte aligned); plan[m] is empty for a level that cannot
-// be streamed within smem_bytes of shared memory.
+// read as uint4 16-byte aligned), but for those with skip[m] set; plan[m] is
+// empty for a level that is left out or cannot be streamed within smem_bytes of
+// shared memory.
 void plan_stream_levels(int32_t k, const std::vector<uint32_t> &xs, const std::vector<int64_t> &off,
-                        int64_t smem_bytes, std::vector<uint32_t> &data, std::vector<std::vector<HostGroup>> &plan);
+                        int64_t smem_bytes, std::vector<uint32_t> &data, std::vector<std::vector<HostGroup>> &plan,
+                        const std::vector<bool> &skip = {});
 
 // Block merge of a level: the terminals are split into the low bits `low` and
 // the others, X = (Xh, Xl).  A unit is one Xh, whose subsets of the level, Xl of

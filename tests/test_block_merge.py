@@ -47,3 +47,52 @@ def test_whole_tables(emv, orc, n, k, wmax, bits):
         s.set_value_bits(bits)
         res = s.solve(csr, table=True)
         assert res.cost == cost and np.array_equal(res.table, want)
+
+
+SKIP_CHECK = r"""
+#include <cstdio>
+#include <cstdlib>
+#include "emv_plan.h"
+using namespace emv;
+int main(int, char **argv)
+{
+    const int k = atoi(argv[1]);
+    std::vector<uint32_t> xs, all, some, blocks;
+    std::vector<int64_t> off;
+    subset_levels(k, xs, off);
+    std::vector<std::vector<HostGroup>> whole, part;
+    std::vector<HostBlockLevel> block;
+    plan_block_levels(k, BLOCK_LOW, xs, off, 224 * 1024, blocks, block);
+    std::vector<bool> skip;
+    for (const HostBlockLevel &L : block) skip.push_back(!L.phases.empty());
+    plan_stream_levels(k, xs, off, 224 * 1024, all, whole);
+    plan_stream_levels(k, xs, off, 224 * 1024, some, part, skip);
+    for (int m = 2; m <= k; m++) {
+        if (skip[m] != part[m].empty()) return printf("level %d\n", m), 1;
+        if (skip[m]) continue;
+        if (part[m].size() != whole[m].size()) return printf("groups of level %d\n", m), 1;
+        for (size_t g = 0; g < part[m].size(); g++)
+            for (size_t p = 0; p < part[m][g].phases.size(); p++) {
+                const HostPhase &a = part[m][g].phases[p], &b = whole[m][g].phases[p];
+                if (a.nrows != b.nrows || a.pairs_at % 4) return printf("phase of level %d\n", m), 1;
+                for (int i = 0; i < a.nrows; i++)
+                    if (some[a.rows_at + i] != all[b.rows_at + i]) return printf("rows of level %d\n", m), 1;
+            }
+    }
+    printf("ok %d\n", some.size() * 4 < all.size());
+}
+"""
+
+
+@pytest.mark.parametrize("k", [6, 9, 11])
+def test_levels_with_a_block_merge_have_no_streamed_plan(tmp_path, k):
+    """The streamed plan of the other levels is as without the omission, and
+    the whole a fraction of the plan of all levels."""
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("g++ not found")
+    src, exe = tmp_path / "skip.cpp", tmp_path / "skip"
+    src.write_text(SKIP_CHECK)
+    subprocess.run([gxx, "-O1", "-std=c++17", "-I", CSRC, str(src), os.path.join(CSRC, "emv_plan.cpp"), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe), str(k)], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0 and out.stdout == "ok 1\n", out.stdout + out.stderr
