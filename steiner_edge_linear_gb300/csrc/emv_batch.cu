@@ -173,16 +173,19 @@ int batch_kernel_setup(emv_ctx *c)
     return EMV_OK;
 }
 
+// Whether some team has more than one CTA.
+static bool batch_teams(const BatchArgs &a) { return a.end[BATCH_SIZES - 2] > 0; }
+
 // Launches k_batch on `blocks` CTAs over prepared descriptors.  Teams wait for
 // their CTAs, so the launch is cooperative unless every team is a single CTA.
 int launch_batch(emv_ctx *c, const BatchArgs &args, int32_t blocks, cudaStream_t st)
 {
     int r = batch_kernel_setup(c);
     if (r) return r;
-    CUDA_TRY(cudaMemsetAsync(args.ctl, 0, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(blocks), st));
+    CUDA_TRY(cudaMemsetAsync(args.ctl, 0, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(c->batch_blocks), st));
     BatchArgs a = args;
     void *p[] = {&a};
-    if (a.end[BATCH_SIZES - 2] > 0)
+    if (batch_teams(a))
         CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_batch, dim3((unsigned)blocks), dim3(RES_THREADS), p,
                                              (size_t)RESIDENT_SMEM, st));
     else
@@ -509,7 +512,7 @@ int64_t batch_arc_stride(int64_t arc_bytes) { return std::max<int64_t>(256, (arc
 BatchArgs batch_args(emv_ctx *c, const BatchPack &pk)
 {
     BatchArgs a;
-    std::memset(&a, 0, sizeof(a));  // padding included: the graph cache compares bytes
+    std::memset(&a, 0, sizeof(a));
     const BatchLane &L = c->blane[pk.lane];
     a.inst = (const BatchInst *)L.desc.ptr;
     a.xs = (const uint32_t *)c->bxs.ptr;
@@ -523,43 +526,60 @@ BatchArgs batch_args(emv_ctx *c, const BatchPack &pk)
     return a;
 }
 
-// Captures {control reset, persistent kernel} once per argument set and replays it.
+// Launches {control reset, persistent kernel} as one graph, captured once per
+// lane and kind of launch.  The arguments of another batch (its classes, its
+// CTAs) go into the kernel's node: a capture and its instantiation for each took
+// as long as the solve of a few small instances.
 int batch_graph_launch(emv_ctx *c, int32_t lane, const BatchArgs &a, int32_t blocks, cudaStream_t st)
 {
-    BatchLane &L = c->blane[lane];
     int r = batch_kernel_setup(c);
     if (r) return r;
-    static_assert(sizeof(BatchArgs) <= sizeof(L.graph_args), "graph key too small");
-    const bool same = L.graph && L.graph_blocks == blocks && std::memcmp(L.graph_args, &a, sizeof(a)) == 0;
-    if (!same) {
-        if (L.graph) cudaGraphExecDestroy(L.graph);
-        L.graph = nullptr;
+    BatchGraphExec &G = c->blane[lane].graph[batch_teams(a)];
+    if (!G.exec || G.ctl != a.ctl) {
+        batch_graph_release(G);
         cudaStream_t cap;
         CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-        cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             r = launch_batch(c, a, blocks, cap);
-            e = cudaStreamEndCapture(cap, &g);
+            e = cudaStreamEndCapture(cap, &G.graph);
         }
         cudaStreamDestroy(cap);
-        if (r) return r;
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            return emv_fail(EMV_ERR_CUDA, "batch graph capture: %s", cudaGetErrorString(e));
+        size_t count = 8;
+        cudaGraphNode_t nodes[8];
+        if (!r && e == cudaSuccess) e = cudaGraphGetNodes(G.graph, nodes, &count);
+        for (size_t i = 0; !r && e == cudaSuccess && i < count; i++) {
+            cudaGraphNodeType type;
+            e = cudaGraphNodeGetType(nodes[i], &type);
+            if (e == cudaSuccess && type == cudaGraphNodeTypeKernel) G.node = nodes[i];
         }
-        e = cudaGraphInstantiate(&L.graph, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) {
+        if (!r && e == cudaSuccess) e = cudaGraphInstantiate(&G.exec, G.graph, 0);
+        if (r || e != cudaSuccess || !G.node) {
             cudaGetLastError();
-            L.graph = nullptr;
-            return emv_fail(EMV_ERR_CUDA, "batch graph instantiate: %s", cudaGetErrorString(e));
+            batch_graph_release(G);
+            return r ? r : emv_fail(EMV_ERR_CUDA, "batch graph: %s", cudaGetErrorString(e));
         }
-        std::memcpy(L.graph_args, &a, sizeof(a));
-        L.graph_blocks = blocks;
+        G.ctl = a.ctl;
+    } else {
+        BatchArgs args = a;
+        void *p[] = {&args};
+        cudaKernelNodeParams kp = {};
+        kp.func = (void *)k_batch;
+        kp.gridDim = dim3((unsigned)blocks);
+        kp.blockDim = dim3(RES_THREADS);
+        kp.sharedMemBytes = RESIDENT_SMEM;
+        kp.kernelParams = p;
+        CUDA_TRY(cudaGraphExecKernelNodeSetParams(G.exec, G.node, &kp));
     }
-    CUDA_TRY(cudaGraphLaunch(L.graph, st));
+    CUDA_TRY(cudaGraphLaunch(G.exec, st));
     return EMV_OK;
+}
+
+void batch_graph_release(BatchGraphExec &G)
+{
+    if (G.exec) cudaGraphExecDestroy(G.exec);
+    if (G.graph) cudaGraphDestroy(G.graph);
+    G = BatchGraphExec();
 }
 
 // --------------------------------------------------------------- autotuner

@@ -159,7 +159,7 @@ extern "C" int emv_destroy(emv_ctx *c)
         if (c->evmax[i]) cudaEventDestroy(c->evmax[i]);
     for (BatchLane &L : c->blane) {
         for (DevBuf *b : {&L.row, &L.adj, &L.term, &L.desc, &L.table, &L.ctrl, &L.arcs}) dev_release(*b);
-        if (L.graph) cudaGraphExecDestroy(L.graph);
+        for (BatchGraphExec &G : L.graph) batch_graph_release(G);
         if (L.stage) cudaFreeHost(L.stage);
     }
     for (cudaEvent_t e : c->bev)

@@ -61,6 +61,15 @@ struct KPlan {
     std::vector<BlockLevel> mblock_levels;                 // per level (nphase 0 = no block merge)
 };
 
+// A captured launch of the batched kernel, and the node its arguments go into.
+struct BatchGraphExec {
+    cudaGraph_t graph = nullptr;
+    cudaGraphNode_t node = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    const void *ctl = nullptr;     // the control words it resets
+};
+void batch_graph_release(BatchGraphExec &G);
+
 // Buffers of one launch of the batched kernel.  A large batch runs as two
 // launches, so that the host packs the second while the first is on the GPU.
 constexpr int BATCH_LANES = 2;
@@ -68,9 +77,7 @@ struct BatchLane {
     DevBuf row, adj, term, desc, table, ctrl, arcs;
     void *stage = nullptr;         // pinned staging of the packed instances
     size_t stage_bytes = 0;
-    cudaGraphExec_t graph = nullptr;
-    char graph_args[160] = {};     // BatchArgs of the captured graph
-    int32_t graph_blocks = 0;      // and its CTAs
+    BatchGraphExec graph[2];       // single-CTA teams; teams (a cooperative launch)
 };
 
 struct emv_ctx {

@@ -237,3 +237,24 @@ def test_batch_in_two_launches(emv):
                 s.batch_solve(bad)
             assert ei.value.status == 1 and f"instance {min(faulty)}:" in str(ei.value)
         assert np.array_equal(s.batch_solve(graphs)[0], costs)
+
+
+def test_batches_of_other_shapes_replay_the_same_graph(emv):
+    """Batches whose classes, CTAs and slices differ are launched without a new
+    capture (40 us of 130): taking turns costs at most a fifth more than the
+    slower of them alone."""
+    shapes = [[emv.Csr.from_stp(emv.StpInstance.regular(n, 4, 1, 9, 4, i)) for i in range(count)]
+              for n, count in ((64, 3), (96, 4), (64, 1))]
+    with emv.Solver(0) as s:
+        want = [[s.solve(g).cost for g in graphs] for graphs in shapes]
+
+        def timed(graphs):
+            t0 = time.perf_counter()
+            costs, _ = s.batch_solve(graphs)
+            took = time.perf_counter() - t0
+            assert list(costs) == want[shapes.index(graphs)]
+            return took
+
+        alone = [np.median([timed(graphs) for _ in range(40)]) for graphs in shapes]
+        turns = np.median([timed(shapes[i % 3]) for i in range(120)])
+    assert turns < 1.2 * max(alone)
