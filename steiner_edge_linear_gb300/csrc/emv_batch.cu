@@ -19,6 +19,7 @@
 #include <vector>
 
 constexpr int32_t BATCH_CUT_MIN = 768;
+constexpr int32_t BATCH_FEW_BLOCKS = 16;
 
 namespace {
 
@@ -271,40 +272,57 @@ static int batch_solve(emv_ctx *c, const emv_instance *inst, int32_t count, int6
     const bool whole = tables_out != nullptr;
     std::vector<int32_t> ids((size_t)count);
     for (int32_t i = 0; i < count; i++) ids[(size_t)i] = i;
-    const BatchOrder ord = batch_order(c, inst, ids, whole, 0);
-    const int32_t cut = batch_cut(ord);
+    BatchOrder ord = batch_order(c, inst, ids, whole, 0);
+    int32_t cut = batch_cut(ord);
     BatchPack pk[BATCH_LANES];
     BatchArgs a[BATCH_LANES];
-    const int lanes = cut < count ? 2 : 1;
-    CUDA_TRY(cudaEventRecord(c->bev[0], st));  // the second lane starts behind the caller's work too
-    int status = EMV_OK;
-    bool failed = false;
+    int lanes = 1;
     auto check = [&](int32_t i) { return check_arrays(i); };
-    for (int l = 0; l < lanes && !status && !failed; l++) {
-        cudaStream_t ls = l ? c->bstream : st;
-        pk[l].lane = l;
-        status = batch_layout(c, inst, ord, l ? cut : 0, l ? count : cut, whole, 0, pk[l]);
-        if (!status) status = batch_fill(c, inst, pk[l], check);
-        for (const BatchInst &d : pk[l].desc) failed |= bad[(size_t)d.orig] != 0;
-        if (status || failed) break;
-        if (l) CUDA_TRY(cudaStreamWaitEvent(ls, c->bev[0], 0));
-        status = batch_upload(c, pk[l], ls);
-        if (status) break;
-        a[l] = batch_args(c, pk[l]);
-        if (l == 0) CUDA_TRY(cudaEventRecord(c->ev[0], st));
-        // The control reset and the persistent launch are replayed as one CUDA graph.
-        status = batch_graph_launch(c, l, a[l], pk[l].blocks, ls);
-        if (!status && l) {
-            CUDA_TRY(cudaEventRecord(c->bev[1], ls));
-            CUDA_TRY(cudaStreamWaitEvent(st, c->bev[1], 0));
+    // A batch whose memory cannot be had in two parts with room to spare is solved
+    // as one, in buffers of its size, at last with the arc slices of a few CTAs or one.
+    bool spare = true;
+    for (int32_t blocks = 0;;) {
+        lanes = cut < count ? 2 : 1;
+        CUDA_TRY(cudaEventRecord(c->bev[0], st));  // the second lane starts behind the caller's work too
+        int status = EMV_OK;
+        bool failed = false;
+        for (int l = 0; l < lanes && !status && !failed; l++) {
+            cudaStream_t ls = l ? c->bstream : st;
+            pk[l].lane = l;
+            status = batch_layout(c, inst, ord, l ? cut : 0, l ? count : cut, whole, blocks, pk[l]);
+            if (!status) status = batch_fill(c, inst, pk[l], check);
+            for (const BatchInst &d : pk[l].desc) failed |= bad[(size_t)d.orig] != 0;
+            if (status || failed) break;
+            if (l) CUDA_TRY(cudaStreamWaitEvent(ls, c->bev[0], 0));
+            status = batch_upload(c, pk[l], spare, ls);
+            if (status) break;
+            a[l] = batch_args(c, pk[l]);
+            if (l == 0) CUDA_TRY(cudaEventRecord(c->ev[0], st));
+            // The control reset and the persistent launch are replayed as one CUDA graph.
+            status = batch_graph_launch(c, l, a[l], pk[l].blocks, ls);
+            if (!status && l) {
+                CUDA_TRY(cudaEventRecord(c->bev[1], ls));
+                CUDA_TRY(cudaStreamWaitEvent(st, c->bev[1], 0));
+            }
         }
-    }
-    if (status || failed) {
+        if (!status && !failed) break;
         if (failed && lanes == 2 && pk[1].desc.empty())  // the second part was not looked at yet
             host_parallel_for(count - cut, [&](int64_t j) { check_arrays(ord.ids[(size_t)(cut + j)]); });
         CUDA_TRY(cudaStreamSynchronize(c->bstream));
         CUDA_TRY(cudaStreamSynchronize(st));
-        return failed ? first_bad() : status;
+        if (failed) return first_bad();
+        if (status != EMV_ERR_OOM || blocks == 1) return status;
+        for (int l = 0; l < BATCH_LANES; l++) {
+            BatchLane &L = c->blane[l];
+            for (DevBuf *b : {&L.row, &L.adj, &L.term, &L.desc, &L.table, &L.arcs}) dev_release(*b);
+            pk[l] = BatchPack();
+        }
+        if (!spare) {
+            blocks = blocks == 0 ? BATCH_FEW_BLOCKS : 1;
+            ord = batch_order(c, inst, ids, whole, blocks);
+        }
+        spare = false;
+        cut = count;
     }
     CUDA_TRY(cudaEventRecord(c->ev[1], st));
     CUDA_TRY(cudaMemcpyAsync(costs_out, c->b_costs.ptr, sizeof(int64_t) * (size_t)count, cudaMemcpyDeviceToHost, st));
@@ -474,19 +492,20 @@ static int reserve_more(DevBuf &b, size_t bytes)
     return dev_reserve(b, bytes + bytes / 4) == EMV_OK ? (int)EMV_OK : dev_reserve(b, bytes);
 }
 
-int batch_upload(emv_ctx *c, BatchPack &pk, cudaStream_t st)
+int batch_upload(emv_ctx *c, BatchPack &pk, bool spare, cudaStream_t st)
 {
     BatchLane &L = c->blane[pk.lane];
-    int r = reserve_more(L.row, sizeof(int32_t) * (size_t)pk.rows);
-    if (!r) r = reserve_more(L.adj, sizeof(int2) * (size_t)std::max<int64_t>(pk.arcs, 1));
-    if (!r) r = reserve_more(L.term, sizeof(int32_t) * (size_t)std::max<int64_t>(pk.terms, 1));
-    if (!r) r = reserve_more(L.desc, sizeof(BatchInst) * (size_t)pk.count);
-    if (!r) r = reserve_more(L.table, sizeof(int32_t) * (size_t)pk.table_words);
+    auto reserve = spare ? reserve_more : dev_reserve;
+    int r = reserve(L.row, sizeof(int32_t) * (size_t)pk.rows);
+    if (!r) r = reserve(L.adj, sizeof(int2) * (size_t)std::max<int64_t>(pk.arcs, 1));
+    if (!r) r = reserve(L.term, sizeof(int32_t) * (size_t)std::max<int64_t>(pk.terms, 1));
+    if (!r) r = reserve(L.desc, sizeof(BatchInst) * (size_t)pk.count);
+    if (!r) r = reserve(L.table, sizeof(int32_t) * (size_t)pk.table_words);
     // costs are written at index orig (the caller's instance index), which can
     // exceed the number of instances in this launch when it is a part or a sample
     if (!r) r = dev_reserve(c->b_costs, sizeof(int64_t) * (size_t)std::max<int64_t>(pk.cost_slots, 1));
     if (!r) r = dev_reserve(L.ctrl, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(c->batch_blocks));
-    if (!r) r = reserve_more(L.arcs, (size_t)batch_arc_stride(pk.arc_bytes) * (size_t)pk.blocks);
+    if (!r) r = reserve(L.arcs, (size_t)batch_arc_stride(pk.arc_bytes) * (size_t)pk.blocks);
     if (!r) r = prepare_batch_subsets(c, st);
     if (r) return r;
     for (int32_t j = 0; j < pk.count; j++) {
@@ -600,7 +619,7 @@ int time_sample(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t>
         r = batch_layout(c, inst, ord, 0, (int32_t)ids.size(), false, blocks, pk);
     }
     if (!r) r = batch_fill(c, inst, pk, nullptr);
-    if (!r) r = batch_upload(c, pk, st);
+    if (!r) r = batch_upload(c, pk, true, st);
     if (r) return r;
     BatchArgs a = batch_args(c, pk);
     ms = 1e30f;

@@ -59,7 +59,8 @@ int batch_layout(emv_ctx *c, const emv_instance *inst, const BatchOrder &ord, in
 // Fills the staging from the instances; check(i) is called for each before it
 // is read and says whether to.
 int batch_fill(emv_ctx *c, const emv_instance *inst, BatchPack &pk, const std::function<bool(int32_t)> &check);
-int batch_upload(emv_ctx *c, BatchPack &pk, cudaStream_t st);
+// spare: buffers that grow take a quarter more where it is free.
+int batch_upload(emv_ctx *c, BatchPack &pk, bool spare, cudaStream_t st);
 emv::BatchArgs batch_args(emv_ctx *c, const BatchPack &pk);
 int launch_batch(emv_ctx *c, const emv::BatchArgs &a, int32_t blocks, cudaStream_t st);
 int batch_graph_launch(emv_ctx *c, int32_t lane, const emv::BatchArgs &a, int32_t blocks, cudaStream_t st);

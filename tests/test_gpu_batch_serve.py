@@ -1,6 +1,7 @@
 """Batched launch and continuous-batching server: every cost equals the
 single-instance solve and the oracle, alone and in the mix; the batched
 launch's whole tables equal the reference-written golden tables."""
+import ctypes
 import time
 
 import numpy as np
@@ -258,3 +259,30 @@ def test_batches_of_other_shapes_replay_the_same_graph(emv):
         alone = [np.median([timed(graphs) for _ in range(40)]) for graphs in shapes]
         turns = np.median([timed(shapes[i % 3]) for i in range(120)])
     assert turns < 1.2 * max(alone)
+
+
+@pytest.mark.parametrize("count,n,k", [(800, 1000, 8), (4, 20000, 10)])
+def test_batch_tables_that_just_fit_the_device(emv, count, n, k):
+    """A batch whose tables and graphs take nearly all free memory (all but 24 MB,
+    a page of 2 MB for each of a dozen buffers) is solved, in one launch
+    instead of two and without spare room, and so is the next."""
+    torch = pytest.importorskip("torch")
+    cudart = ctypes.CDLL("libcudart.so")
+    cudart.cudaMalloc.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_size_t]
+    cudart.cudaFree.argtypes = [ctypes.c_void_p]
+    one = [emv.Csr.from_stp(emv.StpInstance.regular(n, 4, 1, 9, k, seed)) for seed in range(4)]
+    graphs = [one[i % 4] for i in range(count)]
+    need = count * ((4 * n << k) + 4 * (n + 1) + 8 * graphs[0].arcs)
+    with emv.Solver(0) as s:
+        s.batch_solve([emv.Csr.from_stp(emv.StpInstance.regular(64, 4, 1, 9, 4, 1))])
+        want = [s.solve(g, table=True) for g in one]
+        free = torch.cuda.mem_get_info(0)[0]
+        held = ctypes.c_void_p()
+        assert cudart.cudaMalloc(ctypes.byref(held), free - need - (24 << 20)) == 0
+        try:
+            costs, _, tables = s.batch_solve(graphs, tables=True)
+        finally:
+            cudart.cudaFree(held)
+        assert list(costs) == [want[i % 4].cost for i in range(count)]
+        assert all(np.array_equal(t, want[i % 4].table) for i, t in enumerate(tables))
+        assert np.array_equal(s.batch_solve(graphs)[0], costs)
