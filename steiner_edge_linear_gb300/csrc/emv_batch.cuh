@@ -47,7 +47,7 @@ __device__ __forceinline__ bool batch_class(const BatchArgs &a, int32_t c, int32
         if (threadIdx.x == 0) {
             I.row_ptr = B->row_ptr;
             I.adj = B->adj;
-            I.slices = a.scratch + (int64_t)(blockIdx.x - tm.rank) * a.scratch_stride;
+            I.slices = B->slices ? B->slices : a.scratch + (int64_t)(blockIdx.x - tm.rank) * a.scratch_stride;
             I.table = table;
             I.cost = a.costs + B->orig;
             I.unreached = nullptr;

@@ -30,8 +30,8 @@ int32_t batch_class_of(int32_t n, int32_t k);
 bool batch_fits(int32_t n, int32_t k);
 // What the kernel needs to know of a host graph beyond its sizes.
 struct BatchGraph {
-    bool narrow;         // every weight fits a packed arc
-    int64_t arc_bytes;   // sliced arcs
+    bool narrow = false;      // every weight fits a packed arc
+    int64_t arc_bytes = 0;    // sliced arcs
 };
 BatchGraph batch_graph(const int32_t *row_ptr, const int32_t *w, int32_t n, int64_t arcs);
 // Estimated time (us) of levels lo..hi on one CTA.

@@ -32,6 +32,7 @@ struct BatchInst {
     int32_t lo;              // first level to run (1..kt)
     int32_t hi;              // last level to run (lo..kt)
     int32_t pad;
+    char *slices;            // its sliced arcs, or null: in BatchArgs::scratch
 };
 
 struct BatchArgs {

@@ -53,7 +53,7 @@ struct Req {
     bool cancel = false;
     int32_t next_level = 1;
     bool narrow = false;      // BatchGraph of the request
-    int64_t arc_bytes = 0;
+    int64_t arc_bytes = 0;    // of its sliced arcs
     int32_t slot = -1;
     int64_t cost = 0;
     int status = EMV_OK;
@@ -62,12 +62,19 @@ struct Req {
     int32_t *d_row = nullptr;
     int2 *d_adj = nullptr;
     int32_t *d_terms = nullptr;
-    int32_t *d_table = nullptr;
+    int32_t *d_table = nullptr;  // and, table_bytes behind it, the sliced arcs
 };
 
-int64_t footprint(int32_t n, int32_t k, int64_t arcs)
+// The table of a small request: the rows of its first k - 1 terminals.
+int64_t table_bytes(int32_t n, int32_t k) { return (((int64_t)batch_ld(n) << table_terminals(k)) * 4 + 255) / 256 * 256; }
+
+// What a request is charged against the budget: 2^k * n * 4 bytes of table and
+// the graph, or, where that is more, what a small one takes on the device: its
+// table, the graph and its sliced arcs.
+int64_t footprint(int32_t n, int32_t k, int64_t arcs, int64_t slices)
 {
-    return ((int64_t)n << k) * 4 + (int64_t)(n + 1) * 4 + arcs * 8 + (int64_t)k * 4;
+    const int64_t graph = (int64_t)(n + 1) * 4 + arcs * 8 + (int64_t)k * 4;
+    return graph + std::max(((int64_t)n << k) * 4, table_bytes(n, k) + slices);
 }
 
 }  // namespace
@@ -90,7 +97,7 @@ struct emv_server {
     cudaStream_t st_small = nullptr, st_large = nullptr;
     // wave buffers
     std::vector<int32_t> free_slots;
-    DevBuf d_desc, d_costs, d_ctrl, d_arcs;
+    DevBuf d_desc, d_costs, d_ctrl;
     BatchInst *h_desc = nullptr;
     int64_t *h_costs = nullptr;
     int32_t cap_slots = 0;
@@ -133,7 +140,8 @@ int stage_small(emv_server *s, Req *r, std::vector<int2> &adj)
     if (cudaMallocAsync((void **)&r->d_row, sizeof(int32_t) * ((size_t)r->n + 1), st) != cudaSuccess ||
         cudaMallocAsync((void **)&r->d_adj, sizeof(int2) * arcs, st) != cudaSuccess ||
         cudaMallocAsync((void **)&r->d_terms, sizeof(int32_t) * (size_t)r->k, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&r->d_table, sizeof(int32_t) * ((size_t)batch_ld(r->n) << table_terminals(r->k)), st) != cudaSuccess) {
+        cudaMallocAsync((void **)&r->d_table, (size_t)(table_bytes(r->n, r->k) + batch_arc_stride(r->arc_bytes)), st) !=
+            cudaSuccess) {
         cudaGetLastError();
         return emv_fail(EMV_ERR_OOM, "server: device allocation for request %lld", (long long)r->id);
     }
@@ -236,7 +244,7 @@ void scheduler(emv_server *s)
         batch_plan(work, states, most, alone ? 1 << (BATCH_SIZES - 1) : 1, order, size);
         BatchArgs a;
         std::memset(&a, 0, sizeof(a));
-        int64_t ctas = 0, arc_bytes = 0;
+        int64_t ctas = 0;
         for (size_t j = 0; j < wave.size(); j++) {
             const Req *r = wave[(size_t)order[j]];
             BatchInst &d = s->h_desc[j];
@@ -251,12 +259,12 @@ void scheduler(emv_server *s)
             d.size = size[(size_t)order[j]];
             batch_shape(s->ctx_small, d);
             d.narrow = r->narrow;
+            d.slices = (char *)r->d_table + table_bytes(r->n, r->k);
             d.orig = r->slot;
             d.lo = d.hi = r->next_level;
             for (int32_t cl = 0; cl < BATCH_SIZES; cl++)
                 if (d.size >= 1 << (BATCH_SIZES - 1 - cl)) a.end[cl] = (int32_t)j + 1;
             ctas += d.size;
-            arc_bytes = std::max(arc_bytes, r->arc_bytes);
         }
         const int32_t blocks = batch_blocks(s->ctx_small, ctas, cap);
         a.inst = (const BatchInst *)s->d_desc.ptr;
@@ -265,12 +273,9 @@ void scheduler(emv_server *s)
         a.costs = (int64_t *)s->d_costs.ptr;
         a.ctl = (uint32_t *)s->d_ctrl.ptr;
         a.smem = RESIDENT_SMEM;
-        a.scratch_stride = batch_arc_stride(arc_bytes);
-        // grows when a request brings longer arc slices than any before
-        int st = dev_reserve(s->d_arcs, (size_t)a.scratch_stride * (size_t)batch_blocks(s->ctx_small, INT32_MAX, 0));
-        a.scratch = (char *)s->d_arcs.ptr;
         uint32_t err = 0;
-        if (!st && cudaMemcpyAsync(s->d_desc.ptr, s->h_desc, sizeof(BatchInst) * wave.size(), cudaMemcpyHostToDevice,
+        int st = EMV_OK;
+        if (cudaMemcpyAsync(s->d_desc.ptr, s->h_desc, sizeof(BatchInst) * wave.size(), cudaMemcpyHostToDevice,
                             s->st_small) != cudaSuccess)
             st = emv_fail(EMV_ERR_CUDA, "server: descriptor upload");
         if (!st) st = launch_batch(s->ctx_small, a, blocks, s->st_small);
@@ -373,7 +378,6 @@ void server_free(emv_server *s)
     dev_release(s->d_desc);
     dev_release(s->d_costs);
     dev_release(s->d_ctrl);
-    dev_release(s->d_arcs);
     if (s->h_desc) cudaFreeHost(s->h_desc);
     if (s->h_costs) cudaFreeHost(s->h_costs);
     if (s->st_small) cudaStreamDestroy(s->st_small);
@@ -428,8 +432,6 @@ extern "C" int emv_server_create(emv_server **out, const emv_server_opts *opts)
     if (!st) st = prepare_batch_subsets(s->ctx_small, s->st_small);
     if (!st) st = batch_kernel_setup(s->ctx_small);
     if (!st) st = dev_reserve(s->d_ctrl, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(s->ctx_small->batch_blocks));
-    // arc slices of up to 4096 vertices and 32 arcs each; longer ones grow it
-    if (!st) st = dev_reserve(s->d_arcs, (size_t)(4096 * 32 * 4) * (size_t)s->ctx_small->batch_blocks);
     // keep freed pool memory cached in the process (no release at stream syncs)
     cudaMemPool_t pool;
     if (!st && cudaDeviceGetDefaultMemPool(&pool, opts->device) == cudaSuccess) {
@@ -458,7 +460,9 @@ extern "C" int emv_server_submit(emv_server *s, const emv_graph *g, const int32_
         if (terminals[i] < 0 || terminals[i] >= g->n) return emv_fail(EMV_ERR_BAD_INPUT, "terminal out of range");
     st = emv_graph_check(g, nullptr);
     if (st) return st;
-    const int64_t bytes = footprint(g->n, k, g->arcs);
+    const bool large = g->n >= s->opts.large_n || !batch_fits(g->n, k);
+    const BatchGraph bg = large ? BatchGraph{} : batch_graph(g->row_ptr, g->w, g->n, g->arcs);
+    const int64_t bytes = footprint(g->n, k, g->arcs, bg.arc_bytes);
     if (bytes > s->opts.hbm_budget_bytes) {
         std::lock_guard<std::mutex> lk(s->mu);
         s->stats.rejected++;
@@ -476,12 +480,9 @@ extern "C" int emv_server_submit(emv_server *s, const emv_graph *g, const int32_
     r->w.assign(g->w, g->w + g->arcs);
     r->terms.assign(terminals, terminals + k);
     r->bytes = bytes;
-    r->large = g->n >= s->opts.large_n || !batch_fits(g->n, k);
-    if (!r->large) {
-        const BatchGraph bg = batch_graph(g->row_ptr, g->w, g->n, g->arcs);
-        r->narrow = bg.narrow;
-        r->arc_bytes = bg.arc_bytes;
-    }
+    r->large = large;
+    r->narrow = bg.narrow;
+    r->arc_bytes = bg.arc_bytes;
     r->t_submit = Clock::now();
     {
         std::lock_guard<std::mutex> lk(s->mu);

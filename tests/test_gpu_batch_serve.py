@@ -286,3 +286,26 @@ def test_batch_tables_that_just_fit_the_device(emv, count, n, k):
         assert list(costs) == [want[i % 4].cost for i in range(count)]
         assert all(np.array_equal(t, want[i % 4].table) for i, t in enumerate(tables))
         assert np.array_equal(s.batch_solve(graphs)[0], costs)
+
+
+def test_server_memory_follows_its_requests(emv):
+    """A request whose arc slices are far larger than its table (one vertex of 62
+    arcs in every slice, weights past the packed arcs) takes them once, not for
+    every CTA of the GPU, and is charged for them."""
+    torch = pytest.importorskip("torch")
+    n, rng = 25600, np.random.default_rng(4)
+    hubs = np.arange(0, n, 32)
+    ends = np.stack([np.repeat(hubs, 60), rng.integers(0, n // 32, 60 * len(hubs)) * 32 + rng.integers(1, 32, 60 * len(hubs))], 1)
+    ends = np.concatenate([ends, np.stack([np.arange(n - 1), np.arange(1, n)], 1)])
+    edges = np.concatenate([ends, rng.integers(16384, 20000, (len(ends), 1))], 1)
+    csr = emv.Csr.from_stp(emv.StpInstance(n, edges, np.array([5, 9000, 13000, 25000], np.int64)))
+    assert np.diff(csr.row_ptr)[hubs].min() == 61 and np.diff(csr.row_ptr).max() <= 64
+    slices = len(hubs) * 31 * 32 * 16
+    with emv.Solver(0) as s:
+        want = s.solve(csr).cost
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info(0)[0]
+    with emv.Server(0) as srv:
+        assert srv.wait(srv.submit(csr))[0] == want
+        assert before - torch.cuda.mem_get_info(0)[0] < 20 * slices
+        assert srv.stats()["peak_bytes"] >= slices
