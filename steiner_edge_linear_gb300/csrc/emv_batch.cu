@@ -526,7 +526,13 @@ int batch_upload(emv_ctx *c, BatchPack &pk, bool spare, cudaStream_t st)
     return EMV_OK;
 }
 
-int64_t batch_arc_stride(int64_t arc_bytes) { return std::max<int64_t>(256, (arc_bytes + 255) / 256 * 256); }
+// With one element a lane to spare: a closure that keeps arcs in registers loads
+// the first element of its slice also where the slice has none (its vertices have
+// no arcs), and a last slice's would lie behind the others.
+int64_t batch_arc_stride(int64_t arc_bytes)
+{
+    return (arc_bytes + 32 * (int64_t)sizeof(int4) + 255) / 256 * 256;
+}
 
 BatchArgs batch_args(emv_ctx *c, const BatchPack &pk)
 {

@@ -309,3 +309,17 @@ def test_server_memory_follows_its_requests(emv):
         assert srv.wait(srv.submit(csr))[0] == want
         assert before - torch.cuda.mem_get_info(0)[0] < 20 * slices
         assert srv.stats()["peak_bytes"] >= slices
+
+
+def test_autotune_with_a_last_slice_without_arcs(emv):
+    """The autotuner takes instances unchecked: one of 1024 vertices whose last 32
+    have no arcs, with more arcs than shared memory holds."""
+    n, rng = 992, np.random.default_rng(6)
+    ends = np.concatenate([np.stack([np.arange(n - 1), np.arange(1, n)], 1), rng.integers(0, n, (28 * n, 2))])
+    ends = ends[ends[:, 0] != ends[:, 1]]
+    edges = np.concatenate([ends, rng.integers(16384, 20000, (len(ends), 1))], 1)
+    far = emv.Csr.from_stp(emv.StpInstance(1024, edges, np.array([5, 900], np.int64)))
+    near = emv.Csr.from_stp(emv.StpInstance(n, edges, np.array([5, 900], np.int64)))
+    with emv.Solver(0) as s:
+        assert s.batch_autotune([far, near]).max() > 0
+        assert list(s.batch_solve([near, near])[0]) == [s.solve(near).cost] * 2
