@@ -204,6 +204,10 @@ def _single_args(cfg: dict) -> list:
     return ["regular", cfg["n"], cfg["degree"], cfg["wmin"], cfg["wmax"], cfg["k"], cfg["seed"]]
 
 
+# whose emv_kernel a CPU run is ("kind")
+EMV_KERNEL_OF = {"reference": "the reference's emv_kernel", "port": "the oracle's restatement of the reference's emv_kernel"}
+
+
 def cpu_reference_runs(steps: int, warmup: int, threads: int | None = None) -> dict:
     """Times complete solves of the benchmark instance with the reference's own
     emv_kernel (oracle/_ref, built from the reference source with -O3 and
@@ -390,8 +394,8 @@ def run_single(args, dist: Dist, cfg: dict = SINGLE, cfg_name: str = SINGLE_NAME
         t = statistics.median(c["runs_s"])
         out["cpu_baseline"] = {"value": round(1.0 / t, 5), "unit": "solves/s", "cores": c["threads"],
                                "kind": c["kind"], "cost": c["cost"],
-                               "sample": (f"one complete solve of the same instance (all 4096 rows, {t:.2f} s) by the "
-                                          f"reference's emv_kernel, -O3, {c['threads']} OpenMP threads")}
+                               "sample": (f"one complete solve of the same instance (all 4096 rows, {t:.2f} s) by "
+                                          f"{EMV_KERNEL_OF[c['kind']]}, -O3, {c['threads']} OpenMP threads")}
     return out
 
 
@@ -440,9 +444,16 @@ def single_config(cfg: dict, name: str, world: int) -> dict:
 def run_reference(args, dist: Dist) -> dict | None:
     """The reference arm: each timed step is one complete solve of the benchmark
     instance by the reference's own emv_kernel on all host cores (about 20 s on
-    16 Neoverse-V2 cores); warm-up steps solve the first 8 terminals only."""
+    16 Neoverse-V2 cores); warm-up steps solve the first 8 terminals only.
+    Without the reference's source the arm says so: the oracle's restatement does
+    not stand in for it."""
     if dist.rank != 0:
         return None
+    import oracle
+
+    oracle.build(reference=True)
+    if not oracle.reference_available():
+        return {"impl": "reference", "unavailable": "no reference source to build (its tree or a staged copy)"}
     c = cpu_reference_runs(steps=args.steps, warmup=args.warmup)
     t = statistics.median(c["runs_s"])
     value = 1.0 / t
