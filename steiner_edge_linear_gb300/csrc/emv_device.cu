@@ -853,7 +853,9 @@ static int finish_traceback(emv_ctx *c, int32_t n, emv_result *out)
 {
     const int32_t *head = (const int32_t *)((char *)c->pinned + PINNED_TB), *e = head + TB_HEAD;
     const size_t edges = (size_t)head[0];
-    out->timing.traceback_ms = (float)(head[2] * 1e-6);
+    uint64_t ns;
+    std::memcpy(&ns, head + 2, sizeof(ns));
+    out->timing.traceback_ms = (float)(ns * 1e-6);
     if (head[1]) return emv_dev_status_to_emv((uint32_t)head[1]);
     std::vector<int32_t> all;
     if (edges > TB_FIRST_EDGES) {

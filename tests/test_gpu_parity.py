@@ -670,9 +670,13 @@ def test_traceback_waits_for_long_zero_weight_searches(emv, solver):
     """All weights 0: every piece of the tree is one search over a large part of
     the graph, and the pieces queue for the search's arrays for seconds."""
     csr = emv.Csr.from_stp(inst := emv.StpInstance.regular(1 << 19, 4, 0, 0, 12, 3))
+    solver.solve(csr)
+    t0 = time.perf_counter()
     res = solver.solve(csr, tree=True)
+    took = 1e3 * (time.perf_counter() - t0)
     assert res.cost == 0 and res.tree_weight == 0
     check_tree(csr.n, inst.edges, res.tree, csr.terminals, 0)
+    assert 0.9 * took < res.timing["kernel_ms"] + res.timing["traceback_ms"] < took
 
 
 def test_refused_one_launch_solve_traces_nothing(emv, solver):
