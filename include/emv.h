@@ -303,10 +303,10 @@ typedef struct emv_instance {
 typedef struct emv_batch_stats {
     float total_ms;       /* device time of the whole batch            */
     float upload_ms;      /* host->device of CSR and terminals         */
-    int64_t work_items;   /* (instance, level) items executed          */
+    int64_t work_items;   /* instances solved                          */
     int64_t table_bytes;  /* device bytes of all tables                */
-    int32_t merge_tile;   /* autotuned vertices per merge tile         */
-    int32_t relax_rows;   /* autotuned rows per relaxation chunk       */
+    int32_t merge_tile;   /* 32: the unit of the tuned merge widths    */
+    int32_t relax_rows;   /* most rows of a closure, of any instance   */
 } emv_batch_stats;
 
 /* Solves many independent instances (no counterpart in the reference, which

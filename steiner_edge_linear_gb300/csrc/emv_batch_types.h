@@ -8,7 +8,6 @@ namespace emv {
 
 constexpr int BATCH_KMAX = 12;
 constexpr int32_t BATCH_SMEM_BYTES = 200 * 1024;  // admission: 2^k rows of 32 vertices and two rows of n
-constexpr int32_t BATCH_RCAP_MAX = 128;  // most rows per closure that the autotuner tries
 constexpr int32_t BATCH_MW_MAX = 8;      // widest merge vertex block that it tries: 8 columns of 32 vertices
 constexpr int BATCH_SIZES = 8;           // team sizes 128, 64, .. 1
 

@@ -297,8 +297,6 @@ int launch_narrow(emv_ctx *c, const int32_t *row_ptr, const int2 *adj, int32_t n
     return EMV_OK;
 }
 
-int32_t relax_chunk_rows(const emv_ctx *c, int32_t n, bool u16) { return relax_rows_per_chunk(n, c->l2_bytes, u16); }
-
 int32_t relax_chunk_rows_level(const emv_ctx *c, int32_t n, bool u16, int64_t cnt)
 {
     return relax_rows_per_level_chunk(n, c->l2_bytes, u16, cnt);

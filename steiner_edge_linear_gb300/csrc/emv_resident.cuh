@@ -446,7 +446,7 @@ __device__ bool res_close(const ResInst &a, const ResGraph<SRC> &g, bool has_hub
         return res_at<uint16_t>(list + 2 * (end - 1 - (j - (w ? before : 0))));
     };
     auto is_hub = [&](int32_t v) -> bool { return res_at<uint8_t>(g.pairs + v) == RES_HUB_MARK; };
-    // threads with a change among their `per` states when half of all states change
+    // threads with a change among their `per` states when RES_PULL_SHARE of all states change
     float same = 1.0f;
     for (int32_t i = 0; i < per && i < 16; i++) same *= 1.0f - RES_PULL_SHARE;
     const int many = (int)(RES_THREADS * (1.0f - same));

@@ -126,13 +126,12 @@ struct emv_ctx {
     DevBuf b_costs;                // by the caller's instance index
     cudaStream_t bstream = nullptr;  // of the second lane
     cudaEvent_t bev[2] = {};       // the caller's stream reached, the second lane done
-    int32_t tune_rcap[BATCH_CLASSES] = {};
-    int32_t tune_mw[BATCH_CLASSES] = {};  // merge vertex-block width per class (0: default 1)
+    int32_t tune_rcap[BATCH_CLASSES] = {};  // most rows of a closure per class (0: a CTA's share of the widest level)
+    int32_t tune_mw[BATCH_CLASSES] = {};  // most vertices of a merge block per class, in 32s (0: what fits)
 };
 
 int prepare_subsets(emv_ctx *c, int32_t k, cudaStream_t st);
 int reserve_relax(emv_ctx *c, int32_t n);
 constexpr int32_t SWEEP_RATE = 3;  // sweeps of narrow records, or rounds in one launch, for one of k_relax
 int32_t max_sweeps(const emv_ctx *c, int32_t n, int32_t rate);
-int32_t relax_chunk_rows(const emv_ctx *c, int32_t n, bool u16);
 int32_t relax_chunk_rows_level(const emv_ctx *c, int32_t n, bool u16, int64_t cnt);
