@@ -125,7 +125,7 @@ void batch_plan(const std::vector<double> &work, const std::vector<int64_t> &sta
     });
 }
 
-void batch_shape(const emv_ctx *c, BatchInst &d)
+void batch_shape(const emv_ctx *c, int64_t arcs, BatchInst &d)
 {
     const int32_t cls = batch_class_of(d.n, d.k);
     const int32_t rcap = c->tune_rcap[cls] > 0 ? pow2_floor(c->tune_rcap[cls]) : 0;
@@ -133,6 +133,7 @@ void batch_shape(const emv_ctx *c, BatchInst &d)
     d.rows = rcap > 0 ? std::min(most, rcap) : most;
     d.mw = resident_merge_width(d.n, d.kt, d.size, c->tune_mw[cls] > 0 ? 32 * pow2_floor(c->tune_mw[cls]) : 0);
     d.inv_slices = res_inv_slices(d.n);
+    d.spin_limit = res_spin_limit(d.n, arcs, most);
 }
 
 int32_t batch_blocks(const emv_ctx *c, int64_t ctas, int32_t cap)
@@ -418,7 +419,7 @@ int batch_layout(emv_ctx *c, const emv_instance *inst, const BatchOrder &ord, in
         d.k = I.k;
         d.kt = whole ? I.k : table_terminals(I.k);
         d.size = ord.size[(size_t)(from + j)];
-        batch_shape(c, d);
+        batch_shape(c, I.g.arcs, d);
         d.orig = id;
         d.lo = 1;
         d.hi = d.kt;

@@ -63,6 +63,7 @@ __device__ __forceinline__ bool batch_class(const BatchArgs &a, int32_t c, int32
             I.max_rounds = n + 1;
             I.inv_slices = B->inv_slices;
         }
+        tm.limit = B->spin_limit;  // also of the barrier behind the instance
         const int32_t lo = B->lo, hi = B->hi;
         const int32_t base = __ldg(lvl + 1);
         if (threadIdx.x < k) sh.terms[threadIdx.x] = __ldg(B->terms + threadIdx.x);
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_batch(BatchArgs a)
         const int32_t size = 1 << (BATCH_SIZES - 1 - c), teams = (int32_t)gridDim.x / size;
         const int32_t team = (int32_t)blockIdx.x / size, end = a.end[c];
         if (end > beg && team < teams) {
-            ResTeam tm{a.ctl + 32 * (line + team), a.ctl, (int32_t)blockIdx.x % size, size, 0};
+            ResTeam tm{a.ctl + 32 * (line + team), a.ctl, (int32_t)blockIdx.x % size, size, 0, RES_SPIN_LIMIT};
             if (!batch_class(a, c, beg, end, tm, sh, s_inst, s_idx, xs_kt)) return;
         }
         line += teams;

@@ -40,8 +40,8 @@ double batch_work(int32_t n, int32_t kt, int64_t arcs, int32_t lo, int32_t hi);
 // class (then largest first): order[j] is the input's index, size[] by input index.
 void batch_plan(const std::vector<double> &work, const std::vector<int64_t> &states, int32_t blocks, int32_t max_size,
                 std::vector<int32_t> &order, std::vector<int32_t> &size);
-// Fills the fields that follow from n, k, kt and the team size.
-void batch_shape(const emv_ctx *c, emv::BatchInst &d);
+// Fills the fields that follow from n, k, kt, the arcs and the team size.
+void batch_shape(const emv_ctx *c, int64_t arcs, emv::BatchInst &d);
 int prepare_batch_subsets(emv_ctx *c, cudaStream_t st);
 int batch_kernel_setup(emv_ctx *c);
 // Team sizes and launch order of the instances ids[] (blocks > 0: single-CTA

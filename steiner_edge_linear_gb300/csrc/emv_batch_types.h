@@ -30,7 +30,7 @@ struct BatchInst {
     int32_t orig;            // slot of the cost in BatchArgs::costs
     int32_t lo;              // first level to run (1..kt)
     int32_t hi;              // last level to run (lo..kt)
-    int32_t pad;
+    uint32_t spin_limit;     // ResTeam::limit
     char *slices;            // its sliced arcs, or null: in BatchArgs::scratch
 };
 

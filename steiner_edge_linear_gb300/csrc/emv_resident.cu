@@ -14,7 +14,7 @@ namespace emv {
 __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(ResArgs a)
 {
     __shared__ ResShared sh;
-    ResTeam tm{a.out->bar, &a.out->err, (int32_t)blockIdx.x, (int32_t)gridDim.x, 0};
+    ResTeam tm{a.out->bar, &a.out->err, (int32_t)blockIdx.x, (int32_t)gridDim.x, 0, a.spin_limit};
     const int64_t first = (int64_t)blockIdx.x * RES_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * RES_THREADS;
     const ResSmem sm = res_layout(a.inst.n, a.inst.kt, a.smem, a.xs, a.lvl[a.inst.kt + 1]);
     if (threadIdx.x == 0) sh.ok = 1;  // before the barrier that first reads it
@@ -69,6 +69,16 @@ uint32_t res_inv_slices(int32_t n)
 {
     const uint64_t slices = ((uint64_t)n + 31) / 32;
     return slices == 1 ? 0u : (uint32_t)((((uint64_t)1 << 32) + slices - 1) / slices);
+}
+
+// A closure takes up to n + 1 rounds of at most about a nanosecond an arc and
+// 5 us, a poll at least 0.3 us: the band of the longest closures (n = 25 600, 64
+// arcs a vertex, rounds of 0.1 ms as 25 000 vertices have to change one after
+// another) takes 2.5 s a row, while RES_SPIN_LIMIT polls are about 1.5 s.
+uint32_t res_spin_limit(int32_t n, int64_t arcs, int64_t rows)
+{
+    const double polls = (double)rows * n * ((double)arcs / 256 + 16);
+    return RES_SPIN_LIMIT + (uint32_t)std::min(polls, 2e9);
 }
 
 // Whether a solve of n vertices over kt terminals' subsets runs as one
@@ -141,6 +151,7 @@ int resident_launch(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, 
     a.arcs = arcs;
     a.check = check;
     a.smem = RESIDENT_SMEM;
+    a.spin_limit = res_spin_limit(n, arcs, p.rows);
     for (int32_t m = 0; m <= kt + 1; m++) a.lvl[m] = (int32_t)c->kp->xs_off[(size_t)m];
     for (int32_t t = 0; t < k; t++) a.terms[t] = terms[t];
     I.row_ptr = row_ptr;

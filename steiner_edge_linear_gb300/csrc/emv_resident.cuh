@@ -39,7 +39,7 @@ constexpr int RES_HUB = 64;              // a vertex of more arcs is walked by a
 constexpr uint8_t RES_HUB_MARK = 255;    // its arc pairs in ResSmem::pairs
 constexpr uint32_t RES_MAX_W = 1u << 14; // packed arcs hold smaller weights
 constexpr float RES_PULL_SHARE = 0.2f;   // a round after one that changed more of the states pulls
-constexpr uint32_t RES_SPIN_LIMIT = 1u << 22;  // polls of an L2 word, over a second in all
+constexpr uint32_t RES_SPIN_LIMIT = 1u << 22;  // least polls of an L2 word, over a second in all (res_spin_limit)
 constexpr int RES_ACC_WORDS = 2 * RES_THREADS;  // merge minima of a level with at most half as many tasks as threads
 
 // One instance as the device functions below take it.
@@ -67,6 +67,7 @@ struct ResTeam {
     uint32_t *err;            // EMV_DEV_* bits
     int32_t rank, size;
     uint32_t epoch;           // barriers passed
+    uint32_t limit;           // polls at a barrier (res_spin_limit)
 };
 
 // A CTA's static shared memory.
@@ -99,6 +100,7 @@ struct ResArgs {
     int64_t arcs;
     int32_t check;            // leave after the CSR check found a fault
     int32_t smem;             // dynamic shared memory
+    uint32_t spin_limit;
     int32_t lvl[RES_KMAX + 2];
     int32_t terms[EMV_MAX_K];
 };
@@ -136,8 +138,8 @@ __device__ __forceinline__ void res_fail(const ResTeam &t, uint32_t err, ResShar
 }
 
 // Barrier over the team's CTAs.  Arrivals only count up, so no word is reset.
-// Bounded: a CTA that waits longer than RES_SPIN_LIMIT polls records the
-// error; every CTA of the team leaves when it sees one.
+// Bounded: a CTA that waits longer than t.limit polls records the error; every
+// CTA of the team leaves when it sees one.
 __device__ __forceinline__ bool res_barrier(ResTeam &t, ResShared &sh)
 {
     __syncthreads();
@@ -151,7 +153,7 @@ __device__ __forceinline__ bool res_barrier(ResTeam &t, ResShared &sh)
             for (;;) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(t.bar) : "memory");
                 if ((seen & RES_FAILED) || (seen & ~RES_FAILED) >= target) break;
-                if (++spins > RES_SPIN_LIMIT) {
+                if (++spins > t.limit) {
                     res_fail(t, EMV_DEV_BARRIER_TIMEOUT, sh);
                     break;
                 }

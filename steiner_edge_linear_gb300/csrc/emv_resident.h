@@ -21,6 +21,9 @@ bool resident_fits(int32_t n, int32_t kt);
 // so that every CTA has some; cap > 0 bounds it.
 int32_t resident_merge_width(int32_t n, int32_t kt, int32_t ctas, int32_t cap);
 uint32_t res_inv_slices(int32_t n);
+// Polls after which a CTA gives up on the others of its team: CTAs without rows
+// of a level wait for those that close `rows` of them.
+uint32_t res_spin_limit(int32_t n, int64_t arcs, int64_t rows);
 bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, bool host_table, ResidentPlan &p);
 // Enqueues the whole DP over the first kt of the k terminals, CSR check
 // included, and the copy of its result words; fills the table's 2^kt rows

@@ -257,7 +257,7 @@ void scheduler(emv_server *s)
             d.k = r->k;
             d.kt = table_terminals(r->k);
             d.size = size[(size_t)order[j]];
-            batch_shape(s->ctx_small, d);
+            batch_shape(s->ctx_small, r->arcs, d);
             d.narrow = r->narrow;
             d.slices = (char *)r->d_table + table_bytes(r->n, r->k);
             d.orig = r->slot;

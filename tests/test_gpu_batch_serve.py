@@ -323,3 +323,18 @@ def test_autotune_with_a_last_slice_without_arcs(emv):
     with emv.Solver(0) as s:
         assert s.batch_autotune([far, near]).max() > 0
         assert list(s.batch_solve([near, near])[0]) == [s.solve(near).cost] * 2
+
+
+def test_team_waits_for_a_long_closure(emv):
+    """A team's CTAs without rows of a level wait for the one that closes its only
+    row, for seconds where the closure takes a round for every vertex of a long
+    band: each vertex has 64 arcs, of which the two of weight 1 are of use."""
+    n = 25600
+    v = np.arange(n)
+    edges = np.concatenate([np.stack([v[:-j], v[j:], np.full(n - j, 1 if j == 1 else 3 * j)], 1) for j in range(1, 33)])
+    csr = emv.Csr.from_stp(emv.StpInstance(n, edges, np.array([0, 5, 9, n - 1], np.int64)))
+    with emv.Solver(0) as s:
+        costs, st = s.batch_solve([csr])
+        assert costs[0] == n - 1
+        assert st["total_ms"] > 1500
+        assert s.batch_solve([emv.Csr.from_stp(emv.StpInstance.regular(64, 4, 1, 9, 4, 1))])[0][0] > 0
