@@ -74,16 +74,24 @@ bool batch_fits(int32_t n, int32_t k)
            ((int64_t)32 << k) * 4 <= BATCH_SMEM_BYTES && resident_fits(n, k);
 }
 
-BatchGraph batch_graph(const int32_t *row_ptr, const int32_t *w, int32_t n, int64_t arcs)
+uint32_t pack_arcs(const emv_graph &g, int2 *adj)
 {
     uint32_t most = 0;
-    for (int64_t e = 0; e < arcs; e++) most = std::max(most, (uint32_t)w[e]);
+    for (int64_t e = 0; e < g.arcs; e++) {
+        adj[e] = make_int2(g.col[e], g.w[e]);
+        most = std::max(most, (uint32_t)g.w[e]);
+    }
+    return most;
+}
+
+BatchGraph batch_graph(const int32_t *row_ptr, int32_t n, uint32_t most, int32_t hub_min)
+{
     int64_t pairs = 0;
     for (int32_t v0 = 0; v0 < n; v0 += 32) {
         int32_t width = 0;
         for (int32_t v = v0; v < std::min(n, v0 + 32); v++) {
             const int32_t deg = row_ptr[v + 1] - row_ptr[v];
-            if (deg <= RES_HUB) width = std::max(width, (deg + 1) / 2);
+            if (deg <= hub_min) width = std::max(width, (deg + 1) / 2);
         }
         pairs += width;
     }
@@ -134,6 +142,7 @@ void batch_shape(const emv_ctx *c, int64_t arcs, BatchInst &d)
     d.mw = resident_merge_width(d.n, d.kt, d.size, c->tune_mw[cls] > 0 ? 32 * pow2_floor(c->tune_mw[cls]) : 0);
     d.inv_slices = res_inv_slices(d.n);
     d.spin_limit = res_spin_limit(d.n, arcs, most);
+    d.hub_min = res_hub_min(d.n, arcs, d.kt);
 }
 
 int32_t batch_blocks(const emv_ctx *c, int64_t ctas, int32_t cap)
@@ -472,12 +481,11 @@ int batch_fill(emv_ctx *c, const emv_instance *inst, BatchPack &pk, const std::f
         const int32_t id = pk.desc[(size_t)j].orig;
         if (check && !check(id)) return;
         const emv_instance &I = inst[id];
-        const BatchGraph bg = batch_graph(I.g.row_ptr, I.g.w, I.g.n, I.g.arcs);
+        const uint32_t most = pack_arcs(I.g, pk.h_adj + pk.arc_off[(size_t)j]);
+        const BatchGraph bg = batch_graph(I.g.row_ptr, I.g.n, most, pk.desc[(size_t)j].hub_min);
         pk.desc[(size_t)j].narrow = bg.narrow;
         arc_bytes[(size_t)j] = bg.arc_bytes;
         std::memcpy(pk.h_row + pk.row_off[(size_t)j], I.g.row_ptr, sizeof(int32_t) * ((size_t)I.g.n + 1));
-        int2 *ha = pk.h_adj + pk.arc_off[(size_t)j];
-        for (int64_t e = 0; e < I.g.arcs; e++) ha[e] = make_int2(I.g.col[e], I.g.w[e]);
         std::memcpy(pk.h_term + pk.term_off[(size_t)j], I.terminals, sizeof(int32_t) * (size_t)I.k);
     });
     for (int64_t b : arc_bytes) pk.arc_bytes = std::max(pk.arc_bytes, b);

@@ -62,6 +62,7 @@ __device__ __forceinline__ bool batch_class(const BatchArgs &a, int32_t c, int32
             I.mw = B->mw;
             I.max_rounds = n + 1;
             I.inv_slices = B->inv_slices;
+            I.hub_min = B->hub_min;
         }
         tm.limit = B->spin_limit;  // also of the barrier behind the instance
         const int32_t lo = B->lo, hi = B->hi;

@@ -33,7 +33,9 @@ struct BatchGraph {
     bool narrow = false;      // every weight fits a packed arc
     int64_t arc_bytes = 0;    // sliced arcs
 };
-BatchGraph batch_graph(const int32_t *row_ptr, const int32_t *w, int32_t n, int64_t arcs);
+BatchGraph batch_graph(const int32_t *row_ptr, int32_t n, uint32_t largest_weight, int32_t hub_min);
+// Packs the arcs; returns their largest weight.
+uint32_t pack_arcs(const emv_graph &g, int2 *adj);
 // Estimated time (us) of levels lo..hi on one CTA.
 double batch_work(int32_t n, int32_t kt, int64_t arcs, int32_t lo, int32_t hi);
 // Team sizes (at most max_size) for a grid of `blocks` CTAs and the order by

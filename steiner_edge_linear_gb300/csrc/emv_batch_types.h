@@ -31,6 +31,8 @@ struct BatchInst {
     int32_t lo;              // first level to run (1..kt)
     int32_t hi;              // last level to run (lo..kt)
     uint32_t spin_limit;     // ResTeam::limit
+    int32_t hub_min;         // ResInst::hub_min
+    int32_t pad;
     char *slices;            // its sliced arcs, or null: in BatchArgs::scratch
 };
 

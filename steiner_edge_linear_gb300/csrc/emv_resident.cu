@@ -71,6 +71,21 @@ uint32_t res_inv_slices(int32_t n)
     return slices == 1 ? 0u : (uint32_t)((((uint64_t)1 << 32) + slices - 1) / slices);
 }
 
+// Arcs of a vertex up to which it has its place in a slice; more make it a hub.
+// A slice is as wide as its widest vertex, so 64, but in dense graphs twice the
+// mean degree where arc counts of pairs still fit 8 bits: with every vertex a
+// hub, read from adj by a warp, one launch lost to the record kernels and a
+// batch to a CTA an instance.  Before and so: 900 cliques of 100, k = 7 5.6 and
+// 2.1 ms on the device, n = 4000, degree 70, k = 8 3.80 and 1.15 ms; past it the two
+// are equal (clique of 400, k = 4 0.43 and 0.47 ms, k = 8 0.98 and 0.85).  A single
+// row is pushed from few vertices, which suits the warps (clique of 200 0.10 and
+// 0.14 ms).
+int32_t res_hub_min(int32_t n, int64_t arcs, int32_t kt)
+{
+    const int64_t mean = arcs / n;
+    return kt > 1 && mean > 48 && mean <= 254 ? (int32_t)(2 * mean) : 64;
+}
+
 // A closure takes up to n + 1 rounds of at most about a nanosecond an arc and
 // 5 us, a poll at least 0.3 us: the band of the longest closures (n = 25 600, 64
 // arcs a vertex, rounds of 0.1 ms as 25 000 vertices have to change one after
@@ -132,7 +147,8 @@ int resident_launch(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, 
 {
     int r = prepare_subsets(c, kt, st);
     if (!r) r = dev_reserve(c->adj, sizeof(int2) * (size_t)std::max<int64_t>(arcs, 1));
-    if (!r) r = dev_reserve(c->res_arcs, sizeof(int4) * (RES_HUB / 2) * 32 * (((size_t)n + 31) / 32));
+    const int32_t hub_min = res_hub_min(n, arcs, kt);
+    if (!r) r = dev_reserve(c->res_arcs, sizeof(int4) * (size_t)(hub_min / 2) * 32 * (((size_t)n + 31) / 32));
     if (!r) r = dev_reserve(c->res_out, sizeof(ResOut));
     if (r) return r;
     if (!c->res_attr) {
@@ -171,6 +187,7 @@ int resident_launch(emv_ctx *c, const ResidentPlan &p, int32_t n, int64_t arcs, 
     I.mw = p.mw;
     I.max_rounds = max_sweeps(c, n, SWEEP_RATE);
     I.inv_slices = res_inv_slices(n);
+    I.hub_min = hub_min;
     CUDA_TRY(cudaMemsetAsync(a.out, 0, sizeof(ResOut), st));
     CUDA_TRY(cudaEventRecord(c->ev[0], st));
     void *args[] = {&a};

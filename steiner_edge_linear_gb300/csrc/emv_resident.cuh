@@ -35,7 +35,6 @@ namespace emv {
 constexpr int RES_THREADS = 1024;
 constexpr int RES_WARPS = RES_THREADS / 32;
 constexpr int RES_KMAX = 11;             // most terminals whose subsets are solved
-constexpr int RES_HUB = 64;              // a vertex of more arcs is walked by a whole warp
 constexpr uint8_t RES_HUB_MARK = 255;    // its arc pairs in ResSmem::pairs
 constexpr uint32_t RES_MAX_W = 1u << 14; // packed arcs hold smaller weights
 constexpr float RES_PULL_SHARE = 0.2f;   // a round after one that changed more of the states pulls
@@ -59,6 +58,7 @@ struct ResInst {
     int32_t mw;               // vertices of a merge block (multiple of 4)
     int32_t max_rounds;
     uint32_t inv_slices;      // ceil(2^32 / slices), for slices > 1
+    int32_t hub_min;          // a vertex of more arcs is walked by a whole warp (res_hub_min)
 };
 
 // The CTAs that share an instance: all of them on the GPU at once.
@@ -310,7 +310,7 @@ __device__ __forceinline__ void res_merge(const ResInst &a, const ResTeam &tm, c
 // j of the vertex at lane l of slice i: (slice[i] + j) * 32 + l.  A vertex
 // with fewer pairs than its slice's widest (and the second arc of an odd
 // last pair) is padded with an arc to itself that improves nothing; vertices
-// of more than RES_HUB arcs have no pairs here and are read from adj.
+// of more than hub_min arcs have no pairs here and are read from adj.
 enum ResArcs { ARCS_SMEM, ARCS_PACKED, ARCS_WIDE };
 
 template <ResArcs SRC> struct ResElem {
@@ -380,7 +380,7 @@ __device__ __forceinline__ int32_t res_div(uint32_t inv, int32_t wd, int32_t sli
 // read and set after a distance was lowered, so none is lost; it is set
 // whenever a value looked improvable, and a lost race costs a visit.
 //
-// Graphs with vertices of more than RES_HUB arcs list those apart (from the
+// Graphs with vertices of more than hub_min arcs list those apart (from the
 // far end of the warp's part), and after a barrier all warps share them, a
 // warp per vertex: one warp would otherwise walk all hubs of its run.
 // Returns false when max_rounds ran out; `rounds` counts barriers passed.
@@ -825,7 +825,7 @@ __device__ void res_levels(const ResInst &a, ResTeam &tm, const ResSmem &sm, Res
 
 // Widths of the slices in arc pairs, their prefix sums (sm.slice) and the
 // pairs of every vertex; needs at most RES_THREADS slices.  Returns whether a
-// vertex has more than RES_HUB arcs.
+// vertex has more than hub_min arcs.
 __device__ __forceinline__ bool res_slice_starts(const ResInst &a, const ResSmem &sm, int32_t *warp_sums)
 {
     bool hub = false;
@@ -835,9 +835,10 @@ __device__ __forceinline__ bool res_slice_starts(const ResInst &a, const ResSmem
     for (int32_t i = warp; i < slices; i += RES_WARPS) {
         const int32_t v = i * 32 + lane;
         const int32_t deg = v < a.n ? __ldg(a.row_ptr + v + 1) - __ldg(a.row_ptr + v) : 0;
-        const int32_t np = deg > RES_HUB ? 0 : (deg + 1) / 2;
-        hub |= deg > RES_HUB;
-        res_at<uint8_t>(sm.pairs + v) = deg > RES_HUB ? RES_HUB_MARK : (uint8_t)np;
+        const bool big = deg > a.hub_min;
+        const int32_t np = big ? 0 : (deg + 1) / 2;
+        hub |= big;
+        res_at<uint8_t>(sm.pairs + v) = big ? RES_HUB_MARK : (uint8_t)np;
         const int32_t width = __reduce_max_sync(FULL, np);
         if (lane == 0) slice[i] = width;
     }

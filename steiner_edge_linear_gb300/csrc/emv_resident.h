@@ -21,6 +21,7 @@ bool resident_fits(int32_t n, int32_t kt);
 // so that every CTA has some; cap > 0 bounds it.
 int32_t resident_merge_width(int32_t n, int32_t kt, int32_t ctas, int32_t cap);
 uint32_t res_inv_slices(int32_t n);
+int32_t res_hub_min(int32_t n, int64_t arcs, int32_t kt);
 // Polls after which a CTA gives up on the others of its team: CTAs without rows
 // of a level wait for those that close `rows` of them.
 uint32_t res_spin_limit(int32_t n, int64_t arcs, int64_t rows);

@@ -461,7 +461,10 @@ extern "C" int emv_server_submit(emv_server *s, const emv_graph *g, const int32_
     st = emv_graph_check(g, nullptr);
     if (st) return st;
     const bool large = g->n >= s->opts.large_n || !batch_fits(g->n, k);
-    const BatchGraph bg = large ? BatchGraph{} : batch_graph(g->row_ptr, g->w, g->n, g->arcs);
+    BatchGraph bg;
+    if (!large)
+        bg = batch_graph(g->row_ptr, g->n, g->arcs > 0 ? (uint32_t)*std::max_element(g->w, g->w + g->arcs) : 0u,
+                         res_hub_min(g->n, g->arcs, table_terminals(k)));
     const int64_t bytes = footprint(g->n, k, g->arcs, bg.arc_bytes);
     if (bytes > s->opts.hbm_budget_bytes) {
         std::lock_guard<std::mutex> lk(s->mu);
