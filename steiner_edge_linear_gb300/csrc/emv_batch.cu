@@ -342,14 +342,14 @@ static int batch_solve(emv_ctx *c, const emv_instance *inst, int32_t count, int6
     CUDA_TRY(cudaStreamSynchronize(st));
     if (err[0] | err[1]) return emv_dev_status_to_emv(err[0] | err[1]);
     if (tables_out) {
-        for (int l = 0; l < lanes; l++)
-            for (const BatchInst &d : pk[l].desc) {
-                const int32_t i = d.orig;
-                if (!tables_out[i]) continue;
-                const size_t row = sizeof(int32_t) * (size_t)inst[i].g.n;
-                CUDA_TRY(cudaMemcpy2DAsync(tables_out[i], row, d.table, sizeof(int32_t) * (size_t)batch_ld(inst[i].g.n), row,
-                                           (size_t)1 << inst[i].k, cudaMemcpyDeviceToHost, st));
-            }
+        for (int l = 0; l < lanes; l++) {
+            k_close_rows<<<(unsigned)pk[l].count, RES_THREADS, 0, st>>>(a[l].inst);
+            CUDA_TRY(cudaGetLastError());
+            for (const BatchInst &d : pk[l].desc)
+                if (tables_out[d.orig])
+                    CUDA_TRY(cudaMemcpyAsync(tables_out[d.orig], d.table, sizeof(int32_t) * ((size_t)d.n << d.kt),
+                                             cudaMemcpyDeviceToHost, st));
+        }
         CUDA_TRY(cudaStreamSynchronize(st));
     }
     if (stats) {

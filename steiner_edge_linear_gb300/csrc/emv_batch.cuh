@@ -101,4 +101,30 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_batch(BatchArgs a)
     }
 }
 
+// Closes the gaps between the rows of every table whose stride is padded, so that
+// it is copied to the host in one piece: a 2D copy into host pages that were
+// never written takes six times as long (100 tables of 2^8 x 1002 118 ms, 20 so).
+// In place, a CTA an instance: a word moves down only, and a chunk is read
+// before it is written.
+__global__ void __launch_bounds__(RES_THREADS) k_close_rows(const BatchInst *inst)
+{
+    const uint32_t n = (uint32_t)inst[blockIdx.x].n, ld = (uint32_t)batch_ld((int32_t)n), words = n << inst[blockIdx.x].kt;
+    int32_t *table = inst[blockIdx.x].table;
+    constexpr uint32_t PER = 16;
+    if (ld == n) return;
+    for (uint32_t base = threadIdx.x; base - threadIdx.x < words; base += PER * RES_THREADS) {
+        int32_t x[PER];
+#pragma unroll
+        for (uint32_t j = 0; j < PER; j++) {
+            const uint32_t i = base + j * RES_THREADS;
+            if (i < words) x[j] = __ldcg(table + i / n * ld + i % n);
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < PER; j++)
+            if (base + j * RES_THREADS < words) __stcg(table + base + j * RES_THREADS, x[j]);
+        __syncthreads();
+    }
+}
+
 }  // namespace emv

@@ -2,6 +2,7 @@
 single-instance solve and the oracle, alone and in the mix; the batched
 launch's whole tables equal the reference-written golden tables."""
 import ctypes
+import mmap
 import time
 
 import numpy as np
@@ -370,3 +371,42 @@ def test_dense_batches_scale_with_their_arcs(emv):
             graphs = [emv.Csr.from_stp(emv.StpInstance.clique(n, 1, 100, 7, seed)) for seed in range(700)]
             ms.append(min(s.batch_solve(graphs)[1]["total_ms"] for _ in range(5)))
     assert ms[1] < 1.5 * ms[0]
+
+
+@pytest.mark.parametrize("n", [1002, 1004])
+def test_batch_tables_into_new_host_pages(emv, n):
+    """Tables that go to host pages never written before take about as long as
+    tables into warm buffers and a copy of their bytes into new pages together,
+    whether their rows are padded on the device or not."""
+    torch = pytest.importorskip("torch")
+    count, size = 100, 4 * n << 8
+    graphs = [emv.Csr.from_stp(emv.StpInstance.regular(n, 3, 1, 100, 8, s)) for s in range(count)]
+    dev = torch.zeros((count, size // 4), dtype=torch.int32, device="cuda:0")
+    costs, stats = np.zeros(count, np.int64), emv._BatchStats()
+
+    def new_pages(bytes_):
+        return np.frombuffer(mmap.mmap(-1, bytes_), np.int32)
+
+    def timed(call):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        call()
+        return time.perf_counter() - t0
+
+    with emv.Solver(0) as s:
+        insts, _keep = s._instances(graphs)
+
+        def tables_into(bufs):
+            ptrs = (ctypes.c_void_p * count)(*[b.ctypes.data for b in bufs])
+            emv._check(s._lib.emv_batch_solve_tables(s._ctx, insts, count, costs.ctypes.data, ptrs, ctypes.byref(stats), None))
+
+        warm_bufs = [new_pages(size) for _ in range(count)]
+        tables_into(warm_bufs)
+        warm = min(timed(lambda: tables_into(warm_bufs)) for _ in range(4))
+        new, copy = [], []
+        for _ in range(4):
+            bufs, others = ([new_pages(size) for _ in range(count)] for _ in range(2))
+            new.append(timed(lambda: tables_into(bufs)))
+            copy.append(timed(lambda: [torch.from_numpy(o).copy_(d) for o, d in zip(others, dev)]))
+        assert all(np.array_equal(b, w) for b, w in zip(bufs, warm_bufs))
+    assert min(new) < 2 * (warm + min(copy))
