@@ -189,11 +189,11 @@ static bool batch_teams(const BatchArgs &a) { return a.end[BATCH_SIZES - 2] > 0;
 
 // Launches k_batch on `blocks` CTAs over prepared descriptors.  Teams wait for
 // their CTAs, so the launch is cooperative unless every team is a single CTA.
-int launch_batch(emv_ctx *c, const BatchArgs &args, int32_t blocks, cudaStream_t st)
+int launch_batch(emv_ctx *c, const BatchArgs &args, int32_t blocks, int32_t lines, cudaStream_t st)
 {
     int r = batch_kernel_setup(c);
     if (r) return r;
-    CUDA_TRY(cudaMemsetAsync(args.ctl, 0, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(c->batch_blocks), st));
+    CUDA_TRY(cudaMemsetAsync(args.ctl, 0, sizeof(uint32_t) * 32 * (size_t)lines, st));
     BatchArgs a = args;
     void *p[] = {&a};
     if (batch_teams(a))
@@ -575,7 +575,7 @@ int batch_graph_launch(emv_ctx *c, int32_t lane, const BatchArgs &a, int32_t blo
         CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
         cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            r = launch_batch(c, a, blocks, cap);
+            r = launch_batch(c, a, blocks, batch_ctl_lines(c->batch_blocks), cap);  // lines of any batch
             e = cudaStreamEndCapture(cap, &G.graph);
         }
         cudaStreamDestroy(cap);
@@ -640,7 +640,7 @@ int time_sample(emv_ctx *c, const emv_instance *inst, const std::vector<int32_t>
     ms = 1e30f;
     for (int rep = 0; rep < 3; rep++) {
         CUDA_TRY(cudaEventRecord(c->ev[0], st));
-        r = launch_batch(c, a, pk.blocks, st);
+        r = launch_batch(c, a, pk.blocks, batch_ctl_lines(pk.blocks), st);
         if (r) return r;
         CUDA_TRY(cudaEventRecord(c->ev[1], st));
         CUDA_TRY(cudaStreamSynchronize(st));

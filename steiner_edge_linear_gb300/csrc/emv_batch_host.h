@@ -64,7 +64,8 @@ int batch_fill(emv_ctx *c, const emv_instance *inst, BatchPack &pk, const std::f
 // spare: buffers that grow take a quarter more where it is free.
 int batch_upload(emv_ctx *c, BatchPack &pk, bool spare, cudaStream_t st);
 emv::BatchArgs batch_args(emv_ctx *c, const BatchPack &pk);
-int launch_batch(emv_ctx *c, const emv::BatchArgs &a, int32_t blocks, cudaStream_t st);
+// lines: control lines to reset, batch_ctl_lines(blocks) or more.
+int launch_batch(emv_ctx *c, const emv::BatchArgs &a, int32_t blocks, int32_t lines, cudaStream_t st);
 int batch_graph_launch(emv_ctx *c, int32_t lane, const emv::BatchArgs &a, int32_t blocks, cudaStream_t st);
 // Bytes of BatchArgs::scratch for every CTA, from the largest sliced arcs.
 int64_t batch_arc_stride(int64_t arc_bytes);

@@ -278,7 +278,7 @@ void scheduler(emv_server *s)
         if (cudaMemcpyAsync(s->d_desc.ptr, s->h_desc, sizeof(BatchInst) * wave.size(), cudaMemcpyHostToDevice,
                             s->st_small) != cudaSuccess)
             st = emv_fail(EMV_ERR_CUDA, "server: descriptor upload");
-        if (!st) st = launch_batch(s->ctx_small, a, blocks, s->st_small);
+        if (!st) st = launch_batch(s->ctx_small, a, blocks, batch_ctl_lines(blocks), s->st_small);
         if (!st && cudaMemcpyAsync(s->h_costs, s->d_costs.ptr, sizeof(int64_t) * (size_t)s->cap_slots,
                                    cudaMemcpyDeviceToHost, s->st_small) != cudaSuccess)
             st = emv_fail(EMV_ERR_CUDA, "server: cost read");
