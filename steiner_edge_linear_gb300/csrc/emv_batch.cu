@@ -115,13 +115,18 @@ void batch_plan(const std::vector<double> &work, const std::vector<int64_t> &sta
     for (double w : work) total += w;
     // A team large enough that the instance takes at most a third of the
     // batch's fair time (and not below 100 us, where barriers take over), as
-    // far as every CTA still has about a thread's state of the widest level.
+    // far as a CTA has more than two states of the widest level a thread before
+    // its team is doubled, or more than eight where many teams (of more than a
+    // quarter as many instances as CTAs) would take turns on the CTAs: a team of
+    // CTAs with little to do takes longer in all than one CTA.  107 instances on 152 CTAs, with one state throughout, four and
+    // eight: n = 64, 1088 edges, k = 8 0.50, 0.22 and 0.22 ms, n = 33, 560 edges, k = 10
+    // 1.08, 0.45 and 0.34, n = 130, 650 edges, k = 10 1.10, 0.72 and 0.64.
     const double most = std::max(100.0, total / blocks * 0.35);
     size.assign((size_t)count, 1);
     for (int32_t i = 0; i < count; i++) {
         int32_t g = 1;
         while (2 * g <= max_size && 2 * g <= blocks && work[(size_t)i] / g > most &&
-               states[(size_t)i] > (int64_t)RES_THREADS * g)
+               states[(size_t)i] > (int64_t)RES_THREADS * g * ((int64_t)count * std::min(4, 2 * g) <= blocks ? 2 : 8))
             g *= 2;
         size[(size_t)i] = g;
     }

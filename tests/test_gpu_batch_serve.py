@@ -410,3 +410,29 @@ def test_batch_tables_into_new_host_pages(emv, n):
             copy.append(timed(lambda: [torch.from_numpy(o).copy_(d) for o, d in zip(others, dev)]))
         assert all(np.array_equal(b, w) for b, w in zip(bufs, warm_bufs))
     assert min(new) < 2 * (warm + min(copy))
+
+
+@pytest.mark.parametrize("n,k", [(64, 8), (33, 10)])
+def test_batches_of_a_hundred_small_dense_instances(emv, n, k):
+    """Between half as many instances as CTAs and as many, teams of CTAs with less
+    than a thread's work would take turns: 107 instances take at most a quarter
+    longer than a CTA takes for one."""
+    torch = pytest.importorskip("torch")
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(7)
+    graphs = []
+    for _ in range(10):
+        ends = np.concatenate([np.stack([np.arange(n - 1), np.arange(1, n)], 1), rng.integers(0, n, (16 * n, 2))])
+        ends = ends[ends[:, 0] != ends[:, 1]]
+        graphs.append(emv.Csr.from_stp(emv.StpInstance(n, np.concatenate([ends, rng.integers(1, 101, (len(ends), 1))], 1),
+                                                       rng.choice(n, k, replace=False).astype(np.int64))))
+    ms = {}
+    with emv.Solver(0) as s:
+        want = [s.solve(g).cost for g in graphs]
+        for count in (107, 4 * ctas):  # four turns of a CTA each
+            batch = [graphs[i % 10] for i in range(count)]
+            for _ in range(6):
+                costs, st = s.batch_solve(batch)
+                ms[count] = min(ms.get(count, 1e9), st["total_ms"])
+            assert list(costs) == [want[i % 10] for i in range(count)]
+    assert ms[107] < 1.25 * ms[4 * ctas] / 4
