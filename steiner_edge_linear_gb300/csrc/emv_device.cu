@@ -1027,9 +1027,21 @@ extern "C" int emv_solve_dev(emv_ctx *c, const emv_graph *d_g, const int32_t *te
 // reads all arcs in every dense round.  Calls by one launch and by narrow
 // records, random graphs of n vertices and arcs: 300, 88 000 0.16 and 0.20 ms;
 // 1000, 120 000 0.28 and 0.21; 4000, 100 000 0.239 and 0.239; 8192, 80 000 0.23 and
-// 0.22; 8192, 500 000 0.92 and 0.32; grid of 90 x 90 0.38 and 0.95.
+// 0.22; 8192, 500 000 0.92 and 0.32; grid of 90 x 90 0.38 and 0.95.  Beyond, graphs
+// whose arcs crowd in a few vertices stay: narrow records leave 8 neighbouring
+// vertices of such a graph to a warp (5368, 192 000 arcs, half of them at 10 or at
+// 100 vertices 0.32 and 1.53, 0.27 and 0.65 ms; at random 0.28 and 0.25).
 constexpr int32_t SSSP_RESIDENT_N = 8192;
 constexpr int64_t SSSP_RESIDENT_ARCS = 100000;
+static bool sssp_resident(const emv_graph *g)
+{
+    if (g->n > SSSP_RESIDENT_N) return false;
+    if (g->arcs <= SSSP_RESIDENT_ARCS) return true;
+    int64_t most = 0;  // arcs of 8 neighbours
+    for (int32_t v = 0; v < g->n; v += 8)
+        most = std::max(most, (int64_t)g->row_ptr[std::min(v + 8, g->n)] - g->row_ptr[v]);
+    return 64 * most > g->arcs;
+}
 
 extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t *dist_out, float *ms_out, void *stream)
 {
@@ -1044,8 +1056,8 @@ extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t 
     // row 1 = {source}; rows of whole quads
     const int64_t ld = ((int64_t)n + 3) / 4 * 4;
     ResidentPlan plan;
-    const bool resident =
-        n <= SSSP_RESIDENT_N && arcs <= SSSP_RESIDENT_ARCS && resident_plan(c, n, arcs, 1, false, plan);
+    // the line of resident_plan on arcs is that of solves
+    const bool resident = sssp_resident(g) && resident_plan(c, n, 0, 1, false, plan);
     r = dev_reserve(c->table, sizeof(int32_t) * 2 * (size_t)ld);
     if (!r) r = prepare_subsets(c, 1, st);
     if (!r && !resident) r = reserve_relax(c, n);
