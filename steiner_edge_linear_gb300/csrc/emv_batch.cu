@@ -110,28 +110,30 @@ double batch_work(int32_t n, int32_t kt, int64_t arcs, int32_t lo, int32_t hi)
 void batch_plan(const std::vector<double> &work, const std::vector<int64_t> &states, int32_t blocks, int32_t max_size,
                 std::vector<int32_t> &order, std::vector<int32_t> &size)
 {
-    const int32_t count = (int32_t)work.size();
+    const int64_t count = (int64_t)work.size();
     double total = 0;
     for (double w : work) total += w;
     // A team large enough that the instance takes at most a third of the
     // batch's fair time (and not below 100 us, where barriers take over), as
-    // far as a CTA has more than two states of the widest level a thread before
-    // its team is doubled, or more than eight where many teams (of more than a
-    // quarter as many instances as CTAs) would take turns on the CTAs: a team of
-    // CTAs with little to do takes longer in all than one CTA.  107 instances on 152 CTAs, with one state throughout, four and
-    // eight: n = 64, 1088 edges, k = 8 0.50, 0.22 and 0.22 ms, n = 33, 560 edges, k = 10
-    // 1.08, 0.45 and 0.34, n = 130, 650 edges, k = 10 1.10, 0.72 and 0.64.
+    // far as a CTA has more than a state of the widest level a thread before its
+    // team is doubled; two where the teams may have to take turns on the CTAs,
+    // eight where there are more than a quarter as many instances as CTAs: a team
+    // of CTAs with little to do takes longer in all than one CTA.  107 instances
+    // on 152 CTAs, with one state throughout, four and eight: n = 64, 1088 edges,
+    // k = 8 0.50, 0.22 and 0.22 ms, n = 33, 560 edges, k = 10 1.08, 0.45 and 0.34, n =
+    // 130, 650 edges, k = 10 1.10, 0.72 and 0.64; 20 of n = 33, 560 edges with one and
+    // two 0.35 and 0.22; one of n = 500, 40 000 edges, k = 6 0.43 and 0.49.
     const double most = std::max(100.0, total / blocks * 0.35);
     size.assign((size_t)count, 1);
-    for (int32_t i = 0; i < count; i++) {
+    for (int64_t i = 0; i < count; i++) {
         int32_t g = 1;
         while (2 * g <= max_size && 2 * g <= blocks && work[(size_t)i] / g > most &&
-               states[(size_t)i] > (int64_t)RES_THREADS * g * ((int64_t)count * std::min(4, 2 * g) <= blocks ? 2 : 8))
+               states[(size_t)i] > (int64_t)RES_THREADS * g * (count * 2 * g <= blocks ? 1 : count * 4 <= blocks ? 2 : 8))
             g *= 2;
         size[(size_t)i] = g;
     }
     order.resize((size_t)count);
-    for (int32_t i = 0; i < count; i++) order[(size_t)i] = i;
+    for (int64_t i = 0; i < count; i++) order[(size_t)i] = (int32_t)i;
     std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) {
         if (size[(size_t)x] != size[(size_t)y]) return size[(size_t)x] > size[(size_t)y];
         return work[(size_t)x] > work[(size_t)y];

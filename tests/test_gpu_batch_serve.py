@@ -436,3 +436,24 @@ def test_batches_of_a_hundred_small_dense_instances(emv, n, k):
                 ms[count] = min(ms.get(count, 1e9), st["total_ms"])
             assert list(costs) == [want[i % 10] for i in range(count)]
     assert ms[107] < 1.25 * ms[4 * ctas] / 4
+
+
+def test_single_instance_batch_uses_the_gpu_as_a_solve_does(emv):
+    """A batch of one gives its instance as large a team as it can use: on the
+    device it takes at most a third longer than the one-launch solve."""
+    n, m, k = 500, 40000, 6
+    rng = np.random.default_rng(3)
+    ends = np.concatenate([np.stack([np.arange(n - 1), np.arange(1, n)], 1), rng.integers(0, n, (m, 2))])
+    ends = ends[ends[:, 0] != ends[:, 1]]
+    g = emv.Csr.from_stp(emv.StpInstance(n, np.concatenate([ends, rng.integers(1, 101, (len(ends), 1))], 1),
+                                         rng.choice(n, k, replace=False).astype(np.int64)))
+    with emv.Solver(0) as s:
+        solves, batches = [], []
+        for _ in range(8):
+            r = s.solve(g)
+            assert r.timing["relax_launches"] == 1
+            solves.append(r.timing["kernel_ms"])
+            costs, st = s.batch_solve([g])
+            assert costs[0] == r.cost
+            batches.append(st["total_ms"])
+    assert min(batches) < 1.33 * min(solves)
