@@ -1466,9 +1466,12 @@ struct TbArgs {
 // 0 leaf (X = {i}, v = t_i); 1 split d[Y][v] + d[X\Y][v] = D (the lowest
 // pair index; DY = d[Y][v]); 2 arc (u, v) of positive weight with d[X][u] + w
 // = D; 3 none of those (a zero-weight predecessor must exist).  [beg, end):
-// v's arcs, on return of 2 u's.  A step's time is its chain of dependent loads
+// v's arcs, on return of 2 (with WALK set) u's.  A step's time is its chain of dependent loads
 // (arc, value at its head), so the first 32 arcs are requested before the
 // pairs are looked at, and the bounds of a head's own arcs with its value.
+// (Without WALK, in searches, the bounds are left out: with them cliques of 600 and
+// 700 vertices and weights of 0 to 3 took 35 to 68 ms, 26 to 50 so.)
+template <bool WALK>
 __device__ int tb_witness(const TbArgs &a, uint32_t X, int32_t v, int32_t D, int32_t &beg, int32_t &end, uint32_t &Y,
                           int32_t &DY, int32_t &u, int32_t &wt)
 {
@@ -1483,8 +1486,10 @@ __device__ int tb_witness(const TbArgs &a, uint32_t X, int32_t v, int32_t D, int
         if (e < end) {
             arc = a.adj[e];
             du = row[arc.x];
-            ub = a.row_ptr[arc.x];
-            ue = a.row_ptr[arc.x + 1];
+            if (WALK) {
+                ub = a.row_ptr[arc.x];
+                ue = a.row_ptr[arc.x + 1];
+            }
         }
     };
     head(beg + lane);
@@ -1524,8 +1529,10 @@ __device__ int tb_witness(const TbArgs &a, uint32_t X, int32_t v, int32_t D, int
             const int src = __ffs(bal) - 1;
             u = __shfl_sync(FULL, arc.x, src);
             wt = __shfl_sync(FULL, arc.y, src);
-            beg = __shfl_sync(FULL, ub, src);
-            end = __shfl_sync(FULL, ue, src);
+            if (WALK) {
+                beg = __shfl_sync(FULL, ub, src);
+                end = __shfl_sync(FULL, ue, src);
+            }
             return 2;
         }
         e0 += 32;
@@ -1637,7 +1644,7 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(TbArgs a)
             }
             uint32_t Y = 0;
             int32_t DY = 0, u = 0, wt = 0;
-            const int kind = tb_witness(a, X, v, D, beg, end, Y, DY, u, wt);
+            const int kind = tb_witness<true>(a, X, v, D, beg, end, Y, DY, u, wt);
             if (kind == 0) break;
             if (kind == 1) {
                 if (lane == 0) kid = atomicAdd(&s_alloc, 2);
@@ -1700,7 +1707,7 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(TbArgs a)
                 if (x != v) {
                     uint32_t Y2;
                     int32_t d2, u2, w2, xb = a.row_ptr[x], xe = a.row_ptr[x + 1];
-                    if (tb_witness(a, X, x, D, xb, xe, Y2, d2, u2, w2) != 3) {
+                    if (tb_witness<false>(a, X, x, D, xb, xe, Y2, d2, u2, w2) != 3) {
                         target = x;
                         break;
                     }
