@@ -765,6 +765,21 @@ static int check_k(int32_t n, int32_t k, const int32_t *terms)
     return EMV_OK;
 }
 
+// Whether a solve over kt terminals' subsets runs as one launch (then p is its
+// shape).  If not, the graph has been packed, and checked with check set; past
+// the line of resident_plan that tells whether it has hubs.
+static int plan_solve(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr, const int32_t *col, const int32_t *w,
+                      int32_t kt, bool host_table, bool check, cudaStream_t st, ResidentPlan &p, bool &resident)
+{
+    resident = resident_plan(c, n, arcs, kt, host_table, false, p);
+    if (resident) return EMV_OK;
+    const int r = pack_and_check(c, n, arcs, row_ptr, col, w, check, st);
+    if (r || !resident_plan(c, n, arcs, kt, host_table, true, p)) return r;
+    if (!check) CUDA_TRY(cudaStreamSynchronize(st));
+    resident = ((const GraphScan *)((char *)c->pinned + 1024))->hubs > 0;
+    return EMV_OK;
+}
+
 extern "C" int emv_kernel_dev(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *d_row_ptr, const int32_t *d_col,
                               const int32_t *d_w, int32_t k, const int32_t *terminals, int32_t *d_table, int64_t ld,
                               int64_t *cost_out, void *stream)
@@ -778,14 +793,15 @@ extern "C" int emv_kernel_dev(emv_ctx *c, int32_t n, int64_t arcs, const int32_t
     cudaStream_t st = (cudaStream_t)stream;
     c->launches = 0;
     ResidentPlan plan;
-    if (resident_plan(c, n, arcs, k, false, plan)) {
+    bool resident;
+    r = plan_solve(c, n, arcs, d_row_ptr, d_col, d_w, k, false, true, st, plan, resident);
+    if (r) return r;
+    if (resident) {
         r = resident_launch(c, plan, n, arcs, d_row_ptr, d_col, d_w, terminals, k, k, d_table, ld, true, st);
         if (r) return r;
         CUDA_TRY(cudaStreamSynchronize(st));
         return resident_finish(c, n, k, true, true, cost_out, nullptr);
     }
-    r = pack_and_check(c, n, arcs, d_row_ptr, d_col, d_w, true, st);
-    if (r) return r;
     return run_dp(c, n, d_row_ptr, (const int2 *)c->adj.ptr, k, k, terminals, d_table, ld, st, cost_out, nullptr, true);
 }
 
@@ -911,8 +927,8 @@ int solve_on_device(emv_ctx *c, int32_t n, int64_t arcs, const int32_t *row_ptr,
     const int32_t kt = whole ? k : table_terminals(k);
     const size_t tbytes = sizeof(int32_t) * (size_t)ld << kt;
     ResidentPlan plan;
-    const bool resident = resident_plan(c, n, arcs, kt, (flags & EMV_SOLVE_TABLE) && out->table, plan);
-    int r = resident ? EMV_OK : pack_and_check(c, n, arcs, row_ptr, col, w, check, st);
+    bool resident;
+    int r = plan_solve(c, n, arcs, row_ptr, col, w, kt, (flags & EMV_SOLVE_TABLE) && out->table, check, st, plan, resident);
     if (!r) r = dev_reserve(c->table, tbytes);
     if (r) return r;
     int32_t *table = (int32_t *)c->table.ptr;
@@ -1057,7 +1073,7 @@ extern "C" int emv_sssp(emv_ctx *c, const emv_graph *g, int32_t source, int64_t 
     const int64_t ld = ((int64_t)n + 3) / 4 * 4;
     ResidentPlan plan;
     // the line of resident_plan on arcs is that of solves
-    const bool resident = sssp_resident(g) && resident_plan(c, n, 0, 1, false, plan);
+    const bool resident = sssp_resident(g) && resident_plan(c, n, 0, 1, false, false, plan);
     r = dev_reserve(c->table, sizeof(int32_t) * 2 * (size_t)ld);
     if (!r) r = prepare_subsets(c, 1, st);
     if (!r && !resident) r = reserve_relax(c, n);

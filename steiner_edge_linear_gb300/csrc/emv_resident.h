@@ -25,7 +25,8 @@ int32_t res_hub_min(int32_t n, int64_t arcs, int32_t kt);
 // Polls after which a CTA gives up on the others of its team: CTAs without rows
 // of a level wait for those that close `rows` of them.
 uint32_t res_spin_limit(int32_t n, int64_t arcs, int64_t rows);
-bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, bool host_table, ResidentPlan &p);
+// crowded: the graph is known to have vertices of far more arcs than most.
+bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, bool host_table, bool crowded, ResidentPlan &p);
 // Enqueues the whole DP over the first kt of the k terminals, CSR check
 // included, and the copy of its result words; fills the table's 2^kt rows
 // (stride ld) and c->adj.

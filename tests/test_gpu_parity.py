@@ -815,3 +815,28 @@ def test_sssp_of_crowded_arcs_stays_in_one_launch(emv, orc, solver, hubs):
     g = emv.Csr.from_stp(emv.StpInstance(n, np.concatenate([ends, rng.integers(1, 1001, (len(ends), 1))], 1), np.array([0], np.int64)))
     assert np.array_equal(solver.sssp(g, n // 2)[0], orc.sssp(g.n, g.row_ptr, g.col, g.w, n // 2))
     assert min(solver.sssp(g, n // 2)[1] for _ in range(5)) < 0.4
+
+
+@pytest.mark.parametrize("check", [True, False])
+def test_crowded_graphs_past_the_line_run_in_one_launch(emv, orc, solver, check):
+    """Half of the arcs at a hundred vertices: past the line on arcs and vertices
+    such a graph still runs as one launch, from host and from device memory, and
+    the same size without hubs does not."""
+    torch = pytest.importorskip("torch")
+    n, m, k = 14000, 135000, 3
+    rng = np.random.default_rng(6)
+    path = np.stack([np.arange(n - 1), np.arange(1, n)], 1)
+    for hubs in (100, n):
+        ends = np.concatenate([path, np.stack([rng.integers(0, hubs, m), rng.integers(0, n, m)], 1)])
+        ends = ends[ends[:, 0] != ends[:, 1]]
+        g = emv.Csr.from_stp(emv.StpInstance(n, np.concatenate([ends, rng.integers(1, 101, (len(ends), 1))], 1),
+                                             rng.choice(n, k, replace=False).astype(np.int64)))
+        want, cost = orc.emv_table(g.n, g.row_ptr, g.col, g.w, g.terminals, threads=16)
+        res = solver.solve(g, table=True, tree=True, check=check)
+        assert res.cost == cost == res.tree_weight and np.array_equal(res.table, want)
+        assert (res.timing["relax_launches"] == 1) == (hubs == 100)
+        row, col, w = (torch.from_numpy(a).to("cuda:0") for a in (g.row_ptr, g.col, g.w))
+        table = torch.empty((1 << k, n), dtype=torch.int32, device="cuda:0")
+        assert solver.kernel_dev(n, g.arcs, row.data_ptr(), col.data_ptr(), w.data_ptr(), g.terminals, table.data_ptr(), n,
+                                 torch.cuda.current_stream().cuda_stream) == cost
+        assert np.array_equal(table.cpu().numpy(), want)
