@@ -114,9 +114,10 @@ uint32_t res_spin_limit(int32_t n, int64_t arcs, int64_t rows)
 // Levels of more rows than SMs (kt >= 10) take turns on them and read the arcs
 // again each time: kernel times here and there, degree 8, kt = 10: n = 5800 0.62
 // and 1.57 ms, 12 000 1.15 and 1.83, 20 011 1.86 and 2.07; kt = 11, n = 12 000 2.05
-// and 2.84; calls, kt = 10: n = 12 000, degree 20 1.82 and 1.93, 14 000 2.08 and
-// 1.99; kt = 11: n = 16 384, degree 10 3.07 and 3.02, 14 000, degree 20 3.63 and
-// 3.11 (irregular degrees 3.72 and 3.03, 4.55 and 3.22).
+// and 2.84; calls with irregular degrees, kt = 10: n = 12 000, degree 16 2.15 and
+// 2.01, 16 000, degree 16 2.69 and 2.04; kt = 11: n = 12 000, degree 16 3.51 and 3.08,
+// 16 000, degree 10 3.95 and 3.27, degree 5 2.77 and 2.93 (regular; with weights past
+// 16 bits 2.92 and 4.35, with weights of 100 to 120 2.17 and 1.96).
 // The line does not hold for graphs with hubs, which narrow records leave to a
 // warp each: n = 14 414, 288 000 arcs, half of them at a hundred vertices, k = 3 1.5
 // and 6.6 ms.
@@ -126,7 +127,7 @@ uint32_t res_spin_limit(int32_t n, int64_t arcs, int64_t rows)
 constexpr int64_t RESIDENT_MAX_ARCS = 300000;
 bool resident_plan(const emv_ctx *c, int32_t n, int64_t arcs, int32_t kt, bool host_table, bool crowded, ResidentPlan &p)
 {
-    const int64_t most = kt <= 9 ? 270000 + 9000 * kt : 320000 - 80000 * (kt - 10);
+    const int64_t most = kt <= 9 ? 270000 + 9000 * kt : kt == 10 ? 260000 : 200000;
     if (!resident_fits(n, kt) || arcs > RESIDENT_MAX_ARCS || (!crowded && arcs + 5 * (int64_t)n > most)) return false;
     if (kt > 9 && n > 4096 && (n > 16384 || (host_table && (int64_t)n << kt > 1 << 22))) return false;
     const int sms = c->relax_sm_cap > 0 && c->relax_sm_cap < c->sms ? c->relax_sm_cap : c->sms;

@@ -791,7 +791,8 @@ def test_sssp_of_many_arcs_takes_the_whole_gpu(emv, orc, solver):
 
 @pytest.mark.parametrize("n,degree,k,wmax,one", [(20011, 8, 9, 100, True), (24000, 12, 5, 100, False), (30000, 4, 4, 100, True),
                                                  (30000, 8, 4, 100, False), (20000, 14, 8, 30000, False),
-                                                 (4000, 20, 11, 100, True), (4000, 60, 12, 100, False)])
+                                                 (4000, 20, 11, 100, True), (4000, 60, 12, 100, False),
+                                                 (16000, 8, 12, 100, False), (12000, 17, 11, 100, False)])
 def test_one_launch_for_as_many_arcs_as_it_reads_faster(emv, orc, solver, n, degree, k, wmax, one):
     """Both sides of the line on vertices, arcs and terminals up to which a
     small solve runs in one launch."""
