@@ -357,7 +357,7 @@ typedef struct emv_server_opts {
     int32_t device;
     int64_t hbm_budget_bytes;  /* admission bound on the sum of 2^k*n*4 and
                                   graphs (a small request's table, graph
-                                  and arc slices, where those take more) */
+                                  and long arc slices, where those take more) */
     int32_t max_slots;         /* requests resident at once                */
     int32_t large_n;           /* n at or above which a request runs alone */
     int32_t wave_sms;          /* SMs kept for the small requests' waves

@@ -62,19 +62,24 @@ struct Req {
     int32_t *d_row = nullptr;
     int2 *d_adj = nullptr;
     int32_t *d_terms = nullptr;
-    int32_t *d_table = nullptr;  // and, table_bytes behind it, the sliced arcs
+    int32_t *d_table = nullptr;  // and, table_bytes behind it, its own sliced arcs
 };
 
 // The table of a small request: the rows of its first k - 1 terminals.
 int64_t table_bytes(int32_t n, int32_t k) { return (((int64_t)batch_ld(n) << table_terminals(k)) * 4 + 255) / 256 * 256; }
 
+// Sliced arcs of up to this size (4096 vertices of 32 arcs) are written where the
+// team that solves the request has its place, longer ones behind its table.
+constexpr int64_t SLICE_SLOT = 4096 * 32 * 4;
+bool own_slices(int64_t arc_bytes) { return arc_bytes > SLICE_SLOT; }
+
 // What a request is charged against the budget: 2^k * n * 4 bytes of table and
 // the graph, or, where that is more, what a small one takes on the device: its
-// table, the graph and its sliced arcs.
+// table, the graph and its own sliced arcs.
 int64_t footprint(int32_t n, int32_t k, int64_t arcs, int64_t slices)
 {
     const int64_t graph = (int64_t)(n + 1) * 4 + arcs * 8 + (int64_t)k * 4;
-    return graph + std::max(((int64_t)n << k) * 4, table_bytes(n, k) + slices);
+    return graph + std::max(((int64_t)n << k) * 4, table_bytes(n, k) + (own_slices(slices) ? slices : 0));
 }
 
 }  // namespace
@@ -97,7 +102,7 @@ struct emv_server {
     cudaStream_t st_small = nullptr, st_large = nullptr;
     // wave buffers
     std::vector<int32_t> free_slots;
-    DevBuf d_desc, d_costs, d_ctrl;
+    DevBuf d_desc, d_costs, d_ctrl, d_arcs;
     BatchInst *h_desc = nullptr;
     int64_t *h_costs = nullptr;
     int32_t cap_slots = 0;
@@ -140,8 +145,9 @@ int stage_small(emv_server *s, Req *r, std::vector<int2> &adj)
     if (cudaMallocAsync((void **)&r->d_row, sizeof(int32_t) * ((size_t)r->n + 1), st) != cudaSuccess ||
         cudaMallocAsync((void **)&r->d_adj, sizeof(int2) * arcs, st) != cudaSuccess ||
         cudaMallocAsync((void **)&r->d_terms, sizeof(int32_t) * (size_t)r->k, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&r->d_table, (size_t)(table_bytes(r->n, r->k) + batch_arc_stride(r->arc_bytes)), st) !=
-            cudaSuccess) {
+        cudaMallocAsync((void **)&r->d_table,
+                        (size_t)(table_bytes(r->n, r->k) + (own_slices(r->arc_bytes) ? batch_arc_stride(r->arc_bytes) : 0)),
+                        st) != cudaSuccess) {
         cudaGetLastError();
         return emv_fail(EMV_ERR_OOM, "server: device allocation for request %lld", (long long)r->id);
     }
@@ -259,7 +265,7 @@ void scheduler(emv_server *s)
             d.size = size[(size_t)order[j]];
             batch_shape(s->ctx_small, r->arcs, d);
             d.narrow = r->narrow;
-            d.slices = (char *)r->d_table + table_bytes(r->n, r->k);
+            d.slices = own_slices(r->arc_bytes) ? (char *)r->d_table + table_bytes(r->n, r->k) : nullptr;
             d.orig = r->slot;
             d.lo = d.hi = r->next_level;
             for (int32_t cl = 0; cl < BATCH_SIZES; cl++)
@@ -273,6 +279,8 @@ void scheduler(emv_server *s)
         a.costs = (int64_t *)s->d_costs.ptr;
         a.ctl = (uint32_t *)s->d_ctrl.ptr;
         a.smem = RESIDENT_SMEM;
+        a.scratch = (char *)s->d_arcs.ptr;
+        a.scratch_stride = batch_arc_stride(SLICE_SLOT);
         uint32_t err = 0;
         int st = EMV_OK;
         if (cudaMemcpyAsync(s->d_desc.ptr, s->h_desc, sizeof(BatchInst) * wave.size(), cudaMemcpyHostToDevice,
@@ -378,6 +386,7 @@ void server_free(emv_server *s)
     dev_release(s->d_desc);
     dev_release(s->d_costs);
     dev_release(s->d_ctrl);
+    dev_release(s->d_arcs);
     if (s->h_desc) cudaFreeHost(s->h_desc);
     if (s->h_costs) cudaFreeHost(s->h_costs);
     if (s->st_small) cudaStreamDestroy(s->st_small);
@@ -432,6 +441,7 @@ extern "C" int emv_server_create(emv_server **out, const emv_server_opts *opts)
     if (!st) st = prepare_batch_subsets(s->ctx_small, s->st_small);
     if (!st) st = batch_kernel_setup(s->ctx_small);
     if (!st) st = dev_reserve(s->d_ctrl, sizeof(uint32_t) * 32 * (size_t)batch_ctl_lines(s->ctx_small->batch_blocks));
+    if (!st) st = dev_reserve(s->d_arcs, (size_t)batch_arc_stride(SLICE_SLOT) * (size_t)s->ctx_small->batch_blocks);
     // keep freed pool memory cached in the process (no release at stream syncs)
     cudaMemPool_t pool;
     if (!st && cudaDeviceGetDefaultMemPool(&pool, opts->device) == cudaSuccess) {
