@@ -73,17 +73,18 @@ uint32_t res_inv_slices(int32_t n)
 
 // Arcs of a vertex up to which it has its place in a slice; more make it a hub.
 // A slice is as wide as its widest vertex, so 64, but in dense graphs twice the
-// mean degree where arc counts of pairs still fit 8 bits: with every vertex a
+// mean degree as far as arc counts of pairs fit 8 bits: with every vertex a
 // hub, read from adj by a warp, one launch lost to the record kernels and a
 // batch to a CTA an instance.  Before and so: 900 cliques of 100, k = 7 5.6 and
-// 2.1 ms on the device, n = 4000, degree 70, k = 8 3.80 and 1.15 ms; past it the two
-// are equal (clique of 400, k = 4 0.43 and 0.47 ms, k = 8 0.98 and 0.85).  With one
-// row or two a level the slices' latency counts, and a warp a vertex is faster
-// (clique of 200, one source 0.10 and 0.14 ms; n = 517, degree 235, k = 3 0.22 and 0.31).
+// 2.1 ms on the device, 237 of 497, k = 9 58 and 17, n = 4000, degree 70, k = 8 3.80
+// and 1.15 ms.  Past a mean degree of 254 few rows take longer so (clique of 400,
+// k = 4 0.43 and 0.47 ms, k = 6 0.81 and 0.62).  With one row or two a level the
+// slices' latency counts, and a warp a vertex is faster (clique of 200, one source
+// 0.10 and 0.14 ms; n = 517, degree 235, k = 3 0.22 and 0.31).
 int32_t res_hub_min(int32_t n, int64_t arcs, int32_t kt)
 {
     const int64_t mean = arcs / n;
-    return kt > 2 && mean > 48 && mean <= 254 ? (int32_t)(2 * mean) : 64;
+    return kt > 2 && mean > 48 && mean <= (kt > 4 ? 508 : 254) ? (int32_t)std::min<int64_t>(508, 2 * mean) : 64;
 }
 
 // A closure takes up to n + 1 rounds of at most about a nanosecond an arc and

@@ -345,7 +345,8 @@ def test_team_waits_for_a_long_closure(emv):
                                                 ("regular", 300, 49, 30), ("regular", 1000, 180, 20000)])
 def test_dense_graphs_in_one_launch_and_in_batches(emv, orc, kind, n, degree, wmax):
     """Dense graphs keep their arcs in slices up to twice the mean degree: without
-    hubs, hubs only (mean degree past 254), and some of both."""
+    hubs, hubs only (mean degree past 254, below 5 terminals' subsets), and some
+    of both."""
     if kind == "clique":
         inst = emv.StpInstance.clique(n, 1, wmax, 5, 4)
     elif kind == "powlaw":
@@ -362,13 +363,14 @@ def test_dense_graphs_in_one_launch_and_in_batches(emv, orc, kind, n, degree, wm
         assert np.array_equal(s.sssp(csr, 7)[0], orc.sssp(csr.n, csr.row_ptr, csr.col, csr.w, 7))
 
 
-def test_dense_batches_scale_with_their_arcs(emv):
-    """Cliques of 70 vertices, a sixth more arcs than cliques of 65, take at most
-    half as long again on the device (a warp a vertex took 2.3 times as long)."""
+@pytest.mark.parametrize("sizes,count", [((65, 70), 700), ((250, 260), 200)])
+def test_dense_batches_scale_with_their_arcs(emv, sizes, count):
+    """Cliques of a few per cent more vertices, across the degrees of 64 and 254,
+    take at most half as long again on the device."""
     ms = []
     with emv.Solver(0) as s:
-        for n in (65, 70):
-            graphs = [emv.Csr.from_stp(emv.StpInstance.clique(n, 1, 100, 7, seed)) for seed in range(700)]
+        for n in sizes:
+            graphs = [emv.Csr.from_stp(emv.StpInstance.clique(n, 1, 100, 7, seed)) for seed in range(count)]
             ms.append(min(s.batch_solve(graphs)[1]["total_ms"] for _ in range(5)))
     assert ms[1] < 1.5 * ms[0]
 
